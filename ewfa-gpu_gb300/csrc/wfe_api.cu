@@ -425,7 +425,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     }
     int grid = bp.shape[t].grid;
     if (!listed) {
-        const uint32_t per_cta = t >= 5 ? 1u : 4u * (32u / (uint32_t)tier_info(t).G);
+        const uint32_t per_cta = (uint32_t)tier_info(t).pairs_per_cta;
         grid = (int)std::min<uint64_t>((uint64_t)grid, ((uint64_t)n + per_cta - 1) / per_cta);
     }
     grid = std::max(grid, 1);

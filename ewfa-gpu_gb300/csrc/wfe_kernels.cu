@@ -2,7 +2,9 @@
  * wfe_kernels.cu -- the alignment path on sm_103a.
  *
  *   pack_kernel          ASCII -> 2-bit words (src/kernels.cu:313-394)
- *   tier_kernel<Tier>    fused load+pack, wavefront compute+extend, bit-packed
+ *   band_kernel          one pair per thread in a bit-parallel band of 32
+ *                        diagonals: tier 0, and predicted prefix distances
+ *   tier_kernel<Tier>    tiers 1-4: fused load+pack, wavefront compute+extend, bit-packed
  *                        backtrace store, backtrace and CIGAR replay for one
  *                        pair per group of G lanes (src/kernels.cu:27-310 and
  *                        397-625 in one kernel)
@@ -29,6 +31,7 @@
  * diagonal k + op - 2 and adds op at field d-1 (src/kernels.cu:154-171).
  */
 #include "wfe_kernels.cuh"
+#include "wfe_band.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -147,42 +150,18 @@ size_t group_smem_bytes(uint32_t max_len, uint32_t cigar_stride)
     return 16u * (size_t)seq_words_for(max_len) + T::chain_bytes + union_bytes<T>(cigar_stride);
 }
 
-/* The tiers with several pairs per warp also keep, per warp, the packed
- * blocks of a coalesced span load of the warp's pairs (load_warp_span):
- * 160 blocks, 2,560 bytes of input, enough for 8 pairs of 150 bases stored
- * one after another with their file's line marks. */
-constexpr int kSpanWords = 160;
-
 template <class T>
 size_t cta_smem_bytes(uint32_t max_len, uint32_t cigar_stride)
 {
-    const size_t span = T::G < 32 ? (size_t)kWarps * kSpanWords * sizeof(uint32_t) : 0u;
-    return group_smem_bytes<T>(max_len, cigar_stride) * (size_t)(kWarps * T::GPW) + span;
+    return group_smem_bytes<T>(max_len, cigar_stride) * (size_t)(kWarps * T::GPW);
 }
 
-/* The alignment kernel of a tier, in two forms with one body (tier_body):
- *   tier_kernel_bounded<T, PREDICT>  the 4-lane tier 0 and the prediction
- *       pass, launched from the host only, with launch bounds that set its
- *       register budget for 8 resident CTAs per SM;
- *   tier_kernel<T>  the tiers 1-4 that chains launch from the device, with
- *       no launch bounds: a grid launched from the device whose kernel
- *       declares launch bounds and uses dynamic shared memory was measured
- *       to run one CTA per SM at a time, whatever the bounds say. */
-template <class T, bool PREDICT = false>
-__global__ void __launch_bounds__(kThreads, T::MINB)
-tier_kernel_bounded(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t gbytes);
+/* The alignment kernel of tiers 1-4.  Chains launch it from the device, so it
+ * declares no launch bounds: a grid launched from the device whose kernel
+ * declares launch bounds and uses dynamic shared memory was measured to run
+ * one CTA per SM at a time, whatever the bounds say. */
 template <class T>
 __global__ void tier_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t gbytes);
-
-/* Tier 0 carries the short-read workloads; its shape is tuned on the GPU
- * (4 lanes per pair, 11 chunks, 8 resident CTAs per SM by default). */
-#ifndef WFE_T0_J
-#define WFE_T0_J 5
-#endif
-#ifndef WFE_T0_MINB
-#define WFE_T0_MINB 8
-#endif
-using T0 = Tier<4, WFE_T0_J, true, 5, WFE_T0_MINB>; /* distance <= 4*J + 1 (21) */
 
 /* launched from the device too: no launch bounds (see tier_kernel) */
 template <bool GLOBAL_WF, int NT>
@@ -375,7 +354,32 @@ __device__ __forceinline__ void chain_next(const AlignLaunch& A)
     }
 }
 
-template <class T, bool PREDICT>
+/* What becomes of a pair that a tier did not align, by one thread: a pair
+ * past the tier's distance goes to the next tier's list (or is deferred, by a
+ * chain cut short), the others get their status. */
+__device__ __forceinline__ void finish_unaligned(const AlignLaunch& A, uint32_t pi, int state)
+{
+    if (state == ST_OVERFLOW && A.retry) {
+        const uint32_t s = atomicAdd(A.retry_count, 1u);
+        if (A.retry != A.chain.defer) {
+            A.retry[s] = pi;
+        } else {
+            if (s < A.chain.defer_cap) A.retry[s] = A.chain.defer_base + pi;
+            note_deferred(A);
+        }
+        if (A.passed_total) atomicAdd(A.passed_total, 1ull);
+        return;
+    }
+    A.dist[pi] = state == ST_OVERMAX ? A.max_distance + 1 : -1;
+    if (A.status)
+        A.status[pi] = state == ST_OVERMAX  ? (uint8_t)WFE_PAIR_OVER_MAX_DISTANCE
+                       : state == ST_BADWALK ? (uint8_t)WFE_PAIR_BAD_HISTORY
+                       : state == ST_RANGE   ? (uint8_t)WFE_PAIR_OUT_OF_RANGE
+                                             : (uint8_t)WFE_PAIR_TOO_LONG;
+    if (A.cigar_stride) A.cigar[(size_t)pi * A.cigar_stride] = 0;
+}
+
+template <class T>
 __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_words, uint32_t gbytes)
 {
     constexpr int G = T::G, J = T::J, NC = T::NC, DCAP = T::DCAP, GPW = T::GPW;
@@ -433,28 +437,11 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
             pi = A.work ? A.work[item] : item;
             pr = get_pair(A.L, pi);
             const uint32_t mx = max(pr.plen, pr.tlen);
-            state = !pr.in_range ? ST_RANGE
-                    : PREDICT ? ST_RUN
-                    : (mx > A.max_len || mx > 16u * seq_words) ? ST_TOOLONG : ST_RUN;
+            state = !pr.in_range ? ST_RANGE : (mx > A.max_len || mx > 16u * seq_words) ? ST_TOOLONG : ST_RUN;
         }
-        /* a prediction launch aligns only the first kPredictPrefix bases */
-        const uint32_t lp = state == ST_RUN ? (PREDICT ? min(pr.plen, (uint32_t)kPredictPrefix) : pr.plen) : 0u;
-        const uint32_t lt = state == ST_RUN ? (PREDICT ? min(pr.tlen, (uint32_t)kPredictPrefix) : pr.tlen) : 0u;
-        if constexpr (G < 32) {
-            /* the warp's 8 pairs in one coalesced span when they lie together */
-            uint32_t* span = reinterpret_cast<uint32_t*>(smem + (size_t)(kWarps * GPW) * gbytes) + warp * kSpanWords;
-            const uintptr_t a0 = load_warp_span<kSpanWords>(pr.p, lp, pr.t, lt, span, lane);
-            if (a0) {
-                pack_from_span<G>(span, a0, pr.p, lp, QP, g);
-                pack_from_span<G>(span, a0, pr.t, lt, QT, g);
-            } else {
-                load_packed<G, T::RMAX>(pr.p, lp, QP, g, gmask);
-                load_packed<G, T::RMAX>(pr.t, lt, QT, g, gmask);
-            }
-        } else {
-            load_packed<G, T::RMAX>(pr.p, lp, QP, g, gmask);
-            load_packed<G, T::RMAX>(pr.t, lt, QT, g, gmask);
-        }
+        const uint32_t lp = state == ST_RUN ? pr.plen : 0u, lt = state == ST_RUN ? pr.tlen : 0u;
+        load_packed<G, T::RMAX>(pr.p, lp, QP, g, gmask);
+        load_packed<G, T::RMAX>(pr.t, lt, QT, g, gmask);
         __syncwarp();
 
         const int plen = (int)lp, tlen = (int)lt, kt = tlen - plen;
@@ -493,7 +480,7 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
                     const int m = piggyback_max(up, O[c], dn);
                     const unsigned blo = __ballot_sync(kFull, m & 1);
                     const unsigned bhi = __ballot_sync(kFull, m & 2);
-                    if (!PREDICT && lane == 0) ops[rowbase + c - clo] = make_uint2(blo, bhi);
+                    if (lane == 0) ops[rowbase + c - clo] = make_uint2(blo, bhi);
                     const int k = lo_k + g;
                     N[c] = (run && k >= -d && k <= d) ? (m >> 2) : -1;
                 }
@@ -519,11 +506,6 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
             }
         }
 
-        if constexpr (PREDICT) {
-            if (g == 0 && item < count)
-                A.pred[pi] = (uint16_t)(state == ST_DONE ? D : (state == ST_OVERFLOW ? DCAP + 1 : 0xffff));
-            state = ST_IDLE;
-        }
         if (state == ST_DONE) {
             /* backtrace: from (D, kt) back to (0, 0); a walk that leaves the
              * wavefront (never expected) is reported, not followed */
@@ -544,9 +526,6 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
             walk_ok = __shfl_sync(gmask, walk_ok, 0, G);
             if (!walk_ok) state = ST_BADWALK;
         }
-        /* the warp's store is read by every group's walk before any group's
-         * replay reuses its union region */
-        if constexpr (T::SMEM_OPS && GPW > 1) __syncwarp();
         if (state == ST_DONE) {
             __syncwarp(gmask);
             const int len = replay_chain<G>(QP, QT, plen, tlen, chain, D, runs, stage, A.cigar_stride,
@@ -560,29 +539,8 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
                     A.status[pi] = (uint32_t)len > A.cigar_stride ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED
                                                                   : (uint8_t)WFE_PAIR_OK;
             }
-        } else if (state == ST_OVERFLOW && A.retry) {
-            /* hand the pair to the next tier, or defer it (a chain cut short) */
-            if (g == 0) {
-                const uint32_t s = atomicAdd(A.retry_count, 1u);
-                if (A.retry != A.chain.defer) {
-                    A.retry[s] = pi;
-                } else {
-                    if (s < A.chain.defer_cap) A.retry[s] = A.chain.defer_base + pi;
-                    note_deferred(A);
-                }
-                if (A.passed_total) atomicAdd(A.passed_total, 1ull);
-            }
-        } else if (state == ST_OVERFLOW || state == ST_OVERMAX || state == ST_TOOLONG ||
-                   state == ST_BADWALK || state == ST_RANGE) {
-            if (g == 0) {
-                A.dist[pi] = state == ST_OVERMAX ? A.max_distance + 1 : -1;
-                if (A.status)
-                    A.status[pi] = state == ST_OVERMAX  ? (uint8_t)WFE_PAIR_OVER_MAX_DISTANCE
-                                   : state == ST_BADWALK ? (uint8_t)WFE_PAIR_BAD_HISTORY
-                                   : state == ST_RANGE   ? (uint8_t)WFE_PAIR_OUT_OF_RANGE
-                                                         : (uint8_t)WFE_PAIR_TOO_LONG;
-                if (A.cigar_stride) A.cigar[(size_t)pi * A.cigar_stride] = 0;
-            }
+        } else if (state != ST_IDLE && state != ST_RUN) {
+            if (g == 0) finish_unaligned(A, pi, state);
         }
         __syncwarp();
         if (work_next) {
@@ -595,20 +553,381 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
     }
 
     /* the last CTA to finish starts the next tier that has work */
-    if constexpr (!PREDICT) chain_next(A);
-}
-
-template <class T, bool PREDICT>
-__global__ void __launch_bounds__(kThreads, T::MINB)
-tier_kernel_bounded(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t gbytes)
-{
-    tier_body<T, PREDICT>(A, seq_words, gbytes);
+    chain_next(A);
 }
 
 template <class T>
 __global__ void tier_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t gbytes)
 {
-    tier_body<T, false>(A, seq_words, gbytes);
+    tier_body<T>(A, seq_words, gbytes);
+}
+
+/* ------------------------------------------------------------------------ */
+/* Tier 0: one pair per thread, a 32-diagonal band (see wfe_band.cuh),
+ * distances up to 31.  A warp takes 32 pairs.
+ *
+ * Bound by the integer pipe.  About 35 instructions a column -- 18 for the
+ * column, 8 for the transposition, 1 store, the rest the walk back, which
+ * takes one step per edit or block -- and none of it depends on the data but
+ * the walk, so the 32 pairs of a warp stay in step.  The wavefront kernel
+ * that this replaced (4 lanes per pair) spent 981 warp instructions on a
+ * 150-base pair at 5% edits and stepped every pair of a warp to the largest
+ * distance of the eight.  1M such pairs, device-resident: 1,038 us before,
+ * 479 us now; 300k without a context 397 and 189 us; 500k from page-locked
+ * host memory 960 and 883 us (the CPU-GPU link bounds it); 200k pairs of
+ * 50-300 bases at 1-12% edits 473 and 327 us; 64 pairs 17 and 11 us.
+ *
+ * The warp's shared memory (words; a lane owns column `lane` of every row):
+ *   blocks  D0 of 32 columns, transposed: row q holds band bit q's
+ *   ckpt    VP and VN before every block of 32 columns
+ *   planes  the two bit planes of pattern and text, rows of 33 words, so that
+ *           a lane reading its own words and eight lanes writing one pair's
+ *           consecutive words are both free of bank conflicts
+ *   bytes   the CIGAR, written backwards
+ * With texts of up to 32 * kBandBlocks bases the warp keeps every block and
+ * the walk needs nothing else (the bytes then reuse the planes).  Longer
+ * texts keep the checkpoints only, and each block is computed again when the
+ * walk reaches it. */
+constexpr int kBandBlocks = 5;
+constexpr int kSpanWords = 160; /* 16-byte blocks of a span: 8 pairs of 150 bases with their file's line marks */
+static_assert(kSpanWords * 16 <= 4096, "a span must fit in one 4 KiB page (see band_load)");
+constexpr int kPlaneRow = 33;
+constexpr int kSpanRow = kSpanWords + 4; /* a span's words, and those read past its last block */
+constexpr int kBandCkpt = kBandBlocks * 1024;
+constexpr int kBandPlanes = kBandCkpt + kBandBlocks * 64;
+constexpr int kBandStoredWords = kBandPlanes + 2 * kPlaneRow * (2 * kBandBlocks + 1);
+static_assert(4 * kSpanRow <= kBandBlocks * 1024, "the spans use the blocks' space");
+
+__host__ __device__ constexpr uint32_t band_words(uint32_t max_len) { return (max_len + 31u) / 32u; }
+/* words of a CIGAR: 31 operations, 32 runs, and a byte per 127 matches */
+__host__ __device__ constexpr uint32_t band_byte_words(uint32_t max_len) { return (63u + max_len / 127u + 3u) / 4u; }
+static_assert(32 * band_byte_words(32 * kBandBlocks + 31) <= 2 * kPlaneRow * (2 * kBandBlocks + 1),
+              "the bytes reuse the planes' space");
+__host__ __device__ constexpr uint32_t band_smem_words(uint32_t max_len)
+{
+    const uint32_t nw = band_words(max_len) + (max_len == 0u);
+    const uint32_t again = 1024u + 64u * nw + 2u * kPlaneRow * (2u * nw + 1u) + 32u * band_byte_words(max_len);
+    return again > (uint32_t)kBandStoredWords ? again : (uint32_t)kBandStoredWords;
+}
+
+/* Bit planes of the warp's 32 pairs.  Eight neighbouring pairs that lie in
+ * one span of kSpanWords blocks are read by all lanes in consecutive 16-byte
+ * blocks: whole 512-byte rows per instruction, which the CPU-GPU link serves
+ * 20% faster than a short run per pair.  Blocks that fall in gaps between the
+ * pairs are read too: a span is shorter than a 4 KiB page, so it lies within
+ * the page of its first block and the page of its last, and both of those
+ * hold a base, so both are mapped.  The sequences of the other pairs are read
+ * by eight lanes each, 256 bases at a time, in blocks that hold a base.
+ * Words past a sequence's end are not written: rows and columns past the
+ * ends are never used.  A word w >= cap is dropped. */
+__device__ __forceinline__ void band_load(const char* p, uint32_t lp, const char* t, uint32_t lt, uint32_t* words,
+                                          uint32_t* P0, int capP, uint32_t* T0, int capT, int lane)
+{
+    unsigned long long lo = ~0ull, hi = 0ull;
+    if (lp) {
+        lo = (unsigned long long)(uintptr_t)p;
+        hi = lo + lp;
+    }
+    if (lt) {
+        lo = min(lo, (unsigned long long)(uintptr_t)t);
+        hi = max(hi, (unsigned long long)(uintptr_t)t + lt);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(kFull, lo, o));
+        hi = max(hi, __shfl_xor_sync(kFull, hi, o));
+    }
+    lo &= ~15ull;
+    const unsigned long long blocks = hi > lo ? (hi - lo + 15ull) >> 4 : 0ull;
+    const bool spans = blocks <= (unsigned long long)kSpanWords;
+    const int nblk = spans ? (int)blocks : 0;
+    constexpr int R = (kSpanWords + 31) / 32;
+#pragma unroll
+    for (int r = 0; r < 4; r += 2) {
+        uint4 v[2][R];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint4* base = reinterpret_cast<const uint4*>((uintptr_t)__shfl_sync(kFull, lo, 8 * (r + h)));
+            const int nb = __shfl_sync(kFull, nblk, 8 * (r + h));
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int b = lane + 32 * i;
+                v[h][i] = b < nb ? __ldg(base + b) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < R; ++i) words[(r + h) * kSpanRow + lane + 32 * i] = planes16(v[h][i]);
+    }
+    __syncwarp();
+    if (spans) {
+        const uint32_t* mine = words + (lane >> 3) * kSpanRow;
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(which ? t : p);
+            const uint32_t len = which ? lt : lp, sh = (uint32_t)(a & 15u);
+            const int n = min((int)((len + 31u) >> 5), which ? capT : capP);
+            const uint32_t* x = mine + (int)((a - sh - (uintptr_t)lo) >> 4);
+            uint32_t* out = (which ? T0 : P0) + lane;
+            const int plane = kPlaneRow * (which ? capT : capP);
+            uint32_t x0 = n > 0 ? x[0] : 0u;
+            for (int w = 0; w < n; ++w) {
+                const uint32_t x1 = x[2 * w + 1], x2 = x[2 * w + 2];
+                uint32_t b0, b1;
+                planes32(x0, x1, x2, sh, b0, b1);
+                out[w * kPlaneRow] = b0;
+                out[w * kPlaneRow + plane] = b1;
+                x0 = x2;
+            }
+        }
+    }
+    if (__any_sync(kFull, !spans)) {
+        const int g = lane & 7;
+#pragma unroll 1
+        for (int it = 0; it < 16; ++it) {
+            const int own = 2 * it + (lane >> 4), which = (lane >> 3) & 1;
+            const char* sp = reinterpret_cast<const char*>(
+                __shfl_sync(kFull, (unsigned long long)(uintptr_t)p, own));
+            const char* st = reinterpret_cast<const char*>(
+                __shfl_sync(kFull, (unsigned long long)(uintptr_t)t, own));
+            const uint32_t np = __shfl_sync(kFull, lp, own), nt = __shfl_sync(kFull, lt, own);
+            const bool skip = __shfl_sync(kFull, (int)spans, own) != 0;
+            const uintptr_t a = reinterpret_cast<uintptr_t>(which ? st : sp);
+            const uint32_t len = skip ? 0u : (which ? nt : np), sh = (uint32_t)(a & 15u);
+            const uint4* base = reinterpret_cast<const uint4*>(a - sh);
+            const int nb = len ? (int)((sh + len + 15u) >> 4) : 0;
+            const int cap = which ? capT : capP;
+            const int n = min((int)((len + 31u) >> 5), cap);
+            const int most = __reduce_max_sync(kFull, n);
+            uint32_t* out = (which ? T0 : P0) + own;
+            for (int w0 = 0; w0 < most; w0 += 8) {
+                const int w = w0 + g, b = 2 * w;
+                const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+                const uint32_t x0 = planes16(b < nb ? __ldg(base + b) : z);
+                const uint32_t x1 = planes16(b + 1 < nb ? __ldg(base + b + 1) : z);
+                uint32_t x2 = __shfl_down_sync(kFull, x0, 1, 8);
+                if (g == 7) x2 = planes16(b + 2 < nb ? __ldg(base + b + 2) : z);
+                uint32_t b0, b1;
+                planes32(x0, x1, x2, sh, b0, b1);
+                if (w < n) {
+                    out[w * kPlaneRow] = b0;
+                    out[w * kPlaneRow + kPlaneRow * cap] = b1;
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
+/* D0 of the 32 columns of block m, from VP/VN before it (left as they are
+ * after it).  P and T: the lane's columns of the planes; b: see wfe_band.cuh. */
+template <typename F>
+__device__ __forceinline__ void band_block(const uint32_t* P, int planeP, const uint32_t* T, int planeT, int m, int b,
+                                           uint32_t& vp, uint32_t& vn, F&& each)
+{
+    const uint32_t* pw = P + m * kPlaneRow;
+    const uint32_t l0 = m > 0 ? pw[-kPlaneRow] : 0u, l1 = m > 0 ? pw[planeP - kPlaneRow] : 0u;
+    const uint32_t c0 = pw[0], c1 = pw[planeP], n0 = pw[kPlaneRow], n1 = pw[planeP + kPlaneRow];
+    const uint32_t a0 = __funnelshift_l(l0, c0, (uint32_t)b), e0 = __funnelshift_l(c0, n0, (uint32_t)b);
+    const uint32_t a1 = __funnelshift_l(l1, c1, (uint32_t)b), e1 = __funnelshift_l(c1, n1, (uint32_t)b);
+    const uint32_t t0 = T[m * kPlaneRow], t1 = T[m * kPlaneRow + planeT];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const uint32_t x = __funnelshift_r(a0, e0, (uint32_t)j) ^ bit_mask(t0, j);
+        const uint32_t eq = ~(x | (__funnelshift_r(a1, e1, (uint32_t)j) ^ bit_mask(t1, j)));
+        each(j, band_column(eq, vp, vn));
+    }
+}
+
+template <bool PREDICT>
+__global__ void __launch_bounds__(32, 9) band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw)
+{
+    extern __shared__ __align__(16) uint32_t band_smem[];
+    const int lane = (int)(threadIdx.x & 31u);
+    const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+    uint32_t* const work_next = A.chain.work_next ? A.chain.work_next + A.tier : nullptr;
+    uint32_t wb = blockIdx.x * 32u;
+    if (work_next) {
+        uint32_t v = 0;
+        if (lane == 0) v = atomicAdd(work_next, 32u);
+        wb = __shfl_sync(kFull, v, 0);
+    }
+    while (wb < count) {
+        const uint32_t item = wb + (uint32_t)lane;
+        int state = ST_IDLE;
+        uint32_t pi = 0;
+        PairRef pr;
+        pr.p = nullptr; pr.t = nullptr; pr.plen = 0; pr.tlen = 0;
+        if (item < count) {
+            pi = A.work ? A.work[item] : item;
+            pr = get_pair(A.L, pi);
+            const uint32_t mx = max(pr.plen, pr.tlen);
+            state = !pr.in_range ? ST_RANGE
+                    : PREDICT ? ST_RUN
+                    : (mx > A.max_len || mx > 32u * nw) ? ST_TOOLONG : ST_RUN;
+            if constexpr (PREDICT) {
+                pr.plen = min(pr.plen, (uint32_t)kPredictPrefix);
+                pr.tlen = min(pr.tlen, (uint32_t)kPredictPrefix);
+            }
+        }
+        /* a distance past the band: the next tier's, or past the caller's cap */
+        const int past = A.max_distance > 0 && A.max_distance <= kBandDistance ? ST_OVERMAX : ST_OVERFLOW;
+        if (state == ST_RUN && abs((int)pr.tlen - (int)pr.plen) > kBandDistance) state = past;
+        const uint32_t lp = state == ST_RUN ? pr.plen : 0u, lt = state == ST_RUN ? pr.tlen : 0u;
+        const int tlen = (int)lt, kt = tlen - (int)lp, wide = abs(kt);
+        /* diagonals b-31..b hold 0 and kt, with as many on either side */
+        const int b = kBandDistance + min(0, kt) - (kBandDistance - wide) / 2;
+        const int it = b - kt; /* the target's band bit */
+        const int nb = max(1, (__reduce_max_sync(kFull, tlen) + 31) >> 5);
+        const bool stored = nb <= kBandBlocks; /* always, of a prefix */
+        const int capT = stored ? kBandBlocks : (int)nw, capP = capT + 1;
+        uint32_t* const blocks = band_smem;
+        uint32_t* const ckpt = band_smem + (stored ? kBandCkpt : 1024) + lane;
+        uint32_t* const P0 = band_smem + (stored ? kBandPlanes : 1024 + 64 * (int)nw);
+        uint32_t* const T0p = P0 + 2 * kPlaneRow * capP;
+        uint32_t* const bytes = stored ? P0 : T0p + 2 * kPlaneRow * capT;
+        const int top = (int)band_byte_words(stored ? 32u * kBandBlocks : 32u * nw);
+        band_load(pr.p, lp, pr.t, lt, blocks, P0, capP, T0p, capT, lane);
+        const uint32_t* const P = P0 + lane;
+        const uint32_t* const T = T0p + lane;
+        const int planeP = kPlaneRow * capP, planeT = kPlaneRow * capT;
+
+        /* every column, and the distance: |kt| and the increments along the
+         * target's diagonal */
+        uint32_t vp = ~0u << b, vn = ~vp;
+        int D = wide;
+        if (stored && !PREDICT) {
+#pragma unroll 1
+            for (int m = 0; m < nb; ++m) {
+                ckpt[64 * m] = vp;
+                ckpt[64 * m + 32] = vn;
+                uint32_t d0[32];
+                band_block(P, planeP, T, planeT, m, b, vp, vn, [&](int j, uint32_t d) { d0[j] = d; });
+                transpose32(d0);
+                uint32_t* out = blocks + 1024 * m + lane;
+#pragma unroll
+                for (int q = 0; q < 32; ++q) out[32 * q] = d0[q];
+                D += __popc(~out[32 * it] & low_bits(min(32, max(0, tlen - 32 * m))));
+            }
+        } else {
+#pragma unroll 1
+            for (int m = 0; m < nb; ++m) {
+                ckpt[64 * m] = vp;
+                ckpt[64 * m + 32] = vn;
+                uint32_t on = 0;
+                band_block(P, planeP, T, planeT, m, b, vp, vn,
+                           [&](int j, uint32_t d) { on = __funnelshift_r(on, d >> it, 1u); });
+                D += __popc(~on & low_bits(min(32, max(0, tlen - 32 * m))));
+            }
+        }
+        if constexpr (PREDICT) {
+            if (item < count)
+                A.pred[pi] = (uint16_t)(state == ST_RUN ? min(D, kBandDistance + 1)
+                                        : state == past ? kBandDistance + 1 : 0xffff);
+            wb += gridDim.x * 32u;
+            __syncwarp();
+            continue;
+        }
+        if (state == ST_RUN)
+            state = D > kBandDistance ? past : (A.max_distance > 0 && D > A.max_distance) ? ST_OVERMAX : ST_DONE;
+
+        __syncwarp(); /* the bytes may reuse the planes of other lanes */
+
+        /* the walk back from the target (see walk_step) */
+        BackBytes cg{bytes + lane, 0u, 0, top};
+        int m = tlen > 0 ? (tlen - 1) >> 5 : 0, hb = tlen - 32 * m, q = it, s = D, run = 0;
+        bool walking = state == ST_DONE;
+        for (int blk = nb - 1; blk >= 0; --blk) {
+            const uint32_t* inc = blocks + lane;
+            if (!stored) {
+                vp = ckpt[64 * blk];
+                vn = ckpt[64 * blk + 32];
+                uint32_t d0[32];
+                band_block(P, planeP, T, planeT, blk, b, vp, vn, [&](int j, uint32_t d) { d0[j] = d; });
+                transpose32(d0);
+                uint32_t* out = blocks + lane;
+#pragma unroll
+                for (int r = 0; r < 32; ++r) out[32 * r] = d0[r];
+            }
+            while (walking && (stored || m == blk)) {
+                const uint32_t* w = inc + (stored ? 1024 * m : 0);
+                const int best = walk_step(~w[32 * q], ~w[32 * max(q - 1, 0)], ~w[32 * min(q + 1, kBandDistance)],
+                                           ckpt[64 * m], ckpt[64 * m + 32], q, kBandDistance, hb);
+                if (best >= 0) {
+                    const int op = best & 3, x = best >> 2;
+                    cg.push_run(run + hb - x, 32);
+                    cg.push((uint32_t)op_letter(op), 32);
+                    run = 0;
+                    hb = op == kOpDel ? x : x - 1;
+                    q += op == kOpDel ? -1 : (op == kOpIns ? 1 : 0);
+                    --s;
+                    if (s < 0) walking = false; /* never expected */
+                } else {
+                    run += hb;
+                    hb = 0;
+                    if (m == 0) walking = false;
+                }
+                if (hb == 0 && m > 0) {
+                    --m;
+                    hb = 32;
+                }
+            }
+            if (stored) break;
+        }
+        if (state == ST_DONE) {
+            if (s != 0 || q != b) {
+                state = ST_BADWALK;
+            } else {
+                cg.push_run(run, 32);
+                cg.finish(32);
+            }
+        }
+        __syncwarp();
+
+        /* CIGARs: four lanes write a pair's words, eight pairs at a time */
+        const uint32_t cap = A.cigar_stride;
+        if (cap) {
+            const bool aligned = (cap & 3u) == 0u && (reinterpret_cast<uintptr_t>(A.cigar) & 3u) == 0u;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int own = 8 * r + (lane >> 2), g = lane & 3;
+                const bool done = __shfl_sync(kFull, state, own) == ST_DONE;
+                const uint32_t len = (uint32_t)__shfl_sync(kFull, cg.n, own);
+                int8_t* dst = A.cigar + (size_t)__shfl_sync(kFull, pi, own) * cap;
+                if (!done) continue;
+                const uint32_t nbytes = len < cap ? len + 1u : cap;
+                const uint32_t* col = bytes + own;
+                for (uint32_t i = (uint32_t)g; 4u * i < nbytes; i += 4u) {
+                    const uint32_t off = 4u * (uint32_t)top - len + 4u * i; /* byte of the column */
+                    const int k = (int)(off >> 2);
+                    const uint32_t w0 = k < top ? col[32 * k] : 0u, w1 = k + 1 < top ? col[32 * (k + 1)] : 0u;
+                    const uint32_t w = __funnelshift_r(w0, w1, 8u * (off & 3u));
+                    if (aligned) {
+                        reinterpret_cast<uint32_t*>(dst)[i] = w;
+                    } else {
+                        for (uint32_t j = 0; j < 4u && 4u * i + j < nbytes; ++j) dst[4u * i + j] = (int8_t)(w >> (8u * j));
+                    }
+                }
+            }
+        }
+        if (state == ST_DONE) {
+            A.dist[pi] = D;
+            if (A.status)
+                A.status[pi] = (uint32_t)cg.n > cap ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED : (uint8_t)WFE_PAIR_OK;
+        } else if (state != ST_IDLE) {
+            finish_unaligned(A, pi, state);
+        }
+        __syncwarp();
+        if (work_next) {
+            uint32_t v = 0;
+            if (lane == 0) v = atomicAdd(work_next, 32u);
+            wb = __shfl_sync(kFull, v, 0);
+        } else {
+            wb += gridDim.x * 32u;
+        }
+    }
+    chain_next(A);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -991,22 +1310,14 @@ __global__ void bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq
 }
 
 const TierInfo kTiers[kNumTiers] = {
-    {T0::G, T0::J, T0::DCAP, T0::SMEM_OPS},
-    {T1::G, T1::J, T1::DCAP, T1::SMEM_OPS},
-    {T2::G, T2::J, T2::DCAP, T2::SMEM_OPS},
-    {T3::G, T3::J, T3::DCAP, T3::SMEM_OPS},
-    {T4::G, T4::J, T4::DCAP, T4::SMEM_OPS},
-    {kLongThreads, 0, kLongSmemDistance, false},
-    {kLongThreads, 0, 0x7fffffff, false},
+    {kBandDistance, 32},
+    {T1::DCAP, kWarps},
+    {T2::DCAP, kWarps},
+    {T3::DCAP, kWarps},
+    {T4::DCAP, kWarps},
+    {kLongSmemDistance, 1},
+    {0x7fffffff, 1},
 };
-
-/* The kernel a tier's host launches use (see tier_kernel_bounded). */
-template <class T>
-const void* host_kernel()
-{
-    if constexpr (T::G == 32) return (const void*)tier_kernel<T>;
-    else return (const void*)tier_kernel_bounded<T, false>;
-}
 
 template <class T>
 TierShape shape_of(uint32_t max_len, uint32_t cigar_stride, int sm_count)
@@ -1014,7 +1325,7 @@ TierShape shape_of(uint32_t max_len, uint32_t cigar_stride, int sm_count)
     TierShape sh{};
     const size_t smem = cta_smem_bytes<T>(max_len, cigar_stride);
     if (smem > 227u * 1024u) return sh;
-    const void* fn = host_kernel<T>();
+    const void* fn = (const void*)tier_kernel<T>;
     if (allow_smem(fn, smem) != cudaSuccess)
         return sh;
     int nb = 0;
@@ -1050,12 +1361,32 @@ cudaError_t launch(const AlignLaunch& a, int grid, cudaStream_t s)
             a.ops_scratch_bytes < (size_t)tsh.ops_group_bytes * (size_t)grid * (kWarps * T::GPW))
             return cudaErrorInvalidValue;
     }
-    cudaError_t e = allow_smem(host_kernel<T>(), smem);
+    cudaError_t e = allow_smem((const void*)tier_kernel<T>, smem);
     if (e != cudaSuccess) return e;
-    if constexpr (T::G == 32)
-        tier_kernel<T><<<grid, kThreads, smem, s>>>(a, sw, (uint32_t)gb);
-    else
-        tier_kernel_bounded<T><<<grid, kThreads, smem, s>>>(a, sw, (uint32_t)gb);
+    tier_kernel<T><<<grid, kThreads, smem, s>>>(a, sw, (uint32_t)gb);
+    return cudaGetLastError();
+}
+
+TierShape band_shape(uint32_t max_len, int sm_count)
+{
+    TierShape sh{};
+    const size_t smem = 4u * (size_t)band_smem_words(max_len);
+    if (smem > 227u * 1024u || allow_smem((const void*)band_kernel<false>, smem) != cudaSuccess) return sh;
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, band_kernel<false>, 32, smem) != cudaSuccess) return sh;
+    sh.grid = std::max(1, nb) * sm_count;
+    sh.smem = (uint32_t)smem;
+    sh.seq_words = std::max(1u, band_words(max_len));
+    return sh;
+}
+
+cudaError_t launch_band(const AlignLaunch& a, int grid, cudaStream_t s)
+{
+    const size_t smem = 4u * (size_t)band_smem_words(a.max_len);
+    if (smem > 227u * 1024u) return cudaErrorInvalidValue;
+    const cudaError_t e = allow_smem((const void*)band_kernel<false>, smem);
+    if (e != cudaSuccess) return e;
+    band_kernel<false><<<grid, 32, smem, s>>>(a, std::max(1u, band_words(a.max_len)));
     return cudaGetLastError();
 }
 
@@ -1308,7 +1639,7 @@ namespace {
 TierShape compute_tier_shape(int tier, uint32_t max_len, uint32_t cigar_stride, int sm_count)
 {
     switch (tier) {
-    case 0: return shape_of<T0>(max_len, cigar_stride, sm_count);
+    case 0: return band_shape(max_len, sm_count);
     case 1: return shape_of<T1>(max_len, cigar_stride, sm_count);
     case 2: return shape_of<T2>(max_len, cigar_stride, sm_count);
     case 3: return shape_of<T3>(max_len, cigar_stride, sm_count);
@@ -1435,7 +1766,7 @@ cudaError_t launch_tier(int tier, const AlignLaunch& a, int grid, cudaStream_t s
 {
     if (grid <= 0) return cudaErrorInvalidConfiguration;
     switch (tier) {
-    case 0: return launch<T0>(a, grid, s);
+    case 0: return launch_band(a, grid, s);
     case 1: return launch<T1>(a, grid, s);
     case 2: return launch<T2>(a, grid, s);
     case 3: return launch<T3>(a, grid, s);
@@ -1457,10 +1788,8 @@ cudaError_t launch_classify(const Layout& L, uint32_t n, const Buckets& B, cudaS
 cudaError_t launch_predict(const Layout& L, uint32_t n, uint32_t max_len, uint16_t* pred, int grid, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    const uint32_t plen = std::min<uint32_t>(max_len, (uint32_t)kPredictPrefix);
-    const size_t gb = group_smem_bytes<T0>(plen, 0);
-    const size_t smem = cta_smem_bytes<T0>(plen, 0);
-    cudaError_t e = allow_smem((const void*)tier_kernel_bounded<T0, true>, smem);
+    const size_t smem = 4u * (size_t)band_smem_words((uint32_t)kPredictPrefix);
+    cudaError_t e = allow_smem((const void*)band_kernel<true>, smem);
     if (e != cudaSuccess) return e;
     AlignLaunch a{};
     a.L = L;
@@ -1468,9 +1797,8 @@ cudaError_t launch_predict(const Layout& L, uint32_t n, uint32_t max_len, uint16
     a.max_len = max_len;
     a.pred = pred;
     a.tier = 0;
-    const uint32_t per_cta = kWarps * T0::GPW;
-    grid = std::max(1, std::min(grid, (int)((n + per_cta - 1) / per_cta)));
-    tier_kernel_bounded<T0, true><<<grid, kThreads, smem, s>>>(a, seq_words_for(plen), (uint32_t)gb);
+    grid = std::max(1, std::min(grid, (int)((n + 31u) / 32u)));
+    band_kernel<true><<<grid, 32, smem, s>>>(a, band_words((uint32_t)kPredictPrefix));
     return cudaGetLastError();
 }
 

@@ -11,11 +11,9 @@
 
 namespace wfe {
 
-/* Register tiers of the alignment kernel: G lanes per alignment, 2J+1
- * register chunks of G diagonals per lane, largest distance G*J + G/2 - 1. */
 struct TierInfo {
-    int G, J, dcap;
-    bool ops_in_smem;
+    int dcap;          /* largest distance the tier aligns */
+    int pairs_per_cta; /* pairs a CTA takes at a time */
 };
 
 /* Tiers 0-4 are register tiers (one pair per group of G lanes); tiers 5

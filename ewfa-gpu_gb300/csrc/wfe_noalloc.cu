@@ -12,16 +12,16 @@
  * which every GPU that loads this library holds until the process exits.
  *
  * The pairs go through two of the tiers, in rounds of up to 2^20 pairs:
- * tier 0 (4 lanes per pair, distances up to 21, backtrace store in shared
+ * tier 0 (a thread per pair, distances up to 31, all its state in shared
  * memory, so it needs none of the array) aligns every pair, and hands the
- * ones past distance 21 on, through a list at the start of the array, to
+ * ones past distance 31 on, through a list at the start of the array, to
  * the tier-3 kernel (32 lanes per pair, distances up to 271, backtrace store
  * in global memory), pointed at the rest of the array.  A pair's store there
  * takes 20,544 bytes (a triangle of 271 rows), so the rest holds the stores
  * of 612 pairs in flight, 153 CTAs of 4 pairs; that grid is sized so that
  * every resident group has its own slot (about one CTA per SM on a GB300,
  * below the kernel's occupancy: the price of the fixed size, paid only by
- * the pairs past distance 21).  With a max_distance of 21 or less tier 0
+ * the pairs past distance 31).  With a max_distance of 31 or less tier 0
  * does all of it.
  */
 #include <algorithm>
@@ -154,9 +154,9 @@ extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_p
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return WFE_ERR_CUDA;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    /* tier 0: its occupancy (its store is in shared memory).  Its 32 pairs
-     * per CTA each stage a CIGAR in shared memory: for long sequences with
-     * wide CIGAR slots it does not fit, and tier 3 aligns every pair. */
+    /* tier 0: its occupancy (its state is in shared memory).  Sequences of
+     * more than about 9,000 bases do not fit there, and tier 3 aligns every
+     * pair. */
     const wfe::TierShape sh0 = wfe::tier_shape(kFirstTier, max_len, cigar_stride, sms);
     const bool first = sh0.grid > 0;
     const bool deep = !first || max_distance > wfe::tier_info(kFirstTier).dcap;
@@ -196,7 +196,7 @@ extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_p
             a.retry = listed ? list : nullptr;
             a.retry_count = listed ? count : nullptr;
             a.chain.shape[kFirstTier] = sh0;
-            const uint32_t per_cta0 = 4u * (32u / (uint32_t)wfe::tier_info(kFirstTier).G);
+            const uint32_t per_cta0 = (uint32_t)wfe::tier_info(kFirstTier).pairs_per_cta;
             const int grid0 = (int)std::min<uint64_t>((uint64_t)sh0.grid, ((uint64_t)nb + per_cta0 - 1) / per_cta0);
             if (wfe::launch_tier(kFirstTier, a, std::max(grid0, 1), s) != cudaSuccess) return WFE_ERR_CUDA;
         }

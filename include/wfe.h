@@ -190,7 +190,7 @@ int wfe_reset_stats(wfe_ctx* ctx);
  * device and each bucket is aligned with launch shapes sized to its longest
  * sequence -- shared memory per pair, resident CTAs -- starting at its own
  * first tier:
- *   tier 0: 4 lanes per pair, backtrace store in shared memory, distance <= 21
+ *   tier 0: a thread per pair, bit-parallel band of 32 diagonals, distance <= 31
  *   tier 1: 32 lanes per pair, shared-memory store, <= 79
  *   tier 2: 32 lanes, shared-memory store, <= 143
  *   tier 3: 32 lanes, store spilled to global memory, <= 271
@@ -351,13 +351,13 @@ int wfe_cigar_from_history_device(const char* d_ascii, const wfe_pair* d_pairs,
  * device's primary context, or one the application made current); the first
  * call in each context looks that address up (set-up, once per context),
  * so make that first call outside any stream capture.  The pairs are aligned
- * in rounds of up to 2^20: the 4-lane tier (distances up to 21, backtrace in
- * shared memory) takes every pair of a round and hands the ones past
- * distance 21, through a list at the start of the array, to the 32-lane
+ * in rounds of up to 2^20: tier 0 (a thread per pair, distances up to 31, all
+ * its state in shared memory) takes every pair of a round and hands the ones
+ * past distance 31, through a list at the start of the array, to the 32-lane
  * tier 3, whose backtrace stores fill the rest: 612 pairs in flight, 153
  * CTAs of 4 (about one per SM on a 152-SM GB300, below that kernel's
- * occupancy).  Sequences and CIGAR slots too wide for the 4-lane tier's
- * shared memory go to tier 3 alone (816 pairs in flight).  On short reads a
+ * occupancy).  Sequences too long for tier 0's shared memory (past 9,000
+ * bases) go to tier 3 alone (816 pairs in flight).  On short reads a
  * call runs at ~80% of wfe_align_device's speed.
  * Every call shares the array and it keeps the last call's contents
  * (nothing in it has to start at zero: the list's count is set by a

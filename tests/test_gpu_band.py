@@ -1,0 +1,67 @@
+"""The bit-parallel band kernels at the sizes where they can go wrong: columns
+around whole blocks of 32, texts either side of what tier 0 keeps in shared
+memory, distances and length differences either side of the band's limit,
+every byte alignment, pairs next to each other and apart; against the oracle."""
+import numpy as np
+import pytest
+
+import wfe
+from test_gpu_parity import _pinned, compare_with_oracle, torch_cuda
+
+pytestmark = pytest.mark.gpu
+
+
+def bases(rng, n):
+    return np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, n)].tobytes()
+
+
+def edited(rng, text, edits):
+    """`text` after `edits` random edits, a run of insertions or deletions among them now and then."""
+    s = list(text)
+    while edits > 0:
+        k = int(rng.integers(1, 1 + min(edits, 6))) if rng.random() < 0.2 else 1
+        at = int(rng.integers(0, len(s) + 1))
+        kind = rng.integers(0, 3)
+        if kind == 0:
+            s[at:at] = bases(rng, k)
+        elif kind == 1:
+            del s[at:at + k]
+        elif at < len(s):
+            s[at] = b"ACGT"[(b"ACGT".index(s[at]) + 1) % 4]
+        edits -= k
+    return bytes(s)
+
+
+def band_pairs(lengths, edits, seed):
+    rng = np.random.default_rng(seed)
+    seqs = []
+    for n in lengths:
+        unit = bases(rng, max(1, n if rng.random() < 0.7 else 1 + n // 9))
+        text = (unit * (n // len(unit) + 1))[:n]  # repeats have many optimal paths: the tie order decides
+        for e in edits:
+            p = edited(rng, text, e)
+            seqs.append((p, text) if rng.random() < 0.5 else (text, p))
+    return seqs
+
+
+@pytest.mark.parametrize("cap,stride,spread", [(0, 900, 0), (31, 900, 0), (32, 901, 0), (0, 16, 5000)])
+def test_tier_0_band(cap, stride, spread):
+    torch_cuda()
+    lengths = [0, 1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 150, 159, 160, 161, 191, 192, 193, 320, 600]
+    seqs = band_pairs(lengths, [0, 1, 3, 9, 25, 30, 31, 32, 33, 40], 11)
+    for d in range(26, 36):  # the ends' diagonals at the edge of the band
+        t = bases(np.random.default_rng(d), 150)
+        seqs += [(t[d:], t), (t, t[:-d]), (t[:70] + t[70 + d:], t), (b"", t[:d]), (t[:d], b"")]
+    ascii, pairs = wfe.pairs_from_list(seqs)
+    if spread:  # apart, at every alignment: no warp's pairs lie in one span
+        buf, q = np.zeros(spread * 2 * len(pairs), np.uint8), pairs.copy()
+        for i, (p, t) in enumerate(seqs):
+            for off, s, key in ((2 * i * spread + i % 16, p, "p_off"), ((2 * i + 1) * spread + i // 16 % 16, t, "t_off")):
+                buf[off:off + len(s)] = np.frombuffer(s, np.uint8)
+                q[key][i] = off
+        ascii, pairs = buf, q
+    with wfe.Context(max_seq_len=1000, cigar_stride=stride, max_distance=cap) as ctx:
+        dist, cg, st = ctx.align(_pinned(ascii), _pinned(pairs))  # read where they lie
+        assert ctx.stats()["tier_entered"][0] >= len(pairs)
+    assert (dist == 31).any() and (dist == 32).any()
+    compare_with_oracle(ascii, pairs, stride, dist, cg, st, max_distance=cap)
