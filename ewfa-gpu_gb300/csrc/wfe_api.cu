@@ -94,6 +94,7 @@ struct TimedLaunch {
 struct BucketPlan {
     uint32_t max_len = 0;
     int first_tier = 0;
+    bool by_length = false; /* first_tier is the length's default, not the caller's choice */
     int last_tier = 0;
     TierShape shape[kNumTiers] = {};
     LongClasses cls{};      /* tier 5's distance classes (n == 0: none) */
@@ -218,7 +219,7 @@ int default_first_tier(uint32_t max_len)
 /* per bucket: list counts (one more for the last tier's hand-on), finished
  * CTAs and work counters of every tier, then, for every class of tier 5,
  * front and back list counts, finished CTAs and work counters */
-constexpr size_t kChainWords = 3 * kNumTiers + 1 + 4 * kLongClasses;
+constexpr size_t kChainWords = 3 * kNumTiers + 1 + 4 * (kLongClasses + 1) + 2 * kOrderBins;
 constexpr size_t kCountWords = kMaxBuckets * kChainWords;
 
 /* What a stage owns itself: its staging and scratch allocations, pinned
@@ -257,7 +258,9 @@ void plan_bucket(wfe_ctx* ctx, BucketPlan& b)
         b.bound = bound_shape(b.max_len, ctx->sm_count);
         if (b.bound.grid > 0 && ctx->d_long_scratch[5]) {
             b.cls = long_classes(b.max_len, ctx->sm_count, ctx->long_slab[5] * (uint64_t)ctx->scratch_ctas[5]);
-            for (int k = 0; k < b.cls.n; ++k) b.cls.shape[k].scratch = ctx->d_long_scratch[5];
+            for (int k = 0; k < b.cls.n; ++k)
+                b.cls.shape[k].scratch = b.cls.wide[k].scratch = ctx->d_long_scratch[5];
+            b.cls.scan.scratch = b.cls.tile.scratch = ctx->d_long_scratch[5];
         }
     }
 }
@@ -415,13 +418,18 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
         uint32_t* cw = words + 3 * kNumTiers + 1;
         for (int k = 0; k < a.chain.cls.n; ++k) {
             a.chain.cls.list[k] = lists + (size_t)(kNumTiers + k) * B;
-            if (st.own_long_scratch[5]) a.chain.cls.shape[k].scratch = st.own_long_scratch[5];
+            if (st.own_long_scratch[5])
+                a.chain.cls.shape[k].scratch = a.chain.cls.wide[k].scratch = st.own_long_scratch[5];
         }
+        if (st.own_long_scratch[5]) a.chain.cls.scan.scratch = a.chain.cls.tile.scratch = st.own_long_scratch[5];
         a.chain.cls.cap = B;
         a.chain.cls.counts = cw;
-        a.chain.cls.low_counts = cw + kLongClasses;
-        a.chain.cls.cta_done = cw + 2 * kLongClasses;
-        a.chain.cls.work_next = cw + 3 * kLongClasses;
+        a.chain.cls.low_counts = cw + (kLongClasses + 1);
+        a.chain.cls.cta_done = cw + 2 * (kLongClasses + 1);
+        a.chain.cls.work_next = cw + 3 * (kLongClasses + 1);
+        a.chain.cls.order = lists + (size_t)(kNumTiers + kLongClasses) * B;
+        a.chain.cls.order_count = cw + 4 * (kLongClasses + 1);
+        a.chain.cls.order_next = a.chain.cls.order_count + kOrderBins;
     }
     int grid = bp.shape[t].grid;
     if (!listed) {
@@ -434,19 +442,31 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     if (rc != WFE_OK) return rc;
     if (bounded && t == 5 && a.chain.cls.n > 0) {
         /* tier 5 starts with the bound pass, which starts the classes */
-        WFE_CUDA(ctx, launch_bound(a, s));
+        WFE_CUDA(ctx, launch_bound(a, s, &ctx->stats.kernel_launches));
     } else {
-        if (bounded && t == 6) {
-            /* bounds only, then tier 6 */
-            WFE_CUDA(ctx, launch_bound(a, s));
-            ctx->stats.kernel_launches++;
-        }
+        /* bounds only, then tier 6 */
+        if (bounded && t == 6) WFE_CUDA(ctx, launch_bound(a, s, &ctx->stats.kernel_launches));
         WFE_CUDA(ctx, launch_tier(t, a, grid, s));
+        ctx->stats.kernel_launches++;
     }
     if (tl) WFE_CUDA(ctx, cudaEventRecord(tl->stop, s));
-    ctx->stats.kernel_launches++;
     ctx->stats.tier_launches[t]++;
     return WFE_OK;
+}
+
+/* The tier a batch of n pairs starts at.  Sequences of more than
+ * kScanLength bases start at tier 0 by default for the sake of small calls
+ * and of contexts without tier 5's scratch; a large batch that can starts at
+ * tier 5, whose scan costs twice tier 0's band and finds the class of the
+ * pairs that tier 0 would hand on. */
+constexpr uint32_t kScanLength = 400;
+constexpr uint32_t kScanPairs = 8192;
+int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n)
+{
+    const bool scan = bp.by_length && bp.max_len > kScanLength && n >= kScanPairs && ctx->deep_ready && ctx->bound &&
+                      bp.bound.grid > 0 && bp.cls.scan.grid > 0 &&
+                      !(ctx->cfg.max_distance > 0 && ctx->cfg.max_distance <= tier_info(4).dcap);
+    return scan ? std::max(bp.first_tier, 5) : bp.first_tier;
 }
 
 /* Enqueue the alignment of pairs 0..n-1 of one batch on stream s: with one
@@ -462,7 +482,7 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     WFE_CUDA(ctx, cudaMemsetAsync(st.d_counts, 0, sizeof(uint32_t) * kCountWords, s));
     if (ctx->nbuckets == 1 && !ctx->predict) {
         const BucketPlan& bp = ctx->bucket[0];
-        const int t = first_override ? first_override[0] : bp.first_tier;
+        const int t = first_override ? first_override[0] : first_tier_of(ctx, bp, n);
         ctx->single_entered[t] += n;
         return launch_bucket(ctx, st, bp, 0, t, L, false, n, dist, cigar, status, s, base);
     }
@@ -490,10 +510,19 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     bk.counts = st.d_counts;
     bk.count_stride = (uint32_t)kChainWords;
     bk.totals = ctx->d_bucket_total;
+    /* Tier 5's scan and classes do not depend on the bucket's length: the
+     * last bucket's chain takes the tier-5 pairs of all buckets, one scan and
+     * one launch of the classes instead of one per bucket. */
+    const BucketPlan& lp = ctx->bucket[ctx->nbuckets - 1];
+    const int lt = bk.first_tier[ctx->nbuckets - 1];
+    const bool merge = ctx->bound && lt <= 5 && lp.bound.grid > 0 && lp.cls.scan.grid > 0 &&
+                       chain_end(ctx->cfg, lt, lp.last_tier) >= 5;
+    bk.tier5_to = merge ? ctx->nbuckets - 1 : -1;
     WFE_CUDA(ctx, launch_classify(L, n, bk, s));
     ctx->stats.kernel_launches++;
     /* longest bucket first: its chains take longest */
     for (int b = ctx->nbuckets - 1; b >= 0; --b) {
+        if (merge && b + 1 < ctx->nbuckets && bk.first_tier[b] == 5) continue;
         const int r =
             launch_bucket(ctx, st, ctx->bucket[b], b, bk.first_tier[b], L, true, n, dist, cigar, status, s, base);
         if (r != WFE_OK) return r;
@@ -627,6 +656,7 @@ int create_context(const wfe_config* cfg, uint64_t budget5, uint64_t budget6, wf
     ctx->nbuckets = 1;
     ctx->bucket[0].max_len = c.max_seq_len;
     ctx->bucket[0].first_tier = default_first_tier(c.max_seq_len);
+    ctx->bucket[0].by_length = true;
     plan_bucket(ctx, ctx->bucket[0]);
     if (!bucket_usable(ctx->bucket[0])) return bail(cudaErrorInvalidValue); /* sequences too long for shared memory */
 
@@ -698,6 +728,7 @@ int wfe_set_policy(wfe_ctx* ctx, uint32_t nbuckets, const uint32_t* bucket_max_l
         const int32_t ft = first_tier ? first_tier[b] : -1;
         if (ft >= kNumTiers) return WFE_ERR_INVALID_ARGUMENT;
         plan[b].first_tier = ft < 0 ? default_first_tier(m) : ft;
+        plan[b].by_length = ft < 0;
         plan_bucket(ctx, plan[b]);
         if (plan[b].first_tier > plan[b].last_tier || !bucket_usable(plan[b])) return WFE_ERR_INVALID_ARGUMENT;
     }

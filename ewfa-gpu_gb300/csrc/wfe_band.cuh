@@ -194,6 +194,114 @@ __device__ __forceinline__ int walk_step(uint32_t wq, uint32_t wu, uint32_t wd, 
     return best;
 }
 
+/* ---- bands of NW words of 32 diagonals ------------------------------------ */
+
+/* t += v over NW words, with carries */
+template <int NW>
+__device__ __forceinline__ void add_words(uint32_t (&t)[NW], const uint32_t (&v)[NW])
+{
+#ifdef __CUDA_ARCH__
+    asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(t[0]) : "r"(v[0]));
+#pragma unroll
+    for (int i = 1; i < NW - 1; ++i) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(t[i]) : "r"(v[i]));
+    asm volatile("addc.u32 %0, %0, %1;" : "+r"(t[NW - 1]) : "r"(v[NW - 1]));
+#else
+    uint64_t c = 0;
+    for (int i = 0; i < NW; ++i) {
+        c += (uint64_t)t[i] + v[i];
+        t[i] = (uint32_t)c;
+        c >>= 32;
+    }
+#endif
+}
+
+/* One column of a band of NW words (see band_column): column j of a block,
+ * a0/a1 the bit planes of the pattern rows of the block's first column and
+ * of the 32 rows after them, t0/t1 the block's text planes. */
+template <int NW>
+__device__ __forceinline__ void wide_column(const uint32_t (&a0)[NW + 1], const uint32_t (&a1)[NW + 1], uint32_t t0,
+                                            uint32_t t1, int j, uint32_t (&vp)[NW], uint32_t (&vn)[NW],
+                                            uint32_t (&d0)[NW])
+{
+    static_assert(NW >= 2, "one word: band_column");
+    const uint32_t c0 = bit_mask(t0, j), c1 = bit_mask(t1, j);
+    uint32_t eq[NW];
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        const uint32_t x = __funnelshift_r(a0[i], a0[i + 1], (uint32_t)j) ^ c0;
+        eq[i] = ~(x | (__funnelshift_r(a1[i], a1[i + 1], (uint32_t)j) ^ c1));
+        d0[i] = eq[i] & vp[i];
+    }
+    add_words<NW>(d0, vp);
+#pragma unroll
+    for (int i = 0; i < NW; ++i) d0[i] = (d0[i] ^ vp[i]) | eq[i] | vn[i];
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        const uint32_t hp = vn[i] | ~(d0[i] | vp[i]), hn = vp[i] & d0[i];
+        const uint32_t x = __funnelshift_r(d0[i], i + 1 < NW ? d0[i + 1] : 0u, 1u);
+        vp[i] = hn | ~(x | hp);
+        vn[i] = x & hp;
+    }
+}
+
+/* One column of a tile of 32 rows, with the horizontal differences that come
+ * in above it and those that leave below: hp/hn hold the column's at their
+ * highest bit (hi_p/hi_n collect, first column highest). */
+__device__ __forceinline__ void tile_column(uint32_t p0, uint32_t p1, uint32_t c0, uint32_t c1, uint32_t hp_in,
+                                            uint32_t hn_in, uint32_t& vp, uint32_t& vn, uint32_t& hp_out,
+                                            uint32_t& hn_out)
+{
+    const uint32_t x = p0 ^ c0;
+    const uint32_t eq = ~(x | (p1 ^ c1));
+    const uint32_t t = hn_in >> 31;
+    const uint32_t a = (eq | t) & vp;
+    const uint32_t d0 = ((a + vp) ^ vp) | (eq | t | vn);
+    const uint32_t hp = vn | ~(d0 | vp), hn = vp & d0;
+    hp_out = __funnelshift_l(hp, hp_out, 1u);
+    hn_out = __funnelshift_l(hn, hn_out, 1u);
+    const uint32_t sp = __funnelshift_l(hp_in, hp, 1u), sn = __funnelshift_l(hn_in, hn, 1u);
+    vp = sn | ~(d0 | sp);
+    vn = sp & d0;
+}
+
+/* Words of a bit plane of the pattern that start at base r (negative: virtual
+ * rows, any bits), from the lane's column of plane words, n of them, `row`
+ * words apart. */
+template <int N>
+__device__ __forceinline__ void plane_window(const uint32_t* plane, int row, int n, int r, uint32_t (&a)[N])
+{
+    const int w0 = r >> 5;
+    uint32_t x = (unsigned)w0 < (unsigned)n ? plane[(size_t)w0 * row] : 0u;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int w = w0 + k + 1;
+        const uint32_t y = (unsigned)w < (unsigned)n ? plane[(size_t)w * row] : 0u;
+        a[k] = __funnelshift_r(x, y, (uint32_t)(r & 31));
+        x = y;
+    }
+}
+
+/* Move a band of 64 diagonals by `by` (16 or -16) diagonals, downwards for
+ * by > 0: bit i becomes bit i - by.  Rows that enter count one more than
+ * their neighbour in the band (an upper bound, as every value of a band);
+ * returns the change of the value on bit 0. */
+__device__ __forceinline__ int move_band(uint32_t (&vp)[2], uint32_t (&vn)[2], int by)
+{
+    if (by > 0) {
+        const int top = __popc(vp[0] & 0xffffu) - __popc(vn[0] & 0xffffu);
+        vp[0] = __funnelshift_r(vp[0], vp[1], 16u);
+        vn[0] = __funnelshift_r(vn[0], vn[1], 16u);
+        vp[1] = (vp[1] >> 16) | 0xffff0000u;
+        vn[1] >>= 16;
+        return top;
+    }
+    vp[1] = __funnelshift_l(vp[0], vp[1], 16u);
+    vn[1] = __funnelshift_l(vn[0], vn[1], 16u);
+    vp[0] <<= 16;
+    vn[0] = (vn[0] << 16) | 0xffffu;
+    return 16;
+}
+
 }  // namespace wfe
 
 #endif

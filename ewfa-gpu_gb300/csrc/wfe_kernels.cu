@@ -13,6 +13,11 @@
  *                        has a distance bound
  *   bound_kernel         distance bounds from a 32-diagonal band, one warp
  *                        per pair; routes tier 5's pairs to distance classes
+ *   wide_kernel<NW, .>   tier 5 in bulk, one pair per thread, bands of 32 NW
+ *                        diagonals: the scan that bounds distances, and the
+ *                        classes with the most pairs
+ *   tile_kernel          tier 5 in bulk, several lanes per pair
+ *   order_*_kernel       tier 5's list in order of length
  *   classify_kernel      length buckets and predicted tiers
  *   history_cigar_kernel CIGARs from the reference's 128-bit histories
  *                        (src/kernels.cu:397-625)
@@ -82,11 +87,10 @@ __device__ __forceinline__ int op_of(uint2 e, int bit)
 
 /* One distance tier: G lanes per pair, 2J+1 register chunks, backtrace
  * store in shared (SMEM_OPS) or global memory, sequences of up to RMAX*G
- * aligned 16-byte blocks loaded with all loads in flight at once, at least
- * MINB resident CTAs per SM asked of the register allocator. */
-template <int G_, int J_, bool SMEM_OPS_, int RMAX_, int MINB_ = 1>
+ * aligned 16-byte blocks loaded with all loads in flight at once. */
+template <int G_, int J_, bool SMEM_OPS_, int RMAX_>
 struct Tier {
-    static constexpr int G = G_, J = J_, RMAX = RMAX_, MINB = MINB_;
+    static constexpr int G = G_, J = J_, RMAX = RMAX_;
     static constexpr bool SMEM_OPS = SMEM_OPS_;
     static constexpr int NC = 2 * J + 1;
     static constexpr int DCAP = G * J + G / 2 - 1;
@@ -167,6 +171,16 @@ __global__ void tier_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_
 template <bool GLOBAL_WF, int NT>
 __global__ void long_kernel(const __grid_constant__ AlignLaunch A);
 __global__ void bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t unused);
+template <int NW, bool SCAN>
+__global__ void wide_kernel(const __grid_constant__ AlignLaunch A);
+__global__ void tile_kernel(const __grid_constant__ AlignLaunch A);
+__device__ uint32_t tile_chunks(const LongClasses& C);
+/* The classes of a list that the bound pass routes, aligned by a CTA per pair. */
+__device__ __forceinline__ bool class_by_cta(int dlim) { return dlim == 257 || dlim == 577 || dlim == 961; }
+__device__ __forceinline__ bool tile_takes(const LongClasses& C, int c, uint32_t count)
+{
+    return c + 1 < C.n && C.tile.grid > 0 && count > 0u && !(C.wide[c].grid > 0 && count >= kWidePairs);
+}
 using T1 = Tier<32, 2, true, 1>;   /* distance <= 79  */
 using T2 = Tier<32, 4, false, 1>;  /* distance <= 143; backtrace store in global scratch: 8 CTAs per SM */
 using T3 = Tier<32, 8, false, 1>;  /* distance <= 271 */
@@ -202,7 +216,8 @@ __device__ __forceinline__ void note_deferred(const AlignLaunch& A)
  * limit is also what a grid launched from the device runs with. */
 template <typename K>
 __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int u, int grid, int threads,
-                                            uint32_t smem, bool tier_args, uint32_t seq_words, uint32_t gbytes)
+                                            uint32_t smem, bool tier_args, uint32_t seq_words, uint32_t gbytes,
+                                            int bulk = 0)
 {
     void* buf = cudaGetParameterBufferV2((void*)kernel, dim3((unsigned)grid), dim3((unsigned)threads), smem);
     if (!buf) {
@@ -217,6 +232,8 @@ __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int 
     AlignLaunch* n = static_cast<AlignLaunch*>(buf);
     n->tier = u;
     n->cls = -1;
+    n->min_count = n->max_count = 0u;
+    n->bulk = bulk;
     n->work = A.chain.list[u];
     n->work_count = A.chain.counts + u;
     n->retry = u < A.chain.last_tier ? A.chain.list[u + 1] : A.chain.defer;
@@ -251,11 +268,19 @@ __device__ void launch_class_on_device(const AlignLaunch& A, int c, uint32_t cou
 {
     const LongClasses& C = A.chain.cls;
     const TierShape& sh = C.shape[c];
-    const int grid = max(1, min(sh.grid, (int)count));
-    const void* kernel = sh.threads == kLongTinyThreads    ? (const void*)long_kernel<false, kLongTinyThreads>
+    /* one thread per pair or a CTA per pair, by the number of pairs */
+    const bool wide = A.bulk && C.wide[c].grid > 0 && count >= kWidePairs;
+    const TierShape& use = wide ? C.wide[c] : sh;
+    const int grid = max(1, min(use.grid, wide ? ((int)count + 31) / 32 : (int)count));
+    const void* kernel = wide ? (use.dlim == 127   ? (const void*)wide_kernel<4, false>
+                                 : use.dlim == 255 ? (const void*)wide_kernel<8, false>
+                                 : use.dlim == 511 ? (const void*)wide_kernel<16, false>
+                                                   : (const void*)wide_kernel<32, false>)
+                         : sh.threads == kLongTinyThreads    ? (const void*)long_kernel<false, kLongTinyThreads>
                          : sh.threads == kLongSmallThreads ? (const void*)long_kernel<false, kLongSmallThreads>
                                                            : (const void*)long_kernel<false, kLongThreads>;
-    void* buf = cudaGetParameterBufferV2((void*)kernel, dim3((unsigned)grid), dim3((unsigned)sh.threads), sh.smem);
+    void* buf = cudaGetParameterBufferV2((void*)kernel, dim3((unsigned)grid), dim3((unsigned)use.threads),
+                                         use.smem);
     if (!buf) {
         note_launch_error(A, 5);
         return;
@@ -270,8 +295,10 @@ __device__ void launch_class_on_device(const AlignLaunch& A, int c, uint32_t cou
     n->cls = c;
     n->work = C.list[c];
     n->work_count = C.counts + c;
-    n->retry = !last ? C.list[c + 1] : (5 < A.chain.last_tier ? A.chain.list[6] : nullptr);
-    n->retry_count = !last ? C.counts + c + 1 : A.chain.counts + 6;
+    /* a class of the bulk kernels hands on to the last, which has no such limits */
+    const int up = A.bulk ? C.n - 1 : c + 1;
+    n->retry = !last ? C.list[up] : (5 < A.chain.last_tier ? A.chain.list[6] : nullptr);
+    n->retry_count = !last ? C.counts + up : A.chain.counts + 6;
     n->passed_total = last && A.chain.passed ? A.chain.passed + 5 : nullptr;
     if (cudaLaunchDeviceV2(buf, cudaStreamTailLaunch) != cudaSuccess) {
         note_launch_error(A, 5);
@@ -292,7 +319,10 @@ __device__ void launch_tier_on_device(const AlignLaunch& A, int u, uint32_t coun
     case 3: launch_on_device<T3>(A, u, count); break;
     case 4: launch_on_device<T4>(A, u, count); break;
     case 5:
-        if (A.bound && A.chain.cls.n > 0) {
+        if (A.bound && A.chain.cls.n > 0 && A.chain.cls.scan.grid > 0 && count >= kScanMin) {
+            tail_launch(wide_kernel<2, true>, A, u, max(1, min(A.chain.cls.scan.grid, (int)((count + 31u) / 32u))), 32,
+                        0u, false, 0u, 0u, 1);
+        } else if (A.bound && A.chain.cls.n > 0) {
             const TierShape& b = A.chain.bound_shape;
             const uint32_t per_cta = (uint32_t)b.threads / 32u;
             const int grid = max(1, min(b.grid, (int)((count + per_cta - 1u) / per_cta)));
@@ -313,17 +343,52 @@ __device__ void launch_tier_on_device(const AlignLaunch& A, int u, uint32_t coun
     }
 }
 
-/* The launch that follows this one in the chain: within tier 5 with
- * classes (the bound pass, A.cls == -1, or class A.cls), the next class
- * that has work; else the next tier that has work (pairs handed on, or
- * routed to it up front). */
+/* Tail launch of the tile kernel over the classes it takes. */
+__device__ void launch_tile_on_device(const AlignLaunch& A, uint32_t chunks)
+{
+    const LongClasses& C = A.chain.cls;
+    void* buf = cudaGetParameterBufferV2((void*)tile_kernel, dim3((unsigned)max(1, min(C.tile.grid, (int)chunks))),
+                                         dim3((unsigned)C.tile.threads), 0u);
+    if (!buf) {
+        note_launch_error(A, 5);
+        return;
+    }
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&A);
+    unsigned long long* dst = static_cast<unsigned long long*>(buf);
+#pragma unroll 4
+    for (unsigned i = 0; i < sizeof(AlignLaunch) / 8; ++i) dst[i] = src[i];
+    AlignLaunch* n = static_cast<AlignLaunch*>(buf);
+    n->tier = 5;
+    n->cls = kTileClass;
+    n->retry = C.list[C.n - 1];
+    n->retry_count = C.counts + C.n - 1;
+    n->passed_total = nullptr;
+    if (cudaLaunchDeviceV2(buf, cudaStreamTailLaunch) != cudaSuccess) {
+        note_launch_error(A, 5);
+        return;
+    }
+    if (A.chain.launched) atomicAdd(A.chain.launched + 5, 1ull);
+}
+
+/* The launch that follows this one in the chain: within tier 5 with classes,
+ * after the scan (A.bulk) the tile kernel if it takes any class, then the
+ * classes that it does not take, in order; else the next tier that has work
+ * (pairs handed on, or routed to it up front). */
 __device__ void launch_next(const AlignLaunch& A)
 {
     if (A.tier == 5 && A.chain.cls.n > 0) {
-        for (int c = A.cls + 1; c < A.chain.cls.n; ++c) {
-            const uint32_t cnt = *reinterpret_cast<volatile const uint32_t*>(A.chain.cls.counts + c) +
-                                 *reinterpret_cast<volatile const uint32_t*>(A.chain.cls.low_counts + c);
-            if (cnt > 0u) {
+        const LongClasses& C = A.chain.cls;
+        if (A.bulk && A.cls == -1) {
+            const uint32_t chunks = tile_chunks(C);
+            if (chunks > 0u) {
+                launch_tile_on_device(A, chunks);
+                return;
+            }
+        }
+        for (int c = A.cls == kTileClass ? 0 : A.cls + 1; c < C.n; ++c) {
+            const uint32_t front = *reinterpret_cast<volatile const uint32_t*>(C.counts + c);
+            const uint32_t cnt = front + *reinterpret_cast<volatile const uint32_t*>(C.low_counts + c);
+            if (cnt > 0u && !(A.bulk && tile_takes(C, c, front))) {
                 launch_class_on_device(A, c, cnt);
                 return;
             }
@@ -740,6 +805,27 @@ __device__ __forceinline__ void band_block(const uint32_t* P, int planeP, const 
     }
 }
 
+/* A CIGAR of len bytes from the end of a column of backwards-written words
+ * (`top` of them, `row` apart) to its slot, words g, g + G, ... by lane g of
+ * G: up to the terminator (when it fits) and zeros to the end of its word,
+ * or byte by byte where the slots are not word-aligned. */
+__device__ __forceinline__ void store_back_bytes(const uint32_t* col, int row, int top, uint32_t len, uint32_t cap,
+                                                 int8_t* dst, int g, int G, bool aligned)
+{
+    const uint32_t nbytes = len < cap ? len + 1u : cap;
+    for (uint32_t i = (uint32_t)g; 4u * i < nbytes; i += (uint32_t)G) {
+        const uint32_t off = 4u * (uint32_t)top - len + 4u * i; /* byte of the column */
+        const int k = (int)(off >> 2);
+        const uint32_t w0 = k < top ? col[row * k] : 0u, w1 = k + 1 < top ? col[row * (k + 1)] : 0u;
+        const uint32_t w = __funnelshift_r(w0, w1, 8u * (off & 3u));
+        if (aligned) {
+            reinterpret_cast<uint32_t*>(dst)[i] = w;
+        } else {
+            for (uint32_t j = 0; j < 4u && 4u * i + j < nbytes; ++j) dst[4u * i + j] = (int8_t)(w >> (8u * j));
+        }
+    }
+}
+
 template <bool PREDICT>
 __global__ void __launch_bounds__(32, 9) band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw)
 {
@@ -895,20 +981,7 @@ __global__ void __launch_bounds__(32, 9) band_kernel(const __grid_constant__ Ali
                 const bool done = __shfl_sync(kFull, state, own) == ST_DONE;
                 const uint32_t len = (uint32_t)__shfl_sync(kFull, cg.n, own);
                 int8_t* dst = A.cigar + (size_t)__shfl_sync(kFull, pi, own) * cap;
-                if (!done) continue;
-                const uint32_t nbytes = len < cap ? len + 1u : cap;
-                const uint32_t* col = bytes + own;
-                for (uint32_t i = (uint32_t)g; 4u * i < nbytes; i += 4u) {
-                    const uint32_t off = 4u * (uint32_t)top - len + 4u * i; /* byte of the column */
-                    const int k = (int)(off >> 2);
-                    const uint32_t w0 = k < top ? col[32 * k] : 0u, w1 = k + 1 < top ? col[32 * (k + 1)] : 0u;
-                    const uint32_t w = __funnelshift_r(w0, w1, 8u * (off & 3u));
-                    if (aligned) {
-                        reinterpret_cast<uint32_t*>(dst)[i] = w;
-                    } else {
-                        for (uint32_t j = 0; j < 4u && 4u * i + j < nbytes; ++j) dst[4u * i + j] = (int8_t)(w >> (8u * j));
-                    }
-                }
+                if (done) store_back_bytes(bytes + own, 32, top, len, cap, dst, g, 4, aligned);
             }
         }
         if (state == ST_DONE) {
@@ -1155,6 +1228,680 @@ __global__ void long_kernel(const __grid_constant__ AlignLaunch A)
 }
 
 /* ------------------------------------------------------------------------ */
+/* Long pairs in bulk: one pair per thread, a band of 32 * NW diagonals.
+ *
+ * wide_kernel<2, true>, the scan, takes tier 5's list.  Its 64 diagonals
+ * follow the path (they move by 16 when the column's smallest value nears an
+ * edge), so its distance is an upper bound: it routes the pair to the class
+ * whose limit covers it.  A pair at distance 63 or less whose band never had
+ * to move is aligned on the spot, if half of its warp's pairs are.
+ * wide_kernel<NW, false> aligns a class: the bound puts the distance below
+ * 32 * NW, so a fixed band that holds both ends' diagonals is exact.
+ *
+ * Bound by the integer pipe: 13 instructions per word and column and 5 per
+ * column, then one pass over 64 diagonals for the walk back.  The wavefront
+ * kernels (bound_kernel, long_kernel) spend 72 warp instructions on 32 cells
+ * of one pair and 56 more per warp and score, on D^2 / 2 cells; here it is
+ * 32 * NW cells a base, for 32 pairs at once and without divergence, but a
+ * launch lasts a sequence's length of dependent columns, however few its
+ * pairs, and longer the wider its band: a class of fewer than kWidePairs
+ * pairs goes to tile_kernel.  200k pairs of 1,000 bases at 10% edits, in
+ * batches of 20,000: 15.3 ms from tier 0 up, 8.1 ms from the bound pass and
+ * its classes, 2.1 ms so.
+ *
+ * Scratch of a warp (slab; rows of 32 words, a lane's column each): the bit
+ * planes of both sequences, VP/VN before every block of 32 columns, and the
+ * CIGAR bytes (a lane's words together, written backwards).  The walk goes
+ * back block by block: the block's columns are computed again from the
+ * checkpoint, but only 64 diagonals around the path, 32 of them are kept
+ * (transposed in shared memory), and when the walk nears their edge the block
+ * is computed again around where it is.  The 64 diagonals are enough when no
+ * optimal path to the cell where the walk enters can leave them: a path that
+ * touches an edge diagonal e costs at least V(c0, e) + |e - q|, with V the
+ * matrix at the block's first column c0 and q the cell's diagonal (V changes
+ * by at most 1 per row, and a diagonal is left at a cost of 1), and the cell
+ * itself costs at most V(c0, q) + its increments in the block.  Where that
+ * test fails (an indel of dozens of bases inside a block), the pair goes to
+ * the wavefront kernels. */
+struct WideSlab {
+    uint32_t p, t, ckpt, bytes; /* first words */
+    uint32_t np, nt;            /* plane words per sequence */
+    uint32_t bw;                /* words of a lane's CIGAR */
+    uint32_t words;             /* of the whole slab */
+};
+
+template <int NW>
+__host__ __device__ __forceinline__ WideSlab wide_slab(uint32_t max_len)
+{
+    WideSlab s{};
+    s.np = s.nt = (max_len + 31u) / 32u;
+    s.p = 0u;
+    s.t = s.p + 64u * s.np;
+    s.ckpt = s.t + 64u * s.nt;
+    s.bytes = s.ckpt + 64u * (uint32_t)NW * s.nt;
+    /* at most 32 * NW operations, a run before and after each, a byte per 127 matches */
+    s.bw = (64u * (uint32_t)NW + 1u + max_len / 127u + 3u) / 4u;
+    s.words = (s.bytes + 32u * s.bw + 63u) & ~63u;
+    return s;
+}
+
+/* Words [w, end) of a sequence's bit planes, 32 bases each, into rows of the
+ * slab (`row` words; the second plane's row after the first's); four words'
+ * blocks are loaded at once. */
+__device__ __forceinline__ void wide_pack(const char* seq, uint32_t len, uint32_t* out, int row, int w, int end)
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(seq);
+    const uint32_t sh = (uint32_t)(a & 15u);
+    const uint4* base = reinterpret_cast<const uint4*>(a - sh);
+    const int nblk = len ? (int)((sh + len + 15u) >> 4) : 0;
+    uint32_t x0 = w < end ? planes16(__ldg(base + 2 * w)) : 0u;
+    for (; w < end; w += 4) {
+        uint4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[i] = 2 * w + 1 + i < nblk ? __ldg(base + 2 * w + 1 + i) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (w + i >= end) break;
+            const uint32_t x1 = planes16(v[2 * i]), x2 = planes16(v[2 * i + 1]);
+            uint32_t lo, hi;
+            planes32(x0, x1, x2, sh, lo, hi);
+            out[(size_t)(2 * row) * (w + i)] = lo;
+            out[(size_t)(2 * row) * (w + i) + row] = hi;
+            x0 = x2;
+        }
+    }
+}
+
+/* sum of the vertical differences of bits [0, n) of NW words */
+template <int NW>
+__device__ __forceinline__ int column_sum(const uint32_t (&vp)[NW], const uint32_t (&vn)[NW], int n)
+{
+    int s = 0;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+        const uint32_t m = low_bits(min(32, max(0, n - 32 * i)));
+        s += __popc(vp[i] & m) - __popc(vn[i] & m);
+    }
+    return s;
+}
+
+/* The walk back of a pair, by one thread. */
+struct Walk {
+    int m, hb; /* block of 32 columns, and columns into it */
+    int q, b;  /* band bit, and the band's highest diagonal (bit 0) */
+    int W;     /* bits of the band, at least 64 */
+    int s;     /* score left; before the first block: the value on bit q at that block's first column when !known */
+    bool known;
+    int limit; /* !known: a distance past it stops the walk */
+    int run, D;
+    BackBytes cg;
+};
+
+/* The window of a walk: 64 diagonals from band bit e are computed, the 32
+ * from bit e + f kept. */
+struct WalkWindow {
+    int e, f;
+};
+__device__ __forceinline__ WalkWindow walk_window(int q, int W)
+{
+    WalkWindow w;
+    w.e = min(max(q - 32, 0), W - 64);
+    w.f = min(max(q - w.e - 16, 0), 32);
+    return w;
+}
+
+/* Rows of a block in a thread's column of shared memory: D0 of the window's
+ * 32 bits, transposed, and the vertical differences of its 64 before the
+ * block. */
+constexpr int kWalkRows = 36;
+
+/* Fill the rows of block m.  P, T: the thread's columns of the bit planes
+ * (rows of `row` words), np words of the pattern's; src(m, t, vp, vn) gives
+ * the vertical differences before block m of the band's bits 32t .. 32t+31. */
+template <class Src>
+__device__ __forceinline__ void walk_fill(uint32_t* rows, int m, int b, WalkWindow w, const uint32_t* P,
+                                          const uint32_t* T, int row, int np, const Src& src)
+{
+    const uint32_t es = (uint32_t)(w.e & 31);
+    uint32_t xp[2], xn[2];
+    {
+        uint32_t p0, n0, p1, n1, p2 = 0u, n2 = 0u;
+        src(m, w.e >> 5, p0, n0);
+        src(m, (w.e >> 5) + 1, p1, n1);
+        if (es) src(m, (w.e >> 5) + 2, p2, n2);
+        xp[0] = __funnelshift_r(p0, p1, es);
+        xp[1] = __funnelshift_r(p1, p2, es);
+        xn[0] = __funnelshift_r(n0, n1, es);
+        xn[1] = __funnelshift_r(n1, n2, es);
+    }
+    rows[32 * 32] = xp[0];
+    rows[32 * 33] = xp[1];
+    rows[32 * 34] = xn[0];
+    rows[32 * 35] = xn[1];
+    uint32_t a0[3], a1[3];
+    plane_window<3>(P, 2 * row, np, 32 * m - b + w.e, a0);
+    plane_window<3>(P + row, 2 * row, np, 32 * m - b + w.e, a1);
+    const uint32_t t0 = T[(size_t)(2 * row) * m], t1 = T[(size_t)(2 * row) * m + row];
+    uint32_t keep[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        uint32_t d0[2];
+        wide_column<2>(a0, a1, t0, t1, j, xp, xn, d0);
+        keep[j] = __funnelshift_rc(d0[0], d0[1], (uint32_t)w.f);
+    }
+    transpose32(keep);
+#pragma unroll
+    for (int r = 0; r < 32; ++r) rows[32 * r] = keep[r];
+}
+
+/* Walk through block k.m, whose rows are filled with window w, to the block
+ * before it or to the window's edge.  Returns ST_RUN while there is more to
+ * walk, ST_DONE at the origin, ST_OVERMAX past the limit, ST_OVERFLOW when
+ * the window's 64 diagonals do not hold every optimal path. */
+__device__ __forceinline__ int walk_block(Walk& k, const uint32_t* rows, WalkWindow w)
+{
+    const uint32_t xp[2] = {rows[32 * 32], rows[32 * 33]}, xn[2] = {rows[32 * 34], rows[32 * 35]};
+    const int ql = k.q - w.e;
+    int c = ql - w.f; /* the path's row of the 32 */
+    const int ex = __popc(~rows[32 * c] & low_bits(k.hb));
+    if (w.e > 0 || w.e < k.W - 64) {
+        const int su = column_sum<2>(xp, xn, ql);      /* V(q) - V(first) at column c0 */
+        const int sd = column_sum<2>(xp, xn, 63) - su; /* V(last) - V(q) */
+        if ((w.e > 0 && ql - su <= ex) || (w.e < k.W - 64 && 63 - ql + sd <= ex)) return ST_OVERFLOW;
+    }
+    if (!k.known) {
+        k.known = true;
+        k.D = k.s += ex;
+        if (k.s > k.limit) return ST_OVERMAX;
+    }
+    const uint32_t kp = __funnelshift_rc(xp[0], xp[1], (uint32_t)w.f);
+    const uint32_t kn = __funnelshift_rc(xn[0], xn[1], (uint32_t)w.f);
+    /* rows to walk on: the band's own edges may be reached, the others not left */
+    const int lo = w.e + w.f > 0 ? 1 : 0, hi = w.e + w.f + 32 < k.W ? 30 : 31;
+    int state = ST_RUN;
+    bool here = true;
+    do {
+        const int best = walk_step(~rows[32 * c], ~rows[32 * max(c - 1, 0)], ~rows[32 * min(c + 1, 31)], kp, kn, c, 31,
+                                   k.hb);
+        if (best >= 0) {
+            const int op = best & 3, x = best >> 2;
+            k.cg.push_run(k.run + k.hb - x, 1);
+            k.cg.push((uint32_t)op_letter(op), 1);
+            k.run = 0;
+            k.hb = op == kOpDel ? x : x - 1;
+            c += op == kOpDel ? -1 : (op == kOpIns ? 1 : 0);
+            if (--k.s < 0) state = ST_DONE; /* never expected */
+        } else {
+            k.run += k.hb;
+            k.hb = 0;
+            if (k.m == 0) state = ST_DONE;
+        }
+        if (k.hb == 0 && k.m > 0) {
+            --k.m;
+            k.hb = 32;
+            here = false;
+        }
+    } while (state == ST_RUN && here && c >= lo && c <= hi);
+    k.q = w.e + w.f + c;
+    return state;
+}
+
+/* The end of a walk: at the origin with no score left, or not (never expected). */
+__device__ __forceinline__ int walk_end(Walk& k)
+{
+    if (k.s != 0 || k.q != k.b) return ST_BADWALK;
+    k.cg.push_run(k.run, 1);
+    k.cg.finish(1);
+    return ST_DONE;
+}
+
+/* CIGARs and results of up to 32 pairs that one warp walked, bytes at
+ * `bytes`, bw words a pair: eight lanes write a pair's words, four pairs at a
+ * time. */
+__device__ __forceinline__ void store_walked(const AlignLaunch& A, const uint32_t* bytes, int bw, int state, uint32_t pi,
+                                             int D, int n, int lane)
+{
+    const uint32_t cap = A.cigar_stride;
+    if (cap) {
+        const bool aligned = (cap & 3u) == 0u && (reinterpret_cast<uintptr_t>(A.cigar) & 3u) == 0u;
+#pragma unroll 1
+        for (int r = 0; r < 8; ++r) {
+            const int own = 4 * r + (lane >> 3), g = lane & 7;
+            const bool done = __shfl_sync(kFull, state, own) == ST_DONE;
+            const uint32_t len = (uint32_t)__shfl_sync(kFull, n, own);
+            int8_t* dst = A.cigar + (size_t)__shfl_sync(kFull, pi, own) * cap;
+            if (done) store_back_bytes(bytes + (size_t)own * bw, 1, bw, len, cap, dst, g, 8, aligned);
+        }
+    }
+    if (state == ST_DONE) {
+        A.dist[pi] = D;
+        if (A.status) A.status[pi] = (uint32_t)n > cap ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED : (uint8_t)WFE_PAIR_OK;
+    } else if (state != ST_IDLE && state != ST_RUN) {
+        finish_unaligned(A, pi, state);
+    }
+}
+
+/* Routes a scanned pair by the bound on its distance, as the bound pass does. */
+__device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi, int bound, int need);
+
+template <int NW, bool SCAN>
+__device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks)
+{
+    static_assert(!SCAN || NW == 2, "the scan moves a band of two words");
+    constexpr int W = 32 * NW;
+    constexpr int kUnroll = NW <= 4 ? 4 : (NW <= 8 ? 2 : 1);
+    const int lane = (int)(threadIdx.x & 31u);
+    const TierShape& sh = SCAN ? A.chain.cls.scan : A.chain.cls.wide[A.cls];
+    const WideSlab S = wide_slab<NW>(A.max_len);
+    uint32_t* const slab = reinterpret_cast<uint32_t*>(sh.scratch + (size_t)blockIdx.x * sh.slab);
+    uint32_t* const P = slab + S.p + lane;
+    uint32_t* const T = slab + S.t + lane;
+    uint32_t* const ckpt = slab + S.ckpt + lane;
+    /* a class list: its front part, then its back part from the end */
+    const uint32_t front = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+    const uint32_t count = SCAN ? front : min(front + A.chain.cls.low_counts[A.cls], A.n_work);
+    uint32_t* const work_next = SCAN ? A.chain.work_next + A.tier : A.chain.cls.work_next + A.cls;
+    for (;;) {
+        uint32_t wb = 0;
+        if (lane == 0) wb = atomicAdd(work_next, 32u);
+        wb = __shfl_sync(kFull, wb, 0);
+        if (wb >= count) break;
+        const uint32_t item = wb + (uint32_t)lane;
+        int state = ST_IDLE;
+        uint32_t pi = 0;
+        PairRef pr;
+        pr.p = nullptr; pr.t = nullptr; pr.plen = 0; pr.tlen = 0;
+        if (item < count) {
+            pi = !A.work ? item : item < front ? A.work[item] : A.work[A.chain.cls.cap - 1u - (item - front)];
+            pr = get_pair(A.L, pi);
+            state = !pr.in_range ? ST_RANGE : max(pr.plen, pr.tlen) > A.max_len ? ST_TOOLONG : ST_RUN;
+        }
+        /* a class of the caller's cap may get pairs past its band */
+        const int past = A.max_distance > 0 && A.max_distance <= W - 1 ? ST_OVERMAX : ST_OVERFLOW;
+        if (!SCAN && state == ST_RUN && abs((int)pr.tlen - (int)pr.plen) > W - 1) state = past;
+        const int plen = state == ST_RUN ? (int)pr.plen : 0, tlen = state == ST_RUN ? (int)pr.tlen : 0;
+        const int np = (plen + 31) >> 5;
+        const int kt = tlen - plen, wide = abs(kt);
+        wide_pack(pr.p, (uint32_t)plen, P, 32, 0, np);
+        wide_pack(pr.t, (uint32_t)tlen, T, 32, 0, (tlen + 31) >> 5);
+        /* diagonals b-W+1..b: 0 and kt, with as many on either side; a scan
+         * whose ends lie too far apart starts around 0 */
+        bool fixed = !SCAN || wide < W;
+        int b = fixed ? (W - 1) + min(0, kt) - (W - 1 - wide) / 2 : W / 2;
+        int top = b; /* the value on bit 0 */
+        uint32_t vp[NW], vn[NW];
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            vn[i] = low_bits(min(32, max(0, b - 32 * i)));
+            vp[i] = ~vn[i];
+        }
+        for (int m = 0; 32 * m < tlen; ++m) {
+            if constexpr (SCAN) {
+                if (m > 0) {
+                    const int up = __popc(vp[0]) - __popc(vn[0]), down = __popc(vp[1]) - __popc(vn[1]);
+                    /* V(32) > V(0): the path runs above; V(64) < V(32): below */
+                    if (up > 0 || down < 0) {
+                        const int move = up > -down ? -16 : 16;
+                        top += move_band(vp, vn, move);
+                        b -= move;
+                        fixed = false;
+                    }
+                }
+            }
+            uint32_t* ck = ckpt + (size_t)(64 * NW) * m;
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                ck[64 * i] = vp[i];
+                ck[64 * i + 32] = vn[i];
+            }
+            uint32_t a0[NW + 1], a1[NW + 1];
+            plane_window<NW + 1>(P, 64, np, 32 * m - b, a0);
+            plane_window<NW + 1>(P + 32, 64, np, 32 * m - b, a1);
+            const uint32_t t0 = T[64 * m], t1 = T[64 * m + 32];
+            const int n = min(32, tlen - 32 * m);
+            uint32_t on = 0; /* bit 0 of D0, column after column */
+#pragma unroll kUnroll
+            for (int j = 0; j < n; ++j) {
+                uint32_t d0[NW];
+                wide_column<NW>(a0, a1, t0, t1, j, vp, vn, d0);
+                on = __funnelshift_r(on, d0[0], 1u);
+            }
+            top += n - __popc(on);
+        }
+        const int it = b - kt; /* the target's band bit */
+        int D = top + column_sum<NW>(vp, vn, min(max(it, 0), W - 1));
+        if (SCAN) D += it < 0 ? -it : max(0, it - (W - 1)); /* a row away changes the value by at most 1 */
+
+        if (state == ST_RUN) {
+            if (D <= W - 1 && fixed)
+                state = A.max_distance > 0 && D > A.max_distance ? ST_OVERMAX : ST_DONE;
+            else if (!SCAN)
+                state = past;
+        }
+        if constexpr (SCAN) {
+            /* a walk costs the whole warp: with few pairs to align here, a class takes them */
+            const unsigned done = __ballot_sync(kFull, state == ST_DONE), running = __ballot_sync(kFull, state == ST_RUN);
+            if (state == ST_DONE && 2 * __popc(done) < __popc(done | running)) state = ST_RUN;
+            if (state == ST_RUN) {
+                A.bound[pi] = D;
+                route_by_bound(A, pi, D, A.max_distance > 0 ? min(D, A.max_distance) : D);
+            }
+        }
+
+        Walk k{};
+        k.m = tlen > 0 ? (tlen - 1) >> 5 : 0;
+        k.hb = tlen - 32 * k.m;
+        k.q = it;
+        k.b = b;
+        k.W = W;
+        k.s = k.D = D;
+        k.known = true;
+        k.cg = BackBytes{slab + S.bytes + (size_t)lane * S.bw, 0u, 0, (int)S.bw};
+        bool walking = state == ST_DONE;
+        if (walking && tlen == 0) { /* only deletions */
+            for (; k.s > 0; --k.s) k.cg.push((uint32_t)'D', 1);
+            k.q = b;
+            walking = false;
+        }
+        const int most = __reduce_max_sync(kFull, walking ? k.m + 1 : 0);
+        for (int blk = most - 1; blk >= 0; --blk) {
+            while (walking && k.m == blk) {
+                const WalkWindow w = walk_window(k.q, W);
+                walk_fill(blocks + lane, blk, b, w, P, T, 32, np, [&](int m, int t, uint32_t& p, uint32_t& v) {
+                    const uint32_t* c = ckpt + (size_t)(64 * NW) * m + 64 * t;
+                    p = c[0];
+                    v = c[32];
+                });
+                const int st = walk_block(k, blocks + lane, w);
+                walking = st == ST_RUN;
+                if (!walking) state = st;
+            }
+        }
+        if (state == ST_DONE) state = walk_end(k);
+        __syncwarp();
+        store_walked(A, slab + S.bytes, (int)S.bw, state, pi, D, k.cg.n, lane);
+        __syncwarp();
+    }
+    chain_next(A);
+}
+
+/* Launched from the device too, so a register limit and no launch bounds (see
+ * tier_kernel). */
+template <int NW, bool SCAN>
+__global__ void __maxnreg__(NW <= 8 ? 128 : (NW <= 16 ? 168 : 255)) wide_kernel(const __grid_constant__ AlignLaunch A)
+{
+    __shared__ uint32_t blocks[32 * kWalkRows];
+    if constexpr (SCAN) {
+        const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+        if (count < A.min_count) return; /* the bound pass takes the list */
+    }
+    wide_body<NW, SCAN>(A, blocks);
+}
+
+/* ------------------------------------------------------------------------ */
+/* Long pairs by several lanes: G lanes per pair, tiles of 32 x 32 cells.
+ *
+ * Row block bi (32 pattern rows) crosses the column blocks bj = bi + delta of
+ * the band, delta in [dlo, dhi], one per step: tile (bi, bj) is computed at
+ * step bi + bj by lane bi mod G, from the vertical differences that the lane
+ * kept from its previous tile and the horizontal differences that the lane
+ * above handed down a step before, two shuffles for 32 columns of about 21
+ * instructions.  A band of nd tile diagonals has at most (nd + 1) / 2 tiles
+ * per step, so nd <= 2 G.  Differences that come from outside the band count
+ * as +1, an upper bound.  The tile diagonals hold every diagonal of
+ * [32 dlo, 32 dhi]; dlo and dhi are the least that certify the pair's bound.
+ * The vertical differences into each tile are kept for the walk back, which a
+ * warp does for all pairs of the CTA, one per thread (see walk_back).
+ *
+ * A CTA of eight warps takes chunks of up to 32 pairs of a class, the widest
+ * class first and each class from the end of its list (the scan's longest
+ * pairs come last), all classes in one launch: launched one after another,
+ * each class left most of the GPU idle for the length of its longest pair.
+ * A pair takes L / 16 steps whatever its band, so the kernel needs tens of
+ * times fewer pairs than one thread per pair to fill the GPU, for 1.5 to 2
+ * times its instructions.  8,000 pairs of 5,000-7,000 bases at 6-10% edits:
+ * 4.8 ms with a CTA per pair, 2.6 ms so (three callers at once: 3.9 and 1.7 ms
+ * a call); 50,000 pairs of 100-10,000 bases at 1-15%: 13.1 and 6.1 ms (9.4
+ * and 4.4). */
+constexpr int kTileWarps = 8;
+constexpr int kTileThreads = 32 * kTileWarps;
+/* lanes per pair for distances up to dlim: nd <= 2 G for any ends */
+__host__ __device__ constexpr int tile_lanes(int dlim) { return (dlim + 126) / 64 < 2 ? 2 : (dlim + 126) / 64; }
+__host__ __device__ constexpr int tile_groups(int G) { return 32 / G; } /* pairs per warp */
+/* pairs of a CTA: one warp walks them back */
+__host__ __device__ constexpr int tile_pairs(int G)
+{
+    return tile_groups(G) * kTileWarps < 32 ? tile_groups(G) * kTileWarps : 32;
+}
+
+struct TileSlab {
+    uint32_t t, ckpt, start, bytes; /* first words (the pattern's planes at 0) */
+    uint32_t nd, bw;                /* tiles kept per column block; words of a pair's CIGAR */
+    uint64_t words;
+};
+
+__host__ __device__ __forceinline__ TileSlab tile_slab(uint32_t max_len, int dlim)
+{
+    TileSlab s{};
+    const uint32_t G = (uint32_t)tile_lanes(dlim), n = (uint32_t)tile_pairs((int)G), nw = (max_len + 31u) / 32u;
+    s.nd = 2u * G;
+    s.t = 2u * n * nw;
+    s.ckpt = (2u * s.t + 1u) & ~1u;
+    s.start = s.ckpt + 2u * n * nw * s.nd;
+    s.bytes = s.start + n;
+    s.bw = (2u * (uint32_t)dlim + 1u + max_len / 127u + 3u) / 4u;
+    s.words = ((uint64_t)s.bytes + (uint64_t)n * s.bw + 63u) & ~uint64_t(63);
+    return s;
+}
+
+/* CTA loads of the classes that the tile kernel takes */
+__device__ uint32_t tile_chunks(const LongClasses& C)
+{
+    uint32_t n = 0;
+    for (int c = 0; c + 1 < C.n; ++c) {
+        const uint32_t count = *reinterpret_cast<volatile const uint32_t*>(C.counts + c);
+        const uint32_t np = (uint32_t)tile_pairs(tile_lanes(C.shape[c].dlim));
+        if (tile_takes(C, c, count)) n += (count + np - 1u) / np;
+    }
+    return n;
+}
+
+__global__ void __maxnreg__(128) tile_kernel(const __grid_constant__ AlignLaunch A)
+{
+    __shared__ uint32_t blocks[kTileWarps * 32 * kWalkRows];
+    __shared__ uint32_t s_item;
+    __shared__ uint32_t s_pi[32];
+    __shared__ int s_plen[32], s_tlen[32], s_dlo[32], s_dhi[32], s_state[32], s_m[32], s_q[32];
+    __shared__ const char* s_seq[64];
+    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+    const LongClasses& C = A.chain.cls;
+    uint32_t* const slab = reinterpret_cast<uint32_t*>(C.tile.scratch + (size_t)blockIdx.x * C.tile.slab);
+    for (;;) {
+        if (threadIdx.x == 0) s_item = atomicAdd(C.work_next + kTileClass, 1u);
+        __syncthreads();
+        /* chunk s_item, counted from the widest class and from the end of its list */
+        uint32_t chunk = s_item, count = 0;
+        int cls = C.n - 2, npair = 1;
+        for (; cls >= 0; --cls) {
+            count = C.counts[cls];
+            if (!tile_takes(C, cls, count)) continue;
+            npair = tile_pairs(tile_lanes(C.shape[cls].dlim));
+            const uint32_t chunks = (count + (uint32_t)npair - 1u) / (uint32_t)npair;
+            if (chunk < chunks) break;
+            chunk -= chunks;
+        }
+        if (cls < 0) break;
+        const uint32_t first = chunk * (uint32_t)npair;
+        const int limit = C.shape[cls].dlim, G = tile_lanes(limit);
+        const TileSlab S = tile_slab(A.max_len, limit);
+        uint2* const ckpt = reinterpret_cast<uint2*>(slab + S.ckpt);
+        const int past = A.max_distance > 0 && A.max_distance <= limit ? ST_OVERMAX : ST_OVERFLOW;
+        if (warp == 0) {
+            int state = ST_IDLE, plen = 0, tlen = 0, dlo = 0, dhi = 0;
+            const uint32_t item = first + (uint32_t)lane;
+            if (lane < npair && item < count) {
+                const uint32_t pi = C.list[cls][count - 1u - item];
+                const PairRef pr = get_pair(A.L, pi);
+                s_pi[lane] = pi;
+                s_seq[2 * lane] = pr.p;
+                s_seq[2 * lane + 1] = pr.t;
+                state = !pr.in_range ? ST_RANGE : max(pr.plen, pr.tlen) > A.max_len ? ST_TOOLONG : ST_RUN;
+                if (state == ST_RUN) {
+                    const int kt = (int)pr.tlen - (int)pr.plen, wide = abs(kt), bound = A.bound[pi];
+                    const int dub = bound >= 0 ? min(bound, limit) : limit;
+                    if (wide > dub) {
+                        state = past;
+                    } else {
+                        plen = (int)pr.plen;
+                        tlen = (int)pr.tlen;
+                        const int x = (dub - wide) >> 1;
+                        dlo = (min(0, kt) - x) >> 5;
+                        dhi = (max(0, kt) + x + 31) >> 5;
+                        if (dhi - dlo < 2) { /* the walk wants 64 diagonals */
+                            --dlo;
+                            if (dhi - dlo < 2) ++dhi;
+                        }
+                    }
+                }
+            }
+            s_state[lane] = state;
+            s_plen[lane] = plen;
+            s_tlen[lane] = tlen;
+            s_dlo[lane] = dlo;
+            s_dhi[lane] = dhi;
+        }
+        __syncthreads();
+        /* bit planes: every thread a part of a sequence */
+        {
+            const int parts = kTileThreads / (2 * npair);
+            const int seq = (int)threadIdx.x % (2 * npair), part = (int)threadIdx.x / (2 * npair);
+            const int own = seq >> 1;
+            if (part < parts) {
+                const int len = (seq & 1) ? s_tlen[own] : s_plen[own];
+                const int n = (len + 31) >> 5, each = (n + parts - 1) / parts, w0 = part * each;
+                wide_pack(s_seq[seq], (uint32_t)len, slab + ((seq & 1) ? S.t : 0u) + own, npair, w0, min(n, w0 + each));
+            }
+        }
+        __syncthreads();
+        /* forward */
+        {
+            const int groups = tile_groups(G), grp = lane / G, l = lane - grp * G;
+            const int own = warp * groups + grp;
+            const bool in = grp < groups && own < npair && s_state[own & 31] == ST_RUN;
+            const int plen = in ? s_plen[own] : 0, tlen = in ? s_tlen[own] : 0;
+            const int dlo = in ? s_dlo[own] : 0, dhi = in ? s_dhi[own] : 0;
+            const int Bp = (plen + 31) >> 5, Bt = (tlen + 31) >> 5;
+            const int src = grp * G + (l == 0 ? G - 1 : l - 1);
+            /* where the walk starts: the target's diagonal at the last block's first column */
+            const int v0 = 32 * (Bt - 1) - (tlen - plen);
+            const uint32_t* const P = slab + own;
+            const uint32_t* const T = slab + S.t + own;
+            const int steps = __reduce_max_sync(kFull, Bp > 0 && Bt > 0 ? Bp + Bt - 1 : 0);
+            int bi = l, corner = 0;
+            uint32_t vp = 0, vn = 0, p0 = 0, p1 = 0, hp = 0, hn = 0;
+            int low = 0; /* the value below the tile's left edge */
+            for (int s = 0; s < steps; ++s) {
+                const uint32_t up_p = __shfl_sync(kFull, hp, src), up_n = __shfl_sync(kFull, hn, src);
+                const int up_low = __shfl_sync(kFull, low, src);
+                while (bi < Bp && s - bi > bi + dhi) bi += G; /* the row block has left the band */
+                const int bj = s - bi, lead = max(0, bi + dlo);
+                if (bi >= Bp || bj < lead || bj >= Bt) continue;
+                if (bj == lead) {
+                    vp = ~0u;
+                    vn = 0u;
+                    p0 = P[(size_t)(2 * npair) * bi];
+                    p1 = P[(size_t)(2 * npair) * bi + npair];
+                    corner = bj == 0 ? 32 * bi : up_low;
+                }
+                const bool edge = bi == 0 || bj - bi == dhi;
+                const uint32_t in_p = edge ? ~0u : up_p, in_n = edge ? 0u : up_n;
+                ckpt[((size_t)bj * S.nd + (size_t)(bi - bj + dhi)) * npair + own] = make_uint2(vp, vn);
+                if (bj == Bt - 1 && v0 >= 0 && bi == v0 >> 5) {
+                    const uint32_t mask = low_bits(v0 & 31);
+                    slab[S.start + own] = (uint32_t)(corner + __popc(vp & mask) - __popc(vn & mask));
+                }
+                const uint32_t t0 = T[(size_t)(2 * npair) * bj], t1 = T[(size_t)(2 * npair) * bj + npair];
+                low = corner + __popc(vp) - __popc(vn);
+                corner += __popc(in_p) - __popc(in_n);
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    tile_column(p0, p1, bit_mask(t0, j), bit_mask(t1, j), in_p << j, in_n << j, vp, vn, hp, hn);
+            }
+        }
+        __syncthreads();
+        /* The walk back, a pair per lane of the first warp.  The warps fill the
+         * rows of as many blocks at a time, all with the window around where
+         * the walk is: it seldom moves by 15 diagonals in 256 columns. */
+        Walk k{};
+        int state = ST_IDLE;
+        bool walking = false;
+        const int dhi = s_dhi[lane], Bp = (s_plen[lane] + 31) >> 5, nd = dhi - s_dlo[lane] + 1;
+        const int own = lane < npair ? lane : 0;
+        k.b = 32 * dhi;
+        k.W = 32 * (nd - 1) + 1;
+        if (warp == 0) {
+            state = s_state[lane];
+            const int plen = s_plen[lane], tlen = s_tlen[lane], kt = tlen - plen;
+            k.m = tlen > 0 ? (tlen - 1) >> 5 : 0;
+            k.hb = tlen - 32 * k.m;
+            k.q = k.b - kt;
+            k.limit = limit;
+            k.cg = BackBytes{slab + S.bytes + (size_t)own * S.bw, 0u, 0, (int)S.bw};
+            walking = state == ST_RUN;
+            if (walking && (plen == 0 || tlen == 0)) { /* one operation throughout */
+                for (k.s = plen + tlen; k.s > 0; --k.s) k.cg.push(plen ? (uint32_t)'D' : (uint32_t)'I', 1);
+                k.D = plen + tlen;
+                k.q = k.b;
+                state = ST_DONE;
+                walking = false;
+            } else if (walking) {
+                const int v0 = 32 * k.m - kt; /* a virtual row's value is its diagonal */
+                k.s = v0 >= 0 ? (int)slab[S.start + own] : kt;
+            }
+        }
+        for (;;) {
+            if (warp == 0) {
+                s_m[lane] = walking ? k.m : -1;
+                s_q[lane] = k.q;
+            }
+            if (!__syncthreads_or(walking)) break;
+            const int m0 = s_m[lane], m = m0 - warp;
+            const WalkWindow w = walk_window(s_q[lane], k.W);
+            if (m >= 0)
+                walk_fill(blocks + warp * (32 * kWalkRows) + lane, m, k.b, w, slab + own, slab + S.t + own, npair, Bp,
+                          [&](int mm, int t, uint32_t& p, uint32_t& v) {
+                              const int bi = t + mm - dhi;
+                              uint2 c = bi < 0 ? make_uint2(0u, ~0u) : make_uint2(~0u, 0u);
+                              if (bi >= 0 && bi < Bp && t < nd) c = ckpt[((size_t)mm * S.nd + (size_t)t) * npair + own];
+                              p = c.x;
+                              v = c.y;
+                          });
+            __syncthreads();
+            if (warp == 0) {
+                const int lo = w.e + w.f > 0 ? 1 : 0, hi = w.e + w.f + 32 < k.W ? 30 : 31;
+                int c = k.q - w.e - w.f;
+                while (walking && m0 - k.m < kTileWarps && c >= lo && c <= hi) {
+                    const int st = walk_block(k, blocks + (m0 - k.m) * (32 * kWalkRows) + lane, w);
+                    c = k.q - w.e - w.f;
+                    walking = st == ST_RUN;
+                    if (!walking) state = st;
+                }
+            }
+        }
+        if (warp == 0) {
+            if (state == ST_DONE) state = walk_end(k);
+            if (state == ST_OVERMAX) state = past;
+            if (state == ST_DONE && A.max_distance > 0 && k.D > A.max_distance) state = ST_OVERMAX;
+            __syncwarp();
+            store_walked(A, slab + S.bytes, (int)S.bw, state, lane < npair ? s_pi[lane] : 0u, k.D, k.cg.n, lane);
+        }
+        __syncthreads();
+    }
+    chain_next(A);
+}
+
+/* ------------------------------------------------------------------------ */
 /* Distance bounds for the CTA-per-pair tiers, one warp per pair.  The warp
  * runs the recurrence of the tiers restricted to a band of 32 diagonals
  * (lane l: diagonal b + l) that follows the cell furthest along its
@@ -1204,6 +1951,27 @@ __device__ __forceinline__ int extend_words(const uint32_t* P, const uint32_t* T
  * and at least one zero word after them, rounded to 16 bytes */
 __host__ __device__ __forceinline__ uint32_t bound_words(uint32_t seq_words) { return (seq_words + 4u) & ~3u; }
 
+__device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi, int bound, int need)
+{
+    const LongClasses& C = A.chain.cls;
+    const int top = C.shape[C.n - 1].dlim;
+    if (bound > top && need > top && A.retry) {
+        /* past tier 5 (with no cap below its limit): straight on */
+        A.retry[atomicAdd(A.retry_count, 1u)] = pi;
+        if (A.passed_total) atomicAdd(A.passed_total, 1ull);
+        return;
+    }
+    int c = 0, below = 0;
+    while (c + 1 < C.n && (C.shape[c].dlim < need || (!A.bulk && !class_by_cta(C.shape[c].dlim)))) {
+        if (class_by_cta(C.shape[c].dlim)) below = C.shape[c].dlim;
+        ++c;
+    }
+    if (A.bulk || 2 * need >= below + C.shape[c].dlim)
+        C.list[c][atomicAdd(C.counts + c, 1u)] = pi;
+    else
+        C.list[c][C.cap - 1u - atomicAdd(C.low_counts + c, 1u)] = pi;
+}
+
 __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_words)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1216,6 +1984,7 @@ __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_wo
     uint32_t* WP = reinterpret_cast<uint32_t*>(smem) + (size_t)warp * 2u * bw;
     uint32_t* WT = WP + bw;
     const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+    if (A.max_count && count >= A.max_count) return; /* the scan has taken the list */
     for (uint32_t item = blockIdx.x * kW + (uint32_t)warp; item < count; item += gridDim.x * kW) {
         const uint32_t pi = A.work ? A.work[item] : item;
         const PairRef pr = get_pair(A.L, pi);
@@ -1273,21 +2042,7 @@ __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_wo
         if (lane == 0) {
             A.bound[pi] = bound;
             if (route) {
-                const LongClasses& C = A.chain.cls;
-                const int top = C.shape[C.n - 1].dlim;
-                if (bound > top && need > top && A.retry) {
-                    /* past tier 5 (with no cap below its limit): straight on */
-                    A.retry[atomicAdd(A.retry_count, 1u)] = pi;
-                    if (A.passed_total) atomicAdd(A.passed_total, 1ull);
-                } else {
-                    int c = 0;
-                    while (c + 1 < C.n && C.shape[c].dlim < need) ++c;
-                    const int below = c > 0 ? C.shape[c - 1].dlim : 0;
-                    if (2 * need >= below + C.shape[c].dlim)
-                        C.list[c][atomicAdd(C.counts + c, 1u)] = pi;
-                    else
-                        C.list[c][C.cap - 1u - atomicAdd(C.low_counts + c, 1u)] = pi;
-                }
+                route_by_bound(A, pi, bound, need);
             }
         }
         __syncwarp();
@@ -1307,6 +2062,65 @@ bound_kernel_host(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uin
 __global__ void bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t /* unused */)
 {
     bound_body(A, seq_words);
+}
+
+/* Tier 5's list in order of length, longest first (kOrderBins bins of equal
+ * width), for the scan and the classes that it fills: the pairs of a warp then
+ * end together, and the longest do not come last.  Two launches of a few
+ * microseconds: the bins' counts, then every pair to its place.  With fewer
+ * than A.min_count pairs both return at once. */
+__device__ __forceinline__ int order_bin(const AlignLaunch& A, uint32_t item, uint32_t& pi)
+{
+    pi = A.work ? A.work[item] : item;
+    const PairRef pr = get_pair(A.L, pi);
+    const uint32_t len = min(max(pr.plen, pr.tlen), A.max_len);
+    return kOrderBins - 1 - (int)((uint64_t)len * kOrderBins / ((uint64_t)A.max_len + 1u));
+}
+
+__global__ void __launch_bounds__(kOrderBins) order_count_kernel(const __grid_constant__ AlignLaunch A)
+{
+    __shared__ uint32_t bins[kOrderBins];
+    const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+    if (count < A.min_count) return;
+    bins[threadIdx.x] = 0u;
+    __syncthreads();
+    uint32_t pi;
+    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < count; i += gridDim.x * kOrderBins)
+        atomicAdd(&bins[order_bin(A, i, pi)], 1u);
+    __syncthreads();
+    if (bins[threadIdx.x]) atomicAdd(A.chain.cls.order_count + threadIdx.x, bins[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(kOrderBins) order_place_kernel(const __grid_constant__ AlignLaunch A)
+{
+    __shared__ uint32_t start[kOrderBins], mine[kOrderBins], sums[kOrderBins / 32];
+    const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+    if (count < A.min_count) return;
+    const int t = (int)threadIdx.x, lane = t & 31;
+    /* exclusive prefix of the bins */
+    const uint32_t c = A.chain.cls.order_count[t];
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sums[t >> 5] = x;
+    mine[t] = 0u;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < (t >> 5); ++w) before += sums[w];
+    const uint32_t first = before + x - c;
+    uint32_t pi;
+    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < count; i += gridDim.x * kOrderBins)
+        atomicAdd(&mine[order_bin(A, i, pi)], 1u);
+    __syncthreads();
+    start[t] = first + (mine[t] ? atomicAdd(A.chain.cls.order_next + t, mine[t]) : 0u);
+    __syncthreads();
+    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < count; i += gridDim.x * kOrderBins) {
+        const int b = order_bin(A, i, pi);
+        A.chain.cls.order[atomicAdd(&start[b], 1u)] = pi;
+    }
 }
 
 const TierInfo kTiers[kNumTiers] = {
@@ -1404,7 +2218,7 @@ __global__ void __launch_bounds__(256) classify_kernel(Layout L, uint32_t n, Buc
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t lim = (n + 31u) & ~31u; /* whole warps iterate together */
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < lim; i += stride) {
-        int key = -1;
+        int key = -1, bucket = -1;
         if (i < n) {
             const PairRef pr = get_pair(L, i);
             const uint32_t len = max(pr.plen, pr.tlen);
@@ -1424,7 +2238,8 @@ __global__ void __launch_bounds__(256) classify_kernel(Layout L, uint32_t n, Buc
                     while (t < top && (float)B.dcap[t] < est) ++t;
                 }
             }
-            key = b * kListsPerBucket + t;
+            key = (t == 5 && B.tier5_to >= 0 ? B.tier5_to : b) * kListsPerBucket + t;
+            bucket = b;
         }
         const unsigned same = __match_any_sync(kFull, key);
         const int leader = __ffs((int)same) - 1;
@@ -1432,7 +2247,11 @@ __global__ void __launch_bounds__(256) classify_kernel(Layout L, uint32_t n, Buc
         if (key >= 0 && lane == leader) {
             const int b = key / kListsPerBucket, t = key % kListsPerBucket;
             base = atomicAdd(B.counts + (size_t)b * B.count_stride + t, (uint32_t)__popc(same));
-            if (B.totals) atomicAdd(B.totals + b, (unsigned long long)__popc(same));
+        }
+        if (B.totals) {
+            const unsigned alike = __match_any_sync(kFull, bucket);
+            if (bucket >= 0 && lane == __ffs((int)alike) - 1)
+                atomicAdd(B.totals + bucket, (unsigned long long)__popc(alike));
         }
         base = __shfl_sync(kFull, base, leader);
         if (key >= 0) {
@@ -1704,20 +2523,71 @@ TierShape bound_shape(uint32_t max_len, int sm_count)
     return sh;
 }
 
-cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s)
+cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s, uint64_t* launches)
 {
     const TierShape& sh = a.chain.bound_shape;
     if (sh.grid <= 0 || !a.bound || sh.seq_words != seq_words_for(a.max_len)) return cudaErrorInvalidValue;
     cudaError_t e = allow_smem((const void*)bound_kernel_host, sh.smem);
     if (e != cudaSuccess) return e;
+    const TierShape& scan = a.chain.cls.scan;
+    if (a.tier == 5 && a.chain.cls.n > 0 && scan.grid > 0) {
+        AlignLaunch w = a;
+        w.bulk = 1;
+        w.min_count = kScanMin;
+        if (a.work_count || a.n_work >= kScanMin) {
+            const int og = (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 608u);
+            order_count_kernel<<<og, kOrderBins, 0, s>>>(w);
+            order_place_kernel<<<og, kOrderBins, 0, s>>>(w);
+            w.work = a.chain.cls.order;
+            *launches += 3;
+            wide_kernel<2, true><<<std::max(1, std::min(scan.grid, (int)((a.n_work + 31u) / 32u))), 32, 0, s>>>(w);
+            const cudaError_t e1 = cudaGetLastError();
+            if (e1 != cudaSuccess || !a.work_count) return e1;
+        }
+    }
     const uint32_t per_cta = (uint32_t)sh.threads / 32u;
     int grid = sh.grid;
     if (!a.work_count) grid = (int)std::min<uint64_t>((uint64_t)grid, ((uint64_t)a.n_work + per_cta - 1) / per_cta);
-    bound_kernel_host<<<std::max(grid, 1), sh.threads, sh.smem, s>>>(a, sh.seq_words, 0u);
+    ++*launches;
+    AlignLaunch w = a;
+    w.max_count = a.tier == 5 && a.chain.cls.n > 0 && scan.grid > 0 ? kScanMin : 0u;
+    bound_kernel_host<<<std::max(grid, 1), sh.threads, sh.smem, s>>>(w, sh.seq_words, 0u);
     return cudaGetLastError();
 }
 
 namespace {
+
+/* Launch shape of a wide kernel within the tier-5 scratch: as many warps as
+ * fit both (grid 0: too few to be worth it). */
+template <int NW, bool SCAN>
+TierShape wide_shape(uint32_t max_len, int sm_count, uint64_t scratch_bytes)
+{
+    TierShape sh{};
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wide_kernel<NW, SCAN>, 32, 0) != cudaSuccess) return sh;
+    sh.slab = 4u * (uint64_t)wide_slab<NW>(max_len).words;
+    const uint64_t grid = std::min<uint64_t>((uint64_t)std::max(nb, 0) * (uint64_t)sm_count, scratch_bytes / sh.slab);
+    if (grid < (uint64_t)sm_count / 2u) return TierShape{};
+    sh.grid = (int)grid;
+    sh.threads = 32;
+    sh.dlim = 32 * NW - 1;
+    return sh;
+}
+
+/* Launch shape of the tile kernel, its slabs sized for the widest of the first n classes. */
+TierShape tile_shape(uint32_t max_len, const int* dlim, int n, int sm_count, uint64_t scratch_bytes)
+{
+    TierShape sh{};
+    int nb = 0;
+    if (n < 1 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, tile_kernel, kTileThreads, 0) != cudaSuccess)
+        return sh;
+    for (int c = 0; c < n; ++c) sh.slab = std::max<uint64_t>(sh.slab, 4u * tile_slab(max_len, dlim[c]).words);
+    const uint64_t grid = std::min<uint64_t>((uint64_t)std::max(nb, 0) * (uint64_t)sm_count, scratch_bytes / sh.slab);
+    if (grid < (uint64_t)sm_count / 2u) return TierShape{};
+    sh.grid = (int)grid;
+    sh.threads = kTileThreads;
+    return sh;
+}
 
 LongClasses compute_long_classes(uint32_t max_len, int sm_count, uint64_t scratch_bytes)
 {
@@ -1726,7 +2596,7 @@ LongClasses compute_long_classes(uint32_t max_len, int sm_count, uint64_t scratc
     int lim[kLongClasses];
     int n = 0;
     for (int c = 0; c < kLongClasses - 1; ++c)
-        if (2 * kLongClassLimit[c] < top) lim[n++] = kLongClassLimit[c];
+        if (kLongClassLimit[c] < top) lim[n++] = kLongClassLimit[c];
     lim[n++] = top;
     for (int c = 0; c < n; ++c) {
         TierShape sh = lim[c] <= kLongTinyDistance    ? long_shape_for<false, kLongTinyThreads>(max_len, lim[c], sm_count)
@@ -1740,6 +2610,14 @@ LongClasses compute_long_classes(uint32_t max_len, int sm_count, uint64_t scratc
         C.shape[c] = sh;
     }
     C.n = n;
+    C.scan = wide_shape<2, true>(max_len, sm_count, scratch_bytes);
+    for (int c = 0; c + 1 < n; ++c) {
+        C.wide[c] = lim[c] <= 127   ? wide_shape<4, false>(max_len, sm_count, scratch_bytes)
+                    : lim[c] <= 255 ? wide_shape<8, false>(max_len, sm_count, scratch_bytes)
+                    : lim[c] <= 511 ? wide_shape<16, false>(max_len, sm_count, scratch_bytes)
+                    : lim[c] <= 1023 ? wide_shape<32, false>(max_len, sm_count, scratch_bytes) : TierShape{};
+    }
+    C.tile = tile_shape(max_len, lim, n - 1, sm_count, scratch_bytes);
     return C;
 }
 

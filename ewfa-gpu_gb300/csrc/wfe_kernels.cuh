@@ -39,39 +39,57 @@ struct TierShape {
     int threads;        /* tiers 5-6 and the bound pass: threads per CTA */
 };
 
-/* Distance classes of tier 5.  The bound pass (bound_kernel) sends each pair
- * of tier 5 to the first class whose limit covers its distance bound, and
- * every class is a launch of its own with wavefront buffers (shared memory)
- * and backtrace slabs sized to its limit: a class of short distances keeps
- * two to three times the pairs in flight per SM of one launch sized for
- * distance 2047.  Limits 255, 511 and 1023, each kept only while below half
- * of tier 5's own limit, then tier 5's own limit (min(max_len, 2047)).
- * Class 255 runs CTAs of one warp, classes up to distance 1024 CTAs of 128
- * threads, the last one (when larger) 256: a pair of short distance has few
- * cells per step to share, and fewer warps per pair spend fewer instructions
- * on each step's bookkeeping and barrier. */
-constexpr int kLongClasses = 4;
-constexpr int kLongClassLimit[kLongClasses - 1] = {255, 511, 1023};
+/* Distance classes of tier 5, by the upper bound on each pair's distance.
+ * A list of at least kScanMin pairs is bounded by the scan (wide_kernel<2,
+ * true>); the classes are then aligned by the tile kernel, in one launch,
+ * except those with kWidePairs pairs or more, which one thread per pair takes
+ * (wide_kernel), and the last, which holds what the others do not and whose
+ * pairs get a CTA each (long_kernel).  The limits are those of 3, 4, 5, 6, 8,
+ * 10, 16 and 32 lanes per pair: every number of pairs that a warp can hold,
+ * but 7.  Shorter lists are bounded by the bound pass (bound_kernel), and
+ * every pair gets a CTA, in the classes of class_by_cta: each of those is a
+ * launch of its own with wavefront buffers (shared memory) and backtrace
+ * slabs sized to its limit.  Classes up to 257 run CTAs of one warp, classes
+ * up to distance 1024 CTAs of 128 threads, the others 256: a pair of short
+ * distance has few cells per step to share, and fewer warps per pair spend
+ * fewer instructions on each step's bookkeeping and barrier.  Limits at or
+ * past tier 5's own (min(max_len, 2047)) are dropped. */
+constexpr int kLongClasses = 9;
+constexpr int kLongClassLimit[kLongClasses - 1] = {127, 193, 257, 321, 449, 577, 961, 1985};
+/* Where the lines lie: the bulk kernels need about as long for one pair as
+ * for thousands (a sequence's length of dependent columns), a CTA per pair
+ * needs little for one pair and then as much again for every few hundred. */
+constexpr uint32_t kScanMin = 1024;
+constexpr uint32_t kWidePairs = 16384;
 constexpr int kLongTinyThreads = 32;
-constexpr int kLongTinyDistance = 255;   /* classes up to this limit use kLongTinyThreads */
+constexpr int kLongTinyDistance = 257;   /* classes up to this limit use kLongTinyThreads */
 constexpr int kLongSmallThreads = 128;
 constexpr int kLongSmallDistance = 1024; /* classes up to this limit use kLongSmallThreads */
+constexpr int kTileClass = kLongClasses; /* AlignLaunch::cls of the tile kernel */
 /* Work lists of one length bucket: one per tier, then one per class. */
-constexpr int kListsPerBucket = kNumTiers + kLongClasses;
+constexpr int kListsPerBucket = kNumTiers + kLongClasses + 1; /* the last: tier 5's list in order of length */
+constexpr int kOrderBins = 256;
 
 struct LongClasses {
     int n;                           /* classes (0: tier 5 runs as one launch over its list) */
     TierShape shape[kLongClasses];   /* grid, smem, seq_words, dlim, slab, scratch, threads */
-    /* List c holds the pairs of the upper half of the class's distances from
-     * its front (counts[c] of them) and the others from its back
+    TierShape scan;                  /* the scan: grid (0: none), slab, scratch */
+    TierShape wide[kLongClasses];    /* one pair per thread: grid (0: none), slab, scratch */
+    TierShape tile;                  /* several lanes per pair, all classes but the last: grid (0: none), slab, scratch */
+    /* The bound pass puts the pairs of the upper half of a class's distances at
+     * the front of list c (counts[c] of them) and the others at its back
      * (low_counts[c], at cap-1, cap-2, ...): a class launch takes its longer
-     * pairs first, so that its last CTAs are not left with them. */
+     * pairs first, so that its last CTAs are not left with them.  The scan
+     * fills the fronts only. */
     uint32_t* list[kLongClasses];
     uint32_t cap;                    /* entries of each list */
     uint32_t* counts;                /* counts[c]: pairs at the front of list[c] */
     uint32_t* low_counts;            /* low_counts[c]: pairs at its back */
     uint32_t* cta_done;              /* cta_done[c]: CTAs of class c that finished */
     uint32_t* work_next;             /* work_next[c] */
+    uint32_t* order;                 /* tier 5's list in order of length */
+    uint32_t* order_count;           /* pairs per length bin */
+    uint32_t* order_next;            /* pairs placed per length bin */
 };
 
 /* Global scratch of one CTA of tiers 5-6 for distances up to dlim: 2-bit
@@ -127,6 +145,7 @@ struct Buckets {
     uint32_t stride;
     uint32_t* counts;                /* counts of bucket b at counts + b*count_stride */
     uint32_t count_stride;
+    int tier5_to;                    /* bucket whose tier-5 list takes the tier-5 pairs of all (-1: each its own) */
     unsigned long long* totals;      /* pairs classified into each bucket (stats) */
 };
 
@@ -155,6 +174,9 @@ struct AlignLaunch {
     unsigned char* ops_scratch;  /* global op store for tiers that keep it there */
     size_t ops_scratch_bytes;
     int tier;                    /* this launch's tier */
+    int bulk;                    /* tier 5 began with the scan: the classes' pairs are all at the fronts of their lists */
+    uint32_t min_count;          /* the scan of a list: does nothing with fewer pairs */
+    uint32_t max_count;          /* the bound pass: does nothing with as many (0: no limit) */
     Chain chain;                 /* chain.cta_done == NULL: no device-side chaining */
 };
 
@@ -176,10 +198,14 @@ cudaError_t launch_tier(int tier, const AlignLaunch& a, int grid, cudaStream_t s
  * a.bound, one warp per pair; see bound_kernel.  With a.tier == 5 and
  * classes (a.chain.cls.n > 0) the pass also routes every pair to its class
  * and its last CTA starts the first class that has work (tier 5 as a chain
- * of class launches).  bound_shape: its launch shape (grid 0: its shared
- * memory does not fit, and no bound can be computed). */
+ * of class launches); a list of kScanMin pairs and more is put in order of
+ * length and scanned instead (see LongClasses; a list whose length only the
+ * device knows gets the launches of both, and one of them returns at once).
+ * bound_shape: the pass's launch shape (grid 0: its shared memory does not
+ * fit, and no bound can be computed).  The kernels launched are added to
+ * *launches. */
 TierShape bound_shape(uint32_t max_len, int sm_count);
-cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s);
+cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s, uint64_t* launches);
 
 /* Tier 5's distance classes for sequences up to max_len, their slabs carved
  * from a tier-5 scratch of scratch_bytes (0 classes: none fits). */

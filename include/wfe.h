@@ -195,7 +195,8 @@ int wfe_reset_stats(wfe_ctx* ctx);
  *   tier 2: 32 lanes, shared-memory store, <= 143
  *   tier 3: 32 lanes, store spilled to global memory, <= 271
  *   tier 4: 32 lanes, global store, <= 527
- *   tier 5: a CTA per pair, wavefront in shared memory, <= 2047
+ *   tier 5: <= 2047; a CTA per pair, wavefront in shared memory, or, for lists
+ *           of a thousand pairs and more, bit-parallel bands in distance classes
  *   tier 6: a CTA per pair, wavefront in global memory, no limit
  * (a pair above its tier's limit is handed to the next tier on the device).
  * first_tier[b] = -1 picks by length; first_tier may be NULL.  With
@@ -206,11 +207,12 @@ int wfe_reset_stats(wfe_ctx* ctx);
  * start at the same tier (and restart in every tier they outgrow).  Results
  * do not depend on the policy.  The default is one bucket, no prediction.
  * A chain that starts at tier 5 or 6 first bounds the distance of each of its
- * pairs with a narrow band of the wavefront (one warp per pair); the
- * CTA-per-pair tiers then compute only the cells the target cell depends on
- * (about half of them), and a pair whose bound lies past tier 5's limit
- * goes straight to tier 6.  WFE_POLICY_NO_BOUND turns that pass off (for
- * comparison: results are the same).
+ * pairs with a narrow band; each pair then goes to the distance class that
+ * covers its bound, and a pair whose bound lies past tier 5's limit goes
+ * straight to tier 6.  WFE_POLICY_NO_BOUND turns that pass off, and with it the
+ * classes (for comparison: results are the same).  A bucket whose tier is left
+ * to its length (-1) starts large batches of sequences past 400 bases at
+ * tier 5 where it would start small ones at tier 0.
  * Replaces nothing in the reference, which has one fixed launch shape
  * (src/wavefront.cu:173-208); see also wfe_autotune. */
 #define WFE_POLICY_PREDICT 1u  /* route every pair to the tier of its predicted distance */

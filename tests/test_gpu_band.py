@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import wfe
-from test_gpu_parity import _pinned, compare_with_oracle, torch_cuda
+from test_gpu_parity import _pinned, assert_same_cigars, compare_with_oracle, torch_cuda
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,39 @@ def test_tier_0_band(cap, stride, spread):
         assert ctx.stats()["tier_entered"][0] >= len(pairs)
     assert (dist == 31).any() and (dist == 32).any()
     compare_with_oracle(ascii, pairs, stride, dist, cg, st, max_distance=cap)
+
+
+def far_pairs(rng, n, length, edits):
+    """n pairs of up to `length` bases, `edits` edits apart, long indels and repeats among them."""
+    seqs = band_pairs([int(x) for x in rng.integers(max(1, length // 3), length + 1, n)], [edits], int(rng.integers(1 << 30)))
+    out = []
+    for p, t in seqs:
+        if len(t) > 200 and rng.random() < 0.3:
+            at, k = int(rng.integers(0, len(t) - 100)), int(rng.integers(20, 100))
+            t = t[:at] + (bases(rng, k) + t[at:] if rng.random() < 0.5 else t[at + k:])
+        out.append((p, t))
+    return out
+
+
+@pytest.mark.parametrize("cap", [0, 300])
+@pytest.mark.parametrize("n", [600, 20000])  # the classes by several lanes per pair, and by one thread
+@pytest.mark.parametrize("length,edits", [(90, 4), (700, 50), (1100, 110), (1300, 220), (1500, 450), (2200, 900)])
+def test_wide_bands(length, edits, n, cap):
+    torch_cuda()
+    rng = np.random.default_rng(length)
+    seqs = far_pairs(rng, 90, length, edits)
+    t = bases(rng, length)
+    seqs += [(t, t), (b"", t[:60]), (t[:60], b""), (b"", b""), (t[:33], t), (t, t[length // 2:]), (t[:1], t[:1]),
+             (b"", t), (t, b""), (bases(rng, length // 2), bases(rng, length // 2))]
+    ascii, pairs = wfe.pairs_from_list(seqs)
+    pick = rng.permutation(np.arange(n) % len(pairs))
+    with wfe.Context(max_seq_len=2500, cigar_stride=5000, max_distance=cap) as ctx:
+        ctx.set_policy([2500], [5])
+        dist, cg, st = ctx.align(ascii, pairs[pick])
+    for i in range(len(pairs)):  # equal pairs have equal results, whatever their warp
+        same = np.flatnonzero(pick == i)
+        first = same[0]
+        assert (dist[same] == dist[first]).all() and (st[same] == st[first]).all(), i
+        assert_same_cigars(cg[same], np.repeat(cg[first:first + 1], len(same), 0))
+    first = np.array([np.flatnonzero(pick == i)[0] for i in range(len(pairs))])
+    compare_with_oracle(ascii, pairs, 5000, dist[first], cg[first], st[first], max_distance=cap)
