@@ -1239,7 +1239,7 @@ __global__ void long_kernel(const __grid_constant__ AlignLaunch A)
  * 32 * NW, so a fixed band that holds both ends' diagonals is exact.
  *
  * Bound by the integer pipe: 13 instructions per word and column and 5 per
- * column, then one pass over 64 diagonals for the walk back.  The wavefront
+ * column, then one pass over 32 diagonals for the walk back.  The wavefront
  * kernels (bound_kernel, long_kernel) spend 72 warp instructions on 32 cells
  * of one pair and 56 more per warp and score, on D^2 / 2 cells; here it is
  * 32 * NW cells a base, for 32 pairs at once and without divergence, but a
@@ -1247,22 +1247,22 @@ __global__ void long_kernel(const __grid_constant__ AlignLaunch A)
  * pairs, and longer the wider its band: a class of fewer than kWidePairs
  * pairs goes to tile_kernel.  200k pairs of 1,000 bases at 10% edits, in
  * batches of 20,000: 15.3 ms from tier 0 up, 8.1 ms from the bound pass and
- * its classes, 2.1 ms so.
+ * its classes, 1.93 ms so (2.10 with a walk over 64 diagonals).
  *
  * Scratch of a warp (slab; rows of 32 words, a lane's column each): the bit
  * planes of both sequences, VP/VN before every block of 32 columns, and the
  * CIGAR bytes (a lane's words together, written backwards).  The walk goes
  * back block by block: the block's columns are computed again from the
- * checkpoint, but only 64 diagonals around the path, 32 of them are kept
- * (transposed in shared memory), and when the walk nears their edge the block
- * is computed again around where it is.  The 64 diagonals are enough when no
- * optimal path to the cell where the walk enters can leave them: a path that
- * touches an edge diagonal e costs at least V(c0, e) + |e - q|, with V the
- * matrix at the block's first column c0 and q the cell's diagonal (V changes
- * by at most 1 per row, and a diagonal is left at a cost of 1), and the cell
- * itself costs at most V(c0, q) + its increments in the block.  Where that
- * test fails (an indel of dozens of bases inside a block), the pair goes to
- * the wavefront kernels. */
+ * checkpoint, but only 32 diagonals around the path, transposed in shared
+ * memory, and when the walk nears their edge the block is computed again
+ * around where it is.  The 32 diagonals are enough when no optimal path to
+ * the cell where the walk enters can leave them: a path that touches an edge
+ * diagonal e costs at least V(c0, e) + |e - q|, with V the matrix at the
+ * block's first column c0 and q the cell's diagonal (V changes by at most 1
+ * per row, and a diagonal is left at a cost of 1), and the cell itself costs
+ * at most V(c0, q) + its increments in the block.  Where that test fails (an
+ * indel of a dozen bases inside a block), the pair goes to the wavefront
+ * kernels. */
 struct WideSlab {
     uint32_t p, t, ckpt, bytes; /* first words */
     uint32_t np, nt;            /* plane words per sequence */
@@ -1330,7 +1330,7 @@ __device__ __forceinline__ int column_sum(const uint32_t (&vp)[NW], const uint32
 struct Walk {
     int m, hb; /* block of 32 columns, and columns into it */
     int q, b;  /* band bit, and the band's highest diagonal (bit 0) */
-    int W;     /* bits of the band, at least 64 */
+    int W;     /* bits of the band, at least 32 */
     int s;     /* score left; before the first block: the value on bit q at that block's first column when !known */
     bool known;
     int limit; /* !known: a distance past it stops the walk */
@@ -1338,91 +1338,69 @@ struct Walk {
     BackBytes cg;
 };
 
-/* The window of a walk: 64 diagonals from band bit e are computed, the 32
- * from bit e + f kept. */
-struct WalkWindow {
-    int e, f;
-};
-__device__ __forceinline__ WalkWindow walk_window(int q, int W)
-{
-    WalkWindow w;
-    w.e = min(max(q - 32, 0), W - 64);
-    w.f = min(max(q - w.e - 16, 0), 32);
-    return w;
-}
+/* The window of a walk: the 32 diagonals from this band bit. */
+__device__ __forceinline__ int walk_window(int q, int W) { return min(max(q - 16, 0), W - 32); }
 
 /* Rows of a block in a thread's column of shared memory: D0 of the window's
- * 32 bits, transposed, and the vertical differences of its 64 before the
- * block. */
-constexpr int kWalkRows = 36;
+ * 32 bits, transposed, and their vertical differences before the block. */
+constexpr int kWalkRows = 34;
 
 /* Fill the rows of block m.  P, T: the thread's columns of the bit planes
  * (rows of `row` words), np words of the pattern's; src(m, t, vp, vn) gives
  * the vertical differences before block m of the band's bits 32t .. 32t+31. */
 template <class Src>
-__device__ __forceinline__ void walk_fill(uint32_t* rows, int m, int b, WalkWindow w, const uint32_t* P,
-                                          const uint32_t* T, int row, int np, const Src& src)
+__device__ __forceinline__ void walk_fill(uint32_t* rows, int m, int b, int e, const uint32_t* P, const uint32_t* T,
+                                          int row, int np, const Src& src)
 {
-    const uint32_t es = (uint32_t)(w.e & 31);
-    uint32_t xp[2], xn[2];
-    {
-        uint32_t p0, n0, p1, n1, p2 = 0u, n2 = 0u;
-        src(m, w.e >> 5, p0, n0);
-        src(m, (w.e >> 5) + 1, p1, n1);
-        if (es) src(m, (w.e >> 5) + 2, p2, n2);
-        xp[0] = __funnelshift_r(p0, p1, es);
-        xp[1] = __funnelshift_r(p1, p2, es);
-        xn[0] = __funnelshift_r(n0, n1, es);
-        xn[1] = __funnelshift_r(n1, n2, es);
-    }
-    rows[32 * 32] = xp[0];
-    rows[32 * 33] = xp[1];
-    rows[32 * 34] = xn[0];
-    rows[32 * 35] = xn[1];
-    uint32_t a0[3], a1[3];
-    plane_window<3>(P, 2 * row, np, 32 * m - b + w.e, a0);
-    plane_window<3>(P + row, 2 * row, np, 32 * m - b + w.e, a1);
+    const uint32_t es = (uint32_t)(e & 31);
+    uint32_t vp, vn, p1 = 0u, n1 = 0u;
+    src(m, e >> 5, vp, vn);
+    if (es) src(m, (e >> 5) + 1, p1, n1);
+    vp = __funnelshift_r(vp, p1, es);
+    vn = __funnelshift_r(vn, n1, es);
+    rows[32 * 32] = vp;
+    rows[32 * 33] = vn;
+    uint32_t a0[2], a1[2];
+    plane_window<2>(P, 2 * row, np, 32 * m - b + e, a0);
+    plane_window<2>(P + row, 2 * row, np, 32 * m - b + e, a1);
     const uint32_t t0 = T[(size_t)(2 * row) * m], t1 = T[(size_t)(2 * row) * m + row];
-    uint32_t keep[32];
+    uint32_t d0[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-        uint32_t d0[2];
-        wide_column<2>(a0, a1, t0, t1, j, xp, xn, d0);
-        keep[j] = __funnelshift_rc(d0[0], d0[1], (uint32_t)w.f);
+        const uint32_t x = __funnelshift_r(a0[0], a0[1], (uint32_t)j) ^ bit_mask(t0, j);
+        d0[j] = band_column(~(x | (__funnelshift_r(a1[0], a1[1], (uint32_t)j) ^ bit_mask(t1, j))), vp, vn);
     }
-    transpose32(keep);
+    transpose32(d0);
 #pragma unroll
-    for (int r = 0; r < 32; ++r) rows[32 * r] = keep[r];
+    for (int r = 0; r < 32; ++r) rows[32 * r] = d0[r];
 }
 
 /* Walk through block k.m, whose rows are filled with window w, to the block
  * before it or to the window's edge.  Returns ST_RUN while there is more to
  * walk, ST_DONE at the origin, ST_OVERMAX past the limit, ST_OVERFLOW when
- * the window's 64 diagonals do not hold every optimal path. */
-__device__ __forceinline__ int walk_block(Walk& k, const uint32_t* rows, WalkWindow w)
+ * the window's diagonals do not hold every optimal path. */
+__device__ __forceinline__ int walk_block(Walk& k, const uint32_t* rows, int e)
 {
-    const uint32_t xp[2] = {rows[32 * 32], rows[32 * 33]}, xn[2] = {rows[32 * 34], rows[32 * 35]};
-    const int ql = k.q - w.e;
-    int c = ql - w.f; /* the path's row of the 32 */
+    const uint32_t vp = rows[32 * 32], vn = rows[32 * 33];
+    int c = k.q - e; /* the path's row */
     const int ex = __popc(~rows[32 * c] & low_bits(k.hb));
-    if (w.e > 0 || w.e < k.W - 64) {
-        const int su = column_sum<2>(xp, xn, ql);      /* V(q) - V(first) at column c0 */
-        const int sd = column_sum<2>(xp, xn, 63) - su; /* V(last) - V(q) */
-        if ((w.e > 0 && ql - su <= ex) || (w.e < k.W - 64 && 63 - ql + sd <= ex)) return ST_OVERFLOW;
+    {
+        /* V(q) - V(first) and V(last) - V(q) at the block's first column */
+        const uint32_t above = low_bits(c), below = ~above & 0x7fffffffu;
+        const int su = __popc(vp & above) - __popc(vn & above), sd = __popc(vp & below) - __popc(vn & below);
+        if ((e > 0 && c - su <= ex) || (e < k.W - 32 && 31 - c + sd <= ex)) return ST_OVERFLOW;
     }
     if (!k.known) {
         k.known = true;
         k.D = k.s += ex;
         if (k.s > k.limit) return ST_OVERMAX;
     }
-    const uint32_t kp = __funnelshift_rc(xp[0], xp[1], (uint32_t)w.f);
-    const uint32_t kn = __funnelshift_rc(xn[0], xn[1], (uint32_t)w.f);
     /* rows to walk on: the band's own edges may be reached, the others not left */
-    const int lo = w.e + w.f > 0 ? 1 : 0, hi = w.e + w.f + 32 < k.W ? 30 : 31;
+    const int lo = e > 0 ? 1 : 0, hi = e + 32 < k.W ? 30 : 31;
     int state = ST_RUN;
     bool here = true;
     do {
-        const int best = walk_step(~rows[32 * c], ~rows[32 * max(c - 1, 0)], ~rows[32 * min(c + 1, 31)], kp, kn, c, 31,
+        const int best = walk_step(~rows[32 * c], ~rows[32 * max(c - 1, 0)], ~rows[32 * min(c + 1, 31)], vp, vn, c, 31,
                                    k.hb);
         if (best >= 0) {
             const int op = best & 3, x = best >> 2;
@@ -1443,7 +1421,7 @@ __device__ __forceinline__ int walk_block(Walk& k, const uint32_t* rows, WalkWin
             here = false;
         }
     } while (state == ST_RUN && here && c >= lo && c <= hi);
-    k.q = w.e + w.f + c;
+    k.q = e + c;
     return state;
 }
 
@@ -1607,7 +1585,7 @@ __device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks
         const int most = __reduce_max_sync(kFull, walking ? k.m + 1 : 0);
         for (int blk = most - 1; blk >= 0; --blk) {
             while (walking && k.m == blk) {
-                const WalkWindow w = walk_window(k.q, W);
+                const int w = walk_window(k.q, W);
                 walk_fill(blocks + lane, blk, b, w, P, T, 32, np, [&](int m, int t, uint32_t& p, uint32_t& v) {
                     const uint32_t* c = ckpt + (size_t)(64 * NW) * m + 64 * t;
                     p = c[0];
@@ -1619,6 +1597,13 @@ __device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks
             }
         }
         if (state == ST_DONE) state = walk_end(k);
+        if (SCAN && state == ST_OVERFLOW) {
+            /* to the last class, as from the other classes */
+            const LongClasses& C = A.chain.cls;
+            A.bound[pi] = D;
+            C.list[C.n - 1][atomicAdd(C.counts + C.n - 1, 1u)] = pi;
+            state = ST_IDLE;
+        }
         __syncwarp();
         store_walked(A, slab + S.bytes, (int)S.bw, state, pi, D, k.cg.n, lane);
         __syncwarp();
@@ -1629,7 +1614,7 @@ __device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks
 /* Launched from the device too, so a register limit and no launch bounds (see
  * tier_kernel). */
 template <int NW, bool SCAN>
-__global__ void __maxnreg__(NW <= 8 ? 128 : (NW <= 16 ? 168 : 255)) wide_kernel(const __grid_constant__ AlignLaunch A)
+__global__ void __maxnreg__(NW <= 4 ? 96 : (NW <= 8 ? 128 : (NW <= 16 ? 168 : 255))) wide_kernel(const __grid_constant__ AlignLaunch A)
 {
     __shared__ uint32_t blocks[32 * kWalkRows];
     if constexpr (SCAN) {
@@ -1660,10 +1645,11 @@ __global__ void __maxnreg__(NW <= 8 ? 128 : (NW <= 16 ? 168 : 255)) wide_kernel(
  * each class left most of the GPU idle for the length of its longest pair.
  * A pair takes L / 16 steps whatever its band, so the kernel needs tens of
  * times fewer pairs than one thread per pair to fill the GPU, for 1.5 to 2
- * times its instructions.  8,000 pairs of 5,000-7,000 bases at 6-10% edits:
- * 4.8 ms with a CTA per pair, 2.6 ms so (three callers at once: 3.9 and 1.7 ms
- * a call); 50,000 pairs of 100-10,000 bases at 1-15%: 13.1 and 6.1 ms (9.4
- * and 4.4). */
+ * times its instructions.  80 registers keep three CTAs on an SM, so that
+ * two compute while the third walks back (128 and two CTAs: 1.2 times the
+ * time).  8,000 pairs of 5,000-7,000 bases at 6-10% edits: 3.9 ms with a CTA
+ * per pair, 1.42 ms so, a call among others of three contexts; 50,000 pairs of
+ * 100-10,000 bases at 1-15%: 9.3 and 3.7 ms. */
 constexpr int kTileWarps = 8;
 constexpr int kTileThreads = 32 * kTileWarps;
 /* lanes per pair for distances up to dlim: nd <= 2 G for any ends */
@@ -1707,7 +1693,7 @@ __device__ uint32_t tile_chunks(const LongClasses& C)
     return n;
 }
 
-__global__ void __maxnreg__(128) tile_kernel(const __grid_constant__ AlignLaunch A)
+__global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch A)
 {
     __shared__ uint32_t blocks[kTileWarps * 32 * kWalkRows];
     __shared__ uint32_t s_item;
@@ -1758,10 +1744,7 @@ __global__ void __maxnreg__(128) tile_kernel(const __grid_constant__ AlignLaunch
                         const int x = (dub - wide) >> 1;
                         dlo = (min(0, kt) - x) >> 5;
                         dhi = (max(0, kt) + x + 31) >> 5;
-                        if (dhi - dlo < 2) { /* the walk wants 64 diagonals */
-                            --dlo;
-                            if (dhi - dlo < 2) ++dhi;
-                        }
+                        if (dhi == dlo) ++dhi; /* the walk wants 32 diagonals */
                     }
                 }
             }
@@ -1832,7 +1815,8 @@ __global__ void __maxnreg__(128) tile_kernel(const __grid_constant__ AlignLaunch
         __syncthreads();
         /* The walk back, a pair per lane of the first warp.  The warps fill the
          * rows of as many blocks at a time, all with the window around where
-         * the walk is: it seldom moves by 15 diagonals in 256 columns. */
+         * the walk is: it seldom moves by 15 diagonals in 256 columns.  A block
+         * that it enters too near the window's edge is filled again. */
         Walk k{};
         int state = ST_IDLE;
         bool walking = false;
@@ -1867,7 +1851,7 @@ __global__ void __maxnreg__(128) tile_kernel(const __grid_constant__ AlignLaunch
             }
             if (!__syncthreads_or(walking)) break;
             const int m0 = s_m[lane], m = m0 - warp;
-            const WalkWindow w = walk_window(s_q[lane], k.W);
+            const int w = walk_window(s_q[lane], k.W);
             if (m >= 0)
                 walk_fill(blocks + warp * (32 * kWalkRows) + lane, m, k.b, w, slab + own, slab + S.t + own, npair, Bp,
                           [&](int mm, int t, uint32_t& p, uint32_t& v) {
@@ -1879,11 +1863,13 @@ __global__ void __maxnreg__(128) tile_kernel(const __grid_constant__ AlignLaunch
                           });
             __syncthreads();
             if (warp == 0) {
-                const int lo = w.e + w.f > 0 ? 1 : 0, hi = w.e + w.f + 32 < k.W ? 30 : 31;
-                int c = k.q - w.e - w.f;
+                const int lo = w > 0 ? 1 : 0, hi = w + 32 < k.W ? 30 : 31;
+                const int centre = k.q - w;
+                int c = centre;
                 while (walking && m0 - k.m < kTileWarps && c >= lo && c <= hi) {
                     const int st = walk_block(k, blocks + (m0 - k.m) * (32 * kWalkRows) + lane, w);
-                    c = k.q - w.e - w.f;
+                    if (st == ST_OVERFLOW && (k.m < m0 || k.q - w != centre)) break; /* again, around the path */
+                    c = k.q - w;
                     walking = st == ST_RUN;
                     if (!walking) state = st;
                 }
