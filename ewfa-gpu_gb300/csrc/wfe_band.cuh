@@ -244,15 +244,13 @@ __device__ __forceinline__ void wide_column(const uint32_t (&a0)[NW + 1], const 
     }
 }
 
-/* One column of a tile of 32 rows, with the horizontal differences that come
- * in above it and those that leave below: hp/hn hold the column's at their
- * highest bit (hi_p/hi_n collect, first column highest). */
-__device__ __forceinline__ void tile_column(uint32_t p0, uint32_t p1, uint32_t c0, uint32_t c1, uint32_t hp_in,
-                                            uint32_t hn_in, uint32_t& vp, uint32_t& vn, uint32_t& hp_out,
-                                            uint32_t& hn_out)
+/* One column of a tile of 32 rows (eq: the rows that match it), with the
+ * horizontal differences that come in above it, at the highest bits of hp_in
+ * and hn_in, and those that leave below, collected in hp_out and hn_out
+ * (first column highest). */
+__device__ __forceinline__ void tile_column(uint32_t eq, uint32_t hp_in, uint32_t hn_in, uint32_t& vp, uint32_t& vn,
+                                            uint32_t& hp_out, uint32_t& hn_out)
 {
-    const uint32_t x = p0 ^ c0;
-    const uint32_t eq = ~(x | (p1 ^ c1));
     const uint32_t t = hn_in >> 31;
     const uint32_t a = (eq | t) & vp;
     const uint32_t d0 = ((a + vp) ^ vp) | (eq | t | vn);

@@ -1662,8 +1662,8 @@ __host__ __device__ constexpr int tile_pairs(int G)
 }
 
 struct TileSlab {
-    uint32_t t, ckpt, start, bytes; /* first words (the pattern's planes at 0) */
-    uint32_t nd, bw;                /* tiles kept per column block; words of a pair's CIGAR */
+    uint32_t t, chars, ckpt, start, bytes; /* first words (the pattern's planes at 0) */
+    uint32_t nw, nd, bw;            /* words of a plane; tiles kept per column block; words of a pair's CIGAR */
     uint64_t words;
 };
 
@@ -1671,9 +1671,11 @@ __host__ __device__ __forceinline__ TileSlab tile_slab(uint32_t max_len, int dli
 {
     TileSlab s{};
     const uint32_t G = (uint32_t)tile_lanes(dlim), n = (uint32_t)tile_pairs((int)G), nw = (max_len + 31u) / 32u;
+    s.nw = nw;
     s.nd = 2u * G;
     s.t = 2u * n * nw;
-    s.ckpt = (2u * s.t + 1u) & ~1u;
+    s.chars = (2u * s.t + 3u) & ~3u;
+    s.ckpt = s.chars + 8u * n * nw;
     s.start = s.ckpt + 2u * n * nw * s.nd;
     s.bytes = s.start + n;
     s.bw = (2u * (uint32_t)dlim + 1u + max_len / 127u + 3u) / 4u;
@@ -1693,9 +1695,29 @@ __device__ uint32_t tile_chunks(const LongClasses& C)
     return n;
 }
 
+/* The text of a pair as one byte per base, its code times 64, by the eight
+ * threads of a group (g): words of four, from the aligned words that hold a
+ * base. */
+__device__ __forceinline__ void tile_chars(const char* seq, uint32_t len, uint32_t* out, int g)
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(seq);
+    const uint32_t sh = (uint32_t)(a & 3u);
+    const uint32_t* in = reinterpret_cast<const uint32_t*>(a - sh);
+    const int n = (int)((len + 3u) >> 2), last = len ? (int)((sh + len - 1u) >> 2) : -1;
+#pragma unroll 4
+    for (int k = g; k < n; k += 8) {
+        const uint32_t x = __ldg(in + k), y = k < last ? __ldg(in + k + 1) : 0u;
+        out[k] = (__funnelshift_r(x, y, 8u * sh) & 0x06060606u) << 5;
+    }
+}
+
 __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch A)
 {
     __shared__ uint32_t blocks[kTileWarps * 32 * kWalkRows];
+    /* matching rows of each base, per lane: a warp's 512 bytes hold 256 of
+     * each half warp, base c of lane l at 64 c + 4 (l % 16), so that a
+     * byte of the text, with 4 (l % 16) added, is the address's low byte */
+    __shared__ __align__(256) unsigned char match[kTileWarps * 512];
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_pi[32];
     __shared__ int s_plen[32], s_tlen[32], s_dlo[32], s_dhi[32], s_state[32], s_m[32], s_q[32];
@@ -1765,6 +1787,10 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
                 const int n = (len + 31) >> 5, each = (n + parts - 1) / parts, w0 = part * each;
                 wide_pack(s_seq[seq], (uint32_t)len, slab + ((seq & 1) ? S.t : 0u) + own, npair, w0, min(n, w0 + each));
             }
+            const int who = (int)threadIdx.x >> 3;
+            if (who < npair)
+                tile_chars(s_seq[2 * who + 1], (uint32_t)s_tlen[who], slab + S.chars + (size_t)(8u * S.nw) * who,
+                           (int)threadIdx.x & 7);
         }
         __syncthreads();
         /* forward */
@@ -1779,10 +1805,12 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
             /* where the walk starts: the target's diagonal at the last block's first column */
             const int v0 = 32 * (Bt - 1) - (tlen - plen);
             const uint32_t* const P = slab + own;
-            const uint32_t* const T = slab + S.t + own;
+            const uint4* const T = reinterpret_cast<const uint4*>(slab + S.chars + (size_t)(8u * S.nw) * (in ? own : 0));
+            unsigned char* const table = match + warp * 512 + (lane >> 4) * 256;
+            const uint32_t page = (uint32_t)(warp * 512 + (lane >> 4) * 256), mine = 4u * (uint32_t)(lane & 15);
             const int steps = __reduce_max_sync(kFull, Bp > 0 && Bt > 0 ? Bp + Bt - 1 : 0);
             int bi = l, corner = 0;
-            uint32_t vp = 0, vn = 0, p0 = 0, p1 = 0, hp = 0, hn = 0;
+            uint32_t vp = 0, vn = 0, hp = 0, hn = 0;
             int low = 0; /* the value below the tile's left edge */
             for (int s = 0; s < steps; ++s) {
                 const uint32_t up_p = __shfl_sync(kFull, hp, src), up_n = __shfl_sync(kFull, hn, src);
@@ -1793,8 +1821,12 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
                 if (bj == lead) {
                     vp = ~0u;
                     vn = 0u;
-                    p0 = P[(size_t)(2 * npair) * bi];
-                    p1 = P[(size_t)(2 * npair) * bi + npair];
+                    const uint32_t p0 = P[(size_t)(2 * npair) * bi], p1 = P[(size_t)(2 * npair) * bi + npair];
+                    uint32_t* const rows = reinterpret_cast<uint32_t*>(table + mine);
+                    rows[0] = ~(p0 | p1);
+                    rows[16] = p0 & ~p1;
+                    rows[32] = ~p0 & p1;
+                    rows[48] = p0 & p1;
                     corner = bj == 0 ? 32 * bi : up_low;
                 }
                 const bool edge = bi == 0 || bj - bi == dhi;
@@ -1804,12 +1836,17 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
                     const uint32_t mask = low_bits(v0 & 31);
                     slab[S.start + own] = (uint32_t)(corner + __popc(vp & mask) - __popc(vn & mask));
                 }
-                const uint32_t t0 = T[(size_t)(2 * npair) * bj], t1 = T[(size_t)(2 * npair) * bj + npair];
+                const uint4 ca = T[2 * bj], cb = T[2 * bj + 1];
                 low = corner + __popc(vp) - __popc(vn);
                 corner += __popc(in_p) - __popc(in_n);
+                const uint32_t chars[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+                /* the bytes past the text's end hold anything: masked, they are bases too */
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    tile_column(p0, p1, bit_mask(t0, j), bit_mask(t1, j), in_p << j, in_n << j, vp, vn, hp, hn);
+                for (int j = 0; j < 32; ++j) {
+                    const uint32_t at =
+                        __byte_perm((chars[j >> 2] & 0xc0c0c0c0u) | mine * 0x01010101u, page, 0x7650u + (j & 3));
+                    tile_column(*reinterpret_cast<const uint32_t*>(match + at), in_p << j, in_n << j, vp, vn, hp, hn);
+                }
             }
         }
         __syncthreads();
