@@ -79,6 +79,23 @@ __device__ __forceinline__ uint32_t band_column(uint32_t eq, uint32_t& vp, uint3
     return d0;
 }
 
+/* The same column, and the operation by which the wavefront's path leaves each
+ * of its cells, going back (a match leaves by none): the first that fits of a
+ * deletion (the row above has one less), a mismatch (the diagonal before has)
+ * and an insertion (the column before has).  One of the two bits of the
+ * operation codes, `high` or low; bit 0's deletion is not known here. */
+__device__ __forceinline__ uint32_t band_column_ops(uint32_t eq, uint32_t& vp, uint32_t& vn, bool high)
+{
+    const uint32_t d0 = (((eq & vp) + vp) ^ vp) | eq | vn;
+    const uint32_t hp = vn | ~(d0 | vp);
+    const uint32_t hn = vp & d0;
+    const uint32_t x = d0 >> 1;
+    vp = hn | ~(x | hp);
+    vn = x & hp;
+    const uint32_t del = vp << 1;
+    return high ? del | ~d0 : del | (d0 & hp);
+}
+
 /* all ones when bit j of w is set */
 __device__ __forceinline__ uint32_t bit_mask(uint32_t w, int j)
 {

@@ -1331,10 +1331,8 @@ struct Walk {
     int m, hb; /* block of 32 columns, and columns into it */
     int q, b;  /* band bit, and the band's highest diagonal (bit 0) */
     int W;     /* bits of the band, at least 32 */
-    int s;     /* score left; before the first block: the value on bit q at that block's first column when !known */
-    bool known;
-    int limit; /* !known: a distance past it stops the walk */
-    int run, D;
+    int s;     /* score left */
+    int run;
     BackBytes cg;
 };
 
@@ -1377,8 +1375,7 @@ __device__ __forceinline__ void walk_fill(uint32_t* rows, int m, int b, int e, c
 
 /* Walk through block k.m, whose rows are filled with window w, to the block
  * before it or to the window's edge.  Returns ST_RUN while there is more to
- * walk, ST_DONE at the origin, ST_OVERMAX past the limit, ST_OVERFLOW when
- * the window's diagonals do not hold every optimal path. */
+ * walk, ST_DONE at the origin, ST_OVERFLOW when the window's diagonals do not hold every optimal path. */
 __device__ __forceinline__ int walk_block(Walk& k, const uint32_t* rows, int e)
 {
     const uint32_t vp = rows[32 * 32], vn = rows[32 * 33];
@@ -1389,11 +1386,6 @@ __device__ __forceinline__ int walk_block(Walk& k, const uint32_t* rows, int e)
         const uint32_t above = low_bits(c), below = ~above & 0x7fffffffu;
         const int su = __popc(vp & above) - __popc(vn & above), sd = __popc(vp & below) - __popc(vn & below);
         if ((e > 0 && c - su <= ex) || (e < k.W - 32 && 31 - c + sd <= ex)) return ST_OVERFLOW;
-    }
-    if (!k.known) {
-        k.known = true;
-        k.D = k.s += ex;
-        if (k.s > k.limit) return ST_OVERMAX;
     }
     /* rows to walk on: the band's own edges may be reached, the others not left */
     const int lo = e > 0 ? 1 : 0, hi = e + 32 < k.W ? 30 : 31;
@@ -1573,8 +1565,7 @@ __device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks
         k.q = it;
         k.b = b;
         k.W = W;
-        k.s = k.D = D;
-        k.known = true;
+        k.s = D;
         k.cg = BackBytes{slab + S.bytes + (size_t)lane * S.bw, 0u, 0, (int)S.bw};
         bool walking = state == ST_DONE;
         if (walking && tlen == 0) { /* only deletions */
@@ -1637,7 +1628,13 @@ __global__ void __maxnreg__(NW <= 4 ? 96 : (NW <= 8 ? 128 : (NW <= 16 ? 168 : 25
  * as +1, an upper bound.  The tile diagonals hold every diagonal of
  * [32 dlo, 32 dhi]; dlo and dhi are the least that certify the pair's bound.
  * The vertical differences into each tile are kept for the walk back, which a
- * warp does for all pairs of the CTA, one per thread (see walk_back).
+ * warp does for all pairs of the CTA, one per thread: four blocks of 32
+ * columns at a time, from the operation codes of 32 diagonals around the path,
+ * transposed, so that a step is the last set bit of a row.  All warps compute
+ * the codes and, at the end, write the CIGARs from the walk's events: the
+ * walk is a serial chain beside other CTAs' busy warps, and everything that
+ * could be taken out of it was (two fifths of a CTA's time before, one step
+ * comparing three diagonals as walk_step does and writing the bytes).
  *
  * A CTA of eight warps takes chunks of up to 32 pairs of a class, the widest
  * class first and each class from the end of its list (the scan's longest
@@ -1662,8 +1659,8 @@ __host__ __device__ constexpr int tile_pairs(int G)
 }
 
 struct TileSlab {
-    uint32_t t, chars, ckpt, start, bytes; /* first words (the pattern's planes at 0) */
-    uint32_t nw, nd, bw;            /* words of a plane; tiles kept per column block; words of a pair's CIGAR */
+    uint32_t t, chars, ckpt, events; /* first words (the pattern's planes at 0) */
+    uint32_t nw, nd, ne;            /* words of a plane; tiles kept per column block; events of a pair */
     uint64_t words;
 };
 
@@ -1676,10 +1673,9 @@ __host__ __device__ __forceinline__ TileSlab tile_slab(uint32_t max_len, int dli
     s.t = 2u * n * nw;
     s.chars = (2u * s.t + 3u) & ~3u;
     s.ckpt = s.chars + 8u * n * nw;
-    s.start = s.ckpt + 2u * n * nw * s.nd;
-    s.bytes = s.start + n;
-    s.bw = (2u * (uint32_t)dlim + 1u + max_len / 127u + 3u) / 4u;
-    s.words = ((uint64_t)s.bytes + (uint64_t)n * s.bw + 63u) & ~uint64_t(63);
+    s.events = s.ckpt + 2u * n * nw * s.nd;
+    s.ne = (uint32_t)dlim;
+    s.words = ((uint64_t)s.events + (uint64_t)n * s.ne + 63u) & ~uint64_t(63);
     return s;
 }
 
@@ -1711,16 +1707,54 @@ __device__ __forceinline__ void tile_chars(const char* seq, uint32_t len, uint32
     }
 }
 
+constexpr int kTileBlocks = kTileWarps / 2; /* blocks whose codes are computed at a time: two warps each */
+constexpr int kTileRows = 66;              /* of a block: two planes of 32 rows, and the vertical differences */
+
+/* A CIGAR from a walk's n events -- 4 * (matches after the operation) +
+ * operation, last operation first -- and the `lead` matches before the first
+ * operation, by a warp. */
+__device__ __forceinline__ uint32_t store_events(const uint32_t* ev, int n, int lead, int8_t* dst, uint32_t cap,
+                                                 int lane)
+{
+    uint32_t total = 0;
+    for (int base = 0; base <= n; base += 32) {
+        const int d = base + lane;
+        int r = 0, letter = 0, nb = 0;
+        if (d <= n) {
+            r = d == 0 ? lead : (int)(ev[n - d] >> 2);
+            letter = d < n ? (int)op_letter((int)(ev[n - 1 - d] & 3u)) : 0;
+            nb = r / 127 + (r % 127 != 0) + (letter != 0);
+        }
+        int x = nb;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += y;
+        }
+        uint32_t pos = total + (uint32_t)(x - nb);
+        for (int j = r / 127; j > 0; --j, ++pos)
+            if (pos < cap) dst[pos] = (int8_t)-127;
+        if (r % 127) {
+            if (pos < cap) dst[pos] = (int8_t)(-(r % 127));
+            ++pos;
+        }
+        if (letter && pos < cap) dst[pos] = (int8_t)letter;
+        total += (uint32_t)__shfl_sync(kFull, x, 31);
+    }
+    if (lane == 0 && total < cap) dst[total] = 0;
+    return total;
+}
+
 __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch A)
 {
-    __shared__ uint32_t blocks[kTileWarps * 32 * kWalkRows];
+    __shared__ uint32_t blocks[kTileBlocks * 32 * kTileRows];
     /* matching rows of each base, per lane: a warp's 512 bytes hold 256 of
      * each half warp, base c of lane l at 64 c + 4 (l % 16), so that a
      * byte of the text, with 4 (l % 16) added, is the address's low byte */
     __shared__ __align__(256) unsigned char match[kTileWarps * 512];
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_pi[32];
-    __shared__ int s_plen[32], s_tlen[32], s_dlo[32], s_dhi[32], s_state[32], s_m[32], s_q[32];
+    __shared__ int s_plen[32], s_tlen[32], s_dlo[32], s_dhi[32], s_state[32], s_m[32], s_q[32], s_n[32], s_lead[32];
     __shared__ const char* s_seq[64];
     const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
     const LongClasses& C = A.chain.cls;
@@ -1802,19 +1836,15 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
             const int dlo = in ? s_dlo[own] : 0, dhi = in ? s_dhi[own] : 0;
             const int Bp = (plen + 31) >> 5, Bt = (tlen + 31) >> 5;
             const int src = grp * G + (l == 0 ? G - 1 : l - 1);
-            /* where the walk starts: the target's diagonal at the last block's first column */
-            const int v0 = 32 * (Bt - 1) - (tlen - plen);
             const uint32_t* const P = slab + own;
             const uint4* const T = reinterpret_cast<const uint4*>(slab + S.chars + (size_t)(8u * S.nw) * (in ? own : 0));
             unsigned char* const table = match + warp * 512 + (lane >> 4) * 256;
             const uint32_t page = (uint32_t)(warp * 512 + (lane >> 4) * 256), mine = 4u * (uint32_t)(lane & 15);
             const int steps = __reduce_max_sync(kFull, Bp > 0 && Bt > 0 ? Bp + Bt - 1 : 0);
-            int bi = l, corner = 0;
+            int bi = l;
             uint32_t vp = 0, vn = 0, hp = 0, hn = 0;
-            int low = 0; /* the value below the tile's left edge */
             for (int s = 0; s < steps; ++s) {
                 const uint32_t up_p = __shfl_sync(kFull, hp, src), up_n = __shfl_sync(kFull, hn, src);
-                const int up_low = __shfl_sync(kFull, low, src);
                 while (bi < Bp && s - bi > bi + dhi) bi += G; /* the row block has left the band */
                 const int bj = s - bi, lead = max(0, bi + dlo);
                 if (bi >= Bp || bj < lead || bj >= Bt) continue;
@@ -1827,18 +1857,11 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
                     rows[16] = p0 & ~p1;
                     rows[32] = ~p0 & p1;
                     rows[48] = p0 & p1;
-                    corner = bj == 0 ? 32 * bi : up_low;
                 }
                 const bool edge = bi == 0 || bj - bi == dhi;
                 const uint32_t in_p = edge ? ~0u : up_p, in_n = edge ? 0u : up_n;
                 ckpt[((size_t)bj * S.nd + (size_t)(bi - bj + dhi)) * npair + own] = make_uint2(vp, vn);
-                if (bj == Bt - 1 && v0 >= 0 && bi == v0 >> 5) {
-                    const uint32_t mask = low_bits(v0 & 31);
-                    slab[S.start + own] = (uint32_t)(corner + __popc(vp & mask) - __popc(vn & mask));
-                }
                 const uint4 ca = T[2 * bj], cb = T[2 * bj + 1];
-                low = corner + __popc(vp) - __popc(vn);
-                corner += __popc(in_p) - __popc(in_n);
                 const uint32_t chars[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
                 /* the bytes past the text's end hold anything: masked, they are bases too */
 #pragma unroll
@@ -1850,74 +1873,165 @@ __global__ void __maxnreg__(80) tile_kernel(const __grid_constant__ AlignLaunch 
             }
         }
         __syncthreads();
-        /* The walk back, a pair per lane of the first warp.  The warps fill the
-         * rows of as many blocks at a time, all with the window around where
-         * the walk is: it seldom moves by 15 diagonals in 256 columns.  A block
-         * that it enters too near the window's edge is filled again. */
-        Walk k{};
-        int state = ST_IDLE;
+        /* The walk back, a pair per lane of the first warp, with one window of
+         * 32 diagonals around where it is for the next four blocks: it seldom
+         * moves by 15 diagonals in 128 columns.  When it does, or enters a
+         * block too near the window's edge for the test (see wide_kernel), it
+         * goes back to the block's entry and the codes are computed again
+         * from there. */
+        const int dhi = s_dhi[lane], nd = dhi - s_dlo[lane] + 1, W = 32 * (nd - 1) + 1, b = 32 * dhi;
+        const int own = lane < npair ? lane : 0, Bp = (s_plen[lane] + 31) >> 5;
+        uint32_t* const ev = slab + S.events + (size_t)own * S.ne;
+        int state = ST_IDLE, m = 0, hb = 0, q = 0, run = 0, n = 0;
         bool walking = false;
-        const int dhi = s_dhi[lane], Bp = (s_plen[lane] + 31) >> 5, nd = dhi - s_dlo[lane] + 1;
-        const int own = lane < npair ? lane : 0;
-        k.b = 32 * dhi;
-        k.W = 32 * (nd - 1) + 1;
         if (warp == 0) {
             state = s_state[lane];
-            const int plen = s_plen[lane], tlen = s_tlen[lane], kt = tlen - plen;
-            k.m = tlen > 0 ? (tlen - 1) >> 5 : 0;
-            k.hb = tlen - 32 * k.m;
-            k.q = k.b - kt;
-            k.limit = limit;
-            k.cg = BackBytes{slab + S.bytes + (size_t)own * S.bw, 0u, 0, (int)S.bw};
-            walking = state == ST_RUN;
-            if (walking && (plen == 0 || tlen == 0)) { /* one operation throughout */
-                for (k.s = plen + tlen; k.s > 0; --k.s) k.cg.push(plen ? (uint32_t)'D' : (uint32_t)'I', 1);
-                k.D = plen + tlen;
-                k.q = k.b;
+            const int plen = s_plen[lane], tlen = s_tlen[lane];
+            m = tlen > 0 ? (tlen - 1) >> 5 : 0;
+            hb = tlen - 32 * m;
+            q = b - (tlen - plen);
+            walking = state == ST_RUN && plen > 0 && tlen > 0;
+            if (state == ST_RUN && !walking) { /* one operation throughout */
+                for (; n < plen + tlen; ++n) ev[n] = (uint32_t)(plen ? kOpDel : kOpIns);
                 state = ST_DONE;
-                walking = false;
-            } else if (walking) {
-                const int v0 = 32 * k.m - kt; /* a virtual row's value is its diagonal */
-                k.s = v0 >= 0 ? (int)slab[S.start + own] : kt;
             }
         }
         for (;;) {
             if (warp == 0) {
-                s_m[lane] = walking ? k.m : -1;
-                s_q[lane] = k.q;
+                s_m[lane] = walking ? m : -1;
+                s_q[lane] = q;
             }
             if (!__syncthreads_or(walking)) break;
-            const int m0 = s_m[lane], m = m0 - warp;
-            const int w = walk_window(s_q[lane], k.W);
-            if (m >= 0)
-                walk_fill(blocks + warp * (32 * kWalkRows) + lane, m, k.b, w, slab + own, slab + S.t + own, npair, Bp,
-                          [&](int mm, int t, uint32_t& p, uint32_t& v) {
-                              const int bi = t + mm - dhi;
-                              uint2 c = bi < 0 ? make_uint2(0u, ~0u) : make_uint2(~0u, 0u);
-                              if (bi >= 0 && bi < Bp && t < nd) c = ckpt[((size_t)mm * S.nd + (size_t)t) * npair + own];
-                              p = c.x;
-                              v = c.y;
-                          });
+            const int m0 = s_m[lane], e = walk_window(s_q[lane], W);
+            {
+                const int blk = m0 - (warp >> 1);
+                uint32_t* const rows = blocks + (warp >> 1) * (32 * kTileRows) + lane;
+                const bool high = (warp & 1) != 0;
+                if (blk >= 0) {
+                    /* tile t of the column block: rows above the matrix or below the pattern are virtual */
+                    const auto edge = [&](int t) {
+                        const int bi = t + blk - dhi;
+                        return bi < 0 ? make_uint2(0u, ~0u)
+                               : bi < Bp && t < nd ? ckpt[((size_t)blk * S.nd + (size_t)t) * npair + own]
+                                                   : make_uint2(~0u, 0u);
+                    };
+                    const uint32_t es = (uint32_t)(e & 31);
+                    const uint2 c0 = edge(e >> 5), c1 = es ? edge((e >> 5) + 1) : make_uint2(0u, 0u);
+                    uint32_t vp = __funnelshift_r(c0.x, c1.x, es), vn = __funnelshift_r(c0.y, c1.y, es);
+                    if (!high) {
+                        rows[32 * 64] = vp;
+                        rows[32 * 65] = vn;
+                    }
+                    const uint32_t* const P = slab + own;
+                    const uint32_t* const T = slab + S.t + own + (size_t)(2 * npair) * blk;
+                    uint32_t a0[2], a1[2], code[32];
+                    plane_window<2>(P, 2 * npair, Bp, 32 * blk - b + e, a0);
+                    plane_window<2>(P + npair, 2 * npair, Bp, 32 * blk - b + e, a1);
+                    const uint32_t t0 = T[0], t1 = T[npair];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const uint32_t x = __funnelshift_r(a0[0], a0[1], (uint32_t)j) ^ bit_mask(t0, j);
+                        const uint32_t eq = ~(x | (__funnelshift_r(a1[0], a1[1], (uint32_t)j) ^ bit_mask(t1, j)));
+                        code[j] = band_column_ops(eq, vp, vn, high);
+                    }
+                    transpose32(code);
+                    uint32_t* const out = rows + (high ? 32 * 32 : 0);
+#pragma unroll
+                    for (int r = 0; r < 32; ++r) out[32 * r] = code[r];
+                }
+            }
             __syncthreads();
             if (warp == 0) {
-                const int lo = w > 0 ? 1 : 0, hi = w + 32 < k.W ? 30 : 31;
-                const int centre = k.q - w;
-                int c = centre;
-                while (walking && m0 - k.m < kTileWarps && c >= lo && c <= hi) {
-                    const int st = walk_block(k, blocks + (m0 - k.m) * (32 * kWalkRows) + lane, w);
-                    if (st == ST_OVERFLOW && (k.m < m0 || k.q - w != centre)) break; /* again, around the path */
-                    c = k.q - w;
-                    walking = st == ST_RUN;
-                    if (!walking) state = st;
+                /* rows to walk on: the band's own edges may be reached, the others not left */
+                const int lo = e > 0 ? 1 : 0, hi = e + 32 < W ? 30 : 31;
+                int c = q - e;
+                /* the walk at the entry of its block */
+                int c_in = c, hb_in = hb, run_in = run, n_in = n;
+                bool here = walking;
+                while (here) {
+                    const uint32_t* const rows = blocks + (m0 - m) * (32 * kTileRows) + lane;
+                    const uint32_t low = rows[32 * c], high = rows[32 * (32 + c)];
+                    const int at = 31 - __clz((int)((low | high) & low_bits(hb)));
+                    if (at >= 0) {
+                        const int op = (int)((low >> at) & 1u) + 2 * (int)((high >> at) & 1u);
+                        if (n < limit) ev[n] = 4u * (uint32_t)(run + hb - 1 - at) + (uint32_t)op;
+                        ++n;
+                        run = 0;
+                        hb = at + (op == kOpDel ? 1 : 0);
+                        c += op == kOpDel ? -1 : (op == kOpIns ? 1 : 0);
+                    } else {
+                        run += hb;
+                        hb = 0;
+                    }
+                    bool again = c < lo || c > hi;
+                    if (hb == 0) {
+                        /* at the block's first column: could an optimal path leave the window? */
+                        const uint32_t vp = rows[32 * 64], vn = rows[32 * 65];
+                        const uint32_t above = low_bits(c), below = ~above & 0x7fffffffu;
+                        const int su = __popc(vp & above) - __popc(vn & above);
+                        const int sd = __popc(vp & below) - __popc(vn & below);
+                        again = c < 0 || c > 31 || (e > 0 && c_in - su <= n - n_in) ||
+                                (e + 32 < W && 31 - c_in + sd <= n - n_in);
+                    }
+                    if (again) {
+                        here = false;
+                        if (m == m0 && c_in == q - e) { /* nor from a window around the path */
+                            walking = false;
+                            state = ST_OVERFLOW;
+                        }
+                        c = c_in;
+                        hb = hb_in;
+                        run = run_in;
+                        n = n_in;
+                    } else if (n > limit) {
+                        here = walking = false;
+                        state = past;
+                    } else if (hb == 0) {
+                        if (m == 0) {
+                            /* the rows left are deleted */
+                            here = walking = false;
+                            const int left = c + e - b;
+                            state = left < 0 ? ST_BADWALK : n + left > limit ? past : ST_DONE;
+                            for (int v = state == ST_DONE ? left : 0; v > 0; --v) {
+                                ev[n++] = 4u * (uint32_t)run + (uint32_t)kOpDel;
+                                run = 0;
+                            }
+                        } else {
+                            --m;
+                            hb = 32;
+                            c_in = c;
+                            hb_in = hb;
+                            run_in = run;
+                            n_in = n;
+                            here = m0 - m < kTileBlocks && c >= lo && c <= hi;
+                        }
+                    }
                 }
+                q = c + e;
             }
         }
         if (warp == 0) {
-            if (state == ST_DONE) state = walk_end(k);
-            if (state == ST_OVERMAX) state = past;
-            if (state == ST_DONE && A.max_distance > 0 && k.D > A.max_distance) state = ST_OVERMAX;
-            __syncwarp();
-            store_walked(A, slab + S.bytes, (int)S.bw, state, lane < npair ? s_pi[lane] : 0u, k.D, k.cg.n, lane);
+            if (state == ST_DONE && A.max_distance > 0 && n > A.max_distance) state = ST_OVERMAX;
+            s_state[lane] = state;
+            s_n[lane] = n;
+            s_lead[lane] = run;
+        }
+        __syncthreads();
+        /* CIGARs and results, a pair per warp */
+        for (int p = warp; p < npair; p += kTileWarps) {
+            const int st = s_state[p], nev = s_n[p];
+            if (st == ST_IDLE) continue;
+            const uint32_t pi = s_pi[p], cap = A.cigar_stride;
+            if (st == ST_DONE) {
+                const uint32_t len = store_events(slab + S.events + (size_t)p * S.ne, nev, s_lead[p],
+                                                  A.cigar + (size_t)pi * cap, cap, lane);
+                if (lane == 0) {
+                    A.dist[pi] = nev;
+                    if (A.status) A.status[pi] = len > cap ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED : (uint8_t)WFE_PAIR_OK;
+                }
+            } else if (lane == 0) {
+                finish_unaligned(A, pi, st);
+            }
         }
         __syncthreads();
     }
