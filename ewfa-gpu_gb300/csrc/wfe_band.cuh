@@ -102,11 +102,11 @@ __device__ __forceinline__ uint32_t bit_mask(uint32_t w, int j)
     return (uint32_t)((int32_t)(w << (31 - j)) >> 31);
 }
 
-template <int S>
-__device__ __forceinline__ void transpose_step(uint32_t (&a)[32], uint32_t m)
+template <int S, int N>
+__device__ __forceinline__ void transpose_step(uint32_t (&a)[N], uint32_t m)
 {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < N / 2; ++i) {
         const int k = ((i & ~(S - 1)) << 1) | (i & (S - 1));
         const uint32_t x = a[k], y = a[k + S];
         a[k] = (x & m) | ((y << S) & ~m);
@@ -133,6 +133,23 @@ __device__ __forceinline__ void transpose32(uint32_t (&a)[32])
     transpose_step<4>(a, 0x0f0f0f0fu);
     transpose_step<2>(a, 0x33333333u);
     transpose_step<1>(a, 0x55555555u);
+}
+
+/* The same with only bits first .. first + 15 of every a[i], into 16 words:
+ * bit i of out[r] is bit first + r of a[i]. */
+__device__ __forceinline__ void transpose16(const uint32_t (&a)[32], int first, uint32_t (&out)[16])
+{
+#pragma unroll
+    for (int i = 0; i < 16; ++i) out[i] = __byte_perm(a[i] >> first, a[i + 16] >> first, 0x5410);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t x = out[i], y = out[i + 8];
+        out[i] = __byte_perm(x, y, 0x6240);
+        out[i + 8] = __byte_perm(x, y, 0x7351);
+    }
+    transpose_step<4>(out, 0x0f0f0f0fu);
+    transpose_step<2>(out, 0x33333333u);
+    transpose_step<1>(out, 0x55555555u);
 }
 
 /* The lowest n bits, n in [0, 32]. */

@@ -649,30 +649,33 @@ __global__ void tier_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_
  *           a lane reading its own words and eight lanes writing one pair's
  *           consecutive words are both free of bank conflicts
  *   bytes   the CIGAR, written backwards
- * With texts of up to 32 * kBandBlocks bases the warp keeps every block and
- * the walk needs nothing else (the bytes then reuse the planes).  Longer
- * texts keep the checkpoints only, and each block is computed again when the
- * walk reaches it. */
-constexpr int kBandBlocks = 5;
+ * The warp keeps as many of the last blocks as fit, 16 rows of each around
+ * the ends' diagonals.  The blocks before them, and all blocks for a walk that
+ * leaves those rows, are computed again from their checkpoints, with the rows
+ * around the walk, when it reaches them. */
 constexpr int kSpanWords = 160; /* 16-byte blocks of a span: 8 pairs of 150 bases with their file's line marks */
 static_assert(kSpanWords * 16 <= 4096, "a span must fit in one 4 KiB page (see band_load)");
 constexpr int kPlaneRow = 33;
 constexpr int kSpanRow = kSpanWords + 4; /* a span's words, and those read past its last block */
-constexpr int kBandCkpt = kBandBlocks * 1024;
-constexpr int kBandPlanes = kBandCkpt + kBandBlocks * 64;
-constexpr int kBandStoredWords = kBandPlanes + 2 * kPlaneRow * (2 * kBandBlocks + 1);
-static_assert(4 * kSpanRow <= kBandBlocks * 1024, "the spans use the blocks' space");
+static_assert(4 * kSpanRow <= 1024, "the spans use the blocks' space");
 
 __host__ __device__ constexpr uint32_t band_words(uint32_t max_len) { return (max_len + 31u) / 32u; }
-/* words of a CIGAR: 31 operations, 32 runs, and a byte per 127 matches */
-__host__ __device__ constexpr uint32_t band_byte_words(uint32_t max_len) { return (63u + max_len / 127u + 3u) / 4u; }
-static_assert(32 * band_byte_words(32 * kBandBlocks + 31) <= 2 * kPlaneRow * (2 * kBandBlocks + 1),
-              "the bytes reuse the planes' space");
+/* words of a CIGAR of texts of n blocks: 31 operations, 32 runs, and a byte per 127 matches */
+__host__ __device__ constexpr uint32_t band_byte_words(uint32_t n) { return (63u + 32u * n / 127u + 3u) / 4u; }
+/* words of a warp for texts of n blocks without the blocks, and blocks that are always there */
+__host__ __device__ constexpr uint32_t band_fixed_words(uint32_t n)
+{
+    return 64u * n + 2u * kPlaneRow * (2u * n + 1u) + 32u * band_byte_words(n);
+}
+constexpr uint32_t kBandBlockWords = 512;
+/* Words given to a warp: all blocks of texts up to 160 bases (13 warps per SM;
+ * 150-base reads take 0.45 ns a pair, with room for 224 bases 0.51). */
 __host__ __device__ constexpr uint32_t band_smem_words(uint32_t max_len)
 {
-    const uint32_t nw = band_words(max_len) + (max_len == 0u);
-    const uint32_t again = 1024u + 64u * nw + 2u * kPlaneRow * (2u * nw + 1u) + 32u * band_byte_words(max_len);
-    return again > (uint32_t)kBandStoredWords ? again : (uint32_t)kBandStoredWords;
+    const uint32_t n = band_words(max_len) + (max_len == 0u), m = n < 5u ? n : 5u;
+    const uint32_t all = band_fixed_words(m) + (m > 2u ? m : 2u) * kBandBlockWords;
+    const uint32_t one = band_fixed_words(n) + 2u * kBandBlockWords;
+    return all > one ? all : one;
 }
 
 /* Bit planes of the warp's 32 pairs.  Eight neighbouring pairs that lie in
@@ -785,24 +788,41 @@ __device__ __forceinline__ void band_load(const char* p, uint32_t lp, const char
     __syncwarp();
 }
 
-/* D0 of the 32 columns of block m, from VP/VN before it (left as they are
- * after it).  P and T: the lane's columns of the planes; b: see wfe_band.cuh. */
-template <typename F>
-__device__ __forceinline__ void band_block(const uint32_t* P, int planeP, const uint32_t* T, int planeT, int m, int b,
-                                           uint32_t& vp, uint32_t& vn, F&& each)
+extern __shared__ __align__(16) uint32_t band_smem[];
+
+/* D0 of the 32 columns of block m, from VP/VN before it: its rows first ..
+ * first + 15, transposed, to the lane's column at `out`; returns VP/VN after
+ * it.  P and T: where the lane's columns of the planes begin in band_smem, as
+ * out does (pointers would lose their address space); b: see wfe_band.cuh. */
+__device__ __forceinline__ uint2 band_rows(int P, int planeP, int T, int planeT, int m, int b, uint32_t vp,
+                                           uint32_t vn, int first, int out)
 {
-    const uint32_t* pw = P + m * kPlaneRow;
+    const uint32_t* pw = band_smem + P + m * kPlaneRow;
     const uint32_t l0 = m > 0 ? pw[-kPlaneRow] : 0u, l1 = m > 0 ? pw[planeP - kPlaneRow] : 0u;
     const uint32_t c0 = pw[0], c1 = pw[planeP], n0 = pw[kPlaneRow], n1 = pw[planeP + kPlaneRow];
     const uint32_t a0 = __funnelshift_l(l0, c0, (uint32_t)b), e0 = __funnelshift_l(c0, n0, (uint32_t)b);
     const uint32_t a1 = __funnelshift_l(l1, c1, (uint32_t)b), e1 = __funnelshift_l(c1, n1, (uint32_t)b);
-    const uint32_t t0 = T[m * kPlaneRow], t1 = T[m * kPlaneRow + planeT];
+    const uint32_t t0 = band_smem[T + m * kPlaneRow], t1 = band_smem[T + m * kPlaneRow + planeT];
+    uint32_t d0[32], rows[16];
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
         const uint32_t x = __funnelshift_r(a0, e0, (uint32_t)j) ^ bit_mask(t0, j);
         const uint32_t eq = ~(x | (__funnelshift_r(a1, e1, (uint32_t)j) ^ bit_mask(t1, j)));
-        each(j, band_column(eq, vp, vn));
+        d0[j] = band_column(eq, vp, vn);
     }
+    transpose16(d0, first, rows);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) band_smem[out + 32 * r] = rows[r];
+    return make_uint2(vp, vn);
+}
+
+/* One copy of it, for blocks that are computed twice: with the forward pass
+ * inlined, texts of 200-300 bases take 8-10% longer.  The forward pass of
+ * texts that are stored whole is inlined: 5% less on 150 bases. */
+__device__ __noinline__ uint2 band_rows_call(int P, int planeP, int T, int planeT, int m, int b, uint32_t vp,
+                                             uint32_t vn, int first, int out)
+{
+    return band_rows(P, planeP, T, planeT, m, b, vp, vn, first, out);
 }
 
 /* A CIGAR of len bytes from the end of a column of backwards-written words
@@ -827,9 +847,8 @@ __device__ __forceinline__ void store_back_bytes(const uint32_t* col, int row, i
 }
 
 template <bool PREDICT>
-__global__ void __launch_bounds__(32, 9) band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw)
+__global__ void __launch_bounds__(32, 14) band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw, uint32_t words)
 {
-    extern __shared__ __align__(16) uint32_t band_smem[];
     const int lane = (int)(threadIdx.x & 31u);
     const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
     uint32_t* const work_next = A.chain.work_next ? A.chain.work_next + A.tier : nullptr;
@@ -866,47 +885,43 @@ __global__ void __launch_bounds__(32, 9) band_kernel(const __grid_constant__ Ali
         const int b = kBandDistance + min(0, kt) - (kBandDistance - wide) / 2;
         const int it = b - kt; /* the target's band bit */
         const int nb = max(1, (__reduce_max_sync(kFull, tlen) + 31) >> 5);
-        const bool stored = nb <= kBandBlocks; /* always, of a prefix */
-        const int capT = stored ? kBandBlocks : (int)nw, capP = capT + 1;
+        /* rows first .. first + 15 of the band, around both ends' diagonals, or
+         * the target's where they lie too far apart */
+        const bool apart = wide > 12;
+        int first = min(max((apart ? it : (b + it) >> 1) - 8, 0), 16);
+        /* blocks from `kept` on are stored */
+        const int room = (int)(words - band_fixed_words((uint32_t)nb));
+        const int kept = PREDICT ? nb : max(0, nb - room / (int)kBandBlockWords);
         uint32_t* const blocks = band_smem;
-        uint32_t* const ckpt = band_smem + (stored ? kBandCkpt : 1024) + lane;
-        uint32_t* const P0 = band_smem + (stored ? kBandPlanes : 1024 + 64 * (int)nw);
-        uint32_t* const T0p = P0 + 2 * kPlaneRow * capP;
-        uint32_t* const bytes = stored ? P0 : T0p + 2 * kPlaneRow * capT;
-        const int top = (int)band_byte_words(stored ? 32u * kBandBlocks : 32u * nw);
-        band_load(pr.p, lp, pr.t, lt, blocks, P0, capP, T0p, capT, lane);
-        const uint32_t* const P = P0 + lane;
-        const uint32_t* const T = T0p + lane;
-        const int planeP = kPlaneRow * capP, planeT = kPlaneRow * capT;
+        uint32_t* const ckpt = band_smem + room + lane;
+        uint32_t* const P0 = ckpt - lane + 64 * nb;
+        uint32_t* const T0p = P0 + 2 * kPlaneRow * (nb + 1);
+        uint32_t* const bytes = T0p + 2 * kPlaneRow * nb;
+        const int top = (int)band_byte_words((uint32_t)nb);
+        band_load(pr.p, lp, pr.t, lt, blocks, P0, nb + 1, T0p, nb, lane);
+        const int P = room + 64 * nb + lane, T = P + 2 * kPlaneRow * (nb + 1);
+        const int planeP = kPlaneRow * (nb + 1), planeT = kPlaneRow * nb;
 
         /* every column, and the distance: |kt| and the increments along the
          * target's diagonal */
         uint32_t vp = ~0u << b, vn = ~vp;
         int D = wide;
-        if (stored && !PREDICT) {
+        const auto forward = [&](const auto& block) {
 #pragma unroll 1
             for (int m = 0; m < nb; ++m) {
                 ckpt[64 * m] = vp;
                 ckpt[64 * m + 32] = vn;
-                uint32_t d0[32];
-                band_block(P, planeP, T, planeT, m, b, vp, vn, [&](int j, uint32_t d) { d0[j] = d; });
-                transpose32(d0);
-                uint32_t* out = blocks + 1024 * m + lane;
-#pragma unroll
-                for (int q = 0; q < 32; ++q) out[32 * q] = d0[q];
-                D += __popc(~out[32 * it] & low_bits(min(32, max(0, tlen - 32 * m))));
+                const int out = (int)kBandBlockWords * max(0, m - kept) + lane;
+                const uint2 v = block(m, out);
+                vp = v.x;
+                vn = v.y;
+                D += __popc(~blocks[out + 32 * (it - first)] & low_bits(min(32, max(0, tlen - 32 * m))));
             }
-        } else {
-#pragma unroll 1
-            for (int m = 0; m < nb; ++m) {
-                ckpt[64 * m] = vp;
-                ckpt[64 * m + 32] = vn;
-                uint32_t on = 0;
-                band_block(P, planeP, T, planeT, m, b, vp, vn,
-                           [&](int j, uint32_t d) { on = __funnelshift_r(on, d >> it, 1u); });
-                D += __popc(~on & low_bits(min(32, max(0, tlen - 32 * m))));
-            }
-        }
+        };
+        if (kept == 0)
+            forward([&](int m, int out) { return band_rows(P, planeP, T, planeT, m, b, vp, vn, first, out); });
+        else
+            forward([&](int m, int out) { return band_rows_call(P, planeP, T, planeT, m, b, vp, vn, first, out); });
         if constexpr (PREDICT) {
             if (item < count)
                 A.pred[pi] = (uint16_t)(state == ST_RUN ? min(D, kBandDistance + 1)
@@ -918,48 +933,59 @@ __global__ void __launch_bounds__(32, 9) band_kernel(const __grid_constant__ Ali
         if (state == ST_RUN)
             state = D > kBandDistance ? past : (A.max_distance > 0 && D > A.max_distance) ? ST_OVERMAX : ST_DONE;
 
-        __syncwarp(); /* the bytes may reuse the planes of other lanes */
-
         /* the walk back from the target (see walk_step) */
         BackBytes cg{bytes + lane, 0u, 0, top};
-        int m = tlen > 0 ? (tlen - 1) >> 5 : 0, hb = tlen - 32 * m, q = it, s = D, run = 0;
+        int m = 0, hb = 0, q = 0, s = 0, run = 0;
         bool walking = state == ST_DONE;
-        for (int blk = nb - 1; blk >= 0; --blk) {
-            const uint32_t* inc = blocks + lane;
-            if (!stored) {
-                vp = ckpt[64 * blk];
-                vn = ckpt[64 * blk + 32];
-                uint32_t d0[32];
-                band_block(P, planeP, T, planeT, blk, b, vp, vn, [&](int j, uint32_t d) { d0[j] = d; });
-                transpose32(d0);
-                uint32_t* out = blocks + lane;
-#pragma unroll
-                for (int r = 0; r < 32; ++r) out[32 * r] = d0[r];
+        const auto start = [&] {
+            m = tlen > 0 ? (tlen - 1) >> 5 : 0;
+            hb = tlen - 32 * m;
+            q = it;
+            s = D;
+            run = 0;
+            cg.acc = 0u;
+            cg.n = 0;
+        };
+        /* one step on rows first .. first + 15; false once they do not hold
+         * both neighbours (the band's own edges are not passed) */
+        const auto step = [&](const uint32_t* rows) {
+            const uint32_t* w = rows + 32 * (q - first);
+            const int best = walk_step(~w[0], q > first ? ~w[-32] : 0u, q < first + 15 ? ~w[32] : 0u, ckpt[64 * m],
+                                       ckpt[64 * m + 32], q, kBandDistance, hb);
+            if (best >= 0) {
+                const int op = best & 3, x = best >> 2;
+                cg.push_run(run + hb - x, 32);
+                cg.push((uint32_t)op_letter(op), 32);
+                run = 0;
+                hb = op == kOpDel ? x : x - 1;
+                q += op == kOpDel ? -1 : (op == kOpIns ? 1 : 0);
+                if (--s < 0) walking = false; /* never expected */
+            } else {
+                run += hb;
+                hb = 0;
+                if (m == 0) walking = false;
             }
-            while (walking && (stored || m == blk)) {
-                const uint32_t* w = inc + (stored ? 1024 * m : 0);
-                const int best = walk_step(~w[32 * q], ~w[32 * max(q - 1, 0)], ~w[32 * min(q + 1, kBandDistance)],
-                                           ckpt[64 * m], ckpt[64 * m + 32], q, kBandDistance, hb);
-                if (best >= 0) {
-                    const int op = best & 3, x = best >> 2;
-                    cg.push_run(run + hb - x, 32);
-                    cg.push((uint32_t)op_letter(op), 32);
-                    run = 0;
-                    hb = op == kOpDel ? x : x - 1;
-                    q += op == kOpDel ? -1 : (op == kOpIns ? 1 : 0);
-                    --s;
-                    if (s < 0) walking = false; /* never expected */
-                } else {
-                    run += hb;
-                    hb = 0;
-                    if (m == 0) walking = false;
-                }
-                if (hb == 0 && m > 0) {
-                    --m;
-                    hb = 32;
+            if (hb == 0 && m > 0) {
+                --m;
+                hb = 32;
+            }
+            return q >= (first > 0 ? first + 1 : 0) && q <= (first < 16 ? first + 14 : kBandDistance);
+        };
+        start();
+        bool inside = !apart;
+        while (walking && inside && m >= kept) inside = step(blocks + (int)kBandBlockWords * (m - kept) + lane);
+        if (walking && m >= kept) start(); /* left the stored rows */
+        if (__any_sync(kFull, walking)) {
+            const int most = __reduce_max_sync(kFull, walking ? m : 0);
+#pragma unroll 1
+            for (int blk = most; blk >= 0; --blk) {
+                while (walking && m == blk) {
+                    first = min(max(q - 8, 0), 16);
+                    band_rows_call(P, planeP, T, planeT, blk, b, ckpt[64 * blk], ckpt[64 * blk + 32], first, lane);
+                    inside = true;
+                    while (walking && inside && m == blk) inside = step(blocks + lane);
                 }
             }
-            if (stored) break;
         }
         if (state == ST_DONE) {
             if (s != 0 || q != b) {
@@ -2337,7 +2363,7 @@ cudaError_t launch_band(const AlignLaunch& a, int grid, cudaStream_t s)
     if (smem > 227u * 1024u) return cudaErrorInvalidValue;
     const cudaError_t e = allow_smem((const void*)band_kernel<false>, smem);
     if (e != cudaSuccess) return e;
-    band_kernel<false><<<grid, 32, smem, s>>>(a, std::max(1u, band_words(a.max_len)));
+    band_kernel<false><<<grid, 32, smem, s>>>(a, std::max(1u, band_words(a.max_len)), (uint32_t)(smem / 4u));
     return cudaGetLastError();
 }
 
@@ -2813,7 +2839,7 @@ cudaError_t launch_predict(const Layout& L, uint32_t n, uint32_t max_len, uint16
     a.pred = pred;
     a.tier = 0;
     grid = std::max(1, std::min(grid, (int)((n + 31u) / 32u)));
-    band_kernel<true><<<grid, 32, smem, s>>>(a, band_words((uint32_t)kPredictPrefix));
+    band_kernel<true><<<grid, 32, smem, s>>>(a, band_words((uint32_t)kPredictPrefix), (uint32_t)(smem / 4u));
     return cudaGetLastError();
 }
 
