@@ -2240,6 +2240,19 @@ __device__ __forceinline__ int order_bin(const AlignLaunch& A, uint32_t item, ui
     return kOrderBins - 1 - (int)((uint64_t)len * kOrderBins / ((uint64_t)A.max_len + 1u));
 }
 
+/* Adds the items of a CTA's share to bins, one atomic per bin and warp. */
+__device__ __forceinline__ void order_tally(const AlignLaunch& A, uint32_t count, uint32_t* bins)
+{
+    const int lane = (int)(threadIdx.x & 31u);
+    const uint32_t end = (count + 31u) & ~31u; /* whole warps iterate together */
+    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < end; i += gridDim.x * kOrderBins) {
+        uint32_t pi;
+        const int b = i < count ? order_bin(A, i, pi) : -1;
+        const unsigned same = __match_any_sync(kFull, b);
+        if (b >= 0 && lane == __ffs((int)same) - 1) atomicAdd(&bins[b], (uint32_t)__popc(same));
+    }
+}
+
 __global__ void __launch_bounds__(kOrderBins) order_count_kernel(const __grid_constant__ AlignLaunch A)
 {
     __shared__ uint32_t bins[kOrderBins];
@@ -2247,9 +2260,7 @@ __global__ void __launch_bounds__(kOrderBins) order_count_kernel(const __grid_co
     if (count < A.min_count) return;
     bins[threadIdx.x] = 0u;
     __syncthreads();
-    uint32_t pi;
-    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < count; i += gridDim.x * kOrderBins)
-        atomicAdd(&bins[order_bin(A, i, pi)], 1u);
+    order_tally(A, count, bins);
     __syncthreads();
     if (bins[threadIdx.x]) atomicAdd(A.chain.cls.order_count + threadIdx.x, bins[threadIdx.x]);
 }
@@ -2274,15 +2285,21 @@ __global__ void __launch_bounds__(kOrderBins) order_place_kernel(const __grid_co
     uint32_t before = 0;
     for (int w = 0; w < (t >> 5); ++w) before += sums[w];
     const uint32_t first = before + x - c;
-    uint32_t pi;
-    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < count; i += gridDim.x * kOrderBins)
-        atomicAdd(&mine[order_bin(A, i, pi)], 1u);
+    order_tally(A, count, mine);
     __syncthreads();
     start[t] = first + (mine[t] ? atomicAdd(A.chain.cls.order_next + t, mine[t]) : 0u);
     __syncthreads();
-    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < count; i += gridDim.x * kOrderBins) {
-        const int b = order_bin(A, i, pi);
-        A.chain.cls.order[atomicAdd(&start[b], 1u)] = pi;
+    /* neighbours of one bin stay neighbours, a warp at a time: their bytes lie together */
+    const uint32_t end = (count + 31u) & ~31u;
+    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < end; i += gridDim.x * kOrderBins) {
+        uint32_t pi = 0;
+        const int b = i < count ? order_bin(A, i, pi) : -1;
+        const unsigned same = __match_any_sync(kFull, b);
+        const int leader = __ffs((int)same) - 1;
+        uint32_t at = 0;
+        if (b >= 0 && lane == leader) at = atomicAdd(&start[b], (uint32_t)__popc(same));
+        at = __shfl_sync(kFull, at, leader) + (uint32_t)__popc(same & ((1u << lane) - 1u));
+        if (b >= 0) A.chain.cls.order[at] = pi;
     }
 }
 
@@ -2686,6 +2703,14 @@ TierShape bound_shape(uint32_t max_len, int sm_count)
     return sh;
 }
 
+cudaError_t launch_order(const AlignLaunch& a, cudaStream_t s)
+{
+    const int grid = (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 608u);
+    order_count_kernel<<<grid, kOrderBins, 0, s>>>(a);
+    order_place_kernel<<<grid, kOrderBins, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s, uint64_t* launches)
 {
     const TierShape& sh = a.chain.bound_shape;
@@ -2698,9 +2723,8 @@ cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s, uint64_t* launche
         w.bulk = 1;
         w.min_count = kScanMin;
         if (a.work_count || a.n_work >= kScanMin) {
-            const int og = (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 608u);
-            order_count_kernel<<<og, kOrderBins, 0, s>>>(w);
-            order_place_kernel<<<og, kOrderBins, 0, s>>>(w);
+            const cudaError_t e0 = launch_order(w, s);
+            if (e0 != cudaSuccess) return e0;
             w.work = a.chain.cls.order;
             *launches += 3;
             wide_kernel<2, true><<<std::max(1, std::min(scan.grid, (int)((a.n_work + 31u) / 32u))), 32, 0, s>>>(w);

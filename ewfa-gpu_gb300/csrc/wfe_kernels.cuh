@@ -193,6 +193,10 @@ size_t tier_scratch_bytes(int tier, int grid, uint32_t max_len);
 int tier_grid(int tier, uint32_t max_len, uint32_t cigar_stride, int sm_count);
 cudaError_t launch_tier(int tier, const AlignLaunch& a, int grid, cudaStream_t s);
 
+/* a's list (a.work / a.work_count / a.n_work) in order of length, longest
+ * first, to a.chain.cls.order (two kernels). */
+cudaError_t launch_order(const AlignLaunch& a, cudaStream_t s);
+
 /* Upper bounds on the distances of the pairs of a CTA-per-pair tier's work
  * list (a.work / a.work_count / a.n_work, sequences up to a.max_len) into
  * a.bound, one warp per pair; see bound_kernel.  With a.tier == 5 and
