@@ -101,6 +101,10 @@ struct BucketPlan {
     TierShape bound{};      /* the bound pass (grid 0: none) */
 };
 
+/* Running counters on the device: pairs handed on and launches per tier, pairs
+ * per bucket, pairs of planned launches per first tier. */
+constexpr size_t kDevCounters = 3 * kNumTiers + kMaxBuckets;
+
 struct wfe_ctx {
     wfe_config cfg{};
     int sm_count = 0;
@@ -134,6 +138,7 @@ struct wfe_ctx {
     unsigned long long* d_passed = nullptr;    /* pairs each tier handed on, running total */
     unsigned long long* d_launched = nullptr;  /* tier launches made on the device */
     unsigned long long* d_bucket_total = nullptr; /* pairs classified into each bucket */
+    unsigned long long* d_entered = nullptr;   /* pairs of planned launches by first tier */
     uint8_t* h_launch_error = nullptr;         /* byte t: a device-side launch of tier t failed */
     uint8_t* d_launch_error = nullptr;         /* its device address */
     bool launch_error_pinned = false;          /* from cudaHostAlloc (else new[]: pageable memory the
@@ -219,7 +224,7 @@ int default_first_tier(uint32_t max_len)
 /* per bucket: list counts (one more for the last tier's hand-on), finished
  * CTAs and work counters of every tier, then, for every class of tier 5,
  * front and back list counts, finished CTAs and work counters */
-constexpr size_t kChainWords = 3 * kNumTiers + 1 + 4 * (kLongClasses + 1) + 2 * kOrderBins;
+constexpr size_t kChainWords = 3 * kNumTiers + 1 + 4 * (kLongClasses + 1) + 2 * kOrderBins + kPlanSums;
 constexpr size_t kCountWords = kMaxBuckets * kChainWords;
 
 /* What a stage owns itself: its staging and scratch allocations, pinned
@@ -362,6 +367,8 @@ int chain_last(const wfe_ctx* ctx, int first, int last, bool* cut)
 constexpr uint32_t kOrderLength = 320;
 constexpr uint32_t kOrderPairs = 16384;
 
+constexpr int kPlanned = -1; /* first tier of a planned batch (see first_tier_of) */
+
 /* Launch the first tier of one bucket's chain over `work` (NULL: pairs
  * 0..n-1); the last CTA of every tier starts the next tier with work, on the
  * device.  `base` is the index of the batch's first pair in the call (the
@@ -372,7 +379,8 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
 {
     const wfe_config& c = ctx->cfg;
     const uint32_t B = c.batch_size;
-    const int t = first_tier;
+    const bool plan = first_tier == kPlanned; /* tier 0, 1 or 5, chosen on the device */
+    const int t = plan ? 5 : first_tier;
     uint32_t* words = st.d_counts + (size_t)bucket_index * kChainWords;
     uint32_t* lists = st.d_lists + (size_t)bucket_index * kListsPerBucket * B;
     AlignLaunch a{};
@@ -439,6 +447,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     a.chain.cls.order = lists + (size_t)(kNumTiers + kLongClasses) * B;
     a.chain.cls.order_count = cw + 4 * (kLongClasses + 1);
     a.chain.cls.order_next = a.chain.cls.order_count + kOrderBins;
+    const uint32_t* const choice = a.chain.cls.order_next + kOrderBins + kPlanSums - 1;
     int grid = bp.shape[t].grid;
     if (!listed) {
         const uint32_t per_cta = (uint32_t)tier_info(t).pairs_per_cta;
@@ -448,8 +457,15 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     int rc = WFE_OK;
     TimedLaunch* tl = begin_timing(ctx, t, s, &rc);
     if (rc != WFE_OK) return rc;
-    if (bounded && t == 5 && a.chain.cls.n > 0) {
-        /* tier 5 starts with the bound pass, which starts the classes */
+    if (plan) {
+        a.plan = choice;
+        a.plan_tiers = 1;
+        a.entered = ctx->d_entered;
+        WFE_CUDA(ctx, launch_planned(a, s));
+        ctx->stats.kernel_launches += 2; /* and what the plan chooses, counted on the device */
+    } else if (bounded && t == 5 && a.chain.cls.n > 0) {
+        /* tier 5 starts with the bound pass or the scan, which start the classes */
+        a.plan = choice;
         WFE_CUDA(ctx, launch_bound(a, s, &ctx->stats.kernel_launches));
     } else {
         /* bounds only, then tier 6 */
@@ -463,23 +479,27 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
         ctx->stats.kernel_launches++;
     }
     if (tl) WFE_CUDA(ctx, cudaEventRecord(tl->stop, s));
-    ctx->stats.tier_launches[t]++;
+    if (!plan) ctx->stats.tier_launches[t]++;
     return WFE_OK;
 }
 
-/* The tier a batch of n pairs starts at.  Sequences of more than
- * kScanLength bases start at tier 0 by default for the sake of small calls
- * and of contexts without tier 5's scratch; a large batch that can starts at
- * tier 5, whose scan costs twice tier 0's band and finds the class of the
- * pairs that tier 0 would hand on. */
-constexpr uint32_t kScanLength = 400;
-constexpr uint32_t kScanPairs = 8192;
-int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n)
+/* The tier a batch of n pairs starts at.  Where the choice is left to the
+ * length and that says tier 0, a small batch starts at tier 1: 32 lanes per
+ * pair need a few microseconds for a few scores where tier 0 needs the length
+ * of the sequences in columns (300 bases: 31 us against 61 for up to 4,096
+ * pairs, the same at 16,384; 150 bases: 34 and 37 at 1,024, 41 and 37 at
+ * 4,096).  A large batch of sequences past kPlanLength bases is planned
+ * (kPlanned): its error rate decides. */
+constexpr uint32_t kPlanLength = 400;
+int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n, bool device_call)
 {
-    const bool scan = bp.by_length && bp.max_len > kScanLength && n >= kScanPairs && ctx->deep_ready && ctx->bound &&
-                      bp.bound.grid > 0 && bp.cls.scan.grid > 0 &&
+    if (!bp.by_length || bp.first_tier != 0 || bp.shape[1].grid <= 0) return bp.first_tier;
+    if (n < 4096u) return n < 11u * bp.max_len - std::min(1200u, 11u * bp.max_len) ? 1 : 0;
+    if (!device_call) return 0;
+    const bool plan = bp.max_len > kPlanLength && ctx->deep_ready && ctx->bound && bp.bound.grid > 0 &&
+                      bp.cls.scan.grid > 0 &&
                       !(ctx->cfg.max_distance > 0 && ctx->cfg.max_distance <= tier_info(4).dcap);
-    return scan ? std::max(bp.first_tier, 5) : bp.first_tier;
+    return plan ? kPlanned : n < 32768u && bp.max_len > kOrderLength ? 1 : 0;
 }
 
 /* Enqueue the alignment of pairs 0..n-1 of one batch on stream s: with one
@@ -488,15 +508,16 @@ int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n)
  * shapes fit its longest sequence, and by predicted distance to a tier --
  * and every bucket's chain runs from its first tier. */
 int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dist, int8_t* cigar,
-              uint8_t* status, cudaStream_t s, const int* first_override = nullptr, uint32_t base = 0)
+              uint8_t* status, cudaStream_t s, const int* first_override = nullptr, uint32_t base = 0,
+              bool device_call = false)
 {
     if (n == 0) return WFE_OK;
     const uint32_t B = ctx->cfg.batch_size;
     WFE_CUDA(ctx, cudaMemsetAsync(st.d_counts, 0, sizeof(uint32_t) * kCountWords, s));
     if (ctx->nbuckets == 1 && !ctx->predict) {
         const BucketPlan& bp = ctx->bucket[0];
-        const int t = first_override ? first_override[0] : first_tier_of(ctx, bp, n);
-        ctx->single_entered[t] += n;
+        const int t = first_override ? first_override[0] : first_tier_of(ctx, bp, n, device_call);
+        if (t != kPlanned) ctx->single_entered[t] += n;
         return launch_bucket(ctx, st, bp, 0, t, L, false, n, dist, cigar, status, s, base);
     }
     Buckets bk{};
@@ -638,7 +659,7 @@ int create_context(const wfe_config* cfg, uint64_t budget5, uint64_t budget6, wf
         }
     }
     ctx->ops_scratch_bytes = scratch;
-    const size_t nctr = 2 * kNumTiers + kMaxBuckets;
+    const size_t nctr = kDevCounters;
     const size_t passed_at = arena.take(sizeof(unsigned long long) * nctr);
     const size_t B = c.batch_size;
     size_t lists_at[kStages], counts_at[kStages], pred_at[kStages], bound_at[kStages];
@@ -675,6 +696,7 @@ int create_context(const wfe_config* cfg, uint64_t budget5, uint64_t budget6, wf
 
     ctx->d_launched = ctx->d_passed + kNumTiers;
     ctx->d_bucket_total = ctx->d_passed + 2 * kNumTiers;
+    ctx->d_entered = ctx->d_bucket_total + kMaxBuckets;
     /* The record of failed device-side launches is host memory the kernels
      * write in place.  A device that reads the CPU's page tables (ATS over
      * NVLink-C2C) writes ordinary heap memory; elsewhere it is a mapped
@@ -820,13 +842,13 @@ int wfe_get_stats(wfe_ctx* ctx, wfe_stats* out)
         ctx->event_pool.push_back(t.stop);
     }
     ctx->timed.clear();
-    unsigned long long dev[2 * kNumTiers + kMaxBuckets] = {};
+    unsigned long long dev[kDevCounters] = {};
     WFE_CUDA(ctx, cudaMemcpy(dev, ctx->d_passed, sizeof(dev), cudaMemcpyDeviceToHost));
     *out = ctx->stats;
     out->deep_scratch_bytes = ctx->deep_bytes;
     for (int t = 0; t < kNumTiers; ++t) {
         out->tier_passed[t] = dev[t];
-        out->tier_entered[t] = ctx->single_entered[t] + (t > 0 ? dev[t - 1] : 0);
+        out->tier_entered[t] = ctx->single_entered[t] + (t > 0 ? dev[t - 1] : 0) + dev[2 * kNumTiers + kMaxBuckets + t];
         out->tier_launches[t] += dev[kNumTiers + t];
         out->kernel_launches += dev[kNumTiers + t];
     }
@@ -842,7 +864,7 @@ int wfe_reset_stats(wfe_ctx* ctx)
     if (r != WFE_OK) return r;
     ctx->stats = wfe_stats{};
     for (auto& x : ctx->single_entered) x = 0;
-    WFE_CUDA(ctx, cudaMemset(ctx->d_passed, 0, sizeof(unsigned long long) * (2 * kNumTiers + kMaxBuckets)));
+    WFE_CUDA(ctx, cudaMemset(ctx->d_passed, 0, sizeof(unsigned long long) * kDevCounters));
     return WFE_OK;
 }
 
@@ -891,7 +913,7 @@ int wfe_align_device(wfe_ctx* ctx, const char* d_ascii, const wfe_pair* d_pairs,
         L.pairs = d_pairs + b0;
         L.base_off = 0;
         rc = run_chain(ctx, ctx->st[si], L, nb, d_dist + b0, d_cigar ? d_cigar + b0 * ctx->cfg.cigar_stride : nullptr,
-                       d_status ? d_status + b0 : nullptr, si ? ctx->st[1].stream : s);
+                       d_status ? d_status + b0 : nullptr, si ? ctx->st[1].stream : s, nullptr, 0u, true);
         if (rc != WFE_OK) break;
         ctx->stats.batches++;
         ctx->stats.pairs += nb;
@@ -1609,7 +1631,7 @@ extern "C" int wfe_autotune(wfe_ctx* ctx, const char* d_ascii, const wfe_pair* d
     const wfe_stats saved = ctx->stats;
     uint64_t saved_entered[kNumTiers];
     std::copy(ctx->single_entered, ctx->single_entered + kNumTiers, saved_entered);
-    unsigned long long saved_dev[2 * kNumTiers + kMaxBuckets];
+    unsigned long long saved_dev[kDevCounters];
     if ((e = cudaMemcpy(saved_dev, ctx->d_passed, sizeof saved_dev, cudaMemcpyDeviceToHost)) != cudaSuccess) {
         cleanup();
         return fail_cuda(ctx, e);

@@ -174,9 +174,19 @@ __global__ void bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq
 template <int NW, bool SCAN>
 __global__ void wide_kernel(const __grid_constant__ AlignLaunch A);
 __global__ void tile_kernel(const __grid_constant__ AlignLaunch A);
+template <bool PREDICT>
+__global__ void band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw, uint32_t words);
 __device__ uint32_t tile_chunks(const LongClasses& C);
-/* The classes of a list that the bound pass routes, aligned by a CTA per pair. */
-__device__ __forceinline__ bool class_by_cta(int dlim) { return dlim == 257 || dlim == 577 || dlim == 961; }
+/* The classes of a list of `count` pairs that the bound pass routes, aligned
+ * by a CTA per pair.  With so few pairs that nearly every one has a CTA's slot
+ * at once, one launch after another costs more than CTAs that fit the
+ * distance give: the last class alone, or with the shortest (8 pairs of 4-6
+ * kb 0.70 -> 0.36 ms, 256 of 5-7 kb 1.41 -> 0.76 ms). */
+constexpr uint32_t kFewPairs = 384, kSomePairs = 1024;
+__device__ __forceinline__ bool class_by_cta(int dlim, uint32_t count)
+{
+    return count > kFewPairs && (dlim == 257 || (count > kSomePairs && (dlim == 577 || dlim == 961)));
+}
 __device__ __forceinline__ bool tile_takes(const LongClasses& C, int c, uint32_t count)
 {
     return c + 1 < C.n && C.tile.grid > 0 && count > 0u && !(C.wide[c].grid > 0 && count >= kWidePairs);
@@ -185,6 +195,44 @@ using T1 = Tier<32, 2, true, 1>;   /* distance <= 79  */
 using T2 = Tier<32, 4, false, 1>;  /* distance <= 143; backtrace store in global scratch: 8 CTAs per SM */
 using T3 = Tier<32, 8, false, 1>;  /* distance <= 271 */
 using T4 = Tier<32, 16, false, 1>; /* distance <= 527 */
+
+/* Which first kernel a list of `count` pairs takes, from the sums over a
+ * sample of it: pairs, bases (of the longer sequence), predicted distances D
+ * and their squares, and the bulk kernels' work.  Microseconds: the
+ * latency of one pair, or the time of all at the rate of a full GPU, measured
+ * on lists of 8 to 65,536 pairs of 150 to 9,000 bases at 1-20% edits.
+ *   one thread per pair in a 32-diagonal band (tier 0): columns
+ *   32 lanes per pair (tier 1, distances to 79): scores
+ *   a CTA per pair (bound pass and classes): scores, and cells of D^2
+ *   scan and bulk classes: columns times the band's words
+ * A list that the host knows to be short never gets here.  8.5 kb at 1.5%
+ * edits, 2,048 pairs: a CTA per pair 454 us, in bulk 1,631; 5-7 kb at 6-10%:
+ * 2,033 and 1,495; 600 bases at 6%, 4,096 pairs: tier 1 105, bulk 121, tier 0
+ * (and what follows it) 195. */
+__device__ __forceinline__ int plan_choice(const AlignLaunch& A, uint32_t count, const volatile float* sums)
+{
+    const float c = sums[0];
+    if (c <= 0.f) return kPlanCta;
+    const float n = (float)count * 1e-3f, len = sums[1] / c, d = sums[2] / c, dd = sums[3] / c, u = sums[4] / c;
+    const float cta = 60.f + fmaxf(d + 0.0045f * d * d, n * (3.2f + 0.0043f * len + 0.2145f * d + 0.0021f * dd));
+    const float bulk = 50.f + fmaxf(0.2f * len, n * u);
+    int best = bulk < cta ? kPlanBulk : kPlanCta;
+    if (A.plan_tiers) {
+        float t = fminf(bulk, cta);
+        const float reg = 30.f + fmaxf(0.5f * d, n * (0.3f + 0.0015f * len + 0.325f * d));
+        const float spread = 2.f * sqrtf(fmaxf(dd - d * d, d));
+        if (d + spread < 79.f && reg < t) {
+            best = kPlanRegister;
+            t = reg;
+        }
+        const float band = 28.f + fmaxf(0.1f * len, n * 0.0055f * len);
+        if (d + spread < 31.f && band < t) best = kPlanBand;
+    }
+    return best;
+}
+
+/* Whether the plan, if there is one, chose the scan. */
+__device__ __forceinline__ bool planned(const AlignLaunch& A) { return !A.plan || *A.plan == (uint32_t)kPlanBulk; }
 
 /* Record that the device-side launch of tier u failed: a plain store of one
  * byte (one per tier, so no two writers share a byte) into host memory that
@@ -210,14 +258,15 @@ __device__ __forceinline__ void note_deferred(const AlignLaunch& A)
 
 /* Tail launch of tier u over its list of `count` pairs, built in the launch's
  * own parameter buffer: A (a __grid_constant__ kernel parameter, read in
- * place) is copied word by word and the per-tier fields are patched.  No
+ * place) is copied word by word and the per-tier fields are patched
+ * (own_list: its work list stays A's).  No
  * copy of the launch record is made on the stack -- a kernel whose code
  * holds a large stack frame keeps only a few CTAs resident per SM, and that
  * limit is also what a grid launched from the device runs with. */
 template <typename K>
 __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int u, int grid, int threads,
                                             uint32_t smem, bool tier_args, uint32_t seq_words, uint32_t gbytes,
-                                            int bulk = 0)
+                                            int bulk = 0, bool own_list = false)
 {
     void* buf = cudaGetParameterBufferV2((void*)kernel, dim3((unsigned)grid), dim3((unsigned)threads), smem);
     if (!buf) {
@@ -232,10 +281,12 @@ __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int 
     AlignLaunch* n = static_cast<AlignLaunch*>(buf);
     n->tier = u;
     n->cls = -1;
-    n->min_count = n->max_count = 0u;
+    n->plan = nullptr;
     n->bulk = bulk;
-    n->work = A.chain.list[u];
-    n->work_count = A.chain.counts + u;
+    if (!own_list) {
+        n->work = A.chain.list[u];
+        n->work_count = A.chain.counts + u;
+    }
     n->retry = u < A.chain.last_tier ? A.chain.list[u + 1] : A.chain.defer;
     n->retry_count = u < A.chain.last_tier ? A.chain.counts + u + 1 : A.chain.defer_count;
     n->passed_total = A.chain.passed ? A.chain.passed + u : nullptr;
@@ -252,13 +303,22 @@ __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int 
 }
 
 template <class T>
-__device__ __forceinline__ void launch_on_device(const AlignLaunch& A, int u, uint32_t count)
+__device__ __forceinline__ void launch_on_device(const AlignLaunch& A, int u, uint32_t count, bool own_list = false)
 {
     const TierShape& sh = A.chain.shape[u];
     const uint32_t per_cta = (uint32_t)(kWarps * T::GPW);
     const int grid = max(1, min(sh.grid, (int)((count + per_cta - 1u) / per_cta)));
     static_assert(T::G == 32, "only the 32-lane tiers are launched from the device");
-    tail_launch(tier_kernel<T>, A, u, grid, kThreads, sh.smem, true, sh.seq_words, sh.gbytes);
+    tail_launch(tier_kernel<T>, A, u, grid, kThreads, sh.smem, true, sh.seq_words, sh.gbytes, 0, own_list);
+}
+
+/* Tail launch of the bound pass, tier 5's start, over `count` pairs. */
+__device__ __forceinline__ void launch_bound_on_device(const AlignLaunch& A, uint32_t count, bool own_list)
+{
+    const TierShape& b = A.chain.bound_shape;
+    const uint32_t per_cta = (uint32_t)b.threads / 32u;
+    const int grid = max(1, min(b.grid, (int)((count + per_cta - 1u) / per_cta)));
+    tail_launch(bound_kernel, A, 5, grid, b.threads, b.smem, true, b.seq_words, 0u, 0, own_list);
 }
 
 /* Tail launch of distance class c of tier 5 over its list of `count`
@@ -293,6 +353,7 @@ __device__ void launch_class_on_device(const AlignLaunch& A, int c, uint32_t cou
     const bool last = c + 1 >= C.n;
     n->tier = 5;
     n->cls = c;
+    n->plan = nullptr;
     n->work = C.list[c];
     n->work_count = C.counts + c;
     /* a class of the bulk kernels hands on to the last, which has no such limits */
@@ -323,10 +384,7 @@ __device__ void launch_tier_on_device(const AlignLaunch& A, int u, uint32_t coun
             tail_launch(wide_kernel<2, true>, A, u, max(1, min(A.chain.cls.scan.grid, (int)((count + 31u) / 32u))), 32,
                         0u, false, 0u, 0u, 1);
         } else if (A.bound && A.chain.cls.n > 0) {
-            const TierShape& b = A.chain.bound_shape;
-            const uint32_t per_cta = (uint32_t)b.threads / 32u;
-            const int grid = max(1, min(b.grid, (int)((count + per_cta - 1u) / per_cta)));
-            tail_launch(bound_kernel, A, u, grid, b.threads, b.smem, true, b.seq_words, 0u);
+            launch_bound_on_device(A, count, false);
         } else {
             const TierShape& sh = A.chain.shape[u];
             tail_launch(long_kernel<false, kLongThreads>, A, u, max(1, min(sh.grid, (int)count)), kLongThreads,
@@ -360,6 +418,7 @@ __device__ void launch_tile_on_device(const AlignLaunch& A, uint32_t chunks)
     AlignLaunch* n = static_cast<AlignLaunch*>(buf);
     n->tier = 5;
     n->cls = kTileClass;
+    n->plan = nullptr;
     n->retry = C.list[C.n - 1];
     n->retry_count = C.counts + C.n - 1;
     n->passed_total = nullptr;
@@ -847,7 +906,7 @@ __device__ __forceinline__ void store_back_bytes(const uint32_t* col, int row, i
 }
 
 template <bool PREDICT>
-__global__ void __launch_bounds__(32, 14) band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw, uint32_t words)
+__global__ void __maxnreg__(144) band_kernel(const __grid_constant__ AlignLaunch A, uint32_t nw, uint32_t words)
 {
     const int lane = (int)(threadIdx.x & 31u);
     const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
@@ -1479,7 +1538,7 @@ __device__ __forceinline__ void store_walked(const AlignLaunch& A, const uint32_
 }
 
 /* Routes a scanned pair by the bound on its distance, as the bound pass does. */
-__device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi, int bound, int need);
+__device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi, int bound, int need, uint32_t count);
 
 template <int NW, bool SCAN>
 __device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks)
@@ -1581,7 +1640,7 @@ __device__ __forceinline__ void wide_body(const AlignLaunch& A, uint32_t* blocks
             if (state == ST_DONE && 2 * __popc(done) < __popc(done | running)) state = ST_RUN;
             if (state == ST_RUN) {
                 A.bound[pi] = D;
-                route_by_bound(A, pi, D, A.max_distance > 0 ? min(D, A.max_distance) : D);
+                route_by_bound(A, pi, D, A.max_distance > 0 ? min(D, A.max_distance) : D, count);
             }
         }
 
@@ -1634,10 +1693,7 @@ template <int NW, bool SCAN>
 __global__ void __maxnreg__(NW <= 4 ? 96 : (NW <= 8 ? 128 : (NW <= 16 ? 168 : 255))) wide_kernel(const __grid_constant__ AlignLaunch A)
 {
     __shared__ uint32_t blocks[32 * kWalkRows];
-    if constexpr (SCAN) {
-        const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
-        if (count < A.min_count) return; /* the bound pass takes the list */
-    }
+    if (SCAN && !planned(A)) return;
     wide_body<NW, SCAN>(A, blocks);
 }
 
@@ -2114,7 +2170,7 @@ __device__ __forceinline__ int extend_words(const uint32_t* P, const uint32_t* T
  * and at least one zero word after them, rounded to 16 bytes */
 __host__ __device__ __forceinline__ uint32_t bound_words(uint32_t seq_words) { return (seq_words + 4u) & ~3u; }
 
-__device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi, int bound, int need)
+__device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi, int bound, int need, uint32_t count)
 {
     const LongClasses& C = A.chain.cls;
     const int top = C.shape[C.n - 1].dlim;
@@ -2125,8 +2181,8 @@ __device__ __forceinline__ void route_by_bound(const AlignLaunch& A, uint32_t pi
         return;
     }
     int c = 0, below = 0;
-    while (c + 1 < C.n && (C.shape[c].dlim < need || (!A.bulk && !class_by_cta(C.shape[c].dlim)))) {
-        if (class_by_cta(C.shape[c].dlim)) below = C.shape[c].dlim;
+    while (c + 1 < C.n && (C.shape[c].dlim < need || (!A.bulk && !class_by_cta(C.shape[c].dlim, count)))) {
+        if (class_by_cta(C.shape[c].dlim, count)) below = C.shape[c].dlim;
         ++c;
     }
     if (A.bulk || 2 * need >= below + C.shape[c].dlim)
@@ -2147,7 +2203,6 @@ __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_wo
     uint32_t* WP = reinterpret_cast<uint32_t*>(smem) + (size_t)warp * 2u * bw;
     uint32_t* WT = WP + bw;
     const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
-    if (A.max_count && count >= A.max_count) return; /* the scan has taken the list */
     for (uint32_t item = blockIdx.x * kW + (uint32_t)warp; item < count; item += gridDim.x * kW) {
         const uint32_t pi = A.work ? A.work[item] : item;
         const PairRef pr = get_pair(A.L, pi);
@@ -2205,7 +2260,7 @@ __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_wo
         if (lane == 0) {
             A.bound[pi] = bound;
             if (route) {
-                route_by_bound(A, pi, bound, need);
+                route_by_bound(A, pi, bound, need, count);
             }
         }
         __syncwarp();
@@ -2213,16 +2268,10 @@ __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_wo
     if (route) chain_next(A);
 }
 
-/* The bound pass in two forms with one body, as the tier kernels: launched
- * from the host with launch bounds for 6 resident CTAs per SM, and from the
- * device (a chain entering tier 5) without. */
-__global__ void __launch_bounds__(kLongThreads, 6)
-bound_kernel_host(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t /* unused */)
-{
-    bound_body(A, seq_words);
-}
-
-__global__ void bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t /* unused */)
+/* Launched from the host and from the device (a chain entering tier 5): a
+ * bound on the registers for 6 resident CTAs per SM, no launch bounds (see
+ * tier_kernel). */
+__global__ void __maxnreg__(40) bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_words, uint32_t /* unused */)
 {
     bound_body(A, seq_words);
 }
@@ -2230,8 +2279,8 @@ __global__ void bound_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq
 /* Tier 5's list in order of length, longest first (kOrderBins bins of equal
  * width), for the scan and the classes that it fills: the pairs of a warp then
  * end together, and the longest do not come last.  Two launches of a few
- * microseconds: the bins' counts, then every pair to its place.  With fewer
- * than A.min_count pairs both return at once. */
+ * microseconds: the bins' counts, then, unless the plan chooses a kernel that
+ * does not want the order, every pair to its place. */
 __device__ __forceinline__ int order_bin(const AlignLaunch& A, uint32_t item, uint32_t& pi)
 {
     pi = A.work ? A.work[item] : item;
@@ -2241,11 +2290,12 @@ __device__ __forceinline__ int order_bin(const AlignLaunch& A, uint32_t item, ui
 }
 
 /* Adds the items of a CTA's share to bins, one atomic per bin and warp. */
-__device__ __forceinline__ void order_tally(const AlignLaunch& A, uint32_t count, uint32_t* bins)
+__device__ __forceinline__ void order_tally(const AlignLaunch& A, uint32_t count, uint32_t* bins, uint32_t blk,
+                                            uint32_t blks)
 {
     const int lane = (int)(threadIdx.x & 31u);
     const uint32_t end = (count + 31u) & ~31u; /* whole warps iterate together */
-    for (uint32_t i = blockIdx.x * kOrderBins + threadIdx.x; i < end; i += gridDim.x * kOrderBins) {
+    for (uint32_t i = blk * kOrderBins + threadIdx.x; i < end; i += blks * kOrderBins) {
         uint32_t pi;
         const int b = i < count ? order_bin(A, i, pi) : -1;
         const unsigned same = __match_any_sync(kFull, b);
@@ -2253,23 +2303,138 @@ __device__ __forceinline__ void order_tally(const AlignLaunch& A, uint32_t count
     }
 }
 
-__global__ void __launch_bounds__(kOrderBins) order_count_kernel(const __grid_constant__ AlignLaunch A)
+/* The bins' counts, by CTA blk of `blks`. */
+__device__ __forceinline__ void order_count(const AlignLaunch& A, uint32_t count, uint32_t blk, uint32_t blks)
 {
     __shared__ uint32_t bins[kOrderBins];
-    const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
-    if (count < A.min_count) return;
     bins[threadIdx.x] = 0u;
     __syncthreads();
-    order_tally(A, count, bins);
+    order_tally(A, count, bins, blk, blks);
     __syncthreads();
     if (bins[threadIdx.x]) atomicAdd(A.chain.cls.order_count + threadIdx.x, bins[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(kOrderBins) order_count_kernel(const __grid_constant__ AlignLaunch A)
+{
+    order_count(A, A.work_count ? min(*A.work_count, A.n_work) : A.n_work, blockIdx.x, gridDim.x);
+}
+
+/* The first kernel of a list, from a sample of it (plan_choice), by the first
+ * kPlanCtas CTAs, one pair per thread: the distance of the first
+ * kPredictPrefix bases in a band of 32 diagonals, scaled to the length.  The
+ * other CTAs count the bins of the order that the scan wants, meanwhile.  The
+ * last of the first few starts what it chose, on the device, but for the
+ * scan, which follows in the stream, and whose launches see the choice in
+ * words[kPlanSums - 1].  (Batches of 20,000 pairs of 1,000 bases
+ * at 10%: 190 us each without a plan, 192 with it, and 211 with every kernel
+ * launched to see whether it is chosen.) */
+constexpr uint32_t kPlanCtas = kPlanSample / kOrderBins;
+__global__ void __launch_bounds__(kOrderBins) plan_kernel(const __grid_constant__ AlignLaunch A, uint32_t* words)
+{
+    const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
+    float* const sums = reinterpret_cast<float*>(words);
+    const auto choose = [&](int mode) {
+        words[kPlanSums - 1] = (uint32_t)mode;
+        if (A.plan_tiers) {
+            const int tier = mode == kPlanBand ? 0 : mode == kPlanRegister ? 1 : 5;
+            atomicAdd(A.entered + tier, (unsigned long long)count);
+            if (mode == kPlanBulk && A.chain.launched) atomicAdd(A.chain.launched + 5, 1ull);
+        }
+        if (mode == kPlanBand) {
+            const TierShape& b = A.chain.shape[0];
+            tail_launch(band_kernel<false>, A, 0, max(1, min(b.grid, (int)((count + 31u) / 32u))), 32, b.smem, true,
+                        b.seq_words, b.smem / 4u, 0, true);
+        } else if (mode == kPlanRegister) {
+            launch_on_device<T1>(A, 1, count, true);
+        } else if (mode == kPlanCta) {
+            launch_bound_on_device(A, count, true);
+        }
+    };
+    if (count < kScanMin) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) choose(kPlanCta);
+        return;
+    }
+    if (blockIdx.x >= kPlanCtas) {
+        order_count(A, count, blockIdx.x - kPlanCtas, gridDim.x - kPlanCtas);
+        return;
+    }
+    const uint32_t item = (uint32_t)((uint64_t)(blockIdx.x * kOrderBins + threadIdx.x) * count / kPlanSample);
+    const PairRef pr = get_pair(A.L, A.work ? A.work[item] : item);
+    float c = 0.f, len = 0.f, d = 0.f, u = 0.f;
+    if (pr.in_range && max(pr.plen, pr.tlen) <= A.max_len) {
+        constexpr int kWords = kPredictPrefix / 32;
+        const uint32_t lp = min(pr.plen, (uint32_t)kPredictPrefix), lt = min(pr.tlen, (uint32_t)kPredictPrefix);
+        uint32_t p0[kWords + 1], p1[kWords + 1], t0[kWords + 1], t1[kWords + 1];
+        const auto load = [](const char* s, uint32_t n, uint32_t(&lo)[kWords + 1], uint32_t(&hi)[kWords + 1]) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(s);
+            const uint32_t sh = (uint32_t)(a & 15u);
+            const uint4* base = reinterpret_cast<const uint4*>(a - sh);
+            const int nblk = n ? (int)((sh + n + 15u) >> 4) : 0;
+            uint32_t x[2 * kWords + 1];
+#pragma unroll
+            for (int i = 0; i <= 2 * kWords; ++i)
+                x[i] = planes16(i < nblk ? __ldg(base + i) : make_uint4(0u, 0u, 0u, 0u));
+#pragma unroll
+            for (int w = 0; w < kWords; ++w) planes32(x[2 * w], x[2 * w + 1], x[2 * w + 2], sh, lo[w], hi[w]);
+            lo[kWords] = hi[kWords] = 0u;
+        };
+        load(pr.p, lp, p0, p1);
+        load(pr.t, lt, t0, t1);
+        const int kt = (int)lt - (int)lp, wide = abs(kt);
+        int D = wide;
+        if (wide <= kBandDistance) {
+            const int b = kBandDistance + min(0, kt) - (kBandDistance - wide) / 2, it = b - kt;
+            uint32_t vp = ~0u << b, vn = ~vp, l0 = 0u, l1 = 0u;
+#pragma unroll 1
+            for (int m = 0; m < kWords; ++m) {
+                const uint32_t a0 = __funnelshift_l(l0, p0[0], (uint32_t)b), e0 = __funnelshift_l(p0[0], p0[1], (uint32_t)b);
+                const uint32_t a1 = __funnelshift_l(l1, p1[0], (uint32_t)b), e1 = __funnelshift_l(p1[0], p1[1], (uint32_t)b);
+                uint32_t on = 0;
+#pragma unroll 8
+                for (int j = 0; j < 32; ++j) {
+                    const uint32_t x = __funnelshift_r(a0, e0, (uint32_t)j) ^ bit_mask(t0[0], j);
+                    const uint32_t eq = ~(x | (__funnelshift_r(a1, e1, (uint32_t)j) ^ bit_mask(t1[0], j)));
+                    on = __funnelshift_r(on, band_column(eq, vp, vn) >> it, 1u);
+                }
+                D += __popc(~on & low_bits(min(32, max(0, (int)lt - 32 * m))));
+                l0 = p0[0];
+                l1 = p1[0];
+#pragma unroll
+                for (int i = 0; i < kWords; ++i) {
+                    p0[i] = p0[i + 1];
+                    p1[i] = p1[i + 1];
+                    t0[i] = t0[i + 1];
+                    t1[i] = t1[i + 1];
+                }
+            }
+        }
+        c = 1.f;
+        len = (float)max(pr.plen, pr.tlen);
+        d = fmaxf((float)D * fmaxf(1.f, len / (float)kPredictPrefix), fabsf((float)pr.tlen - (float)pr.plen));
+        /* nanoseconds: the scan, then its walk, or the class's band and walk */
+        u = len * (d <= 60.f ? 2.95f : 2.45f + 0.78f * (d / 32.f + 2.5f)) / 444.f;
+    }
+    float v[5] = {c, len, d, d * d, u};
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(kFull, v[i], o);
+        if ((threadIdx.x & 31u) == 0u) atomicAdd(sums + i, v[i]);
+    }
+    if ((threadIdx.x & 31u) == 0u) {
+        __threadfence();
+        if (atomicAdd(words + kPlanSums - 2, 1u) + 1u == kPlanSample / 32u) {
+            __threadfence();
+            choose(plan_choice(A, count, sums));
+        }
+    }
 }
 
 __global__ void __launch_bounds__(kOrderBins) order_place_kernel(const __grid_constant__ AlignLaunch A)
 {
     __shared__ uint32_t start[kOrderBins], mine[kOrderBins], sums[kOrderBins / 32];
     const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
-    if (count < A.min_count) return;
+    if (!planned(A)) return;
     const int t = (int)threadIdx.x, lane = t & 31;
     /* exclusive prefix of the bins */
     const uint32_t c = A.chain.cls.order_count[t];
@@ -2285,7 +2450,7 @@ __global__ void __launch_bounds__(kOrderBins) order_place_kernel(const __grid_co
     uint32_t before = 0;
     for (int w = 0; w < (t >> 5); ++w) before += sums[w];
     const uint32_t first = before + x - c;
-    order_tally(A, count, mine);
+    order_tally(A, count, mine, blockIdx.x, gridDim.x);
     __syncthreads();
     start[t] = first + (mine[t] ? atomicAdd(A.chain.cls.order_next + t, mine[t]) : 0u);
     __syncthreads();
@@ -2691,8 +2856,7 @@ TierShape bound_shape(uint32_t max_len, int sm_count)
     const size_t smem = (size_t)(kLongThreads / 32) * 2u * bound_words(sw) * sizeof(uint32_t);
     int nb = 0;
     if (smem <= 227u * 1024u && allow_smem((const void*)bound_kernel, smem) == cudaSuccess &&
-        allow_smem((const void*)bound_kernel_host, smem) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, bound_kernel_host, kLongThreads, smem) == cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, bound_kernel, kLongThreads, smem) == cudaSuccess) {
         sh.grid = std::max(1, nb) * sm_count;
         sh.smem = (uint32_t)smem;
         sh.seq_words = sw;
@@ -2703,11 +2867,26 @@ TierShape bound_shape(uint32_t max_len, int sm_count)
     return sh;
 }
 
+namespace {
+int order_grid(const AlignLaunch& a) { return (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 608u); }
+}  // namespace
+
 cudaError_t launch_order(const AlignLaunch& a, cudaStream_t s)
 {
-    const int grid = (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 608u);
-    order_count_kernel<<<grid, kOrderBins, 0, s>>>(a);
-    order_place_kernel<<<grid, kOrderBins, 0, s>>>(a);
+    order_count_kernel<<<order_grid(a), kOrderBins, 0, s>>>(a);
+    order_place_kernel<<<order_grid(a), kOrderBins, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_planned(const AlignLaunch& a, cudaStream_t s)
+{
+    if (a.chain.bound_shape.grid <= 0 || !a.bound || a.chain.cls.scan.grid <= 0) return cudaErrorInvalidValue;
+    plan_kernel<<<order_grid(a) + (int)kPlanCtas, kOrderBins, 0, s>>>(a, const_cast<uint32_t*>(a.plan) - (kPlanSums - 1));
+    AlignLaunch w = a;
+    w.bulk = 1;
+    order_place_kernel<<<order_grid(w), kOrderBins, 0, s>>>(w);
+    w.work = w.chain.cls.order;
+    wide_kernel<2, true><<<std::max(1, std::min(w.chain.cls.scan.grid, (int)((w.n_work + 31u) / 32u))), 32, 0, s>>>(w);
     return cudaGetLastError();
 }
 
@@ -2715,30 +2894,19 @@ cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s, uint64_t* launche
 {
     const TierShape& sh = a.chain.bound_shape;
     if (sh.grid <= 0 || !a.bound || sh.seq_words != seq_words_for(a.max_len)) return cudaErrorInvalidValue;
-    cudaError_t e = allow_smem((const void*)bound_kernel_host, sh.smem);
+    cudaError_t e = allow_smem((const void*)bound_kernel, sh.smem);
     if (e != cudaSuccess) return e;
-    const TierShape& scan = a.chain.cls.scan;
-    if (a.tier == 5 && a.chain.cls.n > 0 && scan.grid > 0) {
-        AlignLaunch w = a;
-        w.bulk = 1;
-        w.min_count = kScanMin;
-        if (a.work_count || a.n_work >= kScanMin) {
-            const cudaError_t e0 = launch_order(w, s);
-            if (e0 != cudaSuccess) return e0;
-            w.work = a.chain.cls.order;
-            *launches += 3;
-            wide_kernel<2, true><<<std::max(1, std::min(scan.grid, (int)((a.n_work + 31u) / 32u))), 32, 0, s>>>(w);
-            const cudaError_t e1 = cudaGetLastError();
-            if (e1 != cudaSuccess || !a.work_count) return e1;
-        }
+    if (a.tier == 5 && a.chain.cls.n > 0 && a.chain.cls.scan.grid > 0 && (a.work_count || a.n_work >= kScanMin)) {
+        *launches += 3;
+        return launch_planned(a, s);
     }
+    AlignLaunch w = a;
+    w.plan = nullptr;
     const uint32_t per_cta = (uint32_t)sh.threads / 32u;
     int grid = sh.grid;
     if (!a.work_count) grid = (int)std::min<uint64_t>((uint64_t)grid, ((uint64_t)a.n_work + per_cta - 1) / per_cta);
     ++*launches;
-    AlignLaunch w = a;
-    w.max_count = a.tier == 5 && a.chain.cls.n > 0 && scan.grid > 0 ? kScanMin : 0u;
-    bound_kernel_host<<<std::max(grid, 1), sh.threads, sh.smem, s>>>(w, sh.seq_words, 0u);
+    bound_kernel<<<std::max(grid, 1), sh.threads, sh.smem, s>>>(w, sh.seq_words, 0u);
     return cudaGetLastError();
 }
 

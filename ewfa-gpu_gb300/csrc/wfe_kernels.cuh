@@ -40,13 +40,12 @@ struct TierShape {
 };
 
 /* Distance classes of tier 5, by the upper bound on each pair's distance.
- * A list of at least kScanMin pairs is bounded by the scan (wide_kernel<2,
- * true>); the classes are then aligned by the tile kernel, in one launch,
+ * A list in bulk is bounded by the scan (wide_kernel<2, true>); the classes are then aligned by the tile kernel, in one launch,
  * except those with kWidePairs pairs or more, which one thread per pair takes
  * (wide_kernel), and the last, which holds what the others do not and whose
  * pairs get a CTA each (long_kernel).  The limits are those of 3, 4, 5, 6, 8,
  * 10, 16 and 32 lanes per pair: every number of pairs that a warp can hold,
- * but 7.  Shorter lists are bounded by the bound pass (bound_kernel), and
+ * but 7.  Other lists are bounded by the bound pass (bound_kernel), and
  * every pair gets a CTA, in the classes of class_by_cta: each of those is a
  * launch of its own with wavefront buffers (shared memory) and backtrace
  * slabs sized to its limit.  Classes up to 257 run CTAs of one warp, classes
@@ -56,9 +55,7 @@ struct TierShape {
  * past tier 5's own (min(max_len, 2047)) are dropped. */
 constexpr int kLongClasses = 9;
 constexpr int kLongClassLimit[kLongClasses - 1] = {127, 193, 257, 321, 449, 577, 961, 1985};
-/* Where the lines lie: the bulk kernels need about as long for one pair as
- * for thousands (a sequence's length of dependent columns), a CTA per pair
- * needs little for one pair and then as much again for every few hundred. */
+/* Pairs from which on tier 5 may begin with the scan (see plan_choice). */
 constexpr uint32_t kScanMin = 1024;
 constexpr uint32_t kWidePairs = 16384;
 constexpr int kLongTinyThreads = 32;
@@ -149,6 +146,11 @@ struct Buckets {
     unsigned long long* totals;      /* pairs classified into each bucket (stats) */
 };
 
+/* First kernels that a plan chooses between. */
+enum { kPlanBand = 0, kPlanRegister = 1, kPlanCta = 2, kPlanBulk = 3 };
+constexpr int kPlanSums = 8;       /* words of a plan: five sums, CTAs done, the choice last */
+constexpr uint32_t kPlanSample = 1024; /* pairs it samples */
+
 /* Arguments of one alignment launch over a work list. */
 struct AlignLaunch {
     Layout L;
@@ -175,8 +177,9 @@ struct AlignLaunch {
     size_t ops_scratch_bytes;
     int tier;                    /* this launch's tier */
     int bulk;                    /* tier 5 began with the scan: the classes' pairs are all at the fronts of their lists */
-    uint32_t min_count;          /* the scan of a list: does nothing with fewer pairs */
-    uint32_t max_count;          /* the bound pass: does nothing with as many (0: no limit) */
+    const uint32_t* plan;        /* the choice of launch_planned, the last of its kPlanSums words; NULL: none */
+    int plan_tiers;              /* the plan may choose tiers 0 and 1, too */
+    unsigned long long* entered; /* entered[t]: pairs of planned launches that began at tier t (stats) */
     Chain chain;                 /* chain.cta_done == NULL: no device-side chaining */
 };
 
@@ -197,14 +200,19 @@ cudaError_t launch_tier(int tier, const AlignLaunch& a, int grid, cudaStream_t s
  * first, to a.chain.cls.order (two kernels). */
 cudaError_t launch_order(const AlignLaunch& a, cudaStream_t s);
 
+/* Tier 5 (a.tier) over a's list, from a kernel chosen on the device from a
+ * sample of it: the scan and its classes, the bound pass and a CTA per pair,
+ * or (a.plan_tiers) tier 1 or tier 0 and what they hand on.  a.plan: the last
+ * of kPlanSums words, all zero before. */
+cudaError_t launch_planned(const AlignLaunch& a, cudaStream_t s);
+
 /* Upper bounds on the distances of the pairs of a CTA-per-pair tier's work
  * list (a.work / a.work_count / a.n_work, sequences up to a.max_len) into
  * a.bound, one warp per pair; see bound_kernel.  With a.tier == 5 and
  * classes (a.chain.cls.n > 0) the pass also routes every pair to its class
  * and its last CTA starts the first class that has work (tier 5 as a chain
- * of class launches); a list of kScanMin pairs and more is put in order of
- * length and scanned instead (see LongClasses; a list whose length only the
- * device knows gets the launches of both, and one of them returns at once).
+ * of class launches); a list that may hold kScanMin pairs goes to
+ * launch_planned.
  * bound_shape: the pass's launch shape (grid 0: its shared memory does not
  * fit, and no bound can be computed).  The kernels launched are added to
  * *launches. */

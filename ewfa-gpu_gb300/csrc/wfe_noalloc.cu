@@ -158,13 +158,15 @@ extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_p
      * more than about 9,000 bases do not fit there, and tier 3 aligns every
      * pair. */
     const wfe::TierShape sh0 = wfe::tier_shape(kFirstTier, max_len, cigar_stride, sms);
-    const bool first = sh0.grid > 0;
+    wfe::TierShape sh = wfe::tier_shape(kNoallocTier, max_len, cigar_stride, sms);
+    /* few pairs of sequences past 256 bases: tier 3 takes them in one wave, in
+     * less time than tier 0 needs for the length of the sequences in columns */
+    const bool first = sh0.grid > 0 && !(n <= 512u && max_len > 256u && sh.grid > 0);
     const bool deep = !first || max_distance > wfe::tier_info(kFirstTier).dcap;
     const bool listed = first && deep; /* tier 3 over the pairs tier 0 handed on */
 
     /* tier 3: occupancy, capped by the op-store slots of the array; every
      * group's store holds all rows of the tier (distances up to 271) */
-    wfe::TierShape sh = wfe::tier_shape(kNoallocTier, max_len, cigar_stride, sms);
     if (deep && sh.grid <= 0) return WFE_ERR_SEQ_TOO_LONG; /* sequences + CIGAR slot exceed shared memory */
     const size_t stores_at = listed ? kStoresAt : 0u;
     const uint32_t full_rows = (uint32_t)WFE_NOALLOC_MAX_DISTANCE;

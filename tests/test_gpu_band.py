@@ -61,6 +61,7 @@ def test_tier_0_band(cap, stride, spread):
                 q[key][i] = off
         ascii, pairs = buf, q
     with wfe.Context(max_seq_len=1000, cigar_stride=stride, max_distance=cap) as ctx:
+        ctx.set_policy([1000], [0])
         dist, cg, st = ctx.align(_pinned(ascii), _pinned(pairs))  # read where they lie
         assert ctx.stats()["tier_entered"][0] >= len(pairs)
     assert (dist == 31).any() and (dist == 32).any()
