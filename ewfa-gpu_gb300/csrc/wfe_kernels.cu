@@ -19,7 +19,7 @@
  *   tile_kernel          tier 5 in bulk, several lanes per pair
  *   order_*_kernel       tier 5's list in order of length
  *   classify_kernel      length buckets and predicted tiers
- *   history_cigar_kernel CIGARs from the reference's 128-bit histories
+ *   history_kernel       CIGARs from the reference's 128-bit histories
  *                        (src/kernels.cu:397-625)
  *
  * Wavefront layout of tier_kernel: lane g of a group holds, in register
@@ -713,10 +713,10 @@ __global__ void tier_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_
  * leaves those rows, are computed again from their checkpoints, with the rows
  * around the walk, when it reaches them. */
 constexpr int kSpanWords = 160; /* 16-byte blocks of a span: 8 pairs of 150 bases with their file's line marks */
-static_assert(kSpanWords * 16 <= 4096, "a span must fit in one 4 KiB page (see band_load)");
 constexpr int kPlaneRow = 33;
-constexpr int kSpanRow = kSpanWords + 4; /* a span's words, and those read past its last block */
-static_assert(4 * kSpanRow <= 1024, "the spans use the blocks' space");
+/* a span's words, and those read past its last block */
+__host__ __device__ constexpr int span_row(int span) { return span + 4; }
+static_assert(4 * span_row(kSpanWords) <= 1024, "the spans use the blocks' space");
 
 __host__ __device__ constexpr uint32_t band_words(uint32_t max_len) { return (max_len + 31u) / 32u; }
 /* words of a CIGAR of texts of n blocks: 31 operations, 32 runs, and a byte per 127 matches */
@@ -738,7 +738,7 @@ __host__ __device__ constexpr uint32_t band_smem_words(uint32_t max_len)
 }
 
 /* Bit planes of the warp's 32 pairs.  Eight neighbouring pairs that lie in
- * one span of kSpanWords blocks are read by all lanes in consecutive 16-byte
+ * one span of SPAN blocks are read by all lanes in consecutive 16-byte
  * blocks: whole 512-byte rows per instruction, which the CPU-GPU link serves
  * 20% faster than a short run per pair.  Blocks that fall in gaps between the
  * pairs are read too: a span is shorter than a 4 KiB page, so it lies within
@@ -747,9 +747,12 @@ __host__ __device__ constexpr uint32_t band_smem_words(uint32_t max_len)
  * by eight lanes each, 256 bases at a time, in blocks that hold a base.
  * Words past a sequence's end are not written: rows and columns past the
  * ends are never used.  A word w >= cap is dropped. */
+template <int SPAN>
 __device__ __forceinline__ void band_load(const char* p, uint32_t lp, const char* t, uint32_t lt, uint32_t* words,
                                           uint32_t* P0, int capP, uint32_t* T0, int capT, int lane)
 {
+    static_assert(SPAN * 16 <= 4096, "a span must fit in one 4 KiB page");
+    constexpr int kRow = span_row(SPAN);
     unsigned long long lo = ~0ull, hi = 0ull;
     if (lp) {
         lo = (unsigned long long)(uintptr_t)p;
@@ -766,9 +769,9 @@ __device__ __forceinline__ void band_load(const char* p, uint32_t lp, const char
     }
     lo &= ~15ull;
     const unsigned long long blocks = hi > lo ? (hi - lo + 15ull) >> 4 : 0ull;
-    const bool spans = blocks <= (unsigned long long)kSpanWords;
+    const bool spans = blocks <= (unsigned long long)SPAN;
     const int nblk = spans ? (int)blocks : 0;
-    constexpr int R = (kSpanWords + 31) / 32;
+    constexpr int R = (SPAN + 31) / 32;
 #pragma unroll
     for (int r = 0; r < 4; r += 2) {
         uint4 v[2][R];
@@ -785,11 +788,11 @@ __device__ __forceinline__ void band_load(const char* p, uint32_t lp, const char
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int i = 0; i < R; ++i) words[(r + h) * kSpanRow + lane + 32 * i] = planes16(v[h][i]);
+            for (int i = 0; i < R; ++i) words[(r + h) * kRow + lane + 32 * i] = planes16(v[h][i]);
     }
     __syncwarp();
     if (spans) {
-        const uint32_t* mine = words + (lane >> 3) * kSpanRow;
+        const uint32_t* mine = words + (lane >> 3) * kRow;
 #pragma unroll
         for (int which = 0; which < 2; ++which) {
             const uintptr_t a = reinterpret_cast<uintptr_t>(which ? t : p);
@@ -957,7 +960,7 @@ __global__ void __maxnreg__(144) band_kernel(const __grid_constant__ AlignLaunch
         uint32_t* const T0p = P0 + 2 * kPlaneRow * (nb + 1);
         uint32_t* const bytes = T0p + 2 * kPlaneRow * nb;
         const int top = (int)band_byte_words((uint32_t)nb);
-        band_load(pr.p, lp, pr.t, lt, blocks, P0, nb + 1, T0p, nb, lane);
+        band_load<kSpanWords>(pr.p, lp, pr.t, lt, blocks, P0, nb + 1, T0p, nb, lane);
         const int P = room + 64 * nb + lane, T = P + 2 * kPlaneRow * (nb + 1);
         const int planeP = kPlaneRow * (nb + 1), planeT = kPlaneRow * nb;
 
@@ -2675,59 +2678,122 @@ pack_kernel(Layout L, uint32_t n, uint32_t* out, uint32_t wps)
 }
 
 /* ------------------------------------------------------------------------ */
-/* CIGARs from 128-bit histories (src/kernels.cu:397-625): one group of 4
- * lanes per pair, 8 pairs per warp (a history holds at most 63 operations,
- * and 4 lanes extend 64 bases per trip). */
-constexpr int kHG = 4;
-
-__global__ void __launch_bounds__(kThreads)
-history_cigar_kernel(Layout L, uint32_t n, uint32_t max_len, const int32_t* dist,
-                     const uint64_t* hist, int8_t* cigar, uint32_t stride, uint8_t* status,
-                     uint32_t seq_words, uint32_t gbytes)
+/* CIGARs from 128-bit histories (src/kernels.cu:397-625): one pair per thread,
+ * both sequences of a warp's 32 pairs as bit planes in shared memory.  A step
+ * compares 32 bases, the next of them either after an operation or, if all
+ * match, right after these.  The bytes go to the slot word by word as they
+ * come.  Bound by the integer pipe (2,700 warp instructions for 32 pairs of
+ * 150 bases, two thirds of them the steps) and, with 1.7 waves of warps, by
+ * the latency of each wave's loads; warps of 64 registers, banks free of
+ * conflicts and CIGARs staged in shared memory all took the same time.  With
+ * a group of four lanes per pair before, 200,000 pairs of 150 bases at 5%
+ * took 78 us (now 25), of 250 bases at 10% 177 (73), 100,000 of 500 bases at
+ * 1% 140 (81), 20,000 of 2,000 bases 341 (103), 30 of 100 bases 11 (9). */
+constexpr int kWideSpanWords = 252; /* 16-byte blocks of a span: 8 pairs of 250 bases */
+__host__ __device__ constexpr uint32_t history_smem_words(uint32_t nw, int span)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int G = kHG, GPW = 32 / G;
-    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
-    const int g = lane & (G - 1), grp = lane / G;
-    const unsigned gmask = ((1u << G) - 1u) << (grp * G);
-    unsigned char* gs = smem + (size_t)(warp * GPW + grp) * gbytes;
-    uint2* QP = reinterpret_cast<uint2*>(gs);
-    uint2* QT = QP + seq_words;
-    uint8_t* chain = gs + 16u * (size_t)seq_words;
-    int* runs = reinterpret_cast<int*>(chain + 64);
-    int8_t* stage = reinterpret_cast<int8_t*>(chain + 64 + 256);
-    const uint32_t step = gridDim.x * (uint32_t)(kWarps * GPW);
-    for (uint32_t wb = (blockIdx.x * kWarps + (uint32_t)warp) * GPW; wb < n; wb += step) {
-        const uint32_t pi = wb + (uint32_t)grp;
-        if (pi >= n) continue; /* whole group leaves together */
-        const PairRef pr = get_pair(L, pi);
-        const int D = dist[pi];
-        const bool toolong = max(pr.plen, pr.tlen) > max_len || max(pr.plen, pr.tlen) > 16u * seq_words;
-        if (toolong || D < 0 || D > 63) {
-            if (g == 0) {
-                if (status)
-                    status[pi] = toolong ? (uint8_t)WFE_PAIR_TOO_LONG : (uint8_t)WFE_PAIR_OVER_MAX_DISTANCE;
-                if (stride) cigar[(size_t)pi * stride] = 0;
-            }
-            continue;
+    return 4u * kPlaneRow * (nw + 1u) + 4u * (uint32_t)span_row(span);
+}
+
+template <int SPAN>
+__global__ void __launch_bounds__(32)
+history_kernel(Layout L, uint32_t n, uint32_t max_len, const int32_t* dist, const uint64_t* hist, int8_t* cigar,
+               uint32_t stride, uint8_t* status, uint32_t nw)
+{
+    const int lane = (int)threadIdx.x;
+    const uint32_t pi = blockIdx.x * 32u + threadIdx.x;
+    const int plane = kPlaneRow * (int)(nw + 1u);
+    PairRef pr{};
+    uint64_t w0 = 0, w1 = 0;
+    int D = 0, state = ST_IDLE;
+    if (pi < n) {
+        pr = get_pair(L, pi);
+        D = dist[pi];
+        state = max(pr.plen, pr.tlen) > max_len ? ST_TOOLONG : D < 0 || D > 63 ? ST_OVERMAX : ST_RUN;
+        if (state == ST_RUN) {
+            /* no operations past the distance */
+            w0 = hist[2u * (size_t)pi] & (D < 32 ? (1ull << 2 * D) - 1ull : ~0ull);
+            w1 = D > 32 ? hist[2u * (size_t)pi + 1u] & ((1ull << 2 * (D - 32)) - 1ull) : 0ull;
         }
-        load_packed<G, (G == 4 ? 5 : 3)>(pr.p, pr.plen, QP, g, gmask);
-        load_packed<G, (G == 4 ? 5 : 3)>(pr.t, pr.tlen, QT, g, gmask);
-        const uint64_t w0 = hist[2u * pi], w1 = hist[2u * pi + 1u];
-        for (int d = g; d < D; d += G)
-            chain[d] = (uint8_t)(((d < 32 ? w0 : w1) >> (2 * (d & 31))) & 3u);
-        __syncwarp(gmask);
-        int len = replay_chain<G>(QP, QT, (int)pr.plen, (int)pr.tlen, chain, D, runs, stage, stride, g,
-                                  grp, gmask);
-        const bool bad = len < 0;
-        if (bad) len = -1 - len;
-        if (stride) store_cigar<G>(stage, (uint32_t)len, stride, cigar + (size_t)pi * stride, g, gmask);
-        if (g == 0 && status)
-            status[pi] = bad ? (uint8_t)WFE_PAIR_BAD_HISTORY
-                             : ((uint32_t)len > stride ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED
-                                                       : (uint8_t)WFE_PAIR_OK);
-        __syncwarp(gmask);
     }
+    const bool mine = state == ST_RUN;
+    const int plen = mine ? (int)pr.plen : 0, tlen = mine ? (int)pr.tlen : 0;
+    band_load<SPAN>(pr.p, (uint32_t)plen, pr.t, (uint32_t)tlen, band_smem + 4 * plane, band_smem,
+                    (int)nw + 1, band_smem + 2 * plane, (int)nw + 1, lane);
+    if (pi >= n) return;
+
+    const uint32_t* const P = band_smem + lane;
+    const uint32_t* const T = P + 2 * plane;
+    int8_t* const dst = cigar + (size_t)pi * stride;
+    const bool aligned = (stride & 3u) == 0u && (reinterpret_cast<uintptr_t>(cigar) & 3u) == 0u;
+    uint32_t len = 0;
+    uint64_t acc = 0; /* the len % 4 bytes that are not written yet */
+    /* bytes [len & ~3, end) of the slot */
+    const auto put = [&](uint32_t end) {
+        const uint32_t at = len & ~3u;
+        if (aligned) {
+            if (at < min(end, stride)) *reinterpret_cast<uint32_t*>(dst + at) = (uint32_t)acc;
+        } else {
+            for (uint32_t j = 0; j < 4u && at + j < min(end, stride); ++j) dst[at + j] = (int8_t)(acc >> (8u * j));
+        }
+    };
+    const auto push = [&](uint32_t two, uint32_t k) { /* up to two bytes */
+        acc |= (uint64_t)two << (8u * (len & 3u));
+        if ((len & 3u) + k >= 4u) {
+            put(len + 4u);
+            acc >>= 32;
+        }
+        len += k;
+    };
+    uint32_t o0 = (uint32_t)w0, o1 = (uint32_t)(w0 >> 32), o2 = (uint32_t)w1, o3 = (uint32_t)(w1 >> 32);
+    int v = 0, h = 0, d = 0;
+    uint32_t run = 0;
+    /* every lane goes through the whole of a step, whether its run of matches
+     * ends in it or not: the warp takes as many as its longest pair */
+    while (state == ST_RUN) {
+        const int rem = min(plen - v, tlen - h);
+        uint32_t x = 1u;
+        if (rem > 0) {
+            const uint32_t* p = P + kPlaneRow * (v >> 5);
+            const uint32_t* t = T + kPlaneRow * (h >> 5);
+            x = __funnelshift_r(p[0], p[kPlaneRow], (uint32_t)v) ^ __funnelshift_r(t[0], t[kPlaneRow], (uint32_t)h);
+            x |= __funnelshift_r(p[plane], p[plane + kPlaneRow], (uint32_t)v) ^
+                 __funnelshift_r(t[plane], t[plane + kPlaneRow], (uint32_t)h);
+            if (rem < 32) x |= 1u << rem;
+        }
+        const uint32_t k = x ? (uint32_t)__ffs((int)x) - 1u : 32u;
+        const bool ends = x != 0u;
+        run += k;
+        if (run >= 127u && ends)
+            for (; run >= 127u; run -= 127u) push(256u - 127u, 1u);
+        const uint32_t op = ends ? o0 & 3u : 0u;
+        const uint32_t letter = (0x44584900u >> (8u * op)) & 0xffu; /* I, X, D */
+        const uint32_t r = ends ? run : 0u;
+        push(r ? (256u - r) | letter << 8 : letter, (r ? 1u : 0u) + (op ? 1u : 0u));
+        v += (int)(k + (op >> 1));
+        h += (int)(k + ((op >> 1) ^ (op & 1u)));
+        if (ends) {
+            run = 0;
+            o0 = __funnelshift_r(o0, o1, 2u);
+            o1 = __funnelshift_r(o1, o2, 2u);
+            o2 = __funnelshift_r(o2, o3, 2u);
+            o3 >>= 2;
+            if (op == 0u) state = ST_DONE; /* the end, or a code that is no operation */
+            else ++d;
+        }
+    }
+    const bool bad = d < D;
+    if (stride && state == ST_DONE) {
+        if (len < stride || (len & 3u)) put(len + 1u); /* with the terminator, when it fits */
+    } else if (stride) {
+        dst[0] = 0;
+    }
+    if (status)
+        status[pi] = state == ST_TOOLONG   ? (uint8_t)WFE_PAIR_TOO_LONG
+                     : state == ST_OVERMAX ? (uint8_t)WFE_PAIR_OVER_MAX_DISTANCE
+                     : bad                 ? (uint8_t)WFE_PAIR_BAD_HISTORY
+                     : len > stride        ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED
+                                           : (uint8_t)WFE_PAIR_OK;
 }
 
 }  // namespace
@@ -3061,17 +3127,21 @@ cudaError_t launch_cigar_from_history(const Layout& L, uint32_t n, uint32_t max_
                                       uint32_t stride, uint8_t* status, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    const uint32_t sw = seq_words_for(max_len);
-    const size_t gb = 16u * (size_t)sw + 64u + 256u + round16(stride);
-    const size_t smem = gb * (size_t)(kWarps * (32 / kHG));
-    if (smem > 227u * 1024u) return cudaErrorInvalidValue;
-    cudaError_t e = allow_smem((const void*)history_cigar_kernel, smem);
-    if (e != cudaSuccess) return e;
-    const uint32_t per_cta = kWarps * (32 / kHG);
-    const uint32_t blocks = std::min<uint32_t>((n + per_cta - 1u) / per_cta, 1u << 20);
-    history_cigar_kernel<<<blocks, kThreads, smem, s>>>(L, n, max_len, dist, hist, cigar, stride, status,
-                                                        sw, (uint32_t)gb);
-    return cudaGetLastError();
+    /* long sequences and slots have always been refused together */
+    if (16u * (size_t)seq_words_for(max_len) + 320u + round16(stride) > 227u * 32u) return cudaErrorInvalidValue;
+    const uint32_t nw = std::max(1u, band_words(max_len));
+    const auto launch_as = [&](auto kernel, int span) {
+        const size_t smem = 4u * (size_t)history_smem_words(nw, span);
+        const cudaError_t e = allow_smem((const void*)kernel, smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<n / 32u + (n % 32u != 0u), 32, smem, s>>>(L, n, max_len, dist, hist, cigar, stride, status, nw);
+        return cudaGetLastError();
+    };
+    /* spans of 8 pairs that do not fit the narrower ones (250 bases: 40 us
+     * against 52; 150 bases: 29 against 25) */
+    const bool wide = max_len > (uint32_t)kSpanWords && max_len <= (uint32_t)kWideSpanWords;
+    return wide ? launch_as(history_kernel<kWideSpanWords>, kWideSpanWords)
+                : launch_as(history_kernel<kSpanWords>, kSpanWords);
 }
 
 }  // namespace wfe

@@ -102,3 +102,69 @@ def test_wide_bands(length, edits, n, cap):
         assert_same_cigars(cg[same], np.repeat(cg[first:first + 1], len(same), 0))
     first = np.array([np.flatnonzero(pick == i)[0] for i in range(len(pairs))])
     compare_with_oracle(ascii, pairs, 5000, dist[first], cg[first], st[first], max_distance=cap)
+
+
+def replayed(p, t, record, d, slot):
+    """The slot and status of a backtrace record, replayed base by base into `slot`."""
+    out, v, h, ok = [], 0, 0, True
+    for k in range(d + 1):
+        run = 0
+        while v < len(p) and h < len(t) and p[v] == t[h]:
+            v, h, run = v + 1, h + 1, run + 1
+        out += [256 - 127] * (run // 127) + ([256 - run % 127] if run % 127 else [])
+        op = int(record[k // 32]) >> 2 * (k % 32) & 3 if k < d else 0
+        if k < d and op == 0:
+            ok = False
+            break
+        if op:
+            out.append(b"?IXD"[op])
+            v, h = v + (op != 1), h + (op != 3)
+    body = np.array(out + [0] * (-len(out) % 4 or 4 if len(slot) % 4 == 0 else 1), np.uint8)[:len(slot)]
+    slot[:len(body)] = body.view(np.int8)
+    return wfe.PAIR_BAD_HISTORY if not ok else wfe.PAIR_CIGAR_TRUNCATED if len(out) > len(slot) else wfe.PAIR_OK
+
+
+@pytest.mark.parametrize("stride", [800, 801, 16, 0])
+def test_histories(stride):
+    """Backtrace records to CIGARs, with the narrow and the wide spans: the
+    aligner's own CIGARs from their operations, and the bytes and statuses of
+    records that no alignment leaves."""
+    torch = torch_cuda()
+    rng = np.random.default_rng(5)
+    seqs = band_pairs([0, 1, 15, 31, 32, 33, 64, 65, 127, 128, 129, 150, 254, 255, 300, 480, 512], [0, 1, 2, 9, 30, 60], 17)
+    seqs = [(p, t) for p, t in seqs if max(len(p), len(t)) <= 512]
+    ascii, pairs = wfe.pairs_from_list(seqs)
+    n = len(pairs)
+    with wfe.Context(max_seq_len=512, cigar_stride=800, max_distance=63) as ctx:
+        dist, cg, _ = ctx.align(ascii, pairs)
+    hist = np.zeros((n, 2), np.uint64)
+    for i in np.flatnonzero(dist < 64):
+        ops = [b"?IXD".index(c) for c in cg[i].tobytes()[:cg[i].tobytes().find(0)] if c < 128]
+        assert len(ops) == dist[i]
+        for d, op in enumerate(ops):
+            hist[i, d // 32] |= np.uint64(op << 2 * (d % 32))
+    ok = dist < 64
+    lone = np.arange(n) % 5 == 4  # codes of any kind, distances of any size
+    given, records = dist.copy(), hist.copy()
+    given[lone] = rng.integers(-1, 66, lone.sum())
+    records[lone] = rng.integers(0, 1 << 63, (lone.sum(), 2), dtype=np.uint64) | np.uint64(0x5555555555555555)
+    records[lone & (np.arange(n) % 10 == 9), 0] &= np.uint64(0xfffffffffff0ffff)
+    d_a, d_p = torch.from_numpy(ascii).cuda(), torch.from_numpy(pairs.view(np.uint8)).cuda()
+    d_d, d_h = torch.from_numpy(given).cuda(), torch.from_numpy(records.view(np.int64)).cuda()
+    want, want_st = np.full((n, stride), 7, np.int8), np.zeros(n, np.uint8)
+    for i, (p, t) in enumerate(seqs):
+        if 0 <= given[i] < 64:
+            want_st[i] = replayed(p, t, records[i], given[i], want[i])
+        else:
+            want[i, :1], want_st[i] = 0, wfe.PAIR_OVER_MAX_DISTANCE
+    assert (want_st[lone] == wfe.PAIR_BAD_HISTORY).any()
+    for max_len in (512, 200):
+        out, st = torch.full((n, max(stride, 1)), 7, dtype=torch.int8, device="cuda"), torch.zeros(n, dtype=torch.uint8, device="cuda")
+        wfe.cigar_from_history_device(d_a, d_p, n, max_len, d_d, d_h, out, stride, st, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        got, got_st = out.cpu().numpy()[:, :stride], st.cpu().numpy()
+        fits = np.maximum(pairs["p_len"], pairs["t_len"]) <= max_len
+        np.testing.assert_array_equal(got_st, np.where(fits, want_st, wfe.PAIR_TOO_LONG))
+        np.testing.assert_array_equal(got[fits], want[fits])
+        if stride == 800:
+            assert_same_cigars(got, cg, np.flatnonzero(ok & ~lone & fits))
