@@ -2683,9 +2683,11 @@ pack_kernel(Layout L, uint32_t n, uint32_t* out, uint32_t wps)
  * compares 32 bases, the next of them either after an operation or, if all
  * match, right after these.  The bytes go to the slot word by word as they
  * come.  Bound by the integer pipe (2,700 warp instructions for 32 pairs of
- * 150 bases, two thirds of them the steps) and, with 1.7 waves of warps, by
- * the latency of each wave's loads; warps of 64 registers, banks free of
- * conflicts and CIGARs staged in shared memory all took the same time.  With
+ * 150 bases, two thirds of them the steps) and, with 1.3 waves of warps, by
+ * the latency of each wave's loads: with 80 registers, 24 warps an SM instead
+ * of 32, 200,000 pairs whose inputs are not in L2 took 35 us instead of 33;
+ * banks free of conflicts, CIGARs staged in shared memory and larger CTAs gave
+ * nothing.  With
  * a group of four lanes per pair before, 200,000 pairs of 150 bases at 5%
  * took 78 us (now 25), of 250 bases at 10% 177 (73), 100,000 of 500 bases at
  * 1% 140 (81), 20,000 of 2,000 bases 341 (103), 30 of 100 bases 11 (9). */
@@ -2696,7 +2698,7 @@ __host__ __device__ constexpr uint32_t history_smem_words(uint32_t nw, int span)
 }
 
 template <int SPAN>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(32, 32)
 history_kernel(Layout L, uint32_t n, uint32_t max_len, const int32_t* dist, const uint64_t* hist, int8_t* cigar,
                uint32_t stride, uint8_t* status, uint32_t nw)
 {
