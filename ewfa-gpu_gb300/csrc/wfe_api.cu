@@ -51,7 +51,8 @@ struct Stage {
     uint8_t* d_status = nullptr;
     /* in the context's arena: */
     uint32_t* d_lists = nullptr;  /* a work list of batch_size entries per bucket and tier */
-    uint32_t* d_counts = nullptr; /* per bucket: list counts, finished CTAs, work counters */
+    uint32_t* d_counts = nullptr; /* per bucket: list counts, finished CTAs, work counters; zero between batches */
+    bool counts_dirty = false;    /* unless the launches of a batch failed */
     uint16_t* d_pred = nullptr;   /* predicted prefix distances */
     int32_t* d_bound = nullptr;   /* distance bounds of the pairs of the CTA-per-pair tiers */
     char* h_stage = nullptr;      /* pinned gather buffer for scattered inputs */
@@ -223,8 +224,9 @@ int default_first_tier(uint32_t max_len)
  * tier */
 /* per bucket: list counts (one more for the last tier's hand-on), finished
  * CTAs and work counters of every tier, then, for every class of tier 5,
- * front and back list counts, finished CTAs and work counters */
-constexpr size_t kChainWords = 3 * kNumTiers + 1 + 4 * (kLongClasses + 1) + 2 * kOrderBins + kPlanSums;
+ * front and back list counts, finished CTAs and work counters, then the bins
+ * of an order by length and the words of a plan */
+constexpr size_t kChainWords = kTierWords + kClassWords + 2 * kOrderBins + kPlanSums;
 constexpr size_t kCountWords = kMaxBuckets * kChainWords;
 
 /* What a stage owns itself: its staging and scratch allocations, pinned
@@ -372,10 +374,11 @@ constexpr int kPlanned = -1; /* first tier of a planned batch (see first_tier_of
 /* Launch the first tier of one bucket's chain over `work` (NULL: pairs
  * 0..n-1); the last CTA of every tier starts the next tier with work, on the
  * device.  `base` is the index of the batch's first pair in the call (the
- * deferred pairs of a chain cut short are recorded by it). */
+ * deferred pairs of a chain cut short are recorded by it).  *cleared: the
+ * chain itself leaves the bucket's counters zero. */
 int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_index, int first_tier,
                   const Layout& L, bool listed, uint32_t n, int32_t* dist, int8_t* cigar, uint8_t* status,
-                  cudaStream_t s, uint32_t base)
+                  cudaStream_t s, uint32_t base, bool* cleared)
 {
     const wfe_config& c = ctx->cfg;
     const uint32_t B = c.batch_size;
@@ -427,7 +430,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
      * handed on -- go through the bound pass, which routes them into the
      * classes. */
     const bool bounded = ctx->bound && st.d_bound && bp.bound.grid > 0 && last >= 5;
-    uint32_t* const cw = words + 3 * kNumTiers + 1;
+    uint32_t* const cw = words + kTierWords;
     if (bounded) {
         a.bound = st.d_bound;
         a.chain.bound_shape = bp.bound;
@@ -445,7 +448,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
         a.chain.cls.work_next = cw + 3 * (kLongClasses + 1);
     }
     a.chain.cls.order = lists + (size_t)(kNumTiers + kLongClasses) * B;
-    a.chain.cls.order_count = cw + 4 * (kLongClasses + 1);
+    a.chain.cls.order_count = cw + kClassWords;
     a.chain.cls.order_next = a.chain.cls.order_count + kOrderBins;
     const uint32_t* const choice = a.chain.cls.order_next + kOrderBins + kPlanSums - 1;
     int grid = bp.shape[t].grid;
@@ -454,6 +457,14 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
         grid = (int)std::min<uint64_t>((uint64_t)grid, ((uint64_t)n + per_cta - 1) / per_cta);
     }
     grid = std::max(grid, 1);
+    /* a batch by one chain without an order by length or a plan, as small ones
+     * are: what would be a memset before it is a few stores at its end (64
+     * pairs of 100-200 bases 13.4 -> 12.5 us each in a row, 36.5 -> 33.7
+     * alone) */
+    const bool classes = bounded && t == 5 && a.chain.cls.n > 0;
+    const bool ordered = t == 0 && !listed && L.ascii_bytes == 0 && bp.max_len > kOrderLength && n >= kOrderPairs;
+    *cleared = !listed && !ordered && !plan && !(classes && n >= kScanMin);
+    a.chain.clear = *cleared;
     int rc = WFE_OK;
     TimedLaunch* tl = begin_timing(ctx, t, s, &rc);
     if (rc != WFE_OK) return rc;
@@ -463,14 +474,14 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
         a.entered = ctx->d_entered;
         WFE_CUDA(ctx, launch_planned(a, s));
         ctx->stats.kernel_launches += 2; /* and what the plan chooses, counted on the device */
-    } else if (bounded && t == 5 && a.chain.cls.n > 0) {
+    } else if (classes) {
         /* tier 5 starts with the bound pass or the scan, which start the classes */
         a.plan = choice;
         WFE_CUDA(ctx, launch_bound(a, s, &ctx->stats.kernel_launches));
     } else {
         /* bounds only, then tier 6 */
         if (bounded && t == 6) WFE_CUDA(ctx, launch_bound(a, s, &ctx->stats.kernel_launches));
-        if (t == 0 && !listed && L.ascii_bytes == 0 && bp.max_len > kOrderLength && n >= kOrderPairs) {
+        if (ordered) {
             WFE_CUDA(ctx, launch_order(a, s));
             ctx->stats.kernel_launches += 2;
             a.work = a.chain.cls.order;
@@ -513,12 +524,23 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
 {
     if (n == 0) return WFE_OK;
     const uint32_t B = ctx->cfg.batch_size;
-    WFE_CUDA(ctx, cudaMemsetAsync(st.d_counts, 0, sizeof(uint32_t) * kCountWords, s));
+    const auto clear_counts = [&] { return cudaMemsetAsync(st.d_counts, 0, sizeof(uint32_t) * kCountWords, s); };
+    if (st.counts_dirty) WFE_CUDA(ctx, clear_counts());
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (st.counts_dirty) WFE_CUDA(ctx, cudaStreamIsCapturing(s, &capture));
+    /* until all is enqueued; a memset that was only captured has not run */
+    const bool still_dirty = capture != cudaStreamCaptureStatusNone;
+    st.counts_dirty = true;
+    bool cleared = false;
     if (ctx->nbuckets == 1 && !ctx->predict) {
         const BucketPlan& bp = ctx->bucket[0];
         const int t = first_override ? first_override[0] : first_tier_of(ctx, bp, n, device_call);
         if (t != kPlanned) ctx->single_entered[t] += n;
-        return launch_bucket(ctx, st, bp, 0, t, L, false, n, dist, cigar, status, s, base);
+        const int r = launch_bucket(ctx, st, bp, 0, t, L, false, n, dist, cigar, status, s, base, &cleared);
+        if (r != WFE_OK) return r;
+        if (!cleared) WFE_CUDA(ctx, clear_counts());
+        st.counts_dirty = still_dirty;
+        return WFE_OK;
     }
     Buckets bk{};
     bk.n = ctx->nbuckets;
@@ -558,9 +580,12 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     for (int b = ctx->nbuckets - 1; b >= 0; --b) {
         if (merge && b + 1 < ctx->nbuckets && bk.first_tier[b] == 5) continue;
         const int r =
-            launch_bucket(ctx, st, ctx->bucket[b], b, bk.first_tier[b], L, true, n, dist, cigar, status, s, base);
+            launch_bucket(ctx, st, ctx->bucket[b], b, bk.first_tier[b], L, true, n, dist, cigar, status, s, base,
+                          &cleared);
         if (r != WFE_OK) return r;
     }
+    WFE_CUDA(ctx, clear_counts());
+    st.counts_dirty = still_dirty;
     return WFE_OK;
 }
 
@@ -659,21 +684,22 @@ int create_context(const wfe_config* cfg, uint64_t budget5, uint64_t budget6, wf
         }
     }
     ctx->ops_scratch_bytes = scratch;
-    const size_t nctr = kDevCounters;
-    const size_t passed_at = arena.take(sizeof(unsigned long long) * nctr);
     const size_t B = c.batch_size;
     size_t lists_at[kStages], counts_at[kStages], pred_at[kStages], bound_at[kStages];
+    /* the counters, all zero at first */
+    const size_t passed_at = arena.take(sizeof(unsigned long long) * kDevCounters);
+    const size_t defer_count_at = arena.take(sizeof(uint32_t));
+    for (size_t& at : counts_at) at = arena.take(sizeof(uint32_t) * kCountWords);
+    const size_t zero_bytes = arena.used - passed_at;
     for (int i = 0; i < kStages; ++i) {
         /* a work list per tier of one length bucket; wfe_set_policy adds
          * room for more buckets */
         lists_at[i] = arena.take((size_t)kListsPerBucket * B * sizeof(uint32_t));
-        counts_at[i] = arena.take(sizeof(uint32_t) * kCountWords);
         pred_at[i] = arena.take(B * sizeof(uint16_t));
         bound_at[i] = arena.take(B * sizeof(int32_t));
     }
     /* pairs deferred by host calls that run before tiers 2-6 have scratch */
     const size_t defer_at = arena.take(B * sizeof(uint32_t));
-    const size_t defer_count_at = arena.take(sizeof(uint32_t));
     if ((e = cudaMalloc(&ctx->d_arena, arena.used)) != cudaSuccess) return bail(e);
     unsigned char* A0 = ctx->d_arena;
     ctx->d_defer = reinterpret_cast<uint32_t*>(A0 + defer_at);
@@ -722,10 +748,7 @@ int create_context(const wfe_config* cfg, uint64_t budget5, uint64_t budget6, wf
         if (host_calls) s.ascii_cap = B * 2u * (size_t)c.max_seq_len + 64u;
     }
     /* the counters start at zero; both stages' streams come after this */
-    if ((e = cudaMemsetAsync(ctx->d_passed, 0, sizeof(unsigned long long) * nctr, ctx->st[0].stream)) != cudaSuccess)
-        return bail(e);
-    if ((e = cudaMemsetAsync(ctx->d_defer_count, 0, sizeof(uint32_t), ctx->st[0].stream)) != cudaSuccess)
-        return bail(e);
+    if ((e = cudaMemsetAsync(ctx->d_passed, 0, zero_bytes, ctx->st[0].stream)) != cudaSuccess) return bail(e);
     if ((e = cudaStreamSynchronize(ctx->st[0].stream)) != cudaSuccess) return bail(e);
     if ((c.flags & WFE_FLAG_DEVICE_ONLY) || ctx->bucket[0].first_tier > kShallowLastTier)
         if (ensure_deep(ctx) != WFE_OK) return bail((cudaError_t)ctx->last_cuda_error);

@@ -234,11 +234,23 @@ __device__ __forceinline__ int plan_choice(const AlignLaunch& A, uint32_t count,
 /* Whether the plan, if there is one, chose the scan. */
 __device__ __forceinline__ bool planned(const AlignLaunch& A) { return !A.plan || *A.plan == (uint32_t)kPlanBulk; }
 
+/* The end of a chain: its counters are zero again for the stage's next batch
+ * (Chain::clear).  By the last CTA of its last kernel: nothing reads them any
+ * more. */
+__device__ __forceinline__ void end_chain(const AlignLaunch& A)
+{
+    if (!A.chain.clear) return;
+    for (int i = 0; i < kTierWords; ++i) A.chain.counts[i] = 0u;
+    if (A.tier >= 5 && A.chain.cls.n > 0)
+        for (int i = 0; i < kClassWords; ++i) A.chain.cls.counts[i] = 0u;
+}
+
 /* Record that the device-side launch of tier u failed: a plain store of one
  * byte (one per tier, so no two writers share a byte) into host memory that
- * the host reads once the chain has completed. */
+ * the host reads once the chain has completed.  The chain ends here. */
 __device__ __forceinline__ void note_launch_error(const AlignLaunch& A, int u)
 {
+    end_chain(A);
     if (A.chain.launch_error) {
         *reinterpret_cast<volatile uint8_t*>(A.chain.launch_error + u) = 1u;
         __threadfence_system();
@@ -460,6 +472,7 @@ __device__ void launch_next(const AlignLaunch& A)
             return;
         }
     }
+    end_chain(A);
 }
 
 /* End of a chained kernel: the last CTA to finish starts the next launch. */

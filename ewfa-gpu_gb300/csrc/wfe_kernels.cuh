@@ -66,6 +66,7 @@ constexpr int kTileClass = kLongClasses; /* AlignLaunch::cls of the tile kernel 
 /* Work lists of one length bucket: one per tier, then one per class. */
 constexpr int kListsPerBucket = kNumTiers + kLongClasses + 1; /* the last: tier 5's list in order of length */
 constexpr int kOrderBins = 256;
+constexpr int kClassWords = 4 * (kLongClasses + 1); /* counts, low_counts, cta_done, work_next */
 
 struct LongClasses {
     int n;                           /* classes (0: tier 5 runs as one launch over its list) */
@@ -99,8 +100,11 @@ uint64_t long_slab_bytes(int dlim, bool global_wavefront);
  * handed on.  Each tier kernel's last CTA launches, as a tail launch, the
  * next tier whose list is not empty, so no launch is made for a tier that
  * has no work. */
+constexpr int kTierWords = 3 * kNumTiers + 1; /* counts (one more: the last tier's hand-on), cta_done, work_next */
 struct Chain {
     int last_tier;                   /* last tier of the chain */
+    int clear;                       /* the chain zeroes its counters at its end: the kTierWords from counts on
+                                        and the kClassWords from cls.counts on */
     TierShape shape[kNumTiers];
     uint32_t* list[kNumTiers];       /* list[t]: work of tier t */
     uint32_t* counts;                /* counts[t]: pairs in list[t] */

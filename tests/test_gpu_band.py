@@ -168,3 +168,44 @@ def test_histories(stride):
         np.testing.assert_array_equal(got[fits], want[fits])
         if stride == 800:
             assert_same_cigars(got, cg, np.flatnonzero(ok & ~lone & fits))
+
+
+def test_counters_between_batches():
+    """Batches of every kind on one context, a captured one replayed between
+    them: each finds the counters of its chain zero."""
+    torch = torch_cuda()
+    sets = []
+    for n, lo, hi, p in [(64, 90, 150, .05), (5000, 300, 400, .3), (3000, 700, 900, .2), (20000, 500, 900, .1), (40, 800, 900, .3)]:
+        ascii, pairs = wfe.generate(n, lo, hi, p_min=.01, p_max=p, seed=n)
+        out = tuple(torch.zeros(s, dtype=t, device="cuda") for s, t in
+                    ((n, torch.int32), ((n, 1200), torch.int8), (n, torch.uint8)))
+        sets.append((n, ascii, pairs, torch.from_numpy(ascii).cuda(), torch.from_numpy(pairs.view(np.uint8)).cuda(), out))
+    with wfe.Context(max_seq_len=1200, cigar_stride=1200, batch_size=20000, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        stream = torch.cuda.Stream()
+
+        def run(k):
+            n, _, _, a, p, out = sets[k]
+            ctx.align_device(a, p, n, 1200, *out, stream)
+
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            run(0)
+            stream.synchronize()
+            with torch.cuda.graph(graph, stream=stream):
+                run(0)
+        for policy in (None, ([400, 1200], [0, 5]), ([1200], [5]), ([1200], [0])):
+            if policy:
+                ctx.set_policy(*policy)
+            for k in (4, 0, 3, 2, 1, 2, 3, 4, 0):
+                for d in sets[k][5] + sets[0][5]:
+                    d.zero_()
+                torch.cuda.synchronize()
+                run(k)
+                with torch.cuda.stream(stream):
+                    graph.replay()
+                stream.synchronize()
+                for j in (k, 0):
+                    dist, cg, st = (x.cpu().numpy() for x in sets[j][5])
+                    some = slice(None, None, 1 + sets[j][0] // 300)
+                    compare_with_oracle(sets[j][1], sets[j][2][some], 1200, dist[some], cg[some], st[some])
+                    assert (st == wfe.PAIR_OK).all()
