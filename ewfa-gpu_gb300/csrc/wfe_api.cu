@@ -429,7 +429,8 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
      * can reach the CTA-per-pair tiers: pairs that enter tier 5 -- first or
      * handed on -- go through the bound pass, which routes them into the
      * classes. */
-    const bool bounded = ctx->bound && st.d_bound && bp.bound.grid > 0 && last >= 5;
+    const bool bounded = ctx->bound && st.d_bound && bp.bound.grid > 0 && last >= 5 &&
+                         !(t == 5 && !listed && alone_in_tier_5(n, bp.max_len));
     uint32_t* const cw = words + kTierWords;
     if (bounded) {
         a.bound = st.d_bound;
@@ -459,7 +460,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     grid = std::max(grid, 1);
     /* a batch by one chain without an order by length or a plan, as small ones
      * are: what would be a memset before it is a few stores at its end (64
-     * pairs of 100-200 bases 13.4 -> 12.5 us each in a row, 36.5 -> 33.7
+     * pairs of 150 bases 13.4 -> 12.5 us each in a row, 36.5 -> 33.7
      * alone) */
     const bool classes = bounded && t == 5 && a.chain.cls.n > 0;
     const bool ordered = t == 0 && !listed && L.ascii_bytes == 0 && bp.max_len > kOrderLength && n >= kOrderPairs;

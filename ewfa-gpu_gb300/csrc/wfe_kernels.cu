@@ -271,14 +271,15 @@ __device__ __forceinline__ void note_deferred(const AlignLaunch& A)
 /* Tail launch of tier u over its list of `count` pairs, built in the launch's
  * own parameter buffer: A (a __grid_constant__ kernel parameter, read in
  * place) is copied word by word and the per-tier fields are patched
- * (own_list: its work list stays A's).  No
+ * (own_list: its work list stays A's; bounds: it has distance bounds, or
+ * computes them).  No
  * copy of the launch record is made on the stack -- a kernel whose code
  * holds a large stack frame keeps only a few CTAs resident per SM, and that
  * limit is also what a grid launched from the device runs with. */
 template <typename K>
 __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int u, int grid, int threads,
                                             uint32_t smem, bool tier_args, uint32_t seq_words, uint32_t gbytes,
-                                            int bulk = 0, bool own_list = false)
+                                            int bulk = 0, bool own_list = false, bool bounds = true)
 {
     void* buf = cudaGetParameterBufferV2((void*)kernel, dim3((unsigned)grid), dim3((unsigned)threads), smem);
     if (!buf) {
@@ -295,6 +296,7 @@ __device__ __forceinline__ void tail_launch(K kernel, const AlignLaunch& A, int 
     n->cls = -1;
     n->plan = nullptr;
     n->bulk = bulk;
+    if (!bounds) n->bound = nullptr;
     if (!own_list) {
         n->work = A.chain.list[u];
         n->work_count = A.chain.counts + u;
@@ -324,9 +326,16 @@ __device__ __forceinline__ void launch_on_device(const AlignLaunch& A, int u, ui
     tail_launch(tier_kernel<T>, A, u, grid, kThreads, sh.smem, true, sh.seq_words, sh.gbytes, 0, own_list);
 }
 
-/* Tail launch of the bound pass, tier 5's start, over `count` pairs. */
+/* Tail launch of tier 5's start over `count` pairs: the bound pass, or the
+ * tier itself for pairs that it takes without (alone_in_tier_5). */
 __device__ __forceinline__ void launch_bound_on_device(const AlignLaunch& A, uint32_t count, bool own_list)
 {
+    if (alone_in_tier_5(count, A.max_len)) {
+        const TierShape& sh = A.chain.shape[5];
+        tail_launch(long_kernel<false, kLongThreads>, A, 5, max(1, min(sh.grid, (int)count)), kLongThreads, sh.smem,
+                    false, 0u, 0u, 0, own_list, false);
+        return;
+    }
     const TierShape& b = A.chain.bound_shape;
     const uint32_t per_cta = (uint32_t)b.threads / 32u;
     const int grid = max(1, min(b.grid, (int)((count + per_cta - 1u) / per_cta)));

@@ -55,6 +55,17 @@ struct TierShape {
  * past tier 5's own (min(max_len, 2047)) are dropped. */
 constexpr int kLongClasses = 9;
 constexpr int kLongClassLimit[kLongClasses - 1] = {127, 193, 257, 321, 449, 577, 961, 1985};
+/* Whether tier 5 takes a list without bounds on its distances, as one launch
+ * with a CTA per pair: as many pairs as the GPU has SMs are aligned at once,
+ * in the time of the longest, and the bound pass takes longer than the cells
+ * it saves them (8 pairs of 4-6 kb at 4-8% 362 -> 273 us, 152 of them 518 ->
+ * 455, 152 of 1 kb at 5% 113 -> 66, of 8-9 kb at 1-2% 310 -> 200).  Not where
+ * pairs of 20% edits are past the tier: the bound sends those to tier 6 at
+ * once. */
+__host__ __device__ constexpr bool alone_in_tier_5(uint32_t count, uint32_t max_len)
+{
+    return count <= 152u && max_len <= 5u * (uint32_t)kLongSmemDistance;
+}
 /* Pairs from which on tier 5 may begin with the scan (see plan_choice). */
 constexpr uint32_t kScanMin = 1024;
 constexpr uint32_t kWidePairs = 16384;
