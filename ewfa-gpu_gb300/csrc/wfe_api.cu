@@ -369,7 +369,40 @@ int chain_last(const wfe_ctx* ctx, int first, int last, bool* cut)
 constexpr uint32_t kOrderLength = 320;
 constexpr uint32_t kOrderPairs = 16384;
 
-constexpr int kPlanned = -1; /* first tier of a planned batch (see first_tier_of) */
+constexpr uint32_t kPlanLength = 400; /* sequences from which on large batches are planned */
+constexpr int kPlanned = -1;   /* first tier of a planned batch (see first_tier_of) */
+constexpr int kPlanned1 = -3;  /* tier 1 as first tier, planned: tier 1, or tier 5 */
+constexpr int kBandFirst = -2; /* tier 1 as first tier, its pairs of up to 31 through tier 0's kernel (see band_first) */
+
+/* Whether a bucket of a batch of n pairs can be taken to hold `many`: one of
+ * several, whose lengths reach further the more of the pairs are in others. */
+bool holds_many(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n, uint32_t many)
+{
+    const uint32_t others = ctx->nbuckets == 1 ? 1u : std::max(2u, (ctx->cfg.max_seq_len + bp.max_len - 1u) / std::max(1u, bp.max_len));
+    return n / others >= many;
+}
+
+/* Whether a large batch of short sequences that is to start at tier 1 goes
+ * through the band of tier 0 on the way: a thread per pair takes the pairs of
+ * distances up to 31 in a third of the time, whatever their distance, and the
+ * others are few among sequences of this length (100,000 pairs of 150 bases
+ * at 5% 239 -> 39 us, at 1% 116 -> 31, of 43-173 bases at 9-15% 313 -> 82, of
+ * 200-240 at 10-15%, half of them past 31, 772 -> 285; 16,384 of 150 bases at
+ * 5% 42 -> 12; a list of 6,000 pairs takes the band's latency, 50 us, where tier
+ * 1 takes 31).  They count as pairs of tier 1. */
+constexpr uint32_t kBandLength = 256;
+constexpr uint32_t kBandPairs = 8192;
+bool band_first(const wfe_ctx* ctx, const BucketPlan& bp, int first_tier, uint32_t n)
+{
+    return first_tier == 1 && bp.max_len <= kBandLength && holds_many(ctx, bp, n, kBandPairs) && bp.shape[0].grid > 0;
+}
+
+/* Whether a batch can be planned: the chain reaches tier 5 and has its scan. */
+bool can_plan(const wfe_ctx* ctx, const BucketPlan& bp, bool device_call)
+{
+    return device_call && bp.max_len > kPlanLength && ctx->deep_ready && ctx->bound && bp.bound.grid > 0 &&
+           bp.cls.scan.grid > 0 && !(ctx->cfg.max_distance > 0 && ctx->cfg.max_distance <= tier_info(4).dcap);
+}
 
 /* Launch the first tier of one bucket's chain over `work` (NULL: pairs
  * 0..n-1); the last CTA of every tier starts the next tier with work, on the
@@ -382,14 +415,17 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
 {
     const wfe_config& c = ctx->cfg;
     const uint32_t B = c.batch_size;
-    const bool plan = first_tier == kPlanned; /* tier 0, 1 or 5, chosen on the device */
-    const int t = plan ? 5 : first_tier;
+    const bool from1 = first_tier == kPlanned1;
+    const bool plan = first_tier == kPlanned || from1; /* chosen on the device */
+    const bool band = first_tier == kBandFirst;
+    const int t = plan ? 5 : band ? 0 : first_tier, counted = band ? 1 : t;
     uint32_t* words = st.d_counts + (size_t)bucket_index * kChainWords;
     uint32_t* lists = st.d_lists + (size_t)bucket_index * kListsPerBucket * B;
     AlignLaunch a{};
     a.L = L;
-    a.work = listed ? lists + (size_t)t * B : nullptr;
-    a.work_count = listed ? words + t : nullptr;
+    const int routed = from1 ? 1 : t; /* the list that the pairs were routed to */
+    a.work = listed ? lists + (size_t)routed * B : nullptr;
+    a.work_count = listed ? words + routed : nullptr;
     a.n_work = n;
     a.dist = dist;
     a.cigar = cigar;
@@ -423,7 +459,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     }
     a.retry = t < last ? a.chain.list[t + 1] : a.chain.defer;
     a.retry_count = t < last ? words + t + 1 : a.chain.defer_count;
-    a.passed_total = ctx->d_passed + t;
+    a.passed_total = band ? nullptr : ctx->d_passed + t;
     a.cls = -1;
     /* Distance bounds (and with them tier 5's classes) for every chain that
      * can reach the CTA-per-pair tiers: pairs that enter tier 5 -- first or
@@ -467,12 +503,12 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     *cleared = !listed && !ordered && !plan && !(classes && n >= kScanMin);
     a.chain.clear = *cleared;
     int rc = WFE_OK;
-    TimedLaunch* tl = begin_timing(ctx, t, s, &rc);
+    TimedLaunch* tl = begin_timing(ctx, counted, s, &rc);
     if (rc != WFE_OK) return rc;
     if (plan) {
         a.plan = choice;
-        a.plan_tiers = 1;
-        a.entered = ctx->d_entered;
+        a.plan_tiers = from1 ? kPlanFrom1 : kPlanAll;
+        a.entered = from1 ? nullptr : ctx->d_entered; /* they count as tier 1's */
         WFE_CUDA(ctx, launch_planned(a, s));
         ctx->stats.kernel_launches += 2; /* and what the plan chooses, counted on the device */
     } else if (classes) {
@@ -491,7 +527,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
         ctx->stats.kernel_launches++;
     }
     if (tl) WFE_CUDA(ctx, cudaEventRecord(tl->stop, s));
-    if (!plan) ctx->stats.tier_launches[t]++;
+    if (!plan) ctx->stats.tier_launches[counted]++;
     return WFE_OK;
 }
 
@@ -502,16 +538,23 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
  * pairs, the same at 16,384; 150 bases: 34 and 37 at 1,024, 41 and 37 at
  * 4,096).  A large batch of sequences past kPlanLength bases is planned
  * (kPlanned): its error rate decides. */
-constexpr uint32_t kPlanLength = 400;
 int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n, bool device_call)
 {
     if (!bp.by_length || bp.first_tier != 0 || bp.shape[1].grid <= 0) return bp.first_tier;
     if (n < 4096u) return n < 11u * bp.max_len - std::min(1200u, 11u * bp.max_len) ? 1 : 0;
     if (!device_call) return 0;
-    const bool plan = bp.max_len > kPlanLength && ctx->deep_ready && ctx->bound && bp.bound.grid > 0 &&
-                      bp.cls.scan.grid > 0 &&
-                      !(ctx->cfg.max_distance > 0 && ctx->cfg.max_distance <= tier_info(4).dcap);
-    return plan ? kPlanned : n < 32768u && bp.max_len > kOrderLength ? 1 : 0;
+    return can_plan(ctx, bp, device_call) ? kPlanned : n < 32768u && bp.max_len > kOrderLength ? 1 : 0;
+}
+
+/* How a batch of n pairs whose first tier is `first_tier` starts, if that is tier
+ * 1: a large batch of short sequences with tier 0's kernel, one of longer ones as
+ * the plan says (60,000 pairs of 180-400 bases at 12-15% 674 -> 236 us, at 1-2%
+ * 129 -> 106; at 0.3%, where tier 1 is chosen, the sample adds 20 us to 85; smaller
+ * lists, and lists of a few among longer ones, were up to 9% slower). */
+int from_tier_1(const wfe_ctx* ctx, const BucketPlan& bp, int first_tier, uint32_t n, bool device_call)
+{
+    if (band_first(ctx, bp, first_tier, n)) return kBandFirst;
+    return first_tier == 1 && holds_many(ctx, bp, n, kPlanFrom1Min) && can_plan(ctx, bp, device_call) ? kPlanned1 : first_tier;
 }
 
 /* Enqueue the alignment of pairs 0..n-1 of one batch on stream s: with one
@@ -537,7 +580,8 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
         const BucketPlan& bp = ctx->bucket[0];
         const int t = first_override ? first_override[0] : first_tier_of(ctx, bp, n, device_call);
         if (t != kPlanned) ctx->single_entered[t] += n;
-        const int r = launch_bucket(ctx, st, bp, 0, t, L, false, n, dist, cigar, status, s, base, &cleared);
+        const int first = from_tier_1(ctx, bp, t, n, device_call);
+        const int r = launch_bucket(ctx, st, bp, 0, first, L, false, n, dist, cigar, status, s, base, &cleared);
         if (r != WFE_OK) return r;
         if (!cleared) WFE_CUDA(ctx, clear_counts());
         st.counts_dirty = still_dirty;
@@ -545,9 +589,12 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     }
     Buckets bk{};
     bk.n = ctx->nbuckets;
+    int start[kMaxBuckets];
     for (int b = 0; b < ctx->nbuckets; ++b) {
         bk.max_len[b] = ctx->bucket[b].max_len;
         bk.first_tier[b] = first_override ? first_override[b] : ctx->bucket[b].first_tier;
+        start[b] = from_tier_1(ctx, ctx->bucket[b], bk.first_tier[b], n, device_call);
+        if (start[b] == kBandFirst) bk.first_tier[b] = 0;
         /* routing never goes past the end of the bucket's chain */
         bool cut = false;
         bk.last_tier[b] = chain_last(ctx, bk.first_tier[b], ctx->bucket[b].last_tier, &cut);
@@ -581,8 +628,8 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     for (int b = ctx->nbuckets - 1; b >= 0; --b) {
         if (merge && b + 1 < ctx->nbuckets && bk.first_tier[b] == 5) continue;
         const int r =
-            launch_bucket(ctx, st, ctx->bucket[b], b, bk.first_tier[b], L, true, n, dist, cigar, status, s, base,
-                          &cleared);
+            launch_bucket(ctx, st, ctx->bucket[b], b, start[b], L, true, n, dist, cigar, status, s,
+                          base, &cleared);
         if (r != WFE_OK) return r;
     }
     WFE_CUDA(ctx, clear_counts());

@@ -226,7 +226,7 @@ __device__ __forceinline__ int plan_choice(const AlignLaunch& A, uint32_t count,
             t = reg;
         }
         const float band = 28.f + fmaxf(0.1f * len, n * 0.0055f * len);
-        if (d + spread < 31.f && band < t) best = kPlanBand;
+        if (A.plan_tiers == kPlanAll && d + spread < 31.f && band < t) best = kPlanBand;
     }
     return best;
 }
@@ -2362,7 +2362,7 @@ __global__ void __launch_bounds__(kOrderBins) plan_kernel(const __grid_constant_
         words[kPlanSums - 1] = (uint32_t)mode;
         if (A.plan_tiers) {
             const int tier = mode == kPlanBand ? 0 : mode == kPlanRegister ? 1 : 5;
-            atomicAdd(A.entered + tier, (unsigned long long)count);
+            if (A.entered) atomicAdd(A.entered + tier, (unsigned long long)count);
             if (mode == kPlanBulk && A.chain.launched) atomicAdd(A.chain.launched + 5, 1ull);
         }
         if (mode == kPlanBand) {
@@ -2375,8 +2375,8 @@ __global__ void __launch_bounds__(kOrderBins) plan_kernel(const __grid_constant_
             launch_bound_on_device(A, count, true);
         }
     };
-    if (count < kScanMin) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) choose(kPlanCta);
+    if (count < (A.plan_tiers == kPlanFrom1 ? kPlanFrom1Min : kScanMin)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) choose(A.plan_tiers == kPlanFrom1 ? kPlanRegister : kPlanCta);
         return;
     }
     if (blockIdx.x >= kPlanCtas) {

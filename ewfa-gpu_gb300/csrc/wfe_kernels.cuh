@@ -163,6 +163,8 @@ struct Buckets {
 
 /* First kernels that a plan chooses between. */
 enum { kPlanBand = 0, kPlanRegister = 1, kPlanCta = 2, kPlanBulk = 3 };
+enum { kPlanAll = 1 /* tiers 0 and 1 */, kPlanFrom1 = 2 /* tier 1 */ };
+constexpr uint32_t kPlanFrom1Min = 16384; /* pairs of a list that kPlanFrom1 samples; fewer begin at tier 1 */
 constexpr int kPlanSums = 8;       /* words of a plan: five sums, CTAs done, the choice last */
 constexpr uint32_t kPlanSample = 1024; /* pairs it samples */
 
@@ -193,7 +195,7 @@ struct AlignLaunch {
     int tier;                    /* this launch's tier */
     int bulk;                    /* tier 5 began with the scan: the classes' pairs are all at the fronts of their lists */
     const uint32_t* plan;        /* the choice of launch_planned, the last of its kPlanSums words; NULL: none */
-    int plan_tiers;              /* the plan may choose tiers 0 and 1, too */
+    int plan_tiers;              /* what the plan may choose besides tier 5 (kPlanAll, kPlanFrom1) */
     unsigned long long* entered; /* entered[t]: pairs of planned launches that began at tier t (stats) */
     Chain chain;                 /* chain.cta_done == NULL: no device-side chaining */
 };

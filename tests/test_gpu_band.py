@@ -209,3 +209,23 @@ def test_counters_between_batches():
                     some = slice(None, None, 1 + sets[j][0] // 300)
                     compare_with_oracle(sets[j][1], sets[j][2][some], 1200, dist[some], cg[some], st[some])
                     assert (st == wfe.PAIR_OK).all()
+
+
+@pytest.mark.parametrize("buckets,n,lo,hi,p", [([200], 8192, 40, 180, .2), ([200], 8191, 40, 180, .2), ([256, 500], 40000, 60, 450, .15),
+                                               ([512], 16384, 200, 460, .12), ([512], 16384, 200, 460, .005)])
+def test_large_lists_from_tier_1(buckets, n, lo, hi, p):
+    """A first tier of 1: by the band of tier 0, as planned, or by tier 1
+    itself, the pairs count as tier 1's and come out the same."""
+    torch = torch_cuda()
+    ascii, pairs = wfe.generate(n, lo, hi, p_min=.001, p_max=p, seed=n)
+    d_a, d_p = torch.from_numpy(ascii).cuda(), torch.from_numpy(pairs.view(np.uint8)).cuda()
+    out = tuple(torch.zeros(s, dtype=t, device="cuda") for s, t in
+                ((n, torch.int32), ((n, 600), torch.int8), (n, torch.uint8)))
+    with wfe.Context(max_seq_len=buckets[-1], cigar_stride=600, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        ctx.set_policy(buckets, [1] * len(buckets))
+        for _ in range(2):
+            ctx.align_device(d_a, d_p, n, buckets[-1], *out, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        entered = ctx.stats()["tier_entered"]
+    assert entered[0] == 0 and entered[1] == 2 * n
+    compare_with_oracle(ascii, pairs, 600, *(x.cpu().numpy() for x in out))
