@@ -473,10 +473,12 @@ void run_scheduler(wfe_server* s)
             Batch* b = form_batch(s);
             if (!b) break;
             lk.unlock();
-            b->rc = launch_batch(s, b);
+            /* once its host function is queued, a finisher may have deleted b */
+            const int rc = launch_batch(s, b);
             const uint64_t t1 = now_ns();
-            if (b->rc != WFE_OK) {
+            if (rc != WFE_OK) {
                 /* finishes as failed, without results, once what was queued is done */
+                b->rc = rc;
                 cudaStreamSynchronize(s->lanes[b->lane].stream);
                 batch_done(b);
             }
