@@ -1011,8 +1011,8 @@ def noalloc_throughput(d_ascii, d_pairs, want, stream, steps: int) -> dict:
     got = (d_dist.cpu().numpy(), d_cigar.view(PAIRS, CIGAR_STRIDE).cpu().numpy(), d_status.cpu().numpy())
     return {"value": steps * BATCH / (ms / 1e3), "unit": "alignments/s", "ms_per_step": ms / steps,
             "max_distance": wfe.NOALLOC_MAX_DISTANCE, "same_as_context_path": parity(got, want)["mismatches"] == 0,
-            "note": "no context and no allocation: tier 0 (backtrace store in shared memory) over every pair, "
-                    "then tier 3 over the pairs past distance 21 with its backtrace scratch in a fixed 16 MiB "
+            "note": "no context and no allocation: tier 0 (all its state in shared memory) over every pair, "
+                    "then tier 3 over the pairs past distance 31 with its backtrace scratch in a fixed 16 MiB "
                     "device array (153 CTAs at most), one call per batch"}
 
 
@@ -1317,7 +1317,7 @@ def main():
                                            "issue_slots_busy_pct": profiled("issue_slots_busy_pct"),
                                            "source": "ncu, profiles/" + PROFILE,
                                            "note": "the kernel is bound by its integer pipes, not by HBM"},
-                         "kernel": f"tier_kernel tier {top}" + (" and the tiers it hands pairs on to (one timed "
+                         "kernel": ("band_kernel" if top == 0 else "tier_kernel") + f" tier {top}" + (" and the tiers it hands pairs on to (one timed "
                                                                      "chain)" if any(st["tier_passed"]) else ""),
                          "alg_bytes_per_launch": alg_bytes,
                          "ms_per_launch": ms_max / args.steps,

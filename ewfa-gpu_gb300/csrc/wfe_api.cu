@@ -209,10 +209,9 @@ uint32_t default_cigar_stride(uint32_t max_seq_len)
 }
 
 /* First tier by sequence length, used until a policy says otherwise: short
- * reads almost always finish in the 4-lane tier; longer ones start at the
- * CTA-per-pair tier, whose bound pass sends each pair to the distance class
- * that fits it (on 1,000-base reads at 10% edits 25M alignments/s against
- * 20.7M from tier 2; at 2% edits tier 1 is faster, 125M against 91M). */
+ * reads almost always finish in the band of tier 0; longer ones start at
+ * tier 5, which sends each pair to the distance class that fits it.  Where
+ * this says tier 0, first_tier_of looks at the number of pairs too. */
 int default_first_tier(uint32_t max_len)
 {
     if (max_len <= 1200) return 0;

@@ -17,7 +17,8 @@
  *                        diagonals: the scan that bounds distances, and the
  *                        classes with the most pairs
  *   tile_kernel          tier 5 in bulk, several lanes per pair
- *   order_*_kernel       tier 5's list in order of length
+ *   plan_kernel          the first kernel of a large list, from a sample
+ *   order_*_kernel       a list in order of length
  *   classify_kernel      length buckets and predicted tiers
  *   history_kernel       CIGARs from the reference's 128-bit histories
  *                        (src/kernels.cu:397-625)
@@ -718,10 +719,12 @@ __global__ void tier_kernel(const __grid_constant__ AlignLaunch A, uint32_t seq_
  * the walk, so the 32 pairs of a warp stay in step.  The wavefront kernel
  * that this replaced (4 lanes per pair) spent 981 warp instructions on a
  * 150-base pair at 5% edits and stepped every pair of a warp to the largest
- * distance of the eight.  1M such pairs, device-resident: 1,038 us before,
- * 479 us now; 300k without a context 397 and 189 us; 500k from page-locked
- * host memory 960 and 883 us (the CPU-GPU link bounds it); 200k pairs of
- * 50-300 bases at 1-12% edits 473 and 327 us; 64 pairs 17 and 11 us.
+ * distance of the eight.  1M such pairs, device-resident: 1,032 us before,
+ * 395 us now; 300k without a context 391 and 143 us; 500k from page-locked
+ * host memory 940 and 900 us (the CPU-GPU link bounds it); 200k pairs of
+ * 50-300 bases at 1-12% edits 470 and 186 us.  130 registers (144 allocated)
+ * keep 12 warps on an SM: with 128, 120 or 112 and 13 warps, 1M pairs took
+ * 398, 400 and 405 us.
  *
  * The warp's shared memory (words; a lane owns column `lane` of every row):
  *   blocks  D0 of 32 columns, transposed: row q holds band bit q's
@@ -749,8 +752,9 @@ __host__ __device__ constexpr uint32_t band_fixed_words(uint32_t n)
     return 64u * n + 2u * kPlaneRow * (2u * n + 1u) + 32u * band_byte_words(n);
 }
 constexpr uint32_t kBandBlockWords = 512;
-/* Words given to a warp: all blocks of texts up to 160 bases (13 warps per SM;
- * 150-base reads take 0.45 ns a pair, with room for 224 bases 0.51). */
+/* Words given to a warp: all blocks of texts up to 160 bases (room for 13 warps
+ * per SM, registers for 12; 150-base reads take 0.40 ns a pair; with room for
+ * 224 bases, and 8 warps, an eighth more). */
 __host__ __device__ constexpr uint32_t band_smem_words(uint32_t max_len)
 {
     const uint32_t n = band_words(max_len) + (max_len == 0u), m = n < 5u ? n : 5u;
@@ -1357,7 +1361,7 @@ __global__ void long_kernel(const __grid_constant__ AlignLaunch A)
  * pairs, and longer the wider its band: a class of fewer than kWidePairs
  * pairs goes to tile_kernel.  200k pairs of 1,000 bases at 10% edits, in
  * batches of 20,000: 15.3 ms from tier 0 up, 8.1 ms from the bound pass and
- * its classes, 1.93 ms so (2.10 with a walk over 64 diagonals).
+ * its classes, 1.92 ms so (2.10 with a walk over 64 diagonals).
  *
  * Scratch of a warp (slab; rows of 32 words, a lane's column each): the bit
  * planes of both sequences, VP/VN before every block of 32 columns, and the
@@ -1751,9 +1755,9 @@ __global__ void __maxnreg__(NW <= 4 ? 96 : (NW <= 8 ? 128 : (NW <= 16 ? 168 : 25
  * times fewer pairs than one thread per pair to fill the GPU, for 1.5 to 2
  * times its instructions.  80 registers keep three CTAs on an SM, so that
  * two compute while the third walks back (128 and two CTAs: 1.2 times the
- * time).  8,000 pairs of 5,000-7,000 bases at 6-10% edits: 3.9 ms with a CTA
- * per pair, 1.42 ms so, a call among others of three contexts; 50,000 pairs of
- * 100-10,000 bases at 1-15%: 9.3 and 3.7 ms. */
+ * time; 64, with which four fit: 1.04 times).  8,000 pairs of 5,000-7,000 bases
+ * at 6-10% edits: 3.9 ms with a CTA per pair, 1.36 ms so, a call among others of
+ * three contexts; 50,000 pairs of 100-10,000 bases at 1-15%: 9.3 and 3.55 ms. */
 constexpr int kTileWarps = 8;
 constexpr int kTileThreads = 32 * kTileWarps;
 /* lanes per pair for distances up to dlim: nd <= 2 G for any ends */
@@ -2722,10 +2726,10 @@ __host__ __device__ constexpr uint32_t history_smem_words(uint32_t nw, int span)
 template <int SPAN>
 __global__ void __launch_bounds__(32, 32)
 history_kernel(Layout L, uint32_t n, uint32_t max_len, const int32_t* dist, const uint64_t* hist, int8_t* cigar,
-               uint32_t stride, uint8_t* status, uint32_t nw)
+               uint32_t stride, uint8_t* status, uint32_t nw, uint32_t per_warp)
 {
     const int lane = (int)threadIdx.x;
-    const uint32_t pi = blockIdx.x * 32u + threadIdx.x;
+    const uint32_t pi = threadIdx.x < per_warp ? blockIdx.x * per_warp + threadIdx.x : n;
     const int plane = kPlaneRow * (int)(nw + 1u);
     PairRef pr{};
     uint64_t w0 = 0, w1 = 0;
@@ -3154,11 +3158,16 @@ cudaError_t launch_cigar_from_history(const Layout& L, uint32_t n, uint32_t max_
     /* long sequences and slots have always been refused together */
     if (16u * (size_t)seq_words_for(max_len) + 320u + round16(stride) > 227u * 32u) return cudaErrorInvalidValue;
     const uint32_t nw = std::max(1u, band_words(max_len));
+    /* Few pairs: eight a warp, which read one span and take as many steps as the
+     * longest of eight (4,000 pairs of 250 bases at 10% 20.9 -> 15.0 us, 2,000 of
+     * 1,000 bases 45.7 -> 25.2; 16,384 of 150 bases 10.0 -> 13.1). */
+    const uint32_t per_warp = n <= 8192u ? 8u : 32u;
     const auto launch_as = [&](auto kernel, int span) {
         const size_t smem = 4u * (size_t)history_smem_words(nw, span);
         const cudaError_t e = allow_smem((const void*)kernel, smem);
         if (e != cudaSuccess) return e;
-        kernel<<<n / 32u + (n % 32u != 0u), 32, smem, s>>>(L, n, max_len, dist, hist, cigar, stride, status, nw);
+        kernel<<<n / per_warp + (n % per_warp != 0u), 32, smem, s>>>(L, n, max_len, dist, hist, cigar, stride, status,
+                                                                     nw, per_warp);
         return cudaGetLastError();
     };
     /* spans of 8 pairs that do not fit the narrower ones (250 bases: 40 us

@@ -210,9 +210,13 @@ int wfe_reset_stats(wfe_ctx* ctx);
  * pairs with a narrow band; each pair then goes to the distance class that
  * covers its bound, and a pair whose bound lies past tier 5's limit goes
  * straight to tier 6.  WFE_POLICY_NO_BOUND turns that pass off, and with it the
- * classes (for comparison: results are the same).  A bucket whose tier is left
- * to its length (-1) starts large batches of sequences past 400 bases at
- * tier 5 where it would start small ones at tier 0.
+ * classes (for comparison: results are the same).  As many pairs as the
+ * GPU has SMs are aligned without it, too.
+ * A bucket whose tier is left to its length (-1) and would start at tier 0
+ * starts small batches at tier 1, and device calls of many pairs past 400 bases
+ * at tier 0, 1 or 5, as a sample of the batch says on the device.  Large
+ * batches of a bucket whose first tier is 1 may go through tier 0's kernel on
+ * the way, or start at tier 5; their pairs count as tier 1's.
  * Replaces nothing in the reference, which has one fixed launch shape
  * (src/wavefront.cu:173-208); see also wfe_autotune. */
 #define WFE_POLICY_PREDICT 1u  /* route every pair to the tier of its predicted distance */
@@ -359,8 +363,9 @@ int wfe_cigar_from_history_device(const char* d_ascii, const wfe_pair* d_pairs,
  * tier 3, whose backtrace stores fill the rest: 612 pairs in flight, 153
  * CTAs of 4 (about one per SM on a 152-SM GB300, below that kernel's
  * occupancy).  Sequences too long for tier 0's shared memory (past 9,000
- * bases) go to tier 3 alone (816 pairs in flight).  On short reads a
- * call runs at ~80% of wfe_align_device's speed.
+ * bases), and calls of up to 512 pairs of more than 256 bases, go to tier 3
+ * alone (816 pairs in flight).  On short reads a call of 300,000 pairs takes
+ * 1.2 times as long as wfe_align_device.
  * Every call shares the array and it keeps the last call's contents
  * (nothing in it has to start at zero: the list's count is set by a
  * cudaMemsetAsync on `stream` each round, and every other entry is written

@@ -124,8 +124,8 @@ def replayed(p, t, record, d, slot):
     return wfe.PAIR_BAD_HISTORY if not ok else wfe.PAIR_CIGAR_TRUNCATED if len(out) > len(slot) else wfe.PAIR_OK
 
 
-@pytest.mark.parametrize("stride", [800, 801, 16, 0])
-def test_histories(stride):
+@pytest.mark.parametrize("stride,copies", [(800, 1), (801, 1), (16, 1), (0, 1), (800, 90)])
+def test_histories(stride, copies):
     """Backtrace records to CIGARs, with the narrow and the wide spans: the
     aligner's own CIGARs from their operations, and the bytes and statuses of
     records that no alignment leaves."""
@@ -158,11 +158,16 @@ def test_histories(stride):
         else:
             want[i, :1], want_st[i] = 0, wfe.PAIR_OVER_MAX_DISTANCE
     assert (want_st[lone] == wfe.PAIR_BAD_HISTORY).any()
+    d_p, d_d, d_h, n = d_p.repeat(copies), d_d.repeat(copies), d_h.repeat(copies, 1), n * copies
     for max_len in (512, 200):
         out, st = torch.full((n, max(stride, 1)), 7, dtype=torch.int8, device="cuda"), torch.zeros(n, dtype=torch.uint8, device="cuda")
         wfe.cigar_from_history_device(d_a, d_p, n, max_len, d_d, d_h, out, stride, st, torch.cuda.current_stream())
         torch.cuda.synchronize()
         got, got_st = out.cpu().numpy()[:, :stride], st.cpu().numpy()
+        for c in range(1, copies):
+            np.testing.assert_array_equal(got[:len(seqs)], got[c * len(seqs):(c + 1) * len(seqs)])
+            np.testing.assert_array_equal(got_st[:len(seqs)], got_st[c * len(seqs):(c + 1) * len(seqs)])
+        got, got_st = got[:len(seqs)], got_st[:len(seqs)]
         fits = np.maximum(pairs["p_len"], pairs["t_len"]) <= max_len
         np.testing.assert_array_equal(got_st, np.where(fits, want_st, wfe.PAIR_TOO_LONG))
         np.testing.assert_array_equal(got[fits], want[fits])
