@@ -465,7 +465,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
      * handed on -- go through the bound pass, which routes them into the
      * classes. */
     const bool bounded = ctx->bound && st.d_bound && bp.bound.grid > 0 && last >= 5 &&
-                         !(t == 5 && !listed && alone_in_tier_5(n, bp.max_len));
+                         !(t == 5 && alone_in_tier_5(n, bp.max_len));
     uint32_t* const cw = words + kTierWords;
     if (bounded) {
         a.bound = st.d_bound;
@@ -487,12 +487,10 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
     a.chain.cls.order_count = cw + kClassWords;
     a.chain.cls.order_next = a.chain.cls.order_count + kOrderBins;
     const uint32_t* const choice = a.chain.cls.order_next + kOrderBins + kPlanSums - 1;
-    int grid = bp.shape[t].grid;
-    if (!listed) {
-        const uint32_t per_cta = (uint32_t)tier_info(t).pairs_per_cta;
-        grid = (int)std::min<uint64_t>((uint64_t)grid, ((uint64_t)n + per_cta - 1) / per_cta);
-    }
-    grid = std::max(grid, 1);
+    /* a list holds at most n pairs: 100 pairs in three buckets 57 -> 41 us, much of
+     * it CTAs without work */
+    const uint32_t per_cta = (uint32_t)tier_info(t).pairs_per_cta;
+    const int grid = std::max(1, (int)std::min<uint64_t>((uint64_t)bp.shape[t].grid, ((uint64_t)n + per_cta - 1) / per_cta));
     /* a batch by one chain without an order by length or a plan, as small ones
      * are: what would be a memset before it is a few stores at its end (64
      * pairs of 150 bases 13.4 -> 12.5 us each in a row, 36.5 -> 33.7

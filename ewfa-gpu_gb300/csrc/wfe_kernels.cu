@@ -2380,7 +2380,8 @@ __global__ void __launch_bounds__(kOrderBins) plan_kernel(const __grid_constant_
         }
     };
     if (count < (A.plan_tiers == kPlanFrom1 ? kPlanFrom1Min : kScanMin)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) choose(A.plan_tiers == kPlanFrom1 ? kPlanRegister : kPlanCta);
+        /* an empty list (a bucket that no pair of the batch falls in) starts nothing */
+        if (count > 0u && blockIdx.x == 0 && threadIdx.x == 0) choose(A.plan_tiers == kPlanFrom1 ? kPlanRegister : kPlanCta);
         return;
     }
     if (blockIdx.x >= kPlanCtas) {
@@ -2990,15 +2991,14 @@ cudaError_t launch_bound(const AlignLaunch& a, cudaStream_t s, uint64_t* launche
     if (sh.grid <= 0 || !a.bound || sh.seq_words != seq_words_for(a.max_len)) return cudaErrorInvalidValue;
     cudaError_t e = allow_smem((const void*)bound_kernel, sh.smem);
     if (e != cudaSuccess) return e;
-    if (a.tier == 5 && a.chain.cls.n > 0 && a.chain.cls.scan.grid > 0 && (a.work_count || a.n_work >= kScanMin)) {
+    if (a.tier == 5 && a.chain.cls.n > 0 && a.chain.cls.scan.grid > 0 && a.n_work >= kScanMin) {
         *launches += 3;
         return launch_planned(a, s);
     }
     AlignLaunch w = a;
     w.plan = nullptr;
     const uint32_t per_cta = (uint32_t)sh.threads / 32u;
-    int grid = sh.grid;
-    if (!a.work_count) grid = (int)std::min<uint64_t>((uint64_t)grid, ((uint64_t)a.n_work + per_cta - 1) / per_cta);
+    const int grid = (int)std::min<uint64_t>((uint64_t)sh.grid, ((uint64_t)a.n_work + per_cta - 1) / per_cta);
     ++*launches;
     bound_kernel<<<std::max(grid, 1), sh.threads, sh.smem, s>>>(w, sh.seq_words, 0u);
     return cudaGetLastError();
