@@ -2613,7 +2613,7 @@ __global__ void __launch_bounds__(256) classify_kernel(Layout L, uint32_t n, Buc
                     while (t < top && (float)B.dcap[t] < est) ++t;
                 }
             }
-            key = (t == 5 && B.tier5_to >= 0 ? B.tier5_to : b) * kListsPerBucket + t;
+            key = (t == 5 && B.tier5_to >= 0 ? B.tier5_to : B.to[b]) * kListsPerBucket + t;
             bucket = b;
         }
         const unsigned same = __match_any_sync(kFull, key);

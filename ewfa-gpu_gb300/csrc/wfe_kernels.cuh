@@ -157,6 +157,7 @@ struct Buckets {
     uint32_t stride;
     uint32_t* counts;                /* counts of bucket b at counts + b*count_stride */
     uint32_t count_stride;
+    int to[kMaxBuckets];             /* bucket whose lists take a bucket's pairs */
     int tier5_to;                    /* bucket whose tier-5 list takes the tier-5 pairs of all (-1: each its own) */
     unsigned long long* totals;      /* pairs classified into each bucket (stats) */
 };
