@@ -217,6 +217,7 @@ def test_counters_between_batches():
 
 
 @pytest.mark.parametrize("buckets,n,lo,hi,p", [([200], 8192, 40, 180, .2), ([200], 8191, 40, 180, .2), ([256, 500], 40000, 60, 450, .15),
+                                               ([64, 128, 512], 700, 10, 460, .15),
                                                ([512], 16384, 200, 460, .12), ([512], 16384, 200, 460, .005)])
 def test_large_lists_from_tier_1(buckets, n, lo, hi, p):
     """A first tier of 1: by the band of tier 0, as planned, or by tier 1
