@@ -534,13 +534,17 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
  * of the sequences in columns (300 bases: 31 us against 61 for up to 4,096
  * pairs, the same at 16,384; 150 bases: 34 and 37 at 1,024, 41 and 37 at
  * 4,096).  A large batch of sequences past kPlanLength bases is planned
- * (kPlanned): its error rate decides. */
+ * (kPlanned): its error rate decides.  Other device batches of up to 512 bases
+ * start at tier 0 from 12,288 pairs on (20,000 pairs of 240-330 bases at 4-7%:
+ * 58 us in a row against 92 from tier 1, alone 167 against 131; at 0.5% 34 and
+ * 33), of longer sequences, more of which pass distance 31, from 32,768 on. */
 int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n, bool device_call)
 {
     if (!bp.by_length || bp.first_tier != 0 || bp.shape[1].grid <= 0) return bp.first_tier;
     if (n < 4096u) return n < 11u * bp.max_len - std::min(1200u, 11u * bp.max_len) ? 1 : 0;
     if (!device_call) return 0;
-    return can_plan(ctx, bp, device_call) ? kPlanned : n < 32768u && bp.max_len > kOrderLength ? 1 : 0;
+    if (can_plan(ctx, bp, device_call)) return kPlanned;
+    return n < (bp.max_len > 512u ? 32768u : bp.max_len > kOrderLength ? 12288u : 0u) ? 1 : 0;
 }
 
 /* How a batch of n pairs whose first tier is `first_tier` starts, if that is tier
