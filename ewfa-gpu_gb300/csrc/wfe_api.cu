@@ -551,11 +551,14 @@ int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n, bool dev
  * 1: a large batch of short sequences with tier 0's kernel, one of longer ones as
  * the plan says (60,000 pairs of 180-400 bases at 12-15% 674 -> 236 us, at 1-2%
  * 129 -> 106; at 0.3%, where tier 1 is chosen, the sample adds 20 us to 85; smaller
- * lists, and lists of a few among longer ones, were up to 9% slower). */
+ * lists, and lists of a few among longer ones, were up to 9% slower).  A planned
+ * chain takes the one list that it samples: not where predictions put pairs in the
+ * lists behind it. */
 int from_tier_1(const wfe_ctx* ctx, const BucketPlan& bp, int first_tier, uint32_t n, bool device_call)
 {
     if (band_first(ctx, bp, first_tier, n)) return kBandFirst;
-    return first_tier == 1 && holds_many(ctx, bp, n, kPlanFrom1Min) && can_plan(ctx, bp, device_call) ? kPlanned1 : first_tier;
+    const bool plan = first_tier == 1 && !ctx->predict && holds_many(ctx, bp, n, kPlanFrom1Min) && can_plan(ctx, bp, device_call);
+    return plan ? kPlanned1 : first_tier;
 }
 
 /* Enqueue the alignment of pairs 0..n-1 of one batch on stream s: with one

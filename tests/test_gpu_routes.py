@@ -1,0 +1,39 @@
+"""Calls whose pairs are routed to several lists of a chain: every pair is
+aligned, whichever kernel the chain starts with.  Outputs hold other values
+before each call, so that a pair that no kernel takes is seen."""
+import numpy as np
+import pytest
+
+import wfe
+from test_gpu_parity import compare_with_oracle, torch_cuda
+
+pytestmark = pytest.mark.gpu
+
+
+def align_device(ctx, ascii, pairs, max_len, stride):
+    torch = torch_cuda()
+    n = len(pairs)
+    d_a, d_p = torch.from_numpy(ascii).cuda(), torch.from_numpy(pairs.view(np.uint8)).cuda()
+    out = (torch.full((n,), -7, dtype=torch.int32, device="cuda"), torch.full((n, stride), 55, dtype=torch.int8, device="cuda"),
+           torch.full((n,), 99, dtype=torch.uint8, device="cuda"))
+    ctx.align_device(d_a, d_p, n, max_len, *out, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    return tuple(x.cpu().numpy() for x in out)
+
+
+def check(ascii, pairs, stride, got, some):
+    dist, cg, st = got
+    assert (st == wfe.PAIR_OK).all(), f"{(st != wfe.PAIR_OK).sum()} of {len(pairs)} pairs, statuses {np.unique(st)}"
+    step = slice(None, None, max(1, len(pairs) // some))
+    compare_with_oracle(ascii, pairs[step], stride, dist[step], cg[step], st[step])
+
+
+@pytest.mark.parametrize("p", [.04, .12, .3])  # list 1 full and lists past it; most pairs past it; list 1 empty
+def test_prediction_from_tier_1(p):
+    """Routing by predicted distance puts pairs in the lists past the first
+    tier's, which a plan from tier 1 does not look at."""
+    torch_cuda()
+    ascii, pairs = wfe.generate(50_000, 1000, p_min=p, p_max=p, seed=3)
+    with wfe.Context(max_seq_len=1200, cigar_stride=1400, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        ctx.set_policy([1200], [1], predict=True)
+        check(ascii, pairs, 1400, align_device(ctx, ascii, pairs, 1200, 1400), 400)
