@@ -631,10 +631,11 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     bk.totals = ctx->d_bucket_total;
     /* Tier 5's scan and classes do not depend on the bucket's length: the
      * last bucket's chain takes the tier-5 pairs of all buckets, one scan and
-     * one launch of the classes instead of one per bucket. */
+     * one launch of the classes instead of one per bucket.  Not a chain that is
+     * planned from tier 1, which takes that list alone. */
     const BucketPlan& lp = ctx->bucket[ctx->nbuckets - 1];
     const int lt = bk.first_tier[ctx->nbuckets - 1];
-    const bool merge = ctx->bound && lt <= 5 && lp.bound.grid > 0 && lp.cls.scan.grid > 0 &&
+    const bool merge = ctx->bound && lt <= 5 && start[ctx->nbuckets - 1] != kPlanned1 && lp.bound.grid > 0 && lp.cls.scan.grid > 0 &&
                        chain_end(ctx->cfg, lt, lp.last_tier) >= 5;
     bk.tier5_to = merge ? ctx->nbuckets - 1 : -1;
     WFE_CUDA(ctx, launch_classify(L, n, bk, s));

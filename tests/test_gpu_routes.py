@@ -10,6 +10,20 @@ from test_gpu_parity import compare_with_oracle, torch_cuda
 pytestmark = pytest.mark.gpu
 
 
+def joined(*sets):
+    """The pairs of several generated sets as one, dealt in turn."""
+    ascii = np.concatenate([a for a, _ in sets])
+    shifted, at = [], 0
+    for a, p in sets:
+        q = p.copy()
+        q["p_off"] += at
+        q["t_off"] += at
+        shifted.append(q)
+        at += len(a)
+    pairs = np.concatenate(shifted)
+    return ascii, pairs[np.random.default_rng(1).permutation(len(pairs))]
+
+
 def align_device(ctx, ascii, pairs, max_len, stride):
     torch = torch_cuda()
     n = len(pairs)
@@ -36,4 +50,17 @@ def test_prediction_from_tier_1(p):
     ascii, pairs = wfe.generate(50_000, 1000, p_min=p, p_max=p, seed=3)
     with wfe.Context(max_seq_len=1200, cigar_stride=1400, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
         ctx.set_policy([1200], [1], predict=True)
+        check(ascii, pairs, 1400, align_device(ctx, ascii, pairs, 1200, 1400), 400)
+
+
+@pytest.mark.parametrize("n_long", [0, 20_000])  # an empty last bucket; one whose pairs the plan gives to tier 5
+def test_tier_5_bucket_below_a_planned_one(n_long):
+    """The last bucket's chain, planned from tier 1, beside a bucket that starts at tier 5."""
+    torch_cuda()
+    sets = [wfe.generate(40_000 - n_long, 100, 440, p_min=.01, p_max=.15, seed=4)]
+    if n_long:
+        sets.append(wfe.generate(n_long, 700, 1000, p_min=.1, p_max=.15, seed=5))
+    ascii, pairs = joined(*sets)
+    with wfe.Context(max_seq_len=1200, cigar_stride=1400, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        ctx.set_policy([512, 1200], [5, 1])
         check(ascii, pairs, 1400, align_device(ctx, ascii, pairs, 1200, 1400), 400)
