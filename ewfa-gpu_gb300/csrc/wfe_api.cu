@@ -573,11 +573,14 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     if (n == 0) return WFE_OK;
     const uint32_t B = ctx->cfg.batch_size;
     const auto clear_counts = [&] { return cudaMemsetAsync(st.d_counts, 0, sizeof(uint32_t) * kCountWords, s); };
-    if (st.counts_dirty) WFE_CUDA(ctx, clear_counts());
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (st.counts_dirty) WFE_CUDA(ctx, cudaStreamIsCapturing(s, &capture));
+    WFE_CUDA(ctx, cudaStreamIsCapturing(s, &capture));
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
+    /* a captured batch may be replayed after one whose launches failed part-way:
+     * it clears the counters itself */
+    if (capturing || st.counts_dirty) WFE_CUDA(ctx, clear_counts());
     /* until all is enqueued; a memset that was only captured has not run */
-    const bool still_dirty = capture != cudaStreamCaptureStatusNone;
+    const bool still_dirty = capturing && st.counts_dirty;
     st.counts_dirty = true;
     bool cleared = false;
     if (ctx->nbuckets == 1 && !ctx->predict) {

@@ -1,6 +1,8 @@
 """Calls whose pairs are routed to several lists of a chain: every pair is
 aligned, whichever kernel the chain starts with.  Outputs hold other values
 before each call, so that a pair that no kernel takes is seen."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -64,3 +66,34 @@ def test_tier_5_bucket_below_a_planned_one(n_long):
     with wfe.Context(max_seq_len=1200, cigar_stride=1400, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
         ctx.set_policy([512, 1200], [5, 1])
         check(ascii, pairs, 1400, align_device(ctx, ascii, pairs, 1200, 1400), 400)
+
+
+@pytest.mark.parametrize("n", [64, 900])  # one batch; three, on two streams
+def test_captured_call_clears_its_counters(n):
+    """A captured call begins by clearing the counters of its batches, so that
+    a replay does not depend on how the batch before it ended."""
+    torch = torch_cuda()
+    cuda = ctypes.CDLL("libcuda.so.1")
+    ascii, pairs = wfe.generate(n, 150, p_min=.05, p_max=.05, seed=6)
+    d_a, d_p = torch.from_numpy(ascii).cuda(), torch.from_numpy(pairs.view(np.uint8)).cuda()
+    out = (torch.full((n,), -7, dtype=torch.int32, device="cuda"), torch.zeros((n, 152), dtype=torch.int8, device="cuda"),
+           torch.full((n,), 99, dtype=torch.uint8, device="cuda"))
+    with wfe.Context(max_seq_len=200, cigar_stride=152, batch_size=300, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.stream(stream):
+            ctx.align_device(d_a, d_p, n, 200, *out, stream)
+            stream.synchronize()
+            for x in out:
+                x.fill_(99)
+            with torch.cuda.graph(graph, stream=stream):
+                ctx.align_device(d_a, d_p, n, 200, *out, stream)
+            roots, count = (ctypes.c_void_p * 8)(), ctypes.c_size_t(8)
+            assert cuda.cuGraphGetRootNodes(ctypes.c_void_p(graph.raw_cuda_graph()), roots, ctypes.byref(count)) == 0
+            kinds = [ctypes.c_int(-1) for _ in range(count.value)]
+            assert all(cuda.cuGraphNodeGetType(ctypes.c_void_p(r), ctypes.byref(k)) == 0 for r, k in zip(roots, kinds))
+            assert kinds and all(k.value == 2 for k in kinds)  # CU_GRAPH_NODE_TYPE_MEMSET
+            graph.instantiate()
+            for _ in range(2):
+                graph.replay()
+        stream.synchronize()
+    check(ascii, pairs, 152, tuple(x.cpu().numpy() for x in out), n)
