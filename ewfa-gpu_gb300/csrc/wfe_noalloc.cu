@@ -11,18 +11,19 @@
  * backtrace store of the pairs in flight, lives in the fixed array below,
  * which every GPU that loads this library holds until the process exits.
  *
- * The pairs go through two of the tiers, in rounds of up to 2^20 pairs:
- * tier 0 (a thread per pair, distances up to 31, all its state in shared
- * memory, so it needs none of the array) aligns every pair, and hands the
- * ones past distance 31 on, through a list at the start of the array, to
- * the tier-3 kernel (32 lanes per pair, distances up to 271, backtrace store
- * in global memory), pointed at the rest of the array.  A pair's store there
- * takes 20,544 bytes (a triangle of 271 rows), so the rest holds the stores
- * of 612 pairs in flight, 153 CTAs of 4 pairs; that grid is sized so that
- * every resident group has its own slot (about one CTA per SM on a GB300,
- * below the kernel's occupancy: the price of the fixed size, paid only by
- * the pairs past distance 31).  With a max_distance of 31 or less tier 0
- * does all of it.
+ * The pairs go through two of the tiers, in rounds of up to 2^20 pairs.  The
+ * first, tier 0 (a thread per pair, distances up to 31) or tier 1 (32 lanes per
+ * pair, up to 79; see first_tier_for), keeps its state in shared memory, so it
+ * needs none of the array.  It aligns every pair, and hands the ones past its
+ * distance on, through a list at the start of the array, to the tier-3 kernel
+ * (32 lanes per pair, distances up to 271, backtrace store in global memory),
+ * pointed at the rest of the array.  A pair's store there takes 20,544 bytes (a
+ * triangle of 271 rows), so the rest holds the stores of 612 pairs in flight,
+ * 153 CTAs of 4 pairs; that grid is sized so that every resident group has its
+ * own slot (about one CTA per SM on a GB300, below the kernel's occupancy: the
+ * price of the fixed size, paid only by the pairs handed on).  With a
+ * max_distance within the first tier's it does all of it; some calls go to
+ * tier 3 alone.
  */
 #include <algorithm>
 #include <mutex>
@@ -35,7 +36,6 @@
 namespace {
 
 constexpr size_t kNoallocScratchBytes = (size_t)WFE_NOALLOC_SCRATCH_BYTES;
-constexpr int kFirstTier = 0;
 constexpr int kNoallocTier = 3;
 /* the array: the hand-on list of one round, its count, the tier-3 stores */
 constexpr uint32_t kRoundPairs = 1u << 20;
@@ -128,6 +128,29 @@ cudaError_t scratch_address(void** out)
     return cudaSuccess;
 }
 
+/* The tier that takes a call's pairs first: tier 0, whose time is a sequence's
+ * length in columns, where its sequences are short or its pairs many; tier 1,
+ * whose time is the distance in scores, else; or tier 3 alone.  Microseconds, at
+ * 0.2, 1, 5 and 12% edits:
+ *   6,000 pairs of 150 bases: tier 0 21 22 26 88, tier 1 18 22 35 59; of 220: 33
+ *     35 45 117 and 20 25 44 80; of 300: 47 51 58 481 and 22 28 54 104
+ *   20,000 of 300: 59 62 70 1376 and 45 60 139 292
+ *   20,000 of 400: 71 75 144 2416 and 50 72 179 402; 100,000: 184 193 284 11552 and
+ *     192 289 795 1870
+ *   100,000 of 600: 299 315 3424 18319 and 275 419 1281 4619
+ *   6,000 of 3,000 at 0.2, 1, 5%: 311 636 3326 and 78 146 3478, tier 3 alone 244 559
+ *     2635; of 4,000: 800 1574 5214, 104 205 5070 and 314 767 3961
+ * Tier 3 alone has room for 816 pairs at once (600 of 600 bases at 12%: tier 1
+ * first 236, tier 3 alone 150; at 1% 27 and 30), and sequences past 3,500 bases
+ * are rarely within distance 79. */
+constexpr uint32_t kColumnsLength = 224, kScoresLength = 3500;
+constexpr size_t kFewPairs = 816;
+int first_tier_for(size_t n, uint32_t max_len)
+{
+    if (max_len <= kColumnsLength || (max_len <= 400u && n >= 8192u) || (max_len <= 512u && n >= 32768u)) return 0;
+    return max_len > kScoresLength || (max_len > 256u && n <= kFewPairs) ? kNoallocTier : 1;
+}
+
 }  // namespace
 
 extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_pairs, size_t n,
@@ -154,16 +177,18 @@ extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_p
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return WFE_ERR_CUDA;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    /* tier 0: its occupancy (its state is in shared memory).  Sequences of
-     * more than about 9,000 bases do not fit there, and tier 3 aligns every
-     * pair. */
-    const wfe::TierShape sh0 = wfe::tier_shape(kFirstTier, max_len, cigar_stride, sms);
+    /* the first tier: its occupancy (its state is in shared memory) */
+    int ft = first_tier_for(n, max_len);
     wfe::TierShape sh = wfe::tier_shape(kNoallocTier, max_len, cigar_stride, sms);
-    /* few pairs of sequences past 256 bases: tier 3 takes them in one wave, in
-     * less time than tier 0 needs for the length of the sequences in columns */
-    const bool first = sh0.grid > 0 && !(n <= 512u && max_len > 256u && sh.grid > 0);
-    const bool deep = !first || max_distance > wfe::tier_info(kFirstTier).dcap;
-    const bool listed = first && deep; /* tier 3 over the pairs tier 0 handed on */
+    wfe::TierShape sh0 = ft < kNoallocTier ? wfe::tier_shape(ft, max_len, cigar_stride, sms) : wfe::TierShape{};
+    if (sh0.grid <= 0 && (ft == 1 || sh.grid <= 0)) {
+        /* CIGAR slots too wide to be staged in shared memory: tier 0 keeps none there */
+        ft = 0;
+        sh0 = wfe::tier_shape(ft, max_len, cigar_stride, sms);
+    }
+    const bool first = sh0.grid > 0;
+    const bool deep = !first || max_distance > wfe::tier_info(ft).dcap;
+    const bool listed = first && deep; /* tier 3 over the pairs that the first tier handed on */
 
     /* tier 3: occupancy, capped by the op-store slots of the array; every
      * group's store holds all rows of the tier (distances up to 271) */
@@ -192,15 +217,15 @@ extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_p
         a.max_len = max_len;
         a.passed_total = nullptr; /* a.chain.cta_done stays NULL: the host starts each tier */
         if (first) {
-            /* tier 0 over the round, the pairs past its reach to the list */
+            /* the first tier over the round, the pairs past its reach to the list */
             if (listed && cudaMemsetAsync(count, 0, sizeof(uint32_t), s) != cudaSuccess) return WFE_ERR_CUDA;
-            a.tier = kFirstTier;
+            a.tier = ft;
             a.retry = listed ? list : nullptr;
             a.retry_count = listed ? count : nullptr;
-            a.chain.shape[kFirstTier] = sh0;
-            const uint32_t per_cta0 = (uint32_t)wfe::tier_info(kFirstTier).pairs_per_cta;
+            a.chain.shape[ft] = sh0;
+            const uint32_t per_cta0 = (uint32_t)wfe::tier_info(ft).pairs_per_cta;
             const int grid0 = (int)std::min<uint64_t>((uint64_t)sh0.grid, ((uint64_t)nb + per_cta0 - 1) / per_cta0);
-            if (wfe::launch_tier(kFirstTier, a, std::max(grid0, 1), s) != cudaSuccess) return WFE_ERR_CUDA;
+            if (wfe::launch_tier(ft, a, std::max(grid0, 1), s) != cudaSuccess) return WFE_ERR_CUDA;
         }
         if (!deep) continue;
         /* tier 3 over the list (its count is read on the device), or over

@@ -357,15 +357,16 @@ int wfe_cigar_from_history_device(const char* d_ascii, const wfe_pair* d_pairs,
  * device's primary context, or one the application made current); the first
  * call in each context looks that address up (set-up, once per context),
  * so make that first call outside any stream capture.  The pairs are aligned
- * in rounds of up to 2^20: tier 0 (a thread per pair, distances up to 31, all
- * its state in shared memory) takes every pair of a round and hands the ones
- * past distance 31, through a list at the start of the array, to the 32-lane
- * tier 3, whose backtrace stores fill the rest: 612 pairs in flight, 153
- * CTAs of 4 (about one per SM on a 152-SM GB300, below that kernel's
- * occupancy).  Sequences too long for tier 0's shared memory (past 9,000
- * bases), and calls of up to 512 pairs of more than 256 bases, go to tier 3
- * alone (816 pairs in flight).  On short reads a call of 300,000 pairs takes
- * 1.2 times as long as wfe_align_device.
+ * in rounds of up to 2^20: a first tier whose state is all in shared memory --
+ * tier 0 (a thread per pair, distances up to 31) for sequences of up to 224
+ * bases, and of up to 512 in large calls, tier 1 (32 lanes per pair, distances
+ * up to 79) for others -- takes every pair of a round and hands the ones past its
+ * distance, through a list at the start of the array, to the 32-lane tier 3,
+ * whose backtrace stores fill the rest: 612 pairs in flight, 153 CTAs of 4
+ * (about one per SM on a 152-SM GB300, below that kernel's occupancy).
+ * Sequences of more than 3,500 bases, and calls of up to 816 pairs of more than
+ * 256 bases, go to tier 3 alone (816 pairs in flight).  On short reads a call of
+ * 300,000 pairs takes 1.2 times as long as wfe_align_device.
  * Every call shares the array and it keeps the last call's contents
  * (nothing in it has to start at zero: the list's count is set by a
  * cudaMemsetAsync on `stream` each round, and every other entry is written

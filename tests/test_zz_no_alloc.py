@@ -162,3 +162,41 @@ def test_noalloc_without_status_or_cigars():
     torch.cuda.synchronize()
     od, _, _, _ = oracle.align_batch(a, p["p_off"], p["p_len"], p["t_off"], p["t_len"], 152, max_distance=63)
     np.testing.assert_array_equal(dist.cpu().numpy(), od)
+
+
+@pytest.mark.parametrize("max_len,n,cap", [
+    (224, 600, 271), (225, 600, 271), (225, 600, 79), (256, 816, 80), (257, 816, 271), (257, 817, 31),
+    (400, 8191, 80), (400, 8192, 79), (400, 8192, 31), (401, 8192, 271), (512, 32768, 79), (3500, 817, 271), (3501, 817, 79)])
+def test_noalloc_first_tier_by_length_and_pairs(max_len, n, cap):
+    """Either side of the lines between the first tiers, with distances either
+    side of what each takes and search ranges that end at one of them."""
+    import torch
+
+    long = min(max_len, 40 + 2 * cap) if n > 817 else max_len
+    a, p = wfe.generate(n, max(60, long // 3), int(long / 1.15), p_min=0.0, p_max=0.05 if max_len > 3000 else 0.4, seed=n)
+    d, s = _both(a, p, max_len, cap, 2 * max_len, torch.cuda.Stream())
+    assert (s == wfe.PAIR_OK).any() and (d <= 31).any() and (cap <= 31 or (d > 31).any())
+
+
+def test_noalloc_slots_too_wide_for_shared_memory():
+    """CIGAR slots that tiers 1 and 3 cannot stage, within tier 0's distances: tier 0 alone, however few the pairs."""
+    import torch
+
+    import oracle
+
+    stride = 1 << 16
+    a, p = wfe.generate(700, 200, 300, p_min=0.0, p_max=0.05, seed=8)
+    od, ocg, ost, _ = oracle.align_batch(a, p["p_off"], p["p_len"], p["t_off"], p["t_len"], 800, max_distance=31)
+    d_a, d_p = torch.from_numpy(a).cuda(), torch.from_numpy(p.view(np.uint8)).cuda()
+    for n in (300, 700):
+        dist = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+        cg = torch.full((n, stride), 55, dtype=torch.int8, device="cuda")
+        st = torch.full((n,), 99, dtype=torch.uint8, device="cuda")
+        wfe.align_device_noalloc(d_a, d_p, n, 400, 31, dist, cg, stride, st, None)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(dist.cpu().numpy(), od[:n])
+        np.testing.assert_array_equal(st.cpu().numpy(), ost[:n])
+        got = cg[:, :800].cpu().numpy()
+        assert (ost == wfe.PAIR_OK).any()
+        for i in np.flatnonzero(ost[:n] == wfe.PAIR_OK):
+            assert _cigar_bytes(got[i]) == _cigar_bytes(ocg[i]), f"pair {i}"
