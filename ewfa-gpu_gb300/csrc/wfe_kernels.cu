@@ -1012,8 +1012,7 @@ __global__ void __maxnreg__(144) band_kernel(const __grid_constant__ AlignLaunch
             forward([&](int m, int out) { return band_rows_call(P, planeP, T, planeT, m, b, vp, vn, first, out); });
         if constexpr (PREDICT) {
             if (item < count)
-                A.pred[pi] = (uint16_t)(state == ST_RUN ? min(D, kBandDistance + 1)
-                                        : state == past ? kBandDistance + 1 : 0xffff);
+                A.pred[pi] = (uint16_t)(state == ST_RUN ? min(D, kPredictMost) : state == past ? kPredictMost : 0xffff);
             wb += gridDim.x * 32u;
             __syncwarp();
             continue;

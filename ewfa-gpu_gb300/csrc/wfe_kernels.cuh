@@ -146,6 +146,11 @@ constexpr int kDeferByte = kNumTiers;
  * be routed to by its predicted distance. */
 constexpr int kMaxBuckets = 8;
 constexpr int kPredictPrefix = 128; /* bases of each sequence the distance prediction aligns */
+/* The largest prefix distance that a prediction is made from: a few pairs whose
+ * edits lie in their first bases would else start a tier of their own, two
+ * above the others' (1,000 pairs of 935 bases at 12%: 541 us with prefix
+ * distances up to 32, 315 so). */
+constexpr int kPredictMost = 23;
 struct Buckets {
     int n;
     uint32_t max_len[kMaxBuckets];   /* ascending; a pair goes to the first bucket that holds it */
@@ -245,8 +250,8 @@ LongClasses long_classes(uint32_t max_len, int sm_count, uint64_t scratch_bytes)
  * bucket, into the tier of their predicted distance (see Buckets). */
 cudaError_t launch_classify(const Layout& L, uint32_t n, const Buckets& B, cudaStream_t s);
 
-/* Distance of the first kPredictPrefix bases of every pair (capped at
- * tier 0's limit + 1), for routing: pred[i] for pair i. */
+/* Distance of the first kPredictPrefix bases of every pair (up to
+ * kPredictMost), for routing: pred[i] for pair i. */
 cudaError_t launch_predict(const Layout& L, uint32_t n, uint32_t max_len, uint16_t* pred, int grid,
                            cudaStream_t s);
 

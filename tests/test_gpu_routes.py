@@ -97,3 +97,13 @@ def test_captured_call_clears_its_counters(n):
                 graph.replay()
         stream.synchronize()
     check(ascii, pairs, 152, tuple(x.cpu().numpy() for x in out), n)
+
+
+def test_prediction_of_edits_in_the_first_bases():
+    """A few pairs have twice the edits in their first bases: they start no tier of their own."""
+    ascii, pairs = wfe.generate(1000, 935, p_min=.12, p_max=.12, seed=5)
+    with wfe.Context(max_seq_len=1100, cigar_stride=1100, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        ctx.set_policy([1100], [1], predict=True)
+        got = align_device(ctx, ascii, pairs, 1100, 1100)
+        assert list(ctx.stats()["tier_launches"][3:7]) == [1, 0, 0, 0]
+    check(ascii, pairs, 1100, got, 1000)
