@@ -103,8 +103,8 @@ struct BucketPlan {
 };
 
 /* Running counters on the device: pairs handed on and launches per tier, pairs
- * per bucket, pairs of planned launches per first tier. */
-constexpr size_t kDevCounters = 3 * kNumTiers + kMaxBuckets;
+ * of planned launches and of buckets per first tier. */
+constexpr size_t kDevCounters = 3 * kNumTiers;
 
 struct wfe_ctx {
     wfe_config cfg{};
@@ -138,8 +138,7 @@ struct wfe_ctx {
     uint64_t long_slab[kNumTiers] = {};
     unsigned long long* d_passed = nullptr;    /* pairs each tier handed on, running total */
     unsigned long long* d_launched = nullptr;  /* tier launches made on the device */
-    unsigned long long* d_bucket_total = nullptr; /* pairs classified into each bucket */
-    unsigned long long* d_entered = nullptr;   /* pairs of planned launches by first tier */
+    unsigned long long* d_entered = nullptr;   /* pairs of planned launches and of buckets by first tier */
     uint8_t* h_launch_error = nullptr;         /* byte t: a device-side launch of tier t failed */
     uint8_t* d_launch_error = nullptr;         /* its device address */
     bool launch_error_pinned = false;          /* from cudaHostAlloc (else new[]: pageable memory the
@@ -533,7 +532,7 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
  * pair need a few microseconds for a few scores where tier 0 needs the length
  * of the sequences in columns (300 bases: 31 us against 61 for up to 4,096
  * pairs, the same at 16,384; 150 bases: 34 and 37 at 1,024, 41 and 37 at
- * 4,096).  A large batch of sequences past kPlanLength bases is planned
+ * 4,096; 64 of 600-1,050 bases at 0.5% in two buckets 16 and 64).  A large batch of sequences past kPlanLength bases is planned
  * (kPlanned): its error rate decides.  Other device batches of up to 512 bases
  * start at tier 0 from 12,288 pairs on (20,000 pairs of 240-330 bases at 4-7%:
  * 58 us in a row against 92 from tier 1, alone 167 against 131; at 0.5% 34 and
@@ -542,7 +541,9 @@ int first_tier_of(const wfe_ctx* ctx, const BucketPlan& bp, uint32_t n, bool dev
 {
     if (!bp.by_length || bp.first_tier != 0 || bp.shape[1].grid <= 0) return bp.first_tier;
     if (n < 4096u) return n < 11u * bp.max_len - std::min(1200u, 11u * bp.max_len) ? 1 : 0;
-    if (!device_call) return 0;
+    /* how many of a larger batch are in one of several buckets, or predicted
+     * within a tier, is not known here */
+    if (!device_call || ctx->nbuckets > 1 || ctx->predict) return 0;
     if (can_plan(ctx, bp, device_call)) return kPlanned;
     return n < (bp.max_len > 512u ? 32768u : bp.max_len > kOrderLength ? 12288u : 0u) ? 1 : 0;
 }
@@ -599,7 +600,8 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     int start[kMaxBuckets];
     for (int b = 0; b < ctx->nbuckets; ++b) {
         bk.max_len[b] = ctx->bucket[b].max_len;
-        bk.first_tier[b] = first_override ? first_override[b] : ctx->bucket[b].first_tier;
+        bk.first_tier[b] = first_override ? first_override[b] : first_tier_of(ctx, ctx->bucket[b], n, device_call);
+        bk.entered_tier[b] = bk.first_tier[b];
         start[b] = from_tier_1(ctx, ctx->bucket[b], bk.first_tier[b], n, device_call);
         if (start[b] == kBandFirst) bk.first_tier[b] = 0;
         /* routing never goes past the end of the bucket's chain */
@@ -631,7 +633,7 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
     bk.stride = B;
     bk.counts = st.d_counts;
     bk.count_stride = (uint32_t)kChainWords;
-    bk.totals = ctx->d_bucket_total;
+    bk.entered = ctx->d_entered;
     /* Tier 5's scan and classes do not depend on the bucket's length: the
      * last bucket's chain takes the tier-5 pairs of all buckets, one scan and
      * one launch of the classes instead of one per bucket.  Not a chain that is
@@ -788,8 +790,7 @@ int create_context(const wfe_config* cfg, uint64_t budget5, uint64_t budget6, wf
     if (!bucket_usable(ctx->bucket[0])) return bail(cudaErrorInvalidValue); /* sequences too long for shared memory */
 
     ctx->d_launched = ctx->d_passed + kNumTiers;
-    ctx->d_bucket_total = ctx->d_passed + 2 * kNumTiers;
-    ctx->d_entered = ctx->d_bucket_total + kMaxBuckets;
+    ctx->d_entered = ctx->d_passed + 2 * kNumTiers;
     /* The record of failed device-side launches is host memory the kernels
      * write in place.  A device that reads the CPU's page tables (ATS over
      * NVLink-C2C) writes ordinary heap memory; elsewhere it is a mapped
@@ -938,11 +939,10 @@ int wfe_get_stats(wfe_ctx* ctx, wfe_stats* out)
     out->deep_scratch_bytes = ctx->deep_bytes;
     for (int t = 0; t < kNumTiers; ++t) {
         out->tier_passed[t] = dev[t];
-        out->tier_entered[t] = ctx->single_entered[t] + (t > 0 ? dev[t - 1] : 0) + dev[2 * kNumTiers + kMaxBuckets + t];
+        out->tier_entered[t] = ctx->single_entered[t] + (t > 0 ? dev[t - 1] : 0) + dev[2 * kNumTiers + t];
         out->tier_launches[t] += dev[kNumTiers + t];
         out->kernel_launches += dev[kNumTiers + t];
     }
-    for (int b = 0; b < ctx->nbuckets; ++b) out->tier_entered[ctx->bucket[b].first_tier] += dev[2 * kNumTiers + b];
     return WFE_OK;
 }
 

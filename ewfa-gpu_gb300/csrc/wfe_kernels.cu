@@ -2622,11 +2622,9 @@ __global__ void __launch_bounds__(256) classify_kernel(Layout L, uint32_t n, Buc
             const int b = key / kListsPerBucket, t = key % kListsPerBucket;
             base = atomicAdd(B.counts + (size_t)b * B.count_stride + t, (uint32_t)__popc(same));
         }
-        if (B.totals) {
-            const unsigned alike = __match_any_sync(kFull, bucket);
-            if (bucket >= 0 && lane == __ffs((int)alike) - 1)
-                atomicAdd(B.totals + bucket, (unsigned long long)__popc(alike));
-        }
+        const unsigned alike = __match_any_sync(kFull, bucket);
+        if (bucket >= 0 && lane == __ffs((int)alike) - 1)
+            atomicAdd(B.entered + B.entered_tier[bucket], (unsigned long long)__popc(alike));
         base = __shfl_sync(kFull, base, leader);
         if (key >= 0) {
             const uint32_t rank = (uint32_t)__popc(same & ((1u << lane) - 1u));

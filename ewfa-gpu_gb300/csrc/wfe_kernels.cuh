@@ -164,7 +164,8 @@ struct Buckets {
     uint32_t count_stride;
     int to[kMaxBuckets];             /* bucket whose lists take a bucket's pairs */
     int tier5_to;                    /* bucket whose tier-5 list takes the tier-5 pairs of all (-1: each its own) */
-    unsigned long long* totals;      /* pairs classified into each bucket (stats) */
+    unsigned long long* entered;     /* pairs per tier that their buckets count as first (stats) */
+    int entered_tier[kMaxBuckets];   /* that tier of each bucket */
 };
 
 /* First kernels that a plan chooses between. */

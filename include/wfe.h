@@ -213,10 +213,11 @@ int wfe_reset_stats(wfe_ctx* ctx);
  * classes (for comparison: results are the same).  As many pairs as the
  * GPU has SMs are aligned without it, too.
  * A bucket whose tier is left to its length (-1) and would start at tier 0
- * starts small batches at tier 1, and device calls of many pairs past 400 bases
- * at tier 0, 1 or 5, as a sample of the batch says on the device.  Large
- * batches of a bucket whose first tier is 1 may go through tier 0's kernel on
- * the way, or start at tier 5; their pairs count as tier 1's.
+ * starts batches of few pairs at tier 1.  Where it is the only bucket and
+ * nothing is predicted, device calls of many pairs past 400 bases start at tier
+ * 0, 1 or 5, as a sample of the batch says on the device.  Large batches of a
+ * bucket whose first tier is 1 may go through tier 0's kernel on the way, or,
+ * without predictions, start at tier 5; their pairs count as tier 1's.
  * Replaces nothing in the reference, which has one fixed launch shape
  * (src/wavefront.cu:173-208); see also wfe_autotune. */
 #define WFE_POLICY_PREDICT 1u  /* route every pair to the tier of its predicted distance */

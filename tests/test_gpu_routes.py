@@ -107,3 +107,15 @@ def test_prediction_of_edits_in_the_first_bases():
         got = align_device(ctx, ascii, pairs, 1100, 1100)
         assert list(ctx.stats()["tier_launches"][3:7]) == [1, 0, 0, 0]
     check(ascii, pairs, 1100, got, 1000)
+
+
+@pytest.mark.parametrize("buckets,lo,hi,predict", [([512, 1200], 600, 1000, False), ([512, 1200], 300, 450, False),
+                                                   ([150, 300], 70, 120, False), ([512, 1200], 600, 1000, True)])
+def test_small_batches_of_buckets_left_to_their_lengths(buckets, lo, hi, predict):
+    """Batches of few pairs start at tier 1, with several buckets as with one."""
+    ascii, pairs = wfe.generate(64, lo, hi, p_min=.005, p_max=.005, seed=7)
+    with wfe.Context(max_seq_len=buckets[-1], cigar_stride=1200, flags=wfe.FLAG_DEVICE_ONLY) as ctx:
+        ctx.set_policy(buckets, predict=predict)
+        got = align_device(ctx, ascii, pairs, buckets[-1], 1200)
+        assert list(ctx.stats()["tier_entered"][:2]) == [0, 64]
+    check(ascii, pairs, 1200, got, 64)
