@@ -91,28 +91,26 @@ __device__ __forceinline__ PairRef get_pair(const Layout& L, uint32_t i)
     return r;
 }
 
-/* Packed word w of a sequence of len bytes at s, produced by a group of G
- * lanes, words w0+g for g in [0, G).  The sequence is read in aligned 16-byte
- * blocks (every block holds at least one base of the sequence); the bytes
- * before s are shifted out and the bases at or past len are cleared.
- * Returns the word for lane g (0 if w0+g >= nw).  All lanes of `mask` call. */
-template <int G>
-__device__ __forceinline__ uint32_t packed_word(const char* s, uint32_t len,
-                                                uint32_t w0, int g, unsigned mask)
+/* Packed words w0 .. w0+31 of a sequence of len bytes at s, one per lane of a
+ * warp.  The sequence is read in aligned 16-byte blocks (every block holds at
+ * least one base of the sequence); the bytes before s are shifted out and the
+ * bases at or past len are cleared.  Returns the lane's word (0 past the last).
+ * All lanes call. */
+__device__ __forceinline__ uint32_t packed_word(const char* s, uint32_t len, uint32_t w0, int lane)
 {
     const uint32_t nw = (len + 15u) >> 4;
     const uintptr_t a = reinterpret_cast<uintptr_t>(s);
     const uint32_t sh = (uint32_t)(a & 15u);
     const uint4* base = reinterpret_cast<const uint4*>(a - sh);
     const uint32_t nblk = (sh + len + 15u) >> 4;
-    const uint32_t w = w0 + (uint32_t)g;
+    const uint32_t w = w0 + (uint32_t)lane;
     uint32_t x0 = 0;
     if (w < nw) x0 = pack16(__ldg(base + w));
-    const uint32_t nb = __shfl_down_sync(mask, x0, 1, G);
+    const uint32_t nb = __shfl_down_sync(kFull, x0, 1);
     uint32_t W = x0;
     if (sh != 0) {
         uint32_t x1 = nb;
-        if (g == G - 1 || w + 1 >= nw) x1 = (w + 1 < nblk) ? pack16(__ldg(base + w + 1)) : 0u;
+        if (lane == 31 || w + 1 >= nw) x1 = (w + 1 < nblk) ? pack16(__ldg(base + w + 1)) : 0u;
         W = __funnelshift_l(x1, x0, 2u * sh);
     }
     if (w < nw) {
@@ -124,15 +122,14 @@ __device__ __forceinline__ uint32_t packed_word(const char* s, uint32_t len,
     return W;
 }
 
-/* Pack a sequence into overlapped pairs Q[0..nw) (see top of file) by a
- * group of G lanes; Q[nw-1].x = 0.  When the sequence spans at most RMAX*G
- * aligned blocks, every lane issues all of its block loads first (blocks g,
- * g+G, ...) and the neighbour block for the funnel shift comes from one
- * rotating shuffle per word; longer sequences take the word-by-word loop.
- * The caller syncs the group afterwards. */
-template <int G, int RMAX>
-__device__ __forceinline__ void load_packed(const char* s, uint32_t len, uint2* Q,
-                                            int g, unsigned mask)
+/* Pack a sequence into overlapped pairs Q[0..nw) (see top of file) by a warp;
+ * Q[nw-1].x = 0.  When the sequence spans at most 32 RMAX aligned blocks, every
+ * lane issues all of its block loads first (blocks lane, lane+32, ...) and the
+ * neighbour block for the funnel shift comes from one rotating shuffle per word;
+ * longer sequences take the word-by-word loop.  The caller syncs the warp
+ * afterwards. */
+template <int RMAX>
+__device__ __forceinline__ void load_packed(const char* s, uint32_t len, uint2* Q, int lane)
 {
     const uint32_t nw = (len + 15u) >> 4;
     if (nw == 0) return;
@@ -140,22 +137,22 @@ __device__ __forceinline__ void load_packed(const char* s, uint32_t len, uint2* 
     const uint32_t sh = (uint32_t)(a & 15u);
     const uint4* base = reinterpret_cast<const uint4*>(a - sh);
     const uint32_t nblk = (sh + len + 15u) >> 4;
-    if (nblk <= (uint32_t)(RMAX * G)) {
+    if (nblk <= (uint32_t)(RMAX * 32)) {
         uint32_t x[RMAX + 1];
 #pragma unroll
         for (int r = 0; r < RMAX; ++r) {
-            const uint32_t b = (uint32_t)(g + r * G);
+            const uint32_t b = (uint32_t)(lane + 32 * r);
             x[r] = b < nblk ? pack16(__ldg(base + b)) : 0u;
         }
         x[RMAX] = 0u;
 #pragma unroll
         for (int r = 0; r < RMAX; ++r) {
-            if ((uint32_t)(r * G) >= nw) break;
-            /* block w+1 is lane g+1's block r, or lane 0's block r+1 for the
-             * last lane */
-            const uint32_t y = (g == 0) ? x[r + 1] : x[r];
-            const uint32_t nb = __shfl_sync(mask, y, (g + 1) & (G - 1), G);
-            const uint32_t w = (uint32_t)(g + r * G);
+            if ((uint32_t)(32 * r) >= nw) break;
+            /* block w+1 is the next lane's block r, or lane 0's block r+1 for
+             * the last lane */
+            const uint32_t y = lane == 0 ? x[r + 1] : x[r];
+            const uint32_t nb = __shfl_sync(kFull, y, (lane + 1) & 31);
+            const uint32_t w = (uint32_t)(lane + 32 * r);
             uint32_t W = sh ? __funnelshift_l(nb, x[r], 2u * sh) : x[r];
             if (w < nw) {
                 const uint32_t rem = len - 16u * w;
@@ -165,16 +162,16 @@ __device__ __forceinline__ void load_packed(const char* s, uint32_t len, uint2* 
             }
         }
     } else {
-        for (uint32_t w0 = 0; w0 < nw; w0 += G) {
-            const uint32_t W = packed_word<G>(s, len, w0, g, mask);
-            const uint32_t w = w0 + (uint32_t)g;
+        for (uint32_t w0 = 0; w0 < nw; w0 += 32u) {
+            const uint32_t W = packed_word(s, len, w0, lane);
+            const uint32_t w = w0 + (uint32_t)lane;
             if (w < nw) {
                 Q[w].y = W;
                 if (w > 0) Q[w - 1].x = W;
             }
         }
     }
-    if (g == 0) Q[nw - 1].x = 0u;
+    if (lane == 0) Q[nw - 1].x = 0u;
 }
 
 /* The best of a cell's three candidates, with the operation in the low two
@@ -219,45 +216,34 @@ __device__ __forceinline__ int extend_lane(const uint2* QP, const uint2* QT,
     return h;
 }
 
-/* The same longest common prefix computed by a group of G lanes at once:
- * lane g compares the window 16*g bases further on, a ballot finds the first
- * window that is not a full match.  Returns the run length.  All lanes of
- * the group call with the same arguments.
- * A warp-wide group (G = 32, one pair per warp) first compares the first
- * window on every lane -- the same shared-memory words, so one broadcast
- * read -- and a run shorter than 16 bases, the common case at high error
- * rates, is then known on every lane without the vote and shuffle. */
-template <int G>
-__device__ __forceinline__ int group_extend(const uint2* QP, const uint2* QT, int plen,
-                                            int tlen, int k, int off, int g, int grp,
-                                            unsigned gmask)
+/* The same longest common prefix by a warp: every lane first compares the first
+ * window -- the same shared-memory words, so one broadcast read -- and a run
+ * shorter than 16 bases, the common case at high error rates, is then known on
+ * every lane.  Past that, each lane compares the window 16 * lane bases further
+ * on, and a ballot finds the first that is not a full match.  Returns the run
+ * length.  All lanes call with the same arguments. */
+__device__ __forceinline__ int warp_extend(const uint2* QP, const uint2* QT, int plen, int tlen, int k, int off,
+                                           int lane)
 {
     const int v0 = off - k, h0 = off;
-    int total = 0;
-    if constexpr (G == 32) {
-        int n = 0;
-        if ((unsigned)v0 < (unsigned)plen && (unsigned)h0 < (unsigned)tlen) {
-            const uint32_t x = window(QP, v0) ^ window(QT, h0);
-            n = min(__clz(x) >> 1, min(plen - v0, tlen - h0));
-        }
-        if (n < 16) return n;
-        total = 16;
+    int n = 0;
+    if ((unsigned)v0 < (unsigned)plen && (unsigned)h0 < (unsigned)tlen) {
+        const uint32_t x = window(QP, v0) ^ window(QT, h0);
+        n = min(__clz(x) >> 1, min(plen - v0, tlen - h0));
     }
-    for (;;) {
-        const int v = v0 + total + 16 * g, h = h0 + total + 16 * g;
-        int n = 0;
+    if (n < 16) return n;
+    for (int total = 16;; total += 16 * 32) {
+        const int v = v0 + total + 16 * lane, h = h0 + total + 16 * lane;
+        n = 0;
         if ((unsigned)v < (unsigned)plen && (unsigned)h < (unsigned)tlen) {
             const uint32_t x = window(QP, v) ^ window(QT, h);
             n = min(__clz(x) >> 1, min(plen - v, tlen - h));
         }
-        const unsigned sb = __ballot_sync(gmask, n < 16);
-        const unsigned rel = (G == 32) ? sb : ((sb >> (grp * G)) & ((1u << (G & 31)) - 1u));
-        if (rel) {
-            const int first = __ffs((int)rel) - 1;
-            const int nf = __shfl_sync(gmask, n, first, G);
-            return total + 16 * first + nf;
+        const unsigned ends = __ballot_sync(kFull, n < 16);
+        if (ends) {
+            const int first = __ffs((int)ends) - 1;
+            return total + 16 * first + __shfl_sync(kFull, n, first);
         }
-        total += 16 * G;
     }
 }
 
@@ -267,21 +253,19 @@ __device__ __forceinline__ int8_t op_letter(int op)
 }
 
 /* Encoded CIGAR bytes of steps 0..last of a replayed chain
- * (src/kernels.cu:397-498), by a group of G lanes: runs[d] is the run of M
- * bases before operation d (chain[d], the operation of score d+1).  Lane g
- * takes steps g, g+G, ...: each step's bytes are its run as chunks of at
- * most 127 (-127, ..., -(run % 127)) and then its operation letter (none for
- * step D and for a step at bad_at); an inclusive shuffle scan over the group
- * gives the step's first byte, and every lane writes its own bytes into buf
- * (cap bytes; positions past cap are counted but not written).  Returns the
- * full length on every lane. */
-template <int G>
+ * (src/kernels.cu:397-498), by a warp: runs[d] is the run of M bases before
+ * operation d (chain[d], the operation of score d+1).  A lane takes steps lane,
+ * lane+32, ...: each step's bytes are its run as chunks of at most 127 (-127,
+ * ..., -(run % 127)) and then its operation letter (none for step D and for a
+ * step at bad_at); an inclusive shuffle scan gives the step's first byte, and
+ * every lane writes its own bytes into buf (cap bytes; positions past cap are
+ * counted but not written).  Returns the full length on every lane. */
 __device__ __forceinline__ int encode_runs(const int* runs, const uint8_t* chain, int D, int last, int bad_at,
-                                           int8_t* buf, uint32_t cap, int g, unsigned gmask)
+                                           int8_t* buf, uint32_t cap, int lane)
 {
     int total = 0;
-    for (int base = 0; base <= last; base += G) {
-        const int d = base + g;
+    for (int base = 0; base <= last; base += 32) {
+        const int d = base + lane;
         int r = 0, letter = 0, nb = 0;
         if (d <= last) {
             r = runs[d];
@@ -290,9 +274,9 @@ __device__ __forceinline__ int encode_runs(const int* runs, const uint8_t* chain
         }
         int x = nb;
 #pragma unroll
-        for (int sft = 1; sft < G; sft <<= 1) {
-            const int y = __shfl_up_sync(gmask, x, sft, G);
-            if (g >= sft) x += y;
+        for (int sft = 1; sft < 32; sft <<= 1) {
+            const int y = __shfl_up_sync(kFull, x, sft);
+            if (lane >= sft) x += y;
         }
         uint32_t pos = (uint32_t)(total + x - nb);
         if (d <= last) {
@@ -309,31 +293,30 @@ __device__ __forceinline__ int encode_runs(const int* runs, const uint8_t* chain
                 ++pos;
             }
         }
-        total += __shfl_sync(gmask, x, G - 1, G);
+        total += __shfl_sync(kFull, x, 31);
     }
     return total;
 }
 
 /* Forward replay of an operation chain into an encoded CIGAR
- * (src/kernels.cu:397-498) by a group of G lanes.  chain[d] is the operation
- * of score d+1.
- *   1. In order of d, the run of M bases before operation d comes from a
- *      group-parallel extend from (k, off), starting at (0, 0); runs[d]
- *      keeps it (lane 0 writes).
+ * (src/kernels.cu:397-498) by a warp.  chain[d] is the operation of score
+ * d+1.
+ *   1. In order of d, the run of M bases before operation d comes from
+ *      warp_extend from (k, off), starting at (0, 0); runs[d] keeps it (lane 0
+ *      writes).
  *   2. encode_runs writes the bytes.
  * Returns the full CIGAR length on every lane, or -1 - length if the chain
  * holds a code other than INS/SUB/DEL: the CIGAR then stops after that
  * step's run, like the reference's "Incorrect backtrace" exit
  * (src/kernels.cu:471-478). */
-template <int G>
 __device__ __forceinline__ int replay_chain(const uint2* QP, const uint2* QT, int plen, int tlen,
                                             const uint8_t* chain, int D, int* runs, int8_t* buf,
-                                            uint32_t cap, int g, int grp, unsigned gmask)
+                                            uint32_t cap, int lane)
 {
     int k = 0, off = 0, bad_at = -1;
     for (int d = 0; d <= D; ++d) {
-        const int run = group_extend<G>(QP, QT, plen, tlen, k, off, g, grp, gmask);
-        if (g == 0) runs[d] = run;
+        const int run = warp_extend(QP, QT, plen, tlen, k, off, lane);
+        if (lane == 0) runs[d] = run;
         off += run;
         if (d == D) break;
         const int op = chain[d];
@@ -350,31 +333,29 @@ __device__ __forceinline__ int replay_chain(const uint2* QP, const uint2* QT, in
         }
     }
     const int last = bad_at >= 0 ? bad_at : D;
-    __syncwarp(gmask);
-    const int total = encode_runs<G>(runs, chain, D, last, bad_at, buf, cap, g, gmask);
+    __syncwarp();
+    const int total = encode_runs(runs, chain, D, last, bad_at, buf, cap, lane);
     return bad_at >= 0 ? -1 - total : total;
 }
 
 /* Copy a staged CIGAR of `len` bytes (plus terminator when it fits) from
- * shared to global memory by a group; pads to whole 32-bit words with zeros
+ * shared to global memory by a warp; pads to whole 32-bit words with zeros
  * inside the slot when the slot size allows word stores. */
-template <int G>
-__device__ __forceinline__ void store_cigar(int8_t* stage, uint32_t len, uint32_t cap,
-                                            int8_t* dst, int g, unsigned gmask)
+__device__ __forceinline__ void store_cigar(int8_t* stage, uint32_t len, uint32_t cap, int8_t* dst, int lane)
 {
     uint32_t nbytes = len < cap ? len + 1u : cap;
-    if (g == 0 && len < cap) stage[len] = 0;
+    if (lane == 0 && len < cap) stage[len] = 0;
     if ((cap & 3u) == 0u && (reinterpret_cast<uintptr_t>(dst) & 3u) == 0u) {
         const uint32_t nwords = (nbytes + 3u) >> 2;
-        if (g == 0)
+        if (lane == 0)
             for (uint32_t b = nbytes; b < nwords * 4u; ++b) stage[b] = 0;
-        __syncwarp(gmask);
+        __syncwarp();
         const uint32_t* s32 = reinterpret_cast<const uint32_t*>(stage);
         uint32_t* d32 = reinterpret_cast<uint32_t*>(dst);
-        for (uint32_t i = (uint32_t)g; i < nwords; i += G) d32[i] = s32[i];
+        for (uint32_t i = (uint32_t)lane; i < nwords; i += 32u) d32[i] = s32[i];
     } else {
-        __syncwarp(gmask);
-        for (uint32_t i = (uint32_t)g; i < nbytes; i += G) dst[i] = stage[i];
+        __syncwarp();
+        for (uint32_t i = (uint32_t)lane; i < nbytes; i += 32u) dst[i] = stage[i];
     }
 }
 

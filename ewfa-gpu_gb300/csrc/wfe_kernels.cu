@@ -6,8 +6,8 @@
  *                        diagonals: tier 0, and predicted prefix distances
  *   tier_kernel<Tier>    tiers 1-4: fused load+pack, wavefront compute+extend, bit-packed
  *                        backtrace store, backtrace and CIGAR replay for one
- *                        pair per group of G lanes (src/kernels.cu:27-310 and
- *                        397-625 in one kernel)
+ *                        pair per warp (src/kernels.cu:27-310 and 397-625 in
+ *                        one kernel)
  *   long_kernel<GWF, NT> the same for one pair per CTA of NT threads
  *                        (tiers 5-6), over the target's cone when the pair
  *                        has a distance bound
@@ -23,8 +23,8 @@
  *   history_kernel       CIGARs from the reference's 128-bit histories
  *                        (src/kernels.cu:397-625)
  *
- * Wavefront layout of tier_kernel: lane g of a group holds, in register
- * chunk c (c = 0..2J), diagonal k = G*(c-J) - G/2 + g.  Neighbours k-1 and
+ * Wavefront layout of tier_kernel: lane l of a pair's warp holds, in register
+ * chunk c (c = 0..2J), diagonal k = 32*(c-J) - 16 + l.  Neighbours k-1 and
  * k+1 come from one rotating shuffle each; the lanes at a chunk edge pick up
  * the neighbouring chunk's value.  A chunk is skipped (warp-uniformly) until
  * the wavefront [-d, d] reaches it; lanes outside [-d, d] hold -1, the
@@ -77,40 +77,28 @@ __host__ __device__ constexpr size_t round16(size_t x) { return (x + 15u) & ~siz
 
 /* Backtrace store entry of one chunk of one score step: the two ballots of
  * the warp -- the low and the high bits of the 2-bit operation of every lane's
- * diagonal -- written by lane 0.  Group grp's diagonal g of the chunk is bit
- * grp * G + g.  A warp of several groups (G < 32) keeps one store for all of
- * them, so the ballots are stored as they come, with no per-group shifting and
- * masking in the score loop; the backtrace picks its group's bits. */
+ * diagonal -- written by lane 0.  The chunk's diagonal of lane l is bit l. */
 __device__ __forceinline__ int op_of(uint2 e, int bit)
 {
     return (int)(((e.x >> bit) & 1u) | (((e.y >> bit) & 1u) << 1));
 }
 
-/* One distance tier: G lanes per pair, 2J+1 register chunks, backtrace
- * store in shared (SMEM_OPS) or global memory, sequences of up to RMAX*G
- * aligned 16-byte blocks loaded with all loads in flight at once. */
-template <int G_, int J_, bool SMEM_OPS_, int RMAX_>
+/* One distance tier: a warp per pair, 2J+1 register chunks of 32 diagonals,
+ * backtrace store in shared (SMEM_OPS) or global memory. */
+template <int J_, bool SMEM_OPS_>
 struct Tier {
-    static constexpr int G = G_, J = J_, RMAX = RMAX_;
+    static constexpr int J = J_;
     static constexpr bool SMEM_OPS = SMEM_OPS_;
     static constexpr int NC = 2 * J + 1;
-    static constexpr int DCAP = G * J + G / 2 - 1;
-    static constexpr int GPW = 32 / G;
-    /* Row d of the backtrace store.  The 32-lane tiers keep only the chunks
-     * that score step d touches -- the contiguous range whose diagonals meet
-     * [-d, d] -- row after row (a triangle, 55-68 % of DCAP x NC entries),
-     * which keeps tier 1's store in shared memory small and tiers 2-4's
-     * global scratch mostly in L2.  Tier 0
-     * keeps full rows: its occupancy is set by registers, and it is
-     * issue-bound, so it saves the index arithmetic instead. */
-    static constexpr bool TRI = G == 32;
-    static __host__ __device__ constexpr int chunk_lo(int d)
-    {
-        return !TRI ? 0 : (J - (d - 1 + G / 2) / G < 0 ? 0 : J - (d - 1 + G / 2) / G);
-    }
+    static constexpr int DCAP = 32 * J + 15;
+    /* Row d of the backtrace store: only the chunks that score step d touches
+     * -- the contiguous range whose diagonals meet [-d, d] -- row after row (a
+     * triangle, 55-68 % of DCAP x NC entries), which keeps tier 1's store in
+     * shared memory small and tiers 2-4's global scratch mostly in L2. */
+    static __host__ __device__ constexpr int chunk_lo(int d) { return J - (d + 15) / 32 < 0 ? 0 : J - (d + 15) / 32; }
     static __host__ __device__ constexpr int chunk_hi(int d)
     {
-        return !TRI ? 2 * J : (J + (d + G / 2) / G > 2 * J ? 2 * J : J + (d + G / 2) / G);
+        return J + (d + 16) / 32 > 2 * J ? 2 * J : J + (d + 16) / 32;
     }
     static __host__ __device__ constexpr int row_entries(int d) { return chunk_hi(d) - chunk_lo(d) + 1; }
     /* entries of rows 1..rows */
@@ -120,11 +108,8 @@ struct Tier {
         for (int d = 1; d <= rows && d <= DCAP; ++d) t += row_entries(d);
         return t;
     }
-    /* a group's share of its warp's store (one 8-byte entry per chunk and
-     * score step, shared by the warp's GPW groups) */
-    static constexpr size_t ops_bytes = round16((8u * (size_t)store_entries() + GPW - 1) / GPW);
-    /* one group's store in global scratch (the 32-lane tiers: one group per
-     * warp) for distances up to max_len */
+    static constexpr size_t ops_bytes = round16(8u * (size_t)store_entries());
+    /* one warp's store in global scratch for distances up to max_len */
     static size_t store_bytes(uint32_t max_len)
     {
         return round16(8u * (size_t)store_entries((int)std::min<uint32_t>(max_len, (uint32_t)DCAP)));
@@ -136,12 +121,10 @@ struct Tier {
 
 inline uint32_t seq_words_for(uint32_t max_len) { return std::max<uint32_t>(1u, (max_len + 15u) / 16u); }
 
-/* Shared memory of one group: both sequences, the operation chain, then one
- * region that first holds the group's share of its warp's backtrace store
- * (when it lives in shared memory) and, once the chains have been read from
- * it, the group's CIGAR stage and the runs of the replay.  Within a warp's
- * block the groups' sequences and chains come first, then their union
- * regions one after another, which together hold the warp's store. */
+/* Shared memory of one warp: both sequences, the operation chain, then one
+ * region that first holds the backtrace store (when it lives in shared memory)
+ * and, once the chain has been read from it, the CIGAR stage and the runs of
+ * the replay. */
 template <class T>
 size_t union_bytes(uint32_t cigar_stride)
 {
@@ -150,7 +133,7 @@ size_t union_bytes(uint32_t cigar_stride)
 }
 
 template <class T>
-size_t group_smem_bytes(uint32_t max_len, uint32_t cigar_stride)
+size_t warp_smem_bytes(uint32_t max_len, uint32_t cigar_stride)
 {
     return 16u * (size_t)seq_words_for(max_len) + T::chain_bytes + union_bytes<T>(cigar_stride);
 }
@@ -158,7 +141,7 @@ size_t group_smem_bytes(uint32_t max_len, uint32_t cigar_stride)
 template <class T>
 size_t cta_smem_bytes(uint32_t max_len, uint32_t cigar_stride)
 {
-    return group_smem_bytes<T>(max_len, cigar_stride) * (size_t)(kWarps * T::GPW);
+    return warp_smem_bytes<T>(max_len, cigar_stride) * (size_t)kWarps;
 }
 
 /* The alignment kernel of tiers 1-4.  Chains launch it from the device, so it
@@ -186,16 +169,17 @@ __device__ uint32_t tile_chunks(const LongClasses& C);
 constexpr uint32_t kFewPairs = 384, kSomePairs = 1024;
 __device__ __forceinline__ bool class_by_cta(int dlim, uint32_t count)
 {
-    return count > kFewPairs && (dlim == 257 || (count > kSomePairs && (dlim == 577 || dlim == 961)));
+    constexpr int kMiddle = kCtaClassMiddle[0], kUpper = kCtaClassMiddle[1];
+    return count > kFewPairs && (dlim == kCtaClassShort || (count > kSomePairs && (dlim == kMiddle || dlim == kUpper)));
 }
 __device__ __forceinline__ bool tile_takes(const LongClasses& C, int c, uint32_t count)
 {
     return c + 1 < C.n && C.tile.grid > 0 && count > 0u && !(C.wide[c].grid > 0 && count >= kWidePairs);
 }
-using T1 = Tier<32, 2, true, 1>;   /* distance <= 79  */
-using T2 = Tier<32, 4, false, 1>;  /* distance <= 143; backtrace store in global scratch: 8 CTAs per SM */
-using T3 = Tier<32, 8, false, 1>;  /* distance <= 271 */
-using T4 = Tier<32, 16, false, 1>; /* distance <= 527 */
+using T1 = Tier<2, true>;   /* distance <= 79  */
+using T2 = Tier<4, false>;  /* distance <= 143; backtrace store in global scratch: 8 CTAs per SM */
+using T3 = Tier<8, false>;  /* distance <= 271 */
+using T4 = Tier<16, false>; /* distance <= 527 */
 
 /* Which first kernel a list of `count` pairs takes, from the sums over a
  * sample of it: pairs, bases (of the longer sequence), predicted distances D
@@ -321,9 +305,8 @@ template <class T>
 __device__ __forceinline__ void launch_on_device(const AlignLaunch& A, int u, uint32_t count, bool own_list = false)
 {
     const TierShape& sh = A.chain.shape[u];
-    const uint32_t per_cta = (uint32_t)(kWarps * T::GPW);
+    const uint32_t per_cta = (uint32_t)kWarps;
     const int grid = max(1, min(sh.grid, (int)((count + per_cta - 1u) / per_cta)));
-    static_assert(T::G == 32, "only the 32-lane tiers are launched from the device");
     tail_launch(tier_kernel<T>, A, u, grid, kThreads, sh.smem, true, sh.seq_words, sh.gbytes, 0, own_list);
 }
 
@@ -529,66 +512,52 @@ __device__ __forceinline__ void finish_unaligned(const AlignLaunch& A, uint32_t 
 template <class T>
 __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_words, uint32_t gbytes)
 {
-    constexpr int G = T::G, J = T::J, NC = T::NC, DCAP = T::DCAP, GPW = T::GPW;
+    constexpr int J = T::J, NC = T::NC, DCAP = T::DCAP;
     extern __shared__ __align__(16) unsigned char smem[];
 
     const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
-    const int g = lane & (G - 1), grp = lane / G;
-    const unsigned gmask = (G == 32) ? kFull : (((1u << (G & 31)) - 1u) << (grp * G));
-    const int slot = warp * GPW + grp;
 
-    /* the warp's block: GPW x (sequences, chain), then GPW union regions */
-    const size_t seqchain = 16u * (size_t)seq_words + T::chain_bytes;
-    unsigned char* wblock = smem + (size_t)warp * GPW * gbytes;
-    unsigned char* gs = wblock + (size_t)grp * seqchain;
-    uint2* QP = reinterpret_cast<uint2*>(gs);
+    /* the warp's sequences, chain and union region */
+    unsigned char* ws = smem + (size_t)warp * gbytes;
+    uint2* QP = reinterpret_cast<uint2*>(ws);
     uint2* QT = QP + seq_words;
-    uint8_t* chain = gs + 16u * (size_t)seq_words;
-    unsigned char* unis = wblock + (size_t)GPW * seqchain;
-    unsigned char* uni = unis + (size_t)grp * (gbytes - seqchain);
+    uint8_t* chain = ws + 16u * (size_t)seq_words;
+    unsigned char* uni = chain + T::chain_bytes;
     uint2* ops;
     /* last score step the backtrace store holds: a pair that would go past
      * it (never expected: a distance is at most the longest sequence, and
      * the store holds that many rows) goes on to the next tier instead */
     int store_last = DCAP;
     if constexpr (T::SMEM_OPS) {
-        ops = reinterpret_cast<uint2*>(unis);
+        ops = reinterpret_cast<uint2*>(uni);
     } else {
-        static_assert(T::SMEM_OPS || GPW == 1, "a store in global scratch belongs to one group");
         const TierShape& tsh = A.chain.shape[A.tier];
-        const size_t gslot = (size_t)blockIdx.x * (kWarps * GPW) + (size_t)slot;
-        ops = reinterpret_cast<uint2*>(A.ops_scratch + gslot * tsh.ops_group_bytes);
+        const size_t slot = (size_t)blockIdx.x * kWarps + (size_t)warp;
+        ops = reinterpret_cast<uint2*>(A.ops_scratch + slot * tsh.ops_warp_bytes);
         store_last = min(DCAP, tsh.ops_rows);
     }
     int8_t* stage = reinterpret_cast<int8_t*>(uni);
     int* runs = reinterpret_cast<int*>(uni + round16(A.cigar_stride));
 
     const uint32_t count = A.work_count ? min(*A.work_count, A.n_work) : A.n_work;
-    /* work stealing: each warp takes the next GPW items from the launch's
-     * counter (or, without one, every gridDim-th block of items) */
+    /* work stealing: each warp takes the next item from the launch's counter
+     * (or, without one, every gridDim-th block of items) */
     uint32_t* const work_next = A.chain.work_next ? A.chain.work_next + A.tier : nullptr;
-    const uint32_t step = gridDim.x * (uint32_t)(kWarps * GPW);
-    uint32_t wb = (blockIdx.x * kWarps + (uint32_t)warp) * GPW;
+    const uint32_t step = gridDim.x * (uint32_t)kWarps;
+    uint32_t item = blockIdx.x * kWarps + (uint32_t)warp;
     if (work_next) {
         uint32_t v = 0;
-        if (lane == 0) v = atomicAdd(work_next, (uint32_t)GPW);
-        wb = __shfl_sync(kFull, v, 0);
+        if (lane == 0) v = atomicAdd(work_next, 1u);
+        item = __shfl_sync(kFull, v, 0);
     }
-    for (; wb < count;) {
-        const uint32_t item = wb + (uint32_t)grp;
-        int state = ST_IDLE;
-        uint32_t pi = 0;
-        PairRef pr;
-        pr.p = nullptr; pr.t = nullptr; pr.plen = 0; pr.tlen = 0;
-        if (item < count) {
-            pi = A.work ? A.work[item] : item;
-            pr = get_pair(A.L, pi);
-            const uint32_t mx = max(pr.plen, pr.tlen);
-            state = !pr.in_range ? ST_RANGE : (mx > A.max_len || mx > 16u * seq_words) ? ST_TOOLONG : ST_RUN;
-        }
+    while (item < count) {
+        const uint32_t pi = A.work ? A.work[item] : item;
+        const PairRef pr = get_pair(A.L, pi);
+        const uint32_t mx = max(pr.plen, pr.tlen);
+        int state = !pr.in_range ? ST_RANGE : (mx > A.max_len || mx > 16u * seq_words) ? ST_TOOLONG : ST_RUN;
         const uint32_t lp = state == ST_RUN ? pr.plen : 0u, lt = state == ST_RUN ? pr.tlen : 0u;
-        load_packed<G, T::RMAX>(pr.p, lp, QP, g, gmask);
-        load_packed<G, T::RMAX>(pr.t, lt, QT, g, gmask);
+        load_packed<1>(pr.p, lp, QP, lane);
+        load_packed<1>(pr.t, lt, QT, lane);
         __syncwarp();
 
         const int plen = (int)lp, tlen = (int)lt, kt = tlen - plen;
@@ -598,18 +567,17 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
         int D = 0;
         /* score 0: the lane of diagonal 0 extends from the origin
          * (src/kernels.cu:249-258) */
-        if (state == ST_RUN && g == G / 2) O[J] = extend_lane(QP, QT, plen, tlen, 0, 0);
+        if (state == ST_RUN && lane == 16) O[J] = extend_lane(QP, QT, plen, tlen, 0, 0);
         {
-            const bool hit = state == ST_RUN && g == G / 2 && kt == 0 && O[J] == tlen;
-            if (__ballot_sync(kFull, hit) & gmask) state = ST_DONE;
+            const bool hit = state == ST_RUN && lane == 16 && kt == 0 && O[J] == tlen;
+            if (__any_sync(kFull, hit)) state = ST_DONE;
         }
-        int rowbase = 0;  /* first store entry of step d's row (the same for every group) */
+        int rowbase = 0;  /* first store entry of step d's row */
         int rowD = 0;     /* ... of step D's row */
         for (int d = 1;; rowbase += T::row_entries(d), ++d) {
-            const bool run = state == ST_RUN;
-            if (!__any_sync(kFull, run)) break;
+            if (!__any_sync(kFull, state == ST_RUN)) break; /* a vote: the branch is the warp's */
             if (d > store_last || (A.max_distance > 0 && d > A.max_distance)) {
-                if (run) state = (A.max_distance > 0 && d > A.max_distance) ? ST_OVERMAX : ST_OVERFLOW;
+                state = (A.max_distance > 0 && d > A.max_distance) ? ST_OVERMAX : ST_OVERFLOW;
                 break;
             }
             const int clo = T::chunk_lo(d);
@@ -617,28 +585,28 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
             /* compute (src/kernels.cu:129-152) */
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                const int lo_k = G * (c - J) - G / 2;
+                const int lo_k = 32 * (c - J) - 16;
                 N[c] = -1;
-                if (lo_k <= d && lo_k + G - 1 >= -d) {
+                if (lo_k <= d && lo_k + 31 >= -d) {
                     const int upsrc = (c + 1 < NC) ? O[(c + 1 < NC) ? c + 1 : 0] : -1;
                     const int dnsrc = (c > 0) ? O[(c > 0) ? c - 1 : 0] : -1;
-                    const int up = __shfl_sync(kFull, g == 0 ? upsrc : O[c], (g + 1) & (G - 1), G);
-                    const int dn = __shfl_sync(kFull, g == G - 1 ? dnsrc : O[c], (g + G - 1) & (G - 1), G);
+                    const int up = __shfl_sync(kFull, lane == 0 ? upsrc : O[c], (lane + 1) & 31);
+                    const int dn = __shfl_sync(kFull, lane == 31 ? dnsrc : O[c], (lane + 31) & 31);
                     const int m = piggyback_max(up, O[c], dn);
                     const unsigned blo = __ballot_sync(kFull, m & 1);
                     const unsigned bhi = __ballot_sync(kFull, m & 2);
                     if (lane == 0) ops[rowbase + c - clo] = make_uint2(blo, bhi);
-                    const int k = lo_k + g;
-                    N[c] = (run && k >= -d && k <= d) ? (m >> 2) : -1;
+                    const int k = lo_k + lane;
+                    N[c] = (k >= -d && k <= d) ? (m >> 2) : -1;
                 }
             }
             /* extend and test the target (src/kernels.cu:173-176, 268) */
             bool hit = false;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                const int lo_k = G * (c - J) - G / 2;
-                if (lo_k <= d && lo_k + G - 1 >= -d) {
-                    const int k = lo_k + g;
+                const int lo_k = 32 * (c - J) - 16;
+                if (lo_k <= d && lo_k + 31 >= -d) {
+                    const int k = lo_k + lane;
                     if (N[c] >= 0) {
                         N[c] = extend_lane(QP, QT, plen, tlen, k, N[c]);
                         hit |= (k == kt) && (N[c] == tlen);
@@ -646,7 +614,7 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
                     O[c] = N[c];
                 }
             }
-            if ((__ballot_sync(kFull, hit) & gmask) && run) {
+            if (__any_sync(kFull, hit)) {
                 state = ST_DONE;
                 D = d;
                 rowD = rowbase;
@@ -657,45 +625,43 @@ __device__ __forceinline__ void tier_body(const AlignLaunch& A, uint32_t seq_wor
             /* backtrace: from (D, kt) back to (0, 0); a walk that leaves the
              * wavefront (never expected) is reported, not followed */
             int walk_ok = 1;
-            if (g == 0) {
+            if (lane == 0) {
                 int k = kt;
                 int row = rowD;
                 for (int s = D; s >= 1; --s) {
                     if (k < -s || k > s) { walk_ok = 0; break; }
-                    const int idx = k + G / 2 + G * J;
-                    const int op = op_of(ops[row + idx / G - T::chunk_lo(s)], grp * G + (idx & (G - 1)));
+                    const int idx = k + 16 + 32 * J;
+                    const int op = op_of(ops[row + idx / 32 - T::chunk_lo(s)], idx & 31);
                     chain[s - 1] = (uint8_t)op;
                     k += op - 2;
                     if (s > 1) row -= T::row_entries(s - 1);
                 }
                 if (k != 0) walk_ok = 0;
             }
-            walk_ok = __shfl_sync(gmask, walk_ok, 0, G);
+            walk_ok = __shfl_sync(kFull, walk_ok, 0);
             if (!walk_ok) state = ST_BADWALK;
         }
         if (state == ST_DONE) {
-            __syncwarp(gmask);
-            const int len = replay_chain<G>(QP, QT, plen, tlen, chain, D, runs, stage, A.cigar_stride,
-                                            g, grp, gmask);
+            __syncwarp();
+            const int len = replay_chain(QP, QT, plen, tlen, chain, D, runs, stage, A.cigar_stride, lane);
             if (A.cigar_stride)
-                store_cigar<G>(stage, (uint32_t)len, A.cigar_stride,
-                               A.cigar + (size_t)pi * A.cigar_stride, g, gmask);
-            if (g == 0) {
+                store_cigar(stage, (uint32_t)len, A.cigar_stride, A.cigar + (size_t)pi * A.cigar_stride, lane);
+            if (lane == 0) {
                 A.dist[pi] = D;
                 if (A.status)
                     A.status[pi] = (uint32_t)len > A.cigar_stride ? (uint8_t)WFE_PAIR_CIGAR_TRUNCATED
                                                                   : (uint8_t)WFE_PAIR_OK;
             }
-        } else if (state != ST_IDLE && state != ST_RUN) {
-            if (g == 0) finish_unaligned(A, pi, state);
+        } else if (lane == 0) {
+            finish_unaligned(A, pi, state);
         }
         __syncwarp();
         if (work_next) {
             uint32_t v = 0;
-            if (lane == 0) v = atomicAdd(work_next, (uint32_t)GPW);
-            wb = __shfl_sync(kFull, v, 0);
+            if (lane == 0) v = atomicAdd(work_next, 1u);
+            item = __shfl_sync(kFull, v, 0);
         } else {
-            wb += step;
+            item += step;
         }
     }
 
@@ -1185,8 +1151,8 @@ __global__ void long_kernel(const __grid_constant__ AlignLaunch A)
         const int plen = state == ST_RUN ? (int)pr.plen : 0, tlen = state == ST_RUN ? (int)pr.tlen : 0;
         const int kt = tlen - plen;
         /* warps 0 and 1 load the two sequences (warp 0 both, in a one-warp CTA) */
-        if (warp == 0) load_packed<32, 4>(pr.p, (uint32_t)plen, QP, lane, kFull);
-        if (warp == (kW > 1 ? 1 : 0)) load_packed<32, 4>(pr.t, (uint32_t)tlen, QT, lane, kFull);
+        if (warp == 0) load_packed<4>(pr.p, (uint32_t)plen, QP, lane);
+        if (warp == (kW > 1 ? 1 : 0)) load_packed<4>(pr.t, (uint32_t)tlen, QT, lane);
         __syncthreads();
         int D = 0;
         /* last step: the tier's limit or the caller's cap */
@@ -1301,8 +1267,7 @@ __global__ void long_kernel(const __grid_constant__ AlignLaunch A)
             __syncwarp();
             if (state == ST_DONE) {
                 int8_t* dst = A.cigar_stride ? A.cigar + (size_t)pi * A.cigar_stride : nullptr;
-                const int len = replay_chain<32>(QP, QT, plen, tlen, chain, D, runs, dst, dst ? A.cigar_stride : 0u,
-                                                 lane, 0, kFull);
+                const int len = replay_chain(QP, QT, plen, tlen, chain, D, runs, dst, dst ? A.cigar_stride : 0u, lane);
                 if (lane == 0) {
                     if (dst && (uint32_t)len < A.cigar_stride) dst[len] = 0;
                     A.dist[pi] = D;
@@ -2241,8 +2206,8 @@ __device__ __forceinline__ void bound_body(const AlignLaunch& A, uint32_t seq_wo
             const int plen = (int)pr.plen, tlen = (int)pr.tlen, kt = tlen - plen;
             /* words 0..bw-1 of each sequence: packed_word gives 0 past the end */
             for (uint32_t w0 = 0; w0 < bw; w0 += 32u) {
-                const uint32_t wp = packed_word<32>(pr.p, pr.plen, w0, lane, kFull);
-                const uint32_t wt = packed_word<32>(pr.t, pr.tlen, w0, lane, kFull);
+                const uint32_t wp = packed_word(pr.p, pr.plen, w0, lane);
+                const uint32_t wt = packed_word(pr.t, pr.tlen, w0, lane);
                 if (w0 + (uint32_t)lane < bw) {
                     WP[w0 + lane] = wp;
                     WT[w0 + lane] = wt;
@@ -2522,31 +2487,25 @@ TierShape shape_of(uint32_t max_len, uint32_t cigar_stride, int sm_count)
     sh.grid = std::max(1, nb) * sm_count;
     sh.smem = (uint32_t)smem;
     sh.seq_words = seq_words_for(max_len);
-    sh.gbytes = (uint32_t)group_smem_bytes<T>(max_len, cigar_stride);
+    sh.gbytes = (uint32_t)warp_smem_bytes<T>(max_len, cigar_stride);
     if (!T::SMEM_OPS) {
-        sh.ops_group_bytes = (uint32_t)T::store_bytes(max_len);
+        sh.ops_warp_bytes = (uint32_t)T::store_bytes(max_len);
         sh.ops_rows = T::store_rows(max_len);
     }
     return sh;
 }
 
 template <class T>
-int grid_of(uint32_t max_len, uint32_t cigar_stride, int sm_count)
-{
-    return shape_of<T>(max_len, cigar_stride, sm_count).grid;
-}
-
-template <class T>
 cudaError_t launch(const AlignLaunch& a, int grid, cudaStream_t s)
 {
     const uint32_t sw = seq_words_for(a.max_len);
-    const size_t gb = group_smem_bytes<T>(a.max_len, a.cigar_stride);
+    const size_t gb = warp_smem_bytes<T>(a.max_len, a.cigar_stride);
     const size_t smem = cta_smem_bytes<T>(a.max_len, a.cigar_stride);
     if (smem > 227u * 1024u) return cudaErrorInvalidValue;
     if (!T::SMEM_OPS) {
         const TierShape& tsh = a.chain.shape[a.tier];
-        if (tsh.ops_group_bytes == 0 || tsh.ops_rows <= 0 ||
-            a.ops_scratch_bytes < (size_t)tsh.ops_group_bytes * (size_t)grid * (kWarps * T::GPW))
+        if (tsh.ops_warp_bytes == 0 || tsh.ops_rows <= 0 ||
+            a.ops_scratch_bytes < (size_t)tsh.ops_warp_bytes * (size_t)grid * kWarps)
             return cudaErrorInvalidValue;
     }
     cudaError_t e = allow_smem((const void*)tier_kernel<T>, smem);
@@ -2695,7 +2654,7 @@ pack_kernel(Layout L, uint32_t n, uint32_t* out, uint32_t wps)
         const uint32_t nw = (len + 15u) >> 4;
         for (uint32_t w0 = 0; w0 < wps; w0 += 32u) {
             uint32_t W = 0;
-            if (w0 < nw) W = packed_word<32>(s, len, w0, lane, kFull);
+            if (w0 < nw) W = packed_word(s, len, w0, lane);
             if (w0 + (uint32_t)lane < wps) dst[w0 + lane] = W;
         }
     }
@@ -2829,9 +2788,9 @@ const TierInfo& tier_info(int t) { return kTiers[t]; }
 size_t tier_scratch_bytes(int tier, int grid, uint32_t max_len)
 {
     switch (tier) {
-    case 2: return T2::store_bytes(max_len) * (size_t)grid * (kWarps * T2::GPW);
-    case 3: return T3::store_bytes(max_len) * (size_t)grid * (kWarps * T3::GPW);
-    case 4: return T4::store_bytes(max_len) * (size_t)grid * (kWarps * T4::GPW);
+    case 2: return T2::store_bytes(max_len) * (size_t)grid * kWarps;
+    case 3: return T3::store_bytes(max_len) * (size_t)grid * kWarps;
+    case 4: return T4::store_bytes(max_len) * (size_t)grid * kWarps;
     default: return 0;
     }
 }
@@ -2927,11 +2886,6 @@ TierShape tier_shape(int tier, uint32_t max_len, uint32_t cigar_stride, int sm_c
     return sh;
 }
 
-int tier_grid(int tier, uint32_t max_len, uint32_t cigar_stride, int sm_count)
-{
-    return tier_shape(tier, max_len, cigar_stride, sm_count).grid;
-}
-
 /* cached per (device, max_len, SMs), as tier_shape */
 TierShape bound_shape(uint32_t max_len, int sm_count)
 {
@@ -2960,7 +2914,7 @@ TierShape bound_shape(uint32_t max_len, int sm_count)
 }
 
 namespace {
-int order_grid(const AlignLaunch& a) { return (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 608u); }
+int order_grid(const AlignLaunch& a) { return (int)std::min<uint32_t>((a.n_work + 4u * kOrderBins - 1u) / (4u * kOrderBins), 4u * kSms); }
 }  // namespace
 
 cudaError_t launch_order(const AlignLaunch& a, cudaStream_t s)

@@ -16,9 +16,10 @@ struct TierInfo {
     int pairs_per_cta; /* pairs a CTA takes at a time */
 };
 
-/* Tiers 0-4 are register tiers (one pair per group of G lanes); tiers 5
- * and 6 give each pair a whole CTA with the wavefront in shared (5) or
- * global (6) memory and have no distance limit of their own. */
+/* Tier 0 is a bit-parallel band, one pair per thread; tiers 1-4 keep a pair's
+ * wavefront in a warp's registers; tiers 5 and 6 give each pair a whole CTA
+ * with the wavefront in shared (5) or global (6) memory, or, in bulk, go by
+ * distance classes (5). */
 constexpr int kNumTiers = 7;
 constexpr int kLongThreads = 256;
 constexpr int kLongSmemDistance = 2047; /* largest distance with the wavefront in shared memory */
@@ -29,32 +30,36 @@ struct TierShape {
     int grid;           /* persistent grid (resident CTAs) */
     uint32_t smem;      /* dynamic shared memory per CTA */
     uint32_t seq_words; /* 16-base words per sequence in shared memory */
-    uint32_t gbytes;    /* shared memory per group */
+    uint32_t gbytes;    /* tiers 1-4: shared memory per warp */
     int dlim;           /* tiers 5-6: largest distance the tier computes */
     uint64_t slab;      /* tiers 5-6: bytes of global scratch per CTA */
     unsigned char* scratch; /* tiers 5-6: grid * slab bytes */
-    uint32_t ops_group_bytes; /* tiers 2-4: bytes of one group's backtrace store in the global scratch */
+    uint32_t ops_warp_bytes; /* tiers 2-4: bytes of one warp's backtrace store in the global scratch */
     int ops_rows;       /* tiers 2-4: score steps that store holds (a distance never exceeds the
                            longest sequence, so rows past max_len are never written) */
     int threads;        /* tiers 5-6 and the bound pass: threads per CTA */
 };
 
 /* Distance classes of tier 5, by the upper bound on each pair's distance.
- * A list in bulk is bounded by the scan (wide_kernel<2, true>); the classes are then aligned by the tile kernel, in one launch,
- * except those with kWidePairs pairs or more, which one thread per pair takes
+ * A list in bulk is bounded by the scan (wide_kernel<2, true>); the classes
+ * are then aligned by the tile kernel, in one launch, except those with kWidePairs pairs or more, which one thread per pair takes
  * (wide_kernel), and the last, which holds what the others do not and whose
  * pairs get a CTA each (long_kernel).  The limits are those of 3, 4, 5, 6, 8,
  * 10, 16 and 32 lanes per pair: every number of pairs that a warp can hold,
  * but 7.  Other lists are bounded by the bound pass (bound_kernel), and
  * every pair gets a CTA, in the classes of class_by_cta: each of those is a
  * launch of its own with wavefront buffers (shared memory) and backtrace
- * slabs sized to its limit.  Classes up to 257 run CTAs of one warp, classes
- * up to distance 1024 CTAs of 128 threads, the others 256: a pair of short
+ * slabs sized to its limit.  Classes up to kLongTinyDistance run CTAs of one warp, classes
+ * up to kLongSmallDistance CTAs of 128 threads, the others 256: a pair of short
  * distance has few cells per step to share, and fewer warps per pair spend
  * fewer instructions on each step's bookkeeping and barrier.  Limits at or
  * past tier 5's own (min(max_len, 2047)) are dropped. */
 constexpr int kLongClasses = 9;
 constexpr int kLongClassLimit[kLongClasses - 1] = {127, 193, 257, 321, 449, 577, 961, 1985};
+/* The classes that lists by CTA use, besides the last (see class_by_cta). */
+constexpr int kCtaClassShort = kLongClassLimit[2];
+constexpr int kCtaClassMiddle[2] = {kLongClassLimit[5], kLongClassLimit[6]};
+constexpr uint32_t kSms = 152; /* SMs of the GPU that the rules below were measured on */
 /* Whether tier 5 takes a list without bounds on its distances, as one launch
  * with a CTA per pair: as many pairs as the GPU has SMs are aligned at once,
  * in the time of the longest, and the bound pass takes longer than the cells
@@ -64,13 +69,13 @@ constexpr int kLongClassLimit[kLongClasses - 1] = {127, 193, 257, 321, 449, 577,
  * once. */
 __host__ __device__ constexpr bool alone_in_tier_5(uint32_t count, uint32_t max_len)
 {
-    return count <= 152u && max_len <= 5u * (uint32_t)kLongSmemDistance;
+    return count <= kSms && max_len <= 5u * (uint32_t)kLongSmemDistance;
 }
 /* Pairs from which on tier 5 may begin with the scan (see plan_choice). */
 constexpr uint32_t kScanMin = 1024;
 constexpr uint32_t kWidePairs = 16384;
 constexpr int kLongTinyThreads = 32;
-constexpr int kLongTinyDistance = 257;   /* classes up to this limit use kLongTinyThreads */
+constexpr int kLongTinyDistance = kCtaClassShort; /* classes up to this limit use kLongTinyThreads */
 constexpr int kLongSmallThreads = 128;
 constexpr int kLongSmallDistance = 1024; /* classes up to this limit use kLongSmallThreads */
 constexpr int kTileClass = kLongClasses; /* AlignLaunch::cls of the tile kernel */
@@ -212,12 +217,9 @@ struct AlignLaunch {
 TierShape tier_shape(int tier, uint32_t max_len, uint32_t cigar_stride, int sm_count);
 
 /* Bytes of global op-store scratch tier t needs for `grid` CTAs, each
- * group's store holding the rows of distances up to max_len (capped at the
+ * warp's store holding the rows of distances up to max_len (capped at the
  * tier's own limit). */
 size_t tier_scratch_bytes(int tier, int grid, uint32_t max_len);
-/* Persistent grid of tier t for sequences up to max_len, cigar slots of
- * cigar_stride (occupancy-limited, at least 1). */
-int tier_grid(int tier, uint32_t max_len, uint32_t cigar_stride, int sm_count);
 cudaError_t launch_tier(int tier, const AlignLaunch& a, int grid, cudaStream_t s);
 
 /* a's list (a.work / a.work_count / a.n_work) in order of length, longest

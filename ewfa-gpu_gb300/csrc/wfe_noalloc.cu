@@ -19,7 +19,7 @@
  * (32 lanes per pair, distances up to 271, backtrace store in global memory),
  * pointed at the rest of the array.  A pair's store there takes 20,544 bytes (a
  * triangle of 271 rows), so the rest holds the stores of 612 pairs in flight,
- * 153 CTAs of 4 pairs; that grid is sized so that every resident group has its
+ * 153 CTAs of 4 pairs; that grid is sized so that every resident warp has its
  * own slot (about one CTA per SM on a GB300, below the kernel's occupancy: the
  * price of the fixed size, paid only by the pairs handed on).  With a
  * max_distance within the first tier's it does all of it; some calls go to
@@ -191,13 +191,13 @@ extern "C" int wfe_align_device_noalloc(const char* d_ascii, const wfe_pair* d_p
     const bool listed = first && deep; /* tier 3 over the pairs that the first tier handed on */
 
     /* tier 3: occupancy, capped by the op-store slots of the array; every
-     * group's store holds all rows of the tier (distances up to 271) */
+     * warp's store holds all rows of the tier (distances up to 271) */
     if (deep && sh.grid <= 0) return WFE_ERR_SEQ_TOO_LONG; /* sequences + CIGAR slot exceed shared memory */
     const size_t stores_at = listed ? kStoresAt : 0u;
     const uint32_t full_rows = (uint32_t)WFE_NOALLOC_MAX_DISTANCE;
     const size_t per_cta = wfe::tier_scratch_bytes(kNoallocTier, 1, full_rows);
     const int slots = (int)((kNoallocScratchBytes - stores_at) / per_cta);
-    sh.ops_group_bytes = (uint32_t)(per_cta / 4u); /* 4 groups (one per warp) per CTA */
+    sh.ops_warp_bytes = (uint32_t)(per_cta / 4u); /* 4 warps per CTA */
     sh.ops_rows = (int)full_rows;
 
     unsigned char* base = static_cast<unsigned char*>(scratch);
