@@ -165,12 +165,15 @@ __device__ uint32_t tile_chunks(const LongClasses& C);
  * by a CTA per pair.  With so few pairs that nearly every one has a CTA's slot
  * at once, one launch after another costs more than CTAs that fit the
  * distance give: the last class alone, or with the shortest (8 pairs of 4-6
- * kb 0.70 -> 0.36 ms, 256 of 5-7 kb 1.41 -> 0.76 ms). */
+ * kb 0.70 -> 0.36 ms, 256 of 5-7 kb 1.41 -> 0.76 ms; 600 of 2-8 kb at 3-12% 0.72
+ * -> 0.55, of 1-9 kb 0.77 -> 0.56).  Pairs of one distance between the two
+ * classes lose by it: 600 of 6 kb at 12% 0.61 -> 0.77 ms, 0.63 with the classes
+ * between, which cost the lists above 0.76 and 1.04. */
 constexpr uint32_t kFewPairs = 384, kSomePairs = 1024;
 __device__ __forceinline__ bool class_by_cta(int dlim, uint32_t count)
 {
-    constexpr int kMiddle = kCtaClassMiddle[0], kUpper = kCtaClassMiddle[1];
-    return count > kFewPairs && (dlim == kCtaClassShort || (count > kSomePairs && (dlim == kMiddle || dlim == kUpper)));
+    return count > kFewPairs &&
+           (dlim == kCtaClassShort || (count > kSomePairs && (dlim == kCtaClassMiddle || dlim == kCtaClassUpper)));
 }
 __device__ __forceinline__ bool tile_takes(const LongClasses& C, int c, uint32_t count)
 {

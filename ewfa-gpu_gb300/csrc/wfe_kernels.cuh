@@ -57,8 +57,8 @@ struct TierShape {
 constexpr int kLongClasses = 9;
 constexpr int kLongClassLimit[kLongClasses - 1] = {127, 193, 257, 321, 449, 577, 961, 1985};
 /* The classes that lists by CTA use, besides the last (see class_by_cta). */
-constexpr int kCtaClassShort = kLongClassLimit[2];
-constexpr int kCtaClassMiddle[2] = {kLongClassLimit[5], kLongClassLimit[6]};
+constexpr int kCtaClassShort = kLongClassLimit[2], kCtaClassMiddle = kLongClassLimit[5],
+              kCtaClassUpper = kLongClassLimit[6];
 constexpr uint32_t kSms = 152; /* SMs of the GPU that the rules below were measured on */
 /* Whether tier 5 takes a list without bounds on its distances, as one launch
  * with a CTA per pair: as many pairs as the GPU has SMs are aligned at once,

@@ -53,3 +53,24 @@ def test_pairs_of_one_class(low, limit, length, edits, n):
         same = np.flatnonzero(pick == i)
         assert (dist[same] == dist[first[i]]).all() and (st[same] == st[first[i]]).all(), i
         assert_same_cigars(cg[same], np.repeat(cg[first[i]:first[i] + 1], len(same), 0))
+
+
+@pytest.mark.parametrize("n", [153, 384, 385, 1023])
+def test_lists_by_cta(n):
+    """Lists too short for the bulk kernels: one class, or two, with pairs on
+    either side of the limit between them."""
+    torch_cuda()
+    seqs = [s for low, limit, length, edits in ((0, 127, 900, [30, 75, 110]), (193, 257, 1300, [205, 230, 250]),
+                                               (449, 577, 1900, [540, 620, 700]), (577, 961, 2000, [900, 1100, 1400]))
+            for s in class_pairs(low, limit, length, edits)[::4]]
+    rng = np.random.default_rng(9)
+    t = bases(rng, 2000)
+    seqs += [(t, t[:1040]), (t, t[:1039]), (t, t[:1038]), (t[:900], t), (bases(rng, 1990), bases(rng, 60)), (b"", b"")]
+    ascii, pairs = wfe.pairs_from_list(seqs)
+    assert len(pairs) <= 153
+    pick = rng.permutation(np.arange(n) % len(pairs))
+    with wfe.Context(max_seq_len=2100, cigar_stride=STRIDE) as ctx:
+        ctx.set_policy([2100], [5])
+        dist, cg, st = ctx.align(ascii, pairs[pick])
+    assert (dist > 961).any() and (dist == 961).any() and ((dist > 577) & (dist <= 961)).any()
+    compare_with_oracle(ascii, pairs[pick], STRIDE, dist, cg, st)
