@@ -124,7 +124,7 @@ struct wfe_ctx {
      * made when a call first needs it (deep_ready): until then host calls
      * run their chains as far as tier 1 and defer the pairs that go further
      * (see finish_deferred).  Short reads never reach tier 2, and a context
-     * for them holds ~10 MB instead of ~200. */
+     * for them holds ~15 MB instead of ~230. */
     bool deep_ready = false;
     unsigned char* d_deep = nullptr;
     size_t deep_bytes = 0;
@@ -532,7 +532,8 @@ int launch_bucket(wfe_ctx* ctx, Stage& st, const BucketPlan& bp, int bucket_inde
  * pair need a few microseconds for a few scores where tier 0 needs the length
  * of the sequences in columns (300 bases: 31 us against 61 for up to 4,096
  * pairs, the same at 16,384; 150 bases: 34 and 37 at 1,024, 41 and 37 at
- * 4,096; 64 of 600-1,050 bases at 0.5% in two buckets 16 and 64).  A large batch of sequences past kPlanLength bases is planned
+ * 4,096; 64 of 600-1,050 bases at 0.5% in two buckets 16 and 64).  A large
+ * batch of sequences past kPlanLength bases, of a bucket alone, is planned
  * (kPlanned): its error rate decides.  Other device batches of up to 512 bases
  * start at tier 0 from 12,288 pairs on (20,000 pairs of 240-330 bases at 4-7%:
  * 58 us in a row against 92 from tier 1, alone 167 against 131; at 0.5% 34 and
@@ -640,8 +641,8 @@ int run_chain(wfe_ctx* ctx, Stage& st, const Layout& L, uint32_t n, int32_t* dis
      * planned from tier 1, which takes that list alone. */
     const BucketPlan& lp = ctx->bucket[ctx->nbuckets - 1];
     const int lt = bk.first_tier[ctx->nbuckets - 1];
-    const bool merge = ctx->bound && lt <= 5 && start[ctx->nbuckets - 1] != kPlanned1 && lp.bound.grid > 0 && lp.cls.scan.grid > 0 &&
-                       chain_end(ctx->cfg, lt, lp.last_tier) >= 5;
+    const bool merge = ctx->bound && lt <= 5 && start[ctx->nbuckets - 1] != kPlanned1 && lp.bound.grid > 0 &&
+                       lp.cls.scan.grid > 0 && chain_end(ctx->cfg, lt, lp.last_tier) >= 5;
     bk.tier5_to = merge ? ctx->nbuckets - 1 : -1;
     WFE_CUDA(ctx, launch_classify(L, n, bk, s));
     ctx->stats.kernel_launches++;

@@ -147,8 +147,8 @@ typedef struct wfe_stats {
  * pair's distance passes 79.  Such a host call aligns those pairs again
  * once the scratch exists (from their index in the call; when more than
  * batch_size were deferred, the whole call runs again), with the same
- * results.  A short-read context that never needs it holds ~10 MB of device
- * memory instead of ~200 MB, and frees it sooner.
+ * results.  A short-read context that never needs it holds ~15 MB of device
+ * memory instead of ~230 MB, and frees it sooner.
  * Threading: a context is used by one thread at a time; different contexts
  * may be used from different threads at once.  Every call on a context makes
  * its device the calling thread's current device (as the reference's
@@ -192,8 +192,8 @@ int wfe_reset_stats(wfe_ctx* ctx);
  * first tier:
  *   tier 0: a thread per pair, bit-parallel band of 32 diagonals, distance <= 31
  *   tier 1: 32 lanes per pair, shared-memory store, <= 79
- *   tier 2: 32 lanes, shared-memory store, <= 143
- *   tier 3: 32 lanes, store spilled to global memory, <= 271
+ *   tier 2: 32 lanes, store in global memory, <= 143
+ *   tier 3: 32 lanes, global store, <= 271
  *   tier 4: 32 lanes, global store, <= 527
  *   tier 5: <= 2047; a CTA per pair, wavefront in shared memory, or, for lists
  *           of a thousand pairs and more, bit-parallel bands in distance classes
